@@ -623,6 +623,8 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
             // the grouped GEMM is bound by dequantization, which is paid once per (weight tile, activation tile):
             // prefer the tile that holds an expert's expected rows (plus the spread of a random routing) in one piece
             p.mt = avg <= 48 ? 64 : avg <= 100 ? 128 : 256;
+        } else {
+            p.mt = lb::qgemm_f32_moe_tile(p.t * p.r, p.e);
         }
         if ((uint64_t)lb::moe_max_tiles(p.t * p.r, p.e, p.mt) * p.mt >= lim) fail("too_large", "b200 matmul_id: tile space exceeds 32-bit indexing");
         p.route_bytes = lb::moe_route_bytes(p.t * p.r, p.e, p.mt);
@@ -739,7 +741,8 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
     f.row_pair = route.row_pair;
     f.id_stride = p.wl.total;
     f.id_r = (uint32_t)p.r;
-    cuda_check(lb::launch_qgemm_f32(l.b_dtype, f, dev.stream), "matmul_id gemm launch");
+    f.mt = p.mt;
+    cuda_check(lb::launch_qgemm_f32(l.b_dtype, f, dev.sm_count, dev.stream), "matmul_id gemm launch");
     dev.launches++;
 }
 
@@ -997,7 +1000,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
     f.m = g.m;
     f.n = g.n;
     f.k = g.k;
-    cuda_check(lb::launch_qgemm_f32(l.b_dtype, f, dev.stream), "qgemm_f32 launch");
+    cuda_check(lb::launch_qgemm_f32(l.b_dtype, f, dev.sm_count, dev.stream), "qgemm_f32 launch");
     dev.launches++;
     expr_pass();
 }

@@ -40,11 +40,12 @@ __device__ __forceinline__ float half_bits_to_float(uint32_t h) {
 // else happens to them (`load_contig`, crates/lapid-cpu/src/matmul/mod.rs:165-286); both widenings are exact.
 constexpr int ACT_F32 = 0, ACT_F16 = 1, ACT_BF16 = 2;
 __host__ __device__ constexpr uint32_t act_elem_bytes(int a_type) { return a_type == ACT_F32 ? 4u : 2u; }
+__device__ __forceinline__ float widen_act(uint32_t h, int a_type) {  // the 16 bits of a half type
+    return a_type == ACT_F16 ? __half2float(__ushort_as_half((unsigned short)h)) : __uint_as_float(h << 16);
+}
 // Element i of the row that starts at `row`.
 __device__ __forceinline__ float load_act(const void *row, uint64_t i, int a_type) {
-    if (a_type == ACT_F32) return ((const float *)row)[i];
-    const unsigned short h = ((const unsigned short *)row)[i];
-    return a_type == ACT_F16 ? __half2float(__ushort_as_half(h)) : __uint_as_float((uint32_t)h << 16);
+    return a_type == ACT_F32 ? ((const float *)row)[i] : widen_act(((const unsigned short *)row)[i], a_type);
 }
 // Start of row r = bt*m + i of an activation operand: base + (off + bt*bs + i*rs) elements.
 __device__ __forceinline__ const void *act_row(const void *base, int a_type, uint64_t off, uint64_t bs, uint64_t rs, uint32_t r, uint32_t m) {

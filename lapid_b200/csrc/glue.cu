@@ -9,11 +9,8 @@
 //   silu_mul   out = silu(gate) * up = gate / (1 + exp(-gate)) * up                   elementwise
 //              the SwiGLU product (crates/lapid-nn/src/mlp.rs:84), an Elementwise kernel in lapid
 //
-// Both are memory-trivial (tens of KB at decode sizes) and latency-bound: 128-bit accesses, a row
-// is split over a thread-block cluster of up to 8 CTAs whose partial sums of squares meet through
-// distributed shared memory (so a single decode row still spreads over 8 SMs -- which matters most
-// when the row is the sum of the tensor-parallel ranks' partials, polled from the hand-off slots),
-// programmatic dependent launch like the GEMVs.
+// Both are memory-trivial (tens of KB) and latency-bound at decode sizes: 128-bit accesses, programmatic dependent
+// launch like the GEMVs.
 // They are not part of the quantized-matmul path; f32 results, not bit-matched to lapid-cpu (the
 // order of the sum of squares differs): the tests hold them to 1e-5 relative against f64.
 #include <cooperative_groups.h>
@@ -30,7 +27,68 @@ namespace lb {
 constexpr int GLUE_THREADS = 256;
 constexpr int GLUE_MAX_VEC = 16;  // float4 per thread kept in registers: cols <= 256 * 16 * 4 = 16384
 
-__global__ void __launch_bounds__(GLUE_THREADS) rms_norm_kernel(RmsNormArgs p) {
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float4 scale4(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
+__device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+__device__ __forceinline__ float sumsq4(float4 a, float ss) { return fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, ss)))); }
+
+// One CTA per row, VEC float4 per thread in registers. A decode step has one to eight rows, so what counts there is the
+// chain load -> sum -> store: as many threads as the row has float4s (up to 1024), all loads of a thread issued
+// before the first is used, one barrier. A prompt has enough rows to fill the chip, so memory bandwidth is the bound (x, residual, sum and
+// out: 16 bytes an element). A row split over a cluster of eight CTAs, which this replaces, paid two cluster barriers for
+// every row: 2048 x 8192 took 320 us (0.8 TB/s), now 38 (7.1 TB/s of which part is L2), 77 x 4096 16.5 and 3.0, one row of 4096 inside a
+// decode step 3.5 us less.
+template <int VEC> __global__ void __launch_bounds__(1024) rms_norm_kernel(RmsNormArgs p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ float partial[32];
+    const uint32_t row = blockIdx.x, n4 = p.cols / 4, tid = threadIdx.x, step = blockDim.x;
+    const size_t at = (size_t)row * n4;
+    const float4 *x = (const float4 *)p.x + at, *res = (const float4 *)p.residual + at;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float4 v[VEC], r[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; i++) {
+        const uint32_t c = tid + i * step;
+        v[i] = r[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (c < n4) {
+            v[i] = x[c];
+            if (p.residual) r[i] = res[c];
+        }
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VEC; i++) {
+        if (p.residual) v[i] = add4(v[i], r[i]);
+        ss = sumsq4(v[i], ss);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((tid & 31) == 0) partial[tid >> 5] = ss;
+    __syncthreads();
+    float tot = (tid & 31) < step / 32 ? partial[tid & 31] : 0.0f;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    const float rstd = 1.0f / sqrtf(tot * (1.0f / (float)p.cols) + p.eps);
+#pragma unroll
+    for (int i = 0; i < VEC; i++) {
+        const uint32_t c = tid + i * step;
+        const bool active = c < n4;
+        float4 a = scale4(v[i], rstd);
+        if (active) {
+            if (p.weight) a = mul4(a, ((const float4 *)p.weight)[c]);
+            ((float4 *)p.out)[at + c] = a;
+            if (p.sum_out) ((float4 *)p.sum_out)[at + c] = v[i];
+        }
+        // the same values as the int8 operand of the GEMVs that read `out` (whole warps of the row take the branch together,
+        // lanes past the row pass active = false)
+        if (p.q.qa && (tid & ~31u) + i * step < n4) act_quant_quad(p.q, active, row, 4 * c, a);
+    }
+}
+
+// Tensor-parallel input: x = sum over ranks (in rank order) of the partials they pushed for the call in progress, polled
+// pair by pair from this rank's own slots (protocol: tp_allreduce.cu). The row is split over a cluster of up to 8 CTAs, so that the polling of a
+// single decode row spreads over 8 SMs; their partial sums of squares meet through distributed shared memory.
+__global__ void __launch_bounds__(GLUE_THREADS) tp_rms_norm_kernel(RmsNormArgs p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float partial[GLUE_THREADS / 32];
@@ -39,19 +97,11 @@ __global__ void __launch_bounds__(GLUE_THREADS) rms_norm_kernel(RmsNormArgs p) {
     const uint32_t parts = cluster.num_blocks(), part = cluster.block_rank();
     const uint32_t row = blockIdx.x / parts, n4 = p.cols / 4;
     const uint32_t per = (n4 + parts - 1) / parts, c_lo = part * per, c_hi = min(n4, c_lo + per);  // this CTA's float4 columns
-    // tensor-parallel input: x = sum over ranks (in rank order) of the partials they pushed for the
-    // call in progress, polled pair by pair from this rank's own slots (protocol: tp_allreduce.cu)
-    uint32_t epoch = 0;
-    const uint8_t *slots = nullptr;
-    size_t slot_bytes = 0;
+    const uint32_t epoch = tp_current_epoch(p.tp);
+    const size_t slot_bytes = (size_t)p.tp->max_elems * 8;
+    const uint8_t *slots = (const uint8_t *)p.tp->peer[p.tp->rank] + TP_HEADER + (size_t)(epoch & 1) * p.tp->world * slot_bytes +
+                           (size_t)row * p.cols * 8;
     bool ok = true;
-    if (p.tp) {
-        epoch = tp_current_epoch(p.tp);
-        slot_bytes = (size_t)p.tp->max_elems * 8;
-        slots = (const uint8_t *)p.tp->peer[p.tp->rank] + TP_HEADER + (size_t)(epoch & 1) * p.tp->world * slot_bytes +
-                (size_t)row * p.cols * 8;
-    }
-    const float4 *x = (const float4 *)(p.x + (size_t)row * p.cols);
     const float4 *res = p.residual ? (const float4 *)(p.residual + (size_t)row * p.cols) : nullptr;
     float4 v[GLUE_MAX_VEC];
     float ss = 0.0f;
@@ -59,40 +109,26 @@ __global__ void __launch_bounds__(GLUE_THREADS) rms_norm_kernel(RmsNormArgs p) {
     for (int i = 0; i < GLUE_MAX_VEC; i++) {
         const uint32_t c = c_lo + threadIdx.x + i * GLUE_THREADS;
         if (c < c_hi) {
-            float4 a;
-            if (p.tp) {
-                a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                for (int q = 0; q < p.tp->world; q++) {
-                    const uint8_t *src = slots + (size_t)q * slot_bytes + (size_t)c * 32;
-                    uint4 lo = ld_pairs(src), hi = ld_pairs(src + 16);
-                    for (uint32_t spin = 0; ok && (lo.y != epoch || lo.w != epoch || hi.y != epoch || hi.w != epoch); spin++) {
-                        if (spin >= (p.spin_limit ? p.spin_limit : TP_SPIN_LIMIT)) {
-                            ok = false;
-                            break;
-                        }
-                        __nanosleep(20);
-                        lo = ld_pairs(src);
-                        hi = ld_pairs(src + 16);
+            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int q = 0; q < p.tp->world; q++) {
+                const uint8_t *src = slots + (size_t)q * slot_bytes + (size_t)c * 32;
+                uint4 lo = ld_pairs(src), hi = ld_pairs(src + 16);
+                for (uint32_t spin = 0; ok && (lo.y != epoch || lo.w != epoch || hi.y != epoch || hi.w != epoch); spin++) {
+                    if (spin >= (p.spin_limit ? p.spin_limit : TP_SPIN_LIMIT)) {
+                        ok = false;
+                        break;
                     }
-                    const float4 v = make_float4(__uint_as_float(lo.x), __uint_as_float(lo.z), __uint_as_float(hi.x), __uint_as_float(hi.z));
-                    a.x = q ? a.x + v.x : v.x;
-                    a.y = q ? a.y + v.y : v.y;
-                    a.z = q ? a.z + v.z : v.z;
-                    a.w = q ? a.w + v.w : v.w;
+                    __nanosleep(20);
+                    lo = ld_pairs(src);
+                    hi = ld_pairs(src + 16);
                 }
-            } else {
-                a = x[c];
+                const float4 b = make_float4(__uint_as_float(lo.x), __uint_as_float(lo.z), __uint_as_float(hi.x), __uint_as_float(hi.z));
+                a = q ? add4(a, b) : b;
             }
-            if (res) {
-                const float4 b = res[c];
-                a.x += b.x;
-                a.y += b.y;
-                a.z += b.z;
-                a.w += b.w;
-            }
+            if (res) a = add4(a, res[c]);
             if (p.sum_out) ((float4 *)(p.sum_out + (size_t)row * p.cols))[c] = a;
             v[i] = a;
-            ss = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, ss))));
+            ss = sumsq4(a, ss);
         }
     }
 #pragma unroll
@@ -115,34 +151,21 @@ __global__ void __launch_bounds__(GLUE_THREADS) rms_norm_kernel(RmsNormArgs p) {
         const bool active = c < c_hi;
         float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (active) {
-            a = v[i];
-            a.x *= rstd;
-            a.y *= rstd;
-            a.z *= rstd;
-            a.w *= rstd;
-            if (p.weight) {
-                const float4 g = ((const float4 *)p.weight)[c];
-                a.x *= g.x;
-                a.y *= g.y;
-                a.z *= g.z;
-                a.w *= g.w;
-            }
+            a = scale4(v[i], rstd);
+            if (p.weight) a = mul4(a, ((const float4 *)p.weight)[c]);
             ((float4 *)(p.out + (size_t)row * p.cols))[c] = a;
         }
-        // the same values as the int8 operand of the GEMVs that read `out` (warp-uniform branch: whole warps of
-        // the CTA's column range take it together, lanes past the range pass active = false)
-        if (p.q.qa && c_lo + (threadIdx.x & ~31u) + i * GLUE_THREADS < c_hi) act_quant_quad(p.q, active, row, 4 * c, a);
+        if (p.q.qa && c_lo + (threadIdx.x & ~31u) + i * GLUE_THREADS < c_hi) act_quant_quad(p.q, active, row, 4 * c, a);  // as above
     }
     if (parts > 1) cluster.sync();  // no CTA leaves while a neighbour may still read its partial sum
-    if (p.tp) {  // the last CTA to finish closes the call
-        if (!ok && p.status) atomicOr(p.status, 64);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t *epoch_ctr = (uint32_t *)((uint8_t *)p.tp->peer[p.tp->rank] + 256), *done_ctr = epoch_ctr + 1;
-            if (atomicAdd(done_ctr, 1u) == gridDim.x - 1) {
-                *done_ctr = 0;
-                *(volatile uint32_t *)epoch_ctr = epoch;
-            }
+    // the last CTA to finish closes the call
+    if (!ok && p.status) atomicOr(p.status, 64);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t *epoch_ctr = (uint32_t *)((uint8_t *)p.tp->peer[p.tp->rank] + 256), *done_ctr = epoch_ctr + 1;
+        if (atomicAdd(done_ctr, 1u) == gridDim.x - 1) {
+            *done_ctr = 0;
+            *(volatile uint32_t *)epoch_ctr = epoch;
         }
     }
 }
@@ -169,10 +192,10 @@ __global__ void __launch_bounds__(GLUE_THREADS) silu_mul_kernel(const float *gat
 }
 
 static void pdl_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, unsigned grid, bool pdl, cudaStream_t stream,
-                       unsigned cluster = 1) {
+                       unsigned cluster = 1, unsigned threads = GLUE_THREADS) {
     cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(GLUE_THREADS);
+    cfg.blockDim = dim3(threads);
     cfg.stream = stream;
     int n = 0;
     if (pdl) {
@@ -202,11 +225,21 @@ cudaError_t launch_rms_norm(const RmsNormArgs &a, bool pdl, cudaStream_t stream)
     if (a.rows == 0) return cudaSuccess;
     if (!rms_norm_shape_ok(a.cols)) return cudaErrorInvalidValue;
     if (a.q.qa && (!rms_norm_quant_ok(a.cols) || a.q.k != a.cols || a.q.rows != a.rows)) return cudaErrorInvalidValue;
-    const unsigned parts = rms_norm_parts(a.cols);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    pdl_config(cfg, attr, a.rows * parts, pdl, stream, parts);
-    return cudaLaunchKernelEx(&cfg, rms_norm_kernel, a);
+    if (a.tp) {
+        const unsigned parts = rms_norm_parts(a.cols);
+        pdl_config(cfg, attr, a.rows * parts, pdl, stream, parts);
+        return cudaLaunchKernelEx(&cfg, tp_rms_norm_kernel, a);
+    }
+    // few rows: the most threads a row can use; many: two float4 per thread, so that several rows share an SM
+    const unsigned n4 = a.cols / 4, per = a.rows <= 64 ? 1 : 2;
+    unsigned threads = (n4 + per - 1) / per;
+    threads = threads >= 1024 ? 1024 : (threads + 31) / 32 * 32;
+    pdl_config(cfg, attr, a.rows, pdl, stream, 1, threads);
+    if (n4 <= threads) return cudaLaunchKernelEx(&cfg, rms_norm_kernel<1>, a);
+    if (n4 <= 2 * threads) return cudaLaunchKernelEx(&cfg, rms_norm_kernel<2>, a);
+    return cudaLaunchKernelEx(&cfg, rms_norm_kernel<4>, a);
 }
 
 cudaError_t launch_silu_mul(const float *gate, const float *up, float *out, uint64_t n, uint32_t cols, const ActOut &q, int sm_count,

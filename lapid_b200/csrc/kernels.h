@@ -291,14 +291,17 @@ struct GemmF32Args {
     uint64_t ex_off;
     int64_t ex_s0, ex_s1, ex_s2;
     uint32_t rows, m, n, k;
-    // Expert-indexed launches (moe.cu): rows = the tile space (64-row tiles), w = the expert stack
+    bool a_vec;                  // four activations of a row can be fetched with one aligned load (set by the launcher)
+    // Expert-indexed launches (moe.cu): rows = the tile space (tiles of mt rows: qgemm_f32_moe_tile), w = the expert stack
+    uint32_t mt;
     const int32_t *tile_expert;  // nullptr for an ordinary launch
     const int32_t *row_pair;
     uint64_t id_stride;          // bytes between the experts' matrices
     uint32_t id_r;               // slots per token: pair p reads activation row p / id_r, writes output row p
     const uint8_t *iq_grid;      // i-quants: the format's codebook on this device (set by the launcher)
 };
-cudaError_t launch_qgemm_f32(int fmt, const GemmF32Args &args, cudaStream_t stream);
+cudaError_t launch_qgemm_f32(int fmt, const GemmF32Args &args, int sm_count, cudaStream_t stream);
+uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts);  // activation rows per tile of an expert-indexed launch
 
 // ---- qgemm_tc.cu: tcgen05 tensor-core GEMM (Q4_K weights, bf16 operands, f32 accumulation)
 struct GemmTcArgs {

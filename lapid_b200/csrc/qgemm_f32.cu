@@ -11,90 +11,127 @@
 // the in-order FMA sum over k, i.e. what lapid-cpu's per-expert matmul gives
 // (crates/lapid-cpu/src/moe.rs:80-118 with float_act, :109).
 //
-// CUDA-core kernel: 64x64 output tile per CTA, 4x4 register tile per thread, k in steps of one
-// 32-element group; the W tile is expanded into shared memory once per step (so each weight is
-// dequantized once per 64 activation rows) and A is staged beside it.
+// CUDA-core kernel: the order of the sum is fixed (one chain of fused multiply-adds over k per output), so neither the tensor
+// cores nor a split of K can be used; what bounds it is FMA issue (128 a clock and SM). A BM x BN output tile per CTA,
+// 8 x 8 outputs per thread where the tile is large enough. Two neighbouring activation rows share one packed fma.rn.f32x2
+// (two independent, separately rounded FMAs in one instruction): half the issue slots of scalar FMAs, which leaves room
+// for the shared-memory loads and for expanding the weights. k runs in steps of 16; while a step is multiplied the next
+// one's activations and packed weights are already on their way into registers, and two shared-memory buffers leave one
+// barrier per step. Both operands lie as [k][row] with the row XORed by 8 * (k / 4): the transposing stores hit all 32
+// banks and the 128-bit reads of a warp stay conflict-free.
 #include "common.cuh"
 #include "iquant.cuh"
 #include "kernels.h"
 
 namespace lb {
 
-constexpr int BM = 64, BN = 64, BK = 32, PADF = 4;
+constexpr int BK = 16;
 
-// Eight consecutive elements k0..k0+7 (k0 % 8 == 0) of weight row `row`, bit-exact dequant.
-template <int FMT>
-__device__ __forceinline__ void dequant8(const GemmF32Args &p, uint32_t row, uint32_t k0, float (&y)[8]) {
-    if constexpr (FMT == FMT_Q4K) {
-        const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * Q4K_BYTES;
-        uint32_t e = k0 % QK, j = e >> 6, h = (e >> 5) & 1, l0 = e & 31;
-        float d = half_bits_to_float(b[0] | (b[1] << 8)), dmin = half_bits_to_float(b[2] | (b[3] << 8));
-        int sc, mn;
-        scale_min_k4(2 * j + h, b + 4, sc, mn);
-        float d1 = xmul(d, (float)sc), m1 = xmul(dmin, (float)mn);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            int q = (b[16 + 32 * j + l0 + i] >> (4 * h)) & 15;
-            y[i] = xsub(xmul(d1, (float)q), m1);
+// What one thread fetches for eight consecutive weights of a row, before anything waits for it ...
+template <int FMT> struct Raw8 {
+    uint32_t w[FMT == FMT_Q5K ? 8 : FMT == FMT_Q4K ? 6 : FMT == FMT_Q6K ? 6 : FMT == FMT_MXFP4 ? 4 : is_iq(FMT) ? 4 : 3];
+};
+template <int FMT> __device__ __forceinline__ void load_raw8(const GemmF32Args &p, uint32_t row, uint32_t k0, Raw8<FMT> &r) {
+    if constexpr (FMT == FMT_Q4K || FMT == FMT_Q5K) {  // header (d, dmin, scales), then the eight bytes that hold the nibbles (and the fifth bits)
+        const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * (FMT == FMT_Q4K ? Q4K_BYTES : Q5K_BYTES);
+        const uint32_t e = k0 % QK, l0 = e & 31;
+        const uint4 h = *(const uint4 *)b;
+        const uint2 q = *(const uint2 *)(b + (FMT == FMT_Q4K ? 16 : 48) + 32 * (e >> 6) + l0);
+        r.w[0] = h.x, r.w[1] = h.y, r.w[2] = h.z, r.w[3] = h.w, r.w[4] = q.x, r.w[5] = q.y;
+        if constexpr (FMT == FMT_Q5K) {
+            const uint2 f = *(const uint2 *)(b + 16 + l0);
+            r.w[6] = f.x, r.w[7] = f.y;
         }
-    } else if constexpr (FMT == FMT_Q5K) {
-        const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * Q5K_BYTES;
-        uint32_t e = k0 % QK, j = e >> 6, h = (e >> 5) & 1, l0 = e & 31;
-        float d = half_bits_to_float(b[0] | (b[1] << 8)), dmin = half_bits_to_float(b[2] | (b[3] << 8));
-        int sc, mn;
-        scale_min_k4(2 * j + h, b + 4, sc, mn);
-        float d1 = xmul(d, (float)sc), m1 = xmul(dmin, (float)mn);
+    } else if constexpr (FMT == FMT_Q6K) {  // 2-byte aligned blocks
+        const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * Q6K_BYTES;
+        const uint32_t e = k0 % QK, nh = e >> 7, w = (e >> 5) & 3, l0 = e & 31;
+        const uint8_t *ql = b + 64 * nh + 32 * (w & 1) + l0, *qh = b + 128 + 32 * nh + l0;
+        r.w[0] = ld32_by16(ql), r.w[1] = ld32_by16(ql + 4), r.w[2] = ld32_by16(qh), r.w[3] = ld32_by16(qh + 4);
+        r.w[4] = ld16(b + 208);
+        r.w[5] = b[192 + 8 * nh + 2 * w + (l0 >> 4)];
+    } else if constexpr (FMT == FMT_MXFP4) {  // unaligned blocks: the aligned words around the eight bytes
+        const uint8_t *b = p.w + (((uint64_t)row * p.k + k0) / GROUP) * MXFP4_BYTES;
+        const uintptr_t at = (uintptr_t)(b + 1 + (k0 & 15));
+        const uint32_t *a = (const uint32_t *)(at & ~(uintptr_t)3);
+        const uint32_t sh = 8 * (uint32_t)(at & 3), w0 = a[0], w1 = a[1], w2 = sh ? a[2] : 0u;
+        r.w[0] = b[0];
+        r.w[1] = __funnelshift_r(w0, w1, sh);
+        r.w[2] = __funnelshift_r(w1, w2, sh);
+    } else if constexpr (is_iq(FMT)) {  // grid bytes, sign bits, scale
+        const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * iq_block_bytes(FMT);
+        const uint32_t e = k0 % QK;
+        iq_group8<FMT>(b, (int)(e >> 3), p.iq_grid, r.w[0], r.w[1], r.w[2]);
+        r.w[3] = __float_as_uint(iq_half_scale<FMT>(b, (int)(e >> 4)));
+    } else {
+        const uint64_t g = ((uint64_t)row * p.k + k0) / GROUP;
+        const uint2 q = FMT == FMT_INT4 ? *(const uint2 *)(p.w + g * 16 + (k0 & 15)) : *(const uint2 *)(p.w + (uint64_t)row * p.k + k0);
+        r.w[0] = q.x, r.w[1] = q.y, r.w[2] = ((const uint16_t *)(p.w + p.scales_offset))[g];
+    }
+}
+// ... and the weights themselves, bit-exact dequant (each operation rounded on its own, as the reference rounds it).
+template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, uint32_t k0, float (&y)[8]) {
+    if constexpr (FMT == FMT_Q4K || FMT == FMT_Q5K) {
+        const uint32_t e = k0 % QK, j = e >> 6, h = (e >> 5) & 1;
+        const float d = half_bits_to_float(r.w[0] & 0xffffu), dmin = half_bits_to_float(r.w[0] >> 16);
+        int sc0, mn0, sc1, mn1;
+        scale_min_pair(j, r.w[1], r.w[2], r.w[3], sc0, mn0, sc1, mn1);
+        const float d1 = xmul(d, (float)(h ? sc1 : sc0)), m1 = xmul(dmin, (float)(h ? mn1 : mn0));
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            int q = ((b[48 + 32 * j + l0 + i] >> (4 * h)) & 15) + (((b[16 + l0 + i] >> (2 * j + h)) & 1) << 4);
+            int q = (r.w[4 + (i >> 2)] >> (8 * (i & 3) + 4 * h)) & 15;
+            if constexpr (FMT == FMT_Q5K) q += ((r.w[6 + (i >> 2)] >> (8 * (i & 3) + 2 * j + h)) & 1) << 4;
             y[i] = xsub(xmul(d1, (float)q), m1);
         }
     } else if constexpr (FMT == FMT_Q6K) {
-        const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * Q6K_BYTES;
-        uint32_t e = k0 % QK, nh = e >> 7, w = (e >> 5) & 3, l0 = e & 31;
-        float d = half_bits_to_float(b[208] | (b[209] << 8));
-        float t = xmul(d, (float)(int8_t)b[192 + 8 * nh + 2 * w + (l0 >> 4)]);
+        const uint32_t w = ((k0 % QK) >> 5) & 3;
+        const float t = xmul(half_bits_to_float(r.w[4]), (float)(int8_t)r.w[5]);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            int lo = (b[64 * nh + 32 * (w & 1) + l0 + i] >> (4 * (w >> 1))) & 15;
-            int hi = (b[128 + 32 * nh + l0 + i] >> (2 * w)) & 3;
+            const int lo = (r.w[i >> 2] >> (8 * (i & 3) + 4 * (w >> 1))) & 15, hi = (r.w[2 + (i >> 2)] >> (8 * (i & 3) + 2 * w)) & 3;
             y[i] = xmul(t, (float)((lo | (hi << 4)) - 32));
         }
     } else if constexpr (FMT == FMT_MXFP4) {
-        const uint8_t *b = p.w + (((uint64_t)row * p.k + k0) / GROUP) * MXFP4_BYTES;
-        const uint32_t e = k0 % GROUP;  // 0, 8, 16 or 24
+        const float d = e8m0_half(r.w[0]);
+        const int sh = (k0 & 16) ? 4 : 0;
 #pragma unroll
-        for (int i = 0; i < 8; i++) y[i] = mxfp4_element(b, e + i);
-    } else if constexpr (is_iq(FMT)) {  // one 8-group: y = db * grid byte * sign (crates/lapid-quant/src/iq2.rs:38-90, iq3.rs:18-39)
-        const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * iq_block_bytes(FMT);
-        const uint32_t e = k0 % QK;
-        uint32_t lo, hi, signs;
-        iq_group8<FMT>(b, (int)(e >> 3), p.iq_grid, lo, hi, signs);
-        const float db = iq_half_scale<FMT>(b, (int)(e >> 4));
+        for (int i = 0; i < 8; i++) y[i] = xmul((float)mxfp4_kv((r.w[1 + (i >> 2)] >> (8 * (i & 3) + sh)) & 15u), d);
+    } else if constexpr (is_iq(FMT)) {  // y = db * grid byte * sign (crates/lapid-quant/src/iq2.rs:38-90, iq3.rs:18-39)
+        const float db = __uint_as_float(r.w[3]);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const float v = xmul(db, (float)(((i < 4 ? lo : hi) >> (8 * (i & 3))) & 255u));
-            y[i] = (signs >> i) & 1u ? -v : v;
+            const float v = xmul(db, (float)((r.w[i >> 2] >> (8 * (i & 3))) & 255u));
+            y[i] = (r.w[2] >> i) & 1u ? -v : v;
         }
     } else if constexpr (FMT == FMT_INT4) {
-        const uint64_t g = ((uint64_t)row * p.k + k0) / GROUP;
-        const uint32_t e = k0 % GROUP;  // 0, 8, 16 or 24: elements 16.. are the high nibbles of the same bytes
-        const uint8_t *b = p.w + g * 16 + (e & 15);
-        const float d = half_bits_to_float(((const uint16_t *)(p.w + p.scales_offset))[g]);
+        const float d = half_bits_to_float(r.w[2]);
+        const int sh = (k0 & 16) ? 4 : 0;  // elements 16.. of a group are the high nibbles of the same bytes
 #pragma unroll
-        for (int i = 0; i < 8; i++) y[i] = xmul((float)((int)((e < 16 ? b[i] : (b[i] >> 4)) & 15) - 8), d);
+        for (int i = 0; i < 8; i++) y[i] = xmul((float)((int)((r.w[i >> 2] >> (8 * (i & 3) + sh)) & 15u) - 8), d);
     } else {
-        const int8_t *q = (const int8_t *)p.w + (uint64_t)row * p.k + k0;
-        const uint16_t *s = (const uint16_t *)(p.w + p.scales_offset);
-        float d = half_bits_to_float(s[(uint64_t)row * (p.k / GROUP) + k0 / GROUP]);
+        const float d = half_bits_to_float(r.w[2]);
 #pragma unroll
-        for (int i = 0; i < 8; i++) y[i] = xmul((float)q[i], d);
+        for (int i = 0; i < 8; i++) y[i] = xmul((float)(int8_t)(r.w[i >> 2] >> (8 * (i & 3))), d);
     }
 }
 
-template <int FMT> __global__ void __launch_bounds__(256) qgemm_f32_kernel(GemmF32Args p) {
-    __shared__ float As[BK][BM + PADF];
-    __shared__ float Bs[BK][BN + PADF];
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+
+// TM x TN outputs per thread, TM in pairs of rows; both in runs of four (16-byte shared loads), the runs of a thread BM / 2 (BN / 2) apart
+// when there are two of them.
+template <int FMT, int BM, int BN, int TM, int TN> __global__ void __launch_bounds__((BM / TM) * (BN / TN), 65536 / ((BM / TM) * (BN / TN) * 128))
+qgemm_f32_kernel(GemmF32Args p) {
+    constexpr int THREADS = (BM / TM) * (BN / TN), TX = BN / TN;
+    constexpr int AU = BM * 4, WU = BN * 2;  // loads per step: four activations, eight weights each
+    constexpr int AN = (AU + THREADS - 1) / THREADS, WN = (WU + THREADS - 1) / THREADS;
+    static_assert(WU % THREADS == 0 && BM % 8 == 0 && BN % 32 == 0 && TM % 4 == 0 && TN % 4 == 0, "tile");
+    constexpr int SWA = BM >= 32 ? 8 : BM / 4;  // the XOR stays inside the tile's rows
+    __shared__ __align__(16) float As[2][BK][BM];
+    __shared__ __align__(16) float Bs[2][BK][BN];
     const int tid = threadIdx.x;
     const uint32_t row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
     if (p.tile_expert) {  // expert-indexed launch (moe.cu): this activation tile multiplies one expert's matrix
@@ -102,106 +139,204 @@ template <int FMT> __global__ void __launch_bounds__(256) qgemm_f32_kernel(GemmF
         if (e < 0) return;
         p.w += (uint64_t)e * p.id_stride;
     }
-    const int ty = tid >> 4, tx = tid & 15;
-    float acc[4][4];
+    const int ty = tid / TX, tx = tid % TX;
+    uint64_t acc[TM / 2][TN];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < TM / 2; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < TN; j++) acc[i][j] = 0;
 
-    const int lr = tid >> 2, part = tid & 3;  // loader role: tile row / weight row, 8-element part
-    const uint32_t arow = row0 + lr;
-    const void *aptr = nullptr;
-    if (p.tile_expert) {
-        const int32_t pair = p.row_pair[arow];
-        if (pair >= 0) aptr = (const char *)p.a + (p.a_off + (uint64_t)((uint32_t)pair / p.id_r) * p.a_rs) * act_elem_bytes(p.a_type);
-    } else if (arow < p.rows) {
-        aptr = act_row(p.a, p.a_type, p.a_off, p.a_bs, p.a_rs, arow, p.m);
+    const void *aptr[AN];
+#pragma unroll
+    for (int t = 0; t < AN; t++) {
+        const int u = tid + t * THREADS;
+        const uint32_t arow = row0 + (uint32_t)(u >> 2);
+        aptr[t] = nullptr;
+        if (AU % THREADS != 0 && u >= AU) continue;
+        if (p.tile_expert) {
+            const int32_t pair = p.row_pair[arow];
+            if (pair >= 0) aptr[t] = (const char *)p.a + (p.a_off + (uint64_t)((uint32_t)pair / p.id_r) * p.a_rs) * act_elem_bytes(p.a_type);
+        } else if (arow < p.rows) {
+            aptr[t] = act_row(p.a, p.a_type, p.a_off, p.a_bs, p.a_rs, arow, p.m);
+        }
     }
-    const uint32_t wrow = col0 + lr;
 
-    for (uint32_t k0 = 0; k0 < p.k; k0 += BK) {
-        float av[8], wv[8];
+    float av[AN][4];
+    Raw8<FMT> wv[WN];
+    auto fetch = [&](uint32_t k0) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) av[i] = aptr ? load_act(aptr, k0 + part * 8 + i, p.a_type) : 0.0f;
-        if (wrow < p.n) {
-            dequant8<FMT>(p, wrow, k0 + part * 8, wv);
-        } else {
+        for (int t = 0; t < AN; t++) {
+            const uint32_t k = k0 + 4 * (uint32_t)(tid & 3);  // THREADS is a multiple of 4
+            if (!aptr[t]) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) wv[i] = 0.0f;
+                for (int i = 0; i < 4; i++) av[t][i] = 0.0f;
+            } else if (p.a_vec && p.a_type == ACT_F32) {
+                const float4 v = *(const float4 *)((const float *)aptr[t] + k);
+                av[t][0] = v.x, av[t][1] = v.y, av[t][2] = v.z, av[t][3] = v.w;
+            } else if (p.a_vec) {
+                const uint2 v = *(const uint2 *)((const uint16_t *)aptr[t] + k);
+#pragma unroll
+                for (int i = 0; i < 4; i++) av[t][i] = widen_act(((i < 2 ? v.x : v.y) >> (16 * (i & 1))) & 0xffffu, p.a_type);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++) av[t][i] = load_act(aptr[t], k + i, p.a_type);
+            }
         }
-        __syncthreads();  // previous step's readers are done
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            As[part * 8 + i][lr] = av[i];
-            Bs[part * 8 + i][lr] = wv[i];
+        for (int t = 0; t < WN; t++) {
+            const int u = tid + t * THREADS;
+            const uint32_t wrow = col0 + (uint32_t)(u >> 1);
+            load_raw8<FMT>(p, wrow < p.n ? wrow : p.n - 1, k0 + 8 * (uint32_t)(u & 1), wv[t]);  // columns past the matrix are not stored
         }
-        __syncthreads();
+    };
+    auto stage = [&](int buf, uint32_t k0) {
+#pragma unroll
+        for (int t = 0; t < AN; t++) {
+            const int u = tid + t * THREADS;
+            if (AU % THREADS != 0 && u >= AU) continue;
+            const int q = u & 3;
+#pragma unroll
+            for (int i = 0; i < 4; i++) As[buf][4 * q + i][(u >> 2) ^ (SWA * q)] = av[t][i];
+        }
+#pragma unroll
+        for (int t = 0; t < WN; t++) {
+            const int u = tid + t * THREADS, part = u & 1;
+            float y[8];
+            expand8<FMT>(wv[t], k0 + 8 * (uint32_t)part, y);
+#pragma unroll
+            for (int i = 0; i < 8; i++) Bs[buf][8 * part + i][(u >> 1) ^ (8 * (2 * part + (i >> 2)))] = y[i];
+        }
+    };
+
+    fetch(0);
+    stage(0, 0);
+    __syncthreads();
+    int buf = 0;
+    for (uint32_t k0 = 0; k0 < p.k; k0 += BK, buf ^= 1) {
+        const bool more = k0 + BK < p.k;
+        if (more) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; kk++) {
-            float4 a4 = *(const float4 *)&As[kk][ty * 4];
-            float4 b4 = *(const float4 *)&Bs[kk][tx * 4];
-            float a_[4] = {a4.x, a4.y, a4.z, a4.w}, b_[4] = {b4.x, b4.y, b4.z, b4.w};
+            uint64_t a2[TM / 2];
+            float b[TN];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < TM / 4; i++) {
+                const ulonglong2 v = *(const ulonglong2 *)&As[buf][kk][(4 * ty + i * (BM / (TM / 4))) ^ (SWA * (kk >> 2))];
+                a2[2 * i] = v.x, a2[2 * i + 1] = v.y;
+            }
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a_[i], b_[j], acc[i][j]);
+            for (int j = 0; j < TN / 4; j++) *(float4 *)&b[4 * j] = *(const float4 *)&Bs[buf][kk][(4 * tx + j * (BN / (TN / 4))) ^ (8 * (kk >> 2))];
+#pragma unroll
+            for (int j = 0; j < TN; j++) {
+                const uint64_t b2 = pack2(b[j], b[j]);
+#pragma unroll
+                for (int i = 0; i < TM / 2; i++) fma2(acc[i][j], a2[i], b2);
+            }
+        }
+        if (more) {
+            stage(buf ^ 1, k0 + BK);  // the other buffer's readers passed the barrier of the step before
+            __syncthreads();
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        uint32_t r = row0 + ty * 4 + i;
+    for (int i = 0; i < TM; i++) {
+        const uint32_t r = row0 + 4 * ty + (i >> 2) * (BM / (TM / 4)) + (i & 3);
         if (r >= p.rows) continue;
+        float *o;
+        const float *ex = nullptr;
         if (p.tile_expert) {
             const int32_t pair = p.row_pair[r];
             if (pair < 0) continue;
+            o = p.out + p.out_off + (uint64_t)pair * p.n;
+        } else {
+            const uint32_t bt = r / p.m, ii = r % p.m;
+            o = p.out + p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)ii * p.out_rs;
+            if (p.extra) ex = p.extra + (p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)ii * p.ex_s1);
+        }
+#pragma unroll
+        for (int j4 = 0; j4 < TN / 4; j4++) {
+            const uint32_t col = col0 + 4 * tx + j4 * (BN / (TN / 4));
+            float v[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                uint32_t col = col0 + tx * 4 + j;
-                if (col < p.n) p.out[p.out_off + (uint64_t)pair * p.n + col] = acc[i][j];
+                const uint64_t c = acc[i >> 1][4 * j4 + j];
+                v[j] = __uint_as_float((uint32_t)((i & 1) ? c >> 32 : c));
+                if (ex && col + j < p.n) v[j] += ex[(int64_t)(col + j) * p.ex_s2];
             }
-            continue;
-        }
-        uint32_t bt = r / p.m, ii = r % p.m;
+            if (col + 3 < p.n && ((uintptr_t)(o + col) & 15) == 0) *(float4 *)(o + col) = make_float4(v[0], v[1], v[2], v[3]);
+            else
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            uint32_t col = col0 + tx * 4 + j;
-            if (col >= p.n) continue;
-            float v = acc[i][j];
-            if (p.extra) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)ii * p.ex_s1 + (int64_t)col * p.ex_s2];
-            p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)ii * p.out_rs + col] = v;
+                for (int j = 0; j < 4; j++)
+                    if (col + j < p.n) o[col + j] = v[j];
         }
     }
 }
 
-cudaError_t launch_qgemm_f32(int fmt, const GemmF32Args &a, cudaStream_t stream) {
-    if (a.rows == 0 || a.n == 0) return cudaSuccess;
-    dim3 grid((a.n + BN - 1) / BN, (a.rows + BM - 1) / BM);
+template <int FMT, int BM, int BN, int TM, int TN> static cudaError_t launch_tile(const GemmF32Args &a, cudaStream_t stream) {
+    const dim3 grid((a.n + BN - 1) / BN, (a.rows + BM - 1) / BM);
     if (grid.y > 65535) return cudaErrorInvalidValue;
+    qgemm_f32_kernel<FMT, BM, BN, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, stream>>>(a);
+    return cudaGetLastError();
+}
+
+// Activation rows of a tile. An SM works through ceil(tiles / SMs) tiles, so the tile is the one with the least
+// (tiles per SM) x (tile area) / (rate of that tile): large tiles multiply faster (fewer shared loads and less weight expansion
+// per FMA), small ones fill the chip and waste less on a ragged last tile. The rates are relative FMA rates measured on
+// launches that fill the chip with whole tiles.
+constexpr uint32_t F32_BN = 128;
+static uint32_t pick_bm(uint64_t rows, uint64_t n, int sm_count) {
+    const uint32_t bms[] = {128, 64, 32, 16};
+    const double rate[] = {1.0, 0.9, 0.65, 0.4};
+    uint32_t best = 128;
+    double cost = 1e30;
+    for (int i = 0; i < 4; i++) {
+        const uint64_t tiles = ((rows + bms[i] - 1) / bms[i]) * ((n + F32_BN - 1) / F32_BN), per = (tiles + sm_count - 1) / sm_count;
+        const double c = (double)per * bms[i] / rate[i];
+        if (c < cost) cost = c, best = bms[i];
+    }
+    return best;
+}
+uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts) {
+    const uint64_t avg = pairs / (experts ? experts : 1);
+    return avg <= 10 ? 16 : avg <= 24 ? 32 : avg <= 64 ? 64 : 128;
+}
+
+template <int FMT> static cudaError_t launch_fmt(const GemmF32Args &a, int sm_count, cudaStream_t stream) {
+    switch (a.tile_expert ? a.mt : pick_bm(a.rows, a.n, sm_count)) {
+        case 128: return launch_tile<FMT, 128, F32_BN, 8, 8>(a, stream);
+        case 64: return launch_tile<FMT, 64, F32_BN, 8, 8>(a, stream);
+        case 32: return launch_tile<FMT, 32, F32_BN, 8, 4>(a, stream);
+        case 16: return launch_tile<FMT, 16, F32_BN, 4, 4>(a, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_qgemm_f32(int fmt, const GemmF32Args &args, int sm_count, cudaStream_t stream) {
+    if (args.rows == 0 || args.n == 0) return cudaSuccess;
+    GemmF32Args a = args;
+    const uint64_t quad = a.a_type == ACT_F32 ? 16 : 8;  // four activations in one load
+    a.a_vec = ((uintptr_t)a.a + a.a_off * act_elem_bytes(a.a_type)) % quad == 0 && a.a_rs % 4 == 0 && a.a_bs % 4 == 0;
     switch (fmt) {
-        case FMT_Q4K: qgemm_f32_kernel<FMT_Q4K><<<grid, 256, 0, stream>>>(a); break;
-        case FMT_Q5K: qgemm_f32_kernel<FMT_Q5K><<<grid, 256, 0, stream>>>(a); break;
-        case FMT_Q6K: qgemm_f32_kernel<FMT_Q6K><<<grid, 256, 0, stream>>>(a); break;
-        case FMT_INT8: qgemm_f32_kernel<FMT_INT8><<<grid, 256, 0, stream>>>(a); break;
-        case FMT_INT4: qgemm_f32_kernel<FMT_INT4><<<grid, 256, 0, stream>>>(a); break;
-        case FMT_MXFP4: qgemm_f32_kernel<FMT_MXFP4><<<grid, 256, 0, stream>>>(a); break;
+        case FMT_Q4K: return launch_fmt<FMT_Q4K>(a, sm_count, stream);
+        case FMT_Q5K: return launch_fmt<FMT_Q5K>(a, sm_count, stream);
+        case FMT_Q6K: return launch_fmt<FMT_Q6K>(a, sm_count, stream);
+        case FMT_INT8: return launch_fmt<FMT_INT8>(a, sm_count, stream);
+        case FMT_INT4: return launch_fmt<FMT_INT4>(a, sm_count, stream);
+        case FMT_MXFP4: return launch_fmt<FMT_MXFP4>(a, sm_count, stream);
         case FMT_IQ2XXS:
         case FMT_IQ2XS:
         case FMT_IQ2S:
         case FMT_IQ3XXS: {
             const uint8_t *grids = iq_grids();
             if (!grids) return cudaErrorNotReady;
-            GemmF32Args b = a;
-            b.iq_grid = grids + iq_grid_offset(fmt);
-            if (fmt == FMT_IQ2XXS) qgemm_f32_kernel<FMT_IQ2XXS><<<grid, 256, 0, stream>>>(b);
-            else if (fmt == FMT_IQ2XS) qgemm_f32_kernel<FMT_IQ2XS><<<grid, 256, 0, stream>>>(b);
-            else if (fmt == FMT_IQ2S) qgemm_f32_kernel<FMT_IQ2S><<<grid, 256, 0, stream>>>(b);
-            else qgemm_f32_kernel<FMT_IQ3XXS><<<grid, 256, 0, stream>>>(b);
-            break;
+            a.iq_grid = grids + iq_grid_offset(fmt);
+            if (fmt == FMT_IQ2XXS) return launch_fmt<FMT_IQ2XXS>(a, sm_count, stream);
+            if (fmt == FMT_IQ2XS) return launch_fmt<FMT_IQ2XS>(a, sm_count, stream);
+            if (fmt == FMT_IQ2S) return launch_fmt<FMT_IQ2S>(a, sm_count, stream);
+            return launch_fmt<FMT_IQ3XXS>(a, sm_count, stream);
         }
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 }  // namespace lb
