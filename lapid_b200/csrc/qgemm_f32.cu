@@ -12,20 +12,21 @@
 // (crates/lapid-cpu/src/moe.rs:80-118 with float_act, :109).
 //
 // CUDA-core kernel: the order of the sum is fixed (one chain of fused multiply-adds over k per output), so neither the tensor
-// cores nor a split of K can be used; what bounds it is FMA issue (128 a clock and SM). A BM x BN output tile per CTA,
-// 8 x 8 outputs per thread where the tile is large enough. Two neighbouring activation rows share one packed fma.rn.f32x2
-// (two independent, separately rounded FMAs in one instruction): half the issue slots of scalar FMAs, which leaves room
-// for the shared-memory loads and for expanding the weights. k runs in steps of 16; while a step is multiplied the next
-// one's activations and packed weights are already on their way into registers, and two shared-memory buffers leave one
-// barrier per step. Both operands lie as [k][row] with the row XORed by 8 * (k / 4): the transposing stores hit all 32
-// banks and the 128-bit reads of a warp stay conflict-free.
+// cores nor a split of K can be used; what bounds it is FMA issue (128 a clock and SM: 74 TFLOP/s at 1.96 GHz). Two neighbouring
+// activation rows share one packed fma.rn.f32x2 (two independent, separately rounded FMAs in one instruction): half the issue
+// slots of scalar FMAs, which leaves room for the shared-memory loads and for expanding the weights (scalar: 33.4 against
+// 40.6 TFLOP/s at 512 rows on 14336 x 4096). k runs in steps of BK; while a step is multiplied the next one's activations and packed
+// weights are on their way into registers, and two shared-memory buffers leave one barrier per step. Both operands
+// lie as [k][row] in shared memory with an XOR on the row that keeps the transposing stores and the wide reads of a warp free of bank
+// conflicts. int8 weights, 14336 x 4096: 512 rows 1.43 ms (42 TFLOP/s; the 64 x 64 tiles of scalar FMAs without prefetch that this
+// replaces: 2.71 ms), 1184 rows 48.5 TFLOP/s, where the FMA pipe is busy for about 70 % of the time (ncu: the rest is waits on operands).
+#include <math.h>
+
 #include "common.cuh"
 #include "iquant.cuh"
 #include "kernels.h"
 
 namespace lb {
-
-constexpr int BK = 16;
 
 // What one thread fetches for eight consecutive weights of a row, before anything waits for it ...
 template <int FMT> struct Raw8 {
@@ -67,6 +68,10 @@ template <int FMT> __device__ __forceinline__ void load_raw8(const GemmF32Args &
         const uint2 q = FMT == FMT_INT4 ? *(const uint2 *)(p.w + g * 16 + (k0 & 15)) : *(const uint2 *)(p.w + (uint64_t)row * p.k + k0);
         r.w[0] = q.x, r.w[1] = q.y, r.w[2] = ((const uint16_t *)(p.w + p.scales_offset))[g];
     }
+}
+// Byte i of w minus `bias`, as a float: the byte becomes the low mantissa bits of 2^23 (exact; I2F runs at a sixteenth of the rate)
+__device__ __forceinline__ float byte_float(uint32_t w, int i, float bias) {
+    return xsub(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u | (uint32_t)i)), 8388608.0f + bias);
 }
 // ... and the weights themselves, bit-exact dequant (each operation rounded on its own, as the reference rounds it).
 template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, uint32_t k0, float (&y)[8]) {
@@ -110,7 +115,7 @@ template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, u
     } else {
         const float d = half_bits_to_float(r.w[2]);
 #pragma unroll
-        for (int i = 0; i < 8; i++) y[i] = xmul((float)(int8_t)(r.w[i >> 2] >> (8 * (i & 3))), d);
+        for (int i = 0; i < 8; i++) y[i] = xmul(byte_float(r.w[i >> 2] ^ 0x80808080u, i & 3, 128.0f), d);
     }
 }
 
@@ -123,13 +128,19 @@ __device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) { asm(
 
 // TM x TN outputs per thread, TM in pairs of rows; both in runs of four (16-byte shared loads), the runs of a thread BM / 2 (BN / 2) apart
 // when there are two of them.
-template <int FMT, int BM, int BN, int TM, int TN> __global__ void __launch_bounds__((BM / TM) * (BN / TN), 65536 / ((BM / TM) * (BN / TN) * 128))
+template <int FMT, int BM, int BN, int BK, int TM, int TN> __global__ void __launch_bounds__((BM / TM) * (BN / TN), (TM == 16 ? 256 : 512) / ((BM / TM) * (BN / TN)))
 qgemm_f32_kernel(GemmF32Args p) {
-    constexpr int THREADS = (BM / TM) * (BN / TN), TX = BN / TN;
-    constexpr int AU = BM * 4, WU = BN * 2;  // loads per step: four activations, eight weights each
+    constexpr int THREADS = (BM / TM) * (BN / TN), TX = BN / TN, TR = TN % 4 ? 2 : 4;  // TR: columns per run
+    constexpr int AU = BM * BK / 4, WU = BN * BK / 8, WP = BK / 8;  // loads per step: four activations, eight weights each
     constexpr int AN = (AU + THREADS - 1) / THREADS, WN = (WU + THREADS - 1) / THREADS;
-    static_assert(WU % THREADS == 0 && BM % 8 == 0 && BN % 32 == 0 && TM % 4 == 0 && TN % 4 == 0, "tile");
-    constexpr int SWA = BM >= 32 ? 8 : BM / 4;  // the XOR stays inside the tile's rows
+    static_assert(AU % THREADS == 0 && WU % THREADS == 0 && BM % 16 == 0 && BN % 32 == 0 && TM % 4 == 0 && TN % 2 == 0 && (BK == 16 || BK == 64), "tile");
+    // BK = 16: four lanes fetch a row's 16 activations, two its 16 weights; BK = 64: a warp fetches four activations of each of its
+    // rows, eight lanes a row's 64 weights. The XOR that keeps the transposing stores of a warp apart:
+    auto swz_a = [](int k) { return BK == 16 ? 8 * (k >> 2) : 0; };
+    auto swz_b = [](int k) { return BK == 16 ? 8 * (k >> 2) : 4 * (k >> 3); };
+    auto a_row = [](int u) { return BK == 16 ? u >> 2 : u % BM; };
+    auto a_k = [](int u) { return 4 * (BK == 16 ? u & 3 : u / BM); };
+    static_assert(BK == 64 || BM >= 32, "the XOR stays inside the tile's rows");
     __shared__ __align__(16) float As[2][BK][BM];
     __shared__ __align__(16) float Bs[2][BK][BN];
     const int tid = threadIdx.x;
@@ -150,9 +161,8 @@ qgemm_f32_kernel(GemmF32Args p) {
 #pragma unroll
     for (int t = 0; t < AN; t++) {
         const int u = tid + t * THREADS;
-        const uint32_t arow = row0 + (uint32_t)(u >> 2);
+        const uint32_t arow = row0 + (uint32_t)a_row(u);
         aptr[t] = nullptr;
-        if (AU % THREADS != 0 && u >= AU) continue;
         if (p.tile_expert) {
             const int32_t pair = p.row_pair[arow];
             if (pair >= 0) aptr[t] = (const char *)p.a + (p.a_off + (uint64_t)((uint32_t)pair / p.id_r) * p.a_rs) * act_elem_bytes(p.a_type);
@@ -166,8 +176,8 @@ qgemm_f32_kernel(GemmF32Args p) {
     auto fetch = [&](uint32_t k0) {
 #pragma unroll
         for (int t = 0; t < AN; t++) {
-            const uint32_t k = k0 + 4 * (uint32_t)(tid & 3);  // THREADS is a multiple of 4
-            if (!aptr[t]) {
+            const uint32_t k = k0 + (uint32_t)a_k(tid + t * THREADS);
+            if (!aptr[t] || (BK == 64 && k >= p.k)) {
 #pragma unroll
                 for (int i = 0; i < 4; i++) av[t][i] = 0.0f;
             } else if (p.a_vec && p.a_type == ACT_F32) {
@@ -185,29 +195,35 @@ qgemm_f32_kernel(GemmF32Args p) {
 #pragma unroll
         for (int t = 0; t < WN; t++) {
             const int u = tid + t * THREADS;
-            const uint32_t wrow = col0 + (uint32_t)(u >> 1);
-            load_raw8<FMT>(p, wrow < p.n ? wrow : p.n - 1, k0 + 8 * (uint32_t)(u & 1), wv[t]);  // columns past the matrix are not stored
+            const uint32_t wrow = col0 + (uint32_t)(u / WP);
+            const uint32_t k = k0 + 8 * (uint32_t)(u % WP);
+            if (BK == 16 || k < p.k) load_raw8<FMT>(p, wrow < p.n ? wrow : p.n - 1, k, wv[t]);  // columns past the matrix are not stored
         }
     };
     auto stage = [&](int buf, uint32_t k0) {
 #pragma unroll
         for (int t = 0; t < AN; t++) {
-            const int u = tid + t * THREADS;
-            if (AU % THREADS != 0 && u >= AU) continue;
-            const int q = u & 3;
+            const int u = tid + t * THREADS, k = a_k(u);
 #pragma unroll
-            for (int i = 0; i < 4; i++) As[buf][4 * q + i][(u >> 2) ^ (SWA * q)] = av[t][i];
+            for (int i = 0; i < 4; i++) As[buf][k + i][a_row(u) ^ swz_a(k)] = av[t][i];
         }
 #pragma unroll
         for (int t = 0; t < WN; t++) {
-            const int u = tid + t * THREADS, part = u & 1;
+            const int u = tid + t * THREADS, k = 8 * (u % WP);
             float y[8];
-            expand8<FMT>(wv[t], k0 + 8 * (uint32_t)part, y);
+            if (BK == 16 || k0 + (uint32_t)k < p.k) {
+                expand8<FMT>(wv[t], k0 + (uint32_t)k, y);
+            } else {
 #pragma unroll
-            for (int i = 0; i < 8; i++) Bs[buf][8 * part + i][(u >> 1) ^ (8 * (2 * part + (i >> 2)))] = y[i];
+                for (int i = 0; i < 8; i++) y[i] = 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) Bs[buf][k + i][(u / WP) ^ swz_b(k + i)] = y[i];
         }
     };
 
+    // k is a multiple of 32: the last step of BK = 64 may be half full. The rest is 0 * 0, which leaves every accumulator as it is
+    // (none can be -0: a sum that starts at +0 and rounds to nearest never gets there).
     fetch(0);
     stage(0, 0);
     __syncthreads();
@@ -215,22 +231,31 @@ qgemm_f32_kernel(GemmF32Args p) {
     for (uint32_t k0 = 0; k0 < p.k; k0 += BK, buf ^= 1) {
         const bool more = k0 + BK < p.k;
         if (more) fetch(k0 + BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            uint64_t a2[TM / 2];
-            float b[TN];
+        // operands of step kk + 1 are on their way while kk is multiplied
+        uint64_t a2[2][TM / 2];
+        float b[2][TN];
+        auto operands = [&](int kk) {
 #pragma unroll
             for (int i = 0; i < TM / 4; i++) {
-                const ulonglong2 v = *(const ulonglong2 *)&As[buf][kk][(4 * ty + i * (BM / (TM / 4))) ^ (SWA * (kk >> 2))];
-                a2[2 * i] = v.x, a2[2 * i + 1] = v.y;
+                const ulonglong2 v = *(const ulonglong2 *)&As[buf][kk][(4 * ty + i * (BM / (TM / 4))) ^ swz_a(kk)];
+                a2[kk & 1][2 * i] = v.x, a2[kk & 1][2 * i + 1] = v.y;
             }
 #pragma unroll
-            for (int j = 0; j < TN / 4; j++) *(float4 *)&b[4 * j] = *(const float4 *)&Bs[buf][kk][(4 * tx + j * (BN / (TN / 4))) ^ (8 * (kk >> 2))];
+            for (int j = 0; j < TN / TR; j++) {
+                const float *src = &Bs[buf][kk][(TR * tx + j * (BN / (TN / TR))) ^ swz_b(kk)];
+                if constexpr (TR == 4) *(float4 *)&b[kk & 1][4 * j] = *(const float4 *)src;
+                else *(float2 *)&b[kk & 1][2 * j] = *(const float2 *)src;
+            }
+        };
+        operands(0);
+#pragma unroll 16
+        for (int kk = 0; kk < BK; kk++) {
+            if (kk + 1 < BK) operands(kk + 1);
 #pragma unroll
             for (int j = 0; j < TN; j++) {
-                const uint64_t b2 = pack2(b[j], b[j]);
+                const uint64_t b2 = pack2(b[kk & 1][j], b[kk & 1][j]);
 #pragma unroll
-                for (int i = 0; i < TM / 2; i++) fma2(acc[i][j], a2[i], b2);
+                for (int i = 0; i < TM / 2; i++) fma2(acc[i][j], a2[kk & 1][i], b2);
             }
         }
         if (more) {
@@ -254,59 +279,71 @@ qgemm_f32_kernel(GemmF32Args p) {
             if (p.extra) ex = p.extra + (p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)ii * p.ex_s1);
         }
 #pragma unroll
-        for (int j4 = 0; j4 < TN / 4; j4++) {
-            const uint32_t col = col0 + 4 * tx + j4 * (BN / (TN / 4));
-            float v[4];
+        for (int jr = 0; jr < TN / TR; jr++) {
+            const uint32_t col = col0 + TR * tx + jr * (BN / (TN / TR));
+            float v[TR];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint64_t c = acc[i >> 1][4 * j4 + j];
+            for (int j = 0; j < TR; j++) {
+                const uint64_t c = acc[i >> 1][TR * jr + j];
                 v[j] = __uint_as_float((uint32_t)((i & 1) ? c >> 32 : c));
                 if (ex && col + j < p.n) v[j] += ex[(int64_t)(col + j) * p.ex_s2];
             }
-            if (col + 3 < p.n && ((uintptr_t)(o + col) & 15) == 0) *(float4 *)(o + col) = make_float4(v[0], v[1], v[2], v[3]);
-            else
+            if constexpr (TR == 4) {
+                if (col + 3 < p.n && ((uintptr_t)(o + col) & 15) == 0) {
+                    *(float4 *)(o + col) = make_float4(v[0], v[1], v[2], v[3]);
+                    continue;
+                }
+            }
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (col + j < p.n) o[col + j] = v[j];
+            for (int j = 0; j < TR; j++)
+                if (col + j < p.n) o[col + j] = v[j];
         }
     }
 }
 
-template <int FMT, int BM, int BN, int TM, int TN> static cudaError_t launch_tile(const GemmF32Args &a, cudaStream_t stream) {
+template <int FMT, int BM, int BN, int BK, int TM, int TN> static cudaError_t launch_tile(const GemmF32Args &a, cudaStream_t stream) {
     const dim3 grid((a.n + BN - 1) / BN, (a.rows + BM - 1) / BM);
     if (grid.y > 65535) return cudaErrorInvalidValue;
-    qgemm_f32_kernel<FMT, BM, BN, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, stream>>>(a);
+    qgemm_f32_kernel<FMT, BM, BN, BK, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, stream>>>(a);
     return cudaGetLastError();
 }
 
-// Activation rows of a tile. An SM works through ceil(tiles / SMs) tiles, so the tile is the one with the least
-// (tiles per SM) x (tile area) / (rate of that tile): large tiles multiply faster (fewer shared loads and less weight expansion
-// per FMA), small ones fill the chip and waste less on a ragged last tile. The rates are relative FMA rates measured on
-// launches that fill the chip with whole tiles.
-constexpr uint32_t F32_BN = 128;
-static uint32_t pick_bm(uint64_t rows, uint64_t n, int sm_count) {
-    const uint32_t bms[] = {128, 64, 32, 16};
-    const double rate[] = {1.0, 0.9, 0.65, 0.4};
-    uint32_t best = 128;
+// The tiles, and what one costs: an SM with `per` tiles takes about fixed + per * each (us for k = 4096 on a launch that gives every SM
+// that many; measured with int8 weights, the other formats within a tenth). Large tiles multiply faster (fewer shared loads
+// and less weight expansion per FMA: 46, 38, 34 and 15 outputs a us), small ones fill the chip and waste less on a ragged last tile: 512 rows
+// on 14336 x 4096 weights take 1.43 ms on 64 x 64 and 1.47 on 128 x 128 tiles (3.03 of those per SM), 1024 rows 2.72 and 2.52; on
+// 1024 x 4096 weights 16 rows take 84 us on 16 x 32 tiles and 146 on 64 x 64.
+struct F32Tile {
+    uint32_t bm, bn;
+    double fixed, each, least;
+};
+static const F32Tile F32_TILES[] = {{128, 128, 60, 360, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 122, 0}, {16, 32, 15, 35, 84}};
+static int pick_tile(uint64_t matrices, double rows, uint64_t n, int sm_count) {  // `matrices` products of `rows` rows each
+    int best = 0;
     double cost = 1e30;
     for (int i = 0; i < 4; i++) {
-        const uint64_t tiles = ((rows + bms[i] - 1) / bms[i]) * ((n + F32_BN - 1) / F32_BN), per = (tiles + sm_count - 1) / sm_count;
-        const double c = (double)per * bms[i] / rate[i];
-        if (c < cost) cost = c, best = bms[i];
+        const F32Tile &t = F32_TILES[i];
+        const uint64_t tiles = matrices * (uint64_t)ceil(rows / t.bm) * ((n + t.bn - 1) / t.bn), per = (tiles + sm_count - 1) / sm_count;
+        double c = t.fixed + t.each * (double)per;
+        if (c < t.least) c = t.least;
+        if (c < cost) cost = c, best = i;
     }
     return best;
 }
-uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts) {
-    const uint64_t avg = pairs / (experts ? experts : 1);
-    return avg <= 10 ? 16 : avg <= 24 ? 32 : avg <= 64 ? 64 : 128;
+// Expert-indexed launches: the tile for the experts' expected rows plus the spread of a random routing.
+uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts, uint64_t n, int sm_count) {
+    const uint64_t used = experts < pairs ? experts : pairs;
+    if (!used) return 64;
+    const double avg = (double)pairs / (double)used;
+    return F32_TILES[pick_tile(used, avg + (avg > 1 ? sqrt(avg) : 0), n, sm_count)].bm;
 }
 
 template <int FMT> static cudaError_t launch_fmt(const GemmF32Args &a, int sm_count, cudaStream_t stream) {
-    switch (a.tile_expert ? a.mt : pick_bm(a.rows, a.n, sm_count)) {
-        case 128: return launch_tile<FMT, 128, F32_BN, 8, 8>(a, stream);
-        case 64: return launch_tile<FMT, 64, F32_BN, 8, 8>(a, stream);
-        case 32: return launch_tile<FMT, 32, F32_BN, 8, 4>(a, stream);
-        case 16: return launch_tile<FMT, 16, F32_BN, 4, 4>(a, stream);
+    switch (a.tile_expert ? a.mt : F32_TILES[pick_tile(1, a.rows, a.n, sm_count)].bm) {
+        case 128: return launch_tile<FMT, 128, 128, 16, 16, 8>(a, stream);
+        case 64: return launch_tile<FMT, 64, 64, 16, 8, 4>(a, stream);
+        case 32: return launch_tile<FMT, 32, 128, 16, 8, 4>(a, stream);
+        case 16: return launch_tile<FMT, 16, 32, 64, 4, 2>(a, stream);
         default: return cudaErrorInvalidValue;
     }
 }

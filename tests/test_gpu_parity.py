@@ -580,6 +580,30 @@ def _gemm_f32_cases(be, oracle, fmt, name):
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (name, batch, m, n, k)
 
 
+@pytest.mark.parametrize("fmt,name", FMTS)
+@pytest.mark.parametrize("m,n,k,pad", [(16, 33, 288, 1), (17, 31, 96, 0), (65, 4225, 256, 0), (31, 18900, 288, 4), (127, 18900, 320, 2)])
+def test_gemm_f32_tiles_bit_exact(be, oracle, fmt, name, m, n, k, pad):
+    """Each tile of the exact-f32 GEMM at its edges (16 x 32 with a half last step of k, 64 x 64, 32 x 128, 128 x 128), with rows
+    that are and are not aligned for wide loads. Exact: the order of every sum is fixed."""
+    if int(fmt) in (6, 7, 8):
+        k = -(-k // 256) * 256
+    rows = min(n, 200)   # the oracle checks the first and the last weight rows
+    w = np.random.default_rng(900 + m).standard_normal(n * k, dtype=np.float32) * np.float32(0.02)
+    qb = quant.quantize(be, fmt, w, n, k)
+    rs = k + pad
+    a = rnd(m * rs, 901 + m)
+    be.set_option("gemm", "f32")
+    try:
+        got = run_matmul(be, fmt, a, qb, m, n, k, a_row_stride=rs).reshape(m, n)
+    finally:
+        be.set_option("gemm", "tc")
+    for j0 in {0, n - rows}:
+        part = oracle.quantize(int(fmt), w[j0 * k:(j0 + rows) * k], rows, k)   # rows are quantized one by one
+        want, path = oracle.matmul(int(fmt), a, part, rows, k, m=m, a_view=(0, m * rs, rs), fma=True)
+        assert path == "f32_act"
+        assert np.array_equal(np.ascontiguousarray(got[:, j0:j0 + rows]).view(np.uint32), want.reshape(m, rows).view(np.uint32)), (name, m, n, k, j0)
+
+
 # ------------------------------------------------------------------ tensor-core GEMM path (Q4_K)
 def bf16_round(x):
     u = np.ascontiguousarray(x, np.float32).view(np.uint32).astype(np.uint64)
