@@ -62,8 +62,8 @@ __device__ __forceinline__ void quantize_group(const ActQuantArgs &p, uint32_t r
 __global__ void __launch_bounds__(256) act_quant_kernel(ActQuantArgs p) {
     // Under programmatic dependent launch: let the consumer's CTAs start staging weights now,
     // and do not read the activations before the producer grid has completed.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const uint32_t kg = p.k / GROUP;
     const uint64_t n_groups = (uint64_t)p.rows * kg;
@@ -75,8 +75,8 @@ __global__ void __launch_bounds__(256) act_quant_kernel(ActQuantArgs p) {
 // Several independent activation operands in one launch (the pre-passes of a launch list whose
 // inputs are not produced inside the list).
 __global__ void __launch_bounds__(256) act_quant_batch_kernel(ActQuantBatch b) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const uint64_t total = b.group_end[b.count - 1];
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);

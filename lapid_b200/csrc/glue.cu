@@ -39,12 +39,12 @@ __device__ __forceinline__ float sumsq4(float4 a, float ss) { return fmaf(a.x, a
 // every row: 2048 x 8192 took 320 us (0.8 TB/s), now 38 (7.1 TB/s of which part is L2), 77 x 4096 16.5 and 3.0, one row of 4096 inside a
 // decode step 3.5 us less.
 template <int VEC> __global__ void __launch_bounds__(1024) rms_norm_kernel(RmsNormArgs p) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float partial[32];
     const uint32_t row = blockIdx.x, n4 = p.cols / 4, tid = threadIdx.x, step = blockDim.x;
     const size_t at = (size_t)row * n4;
     const float4 *x = (const float4 *)p.x + at, *res = (const float4 *)p.residual + at;
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     float4 v[VEC], r[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; i++) {
@@ -89,8 +89,8 @@ template <int VEC> __global__ void __launch_bounds__(1024) rms_norm_kernel(RmsNo
 // pair by pair from this rank's own slots (protocol: tp_allreduce.cu). The row is split over a cluster of up to 8 CTAs, so that the polling of a
 // single decode row spreads over 8 SMs; their partial sums of squares meet through distributed shared memory.
 __global__ void __launch_bounds__(GLUE_THREADS) tp_rms_norm_kernel(RmsNormArgs p) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float partial[GLUE_THREADS / 32];
     __shared__ float cta_ss;
     cg::cluster_group cluster = cg::this_cluster();
@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(GLUE_THREADS) tp_rms_norm_kernel(RmsNormArgs p
 
 __global__ void __launch_bounds__(GLUE_THREADS) silu_mul_kernel(const float *gate, const float *up, float *out, uint64_t n4, uint32_t cols4,
                                                                 ActOut q) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // whole warps iterate together (the quantized copy needs every lane of a warp in the call)
     for (uint64_t base = (uint64_t)blockIdx.x * GLUE_THREADS + (threadIdx.x & ~31u); base < n4; base += (uint64_t)gridDim.x * GLUE_THREADS) {
         const uint64_t i = base + (threadIdx.x & 31u);
@@ -259,8 +259,8 @@ cudaError_t launch_silu_mul(const float *gate, const float *up, float *out, uint
 __global__ void __launch_bounds__(256) epilogue_expr_kernel(EpiProg prog, float *out, uint64_t out_off, uint64_t out_bs, uint64_t out_rs,
                                                             const float *extra, uint64_t ex_off, int64_t ex_s0, int64_t ex_s1, int64_t ex_s2,
                                                             uint32_t batch, uint32_t m, uint32_t n) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint64_t total = (uint64_t)batch * m * n;
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t row = e / n, j = e - row * n, bt = row / m, i = row - bt * m;

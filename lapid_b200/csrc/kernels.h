@@ -121,7 +121,8 @@ struct GemvArgs {
     // 1: everything the kernel READS (weights, quantized activations) was complete before the kernel in front of it
     // in the stream started, so under programmatic dependent launch it may read and compute without waiting for that
     // kernel and only has to wait before it WRITES. Set by the host for launches whose activations were quantized by
-    // the pre-pass at the head of an execute list, when a fully serialised launch lies in between. Kernels may ignore it.
+    // the pre-pass at the head of an execute list, when a launch lies in between whose CTAs wait before they let it
+    // start (lapid_b200_device::after_hoist). Kernels may ignore it.
     uint32_t early;
 };
 // rows in 1..8. Returns cudaErrorInvalidValue for an unsupported combination.

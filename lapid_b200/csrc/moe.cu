@@ -27,8 +27,8 @@ namespace lb {
 constexpr int ROUTE_THREADS = 1024;
 
 __global__ void __launch_bounds__(ROUTE_THREADS) moe_route_kernel(MoeRouteArgs a) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ uint32_t warp_sum[ROUTE_THREADS / 32];
     __shared__ uint32_t base_tile;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

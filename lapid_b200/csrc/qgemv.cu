@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_kernel(GemvArgs p) {
         if ((uint32_t)i < items) issue(i);
         cp_async_commit();
     }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     float acc[M][C];
     const int blk_l = lane >> 2, pr = lane & 3;  // lane -> (super-block of the stage, 64-element part)

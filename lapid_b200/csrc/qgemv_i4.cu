@@ -19,8 +19,8 @@ namespace i4 {
 constexpr int WARPS = 8;
 
 template <int M> __global__ void __launch_bounds__(WARPS * 32) qgemv_i4_kernel(GemvArgs p) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t k = p.k, kg = k / GROUP;
     if (p.ids) {

@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(Shape<M>::WARPS * 32, Shape<M>::MIN_CTAS) qgem
     issue();
     issue();
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if constexpr (!EARLY) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     bool waited = !EARLY;
     float *pend = act_d + (size_t)p.rows * kg + warp * PEND_ROWS;  // EARLY: behind the activation scales
     uint32_t npend = 0;

@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvArgs p)
     issue();
     issue();
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     __shared__ TpPushCtx tp_ctx;
     if (p.tp && threadIdx.x == 0) tp_push_ctx_load(&tp_ctx, p.tp);

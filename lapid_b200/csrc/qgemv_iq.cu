@@ -88,7 +88,6 @@ __device__ __forceinline__ void unpack32(const uint8_t *b, int ib, const uint8_t
 // leave most warp slots of an SM empty); their partial sums meet in shared memory and are added in warp order.
 template <int FMT, int M, int ROWS, int WARPS, int KS>
 __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const uint8_t *__restrict__ grid_global) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ __align__(16) uint8_t grid[iq_grid_bytes(FMT)];
     {  // the codebook never changes: it may be read before the launch this one depends on has finished
         const uint4 *src = (const uint4 *)grid_global;
@@ -97,6 +96,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
     }
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t k = p.k, kg = k / GROUP, nblk = k / QK;
     constexpr int BB = iq_block_bytes(FMT);

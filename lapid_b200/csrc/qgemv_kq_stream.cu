@@ -149,7 +149,7 @@ qgemv_kq_stream_kernel(const __grid_constant__ Maps<NG> maps, const Head head, G
         trace[TR_UNITS] = u_hi - u_lo;
     }
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (early & 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint64_t *full = (uint64_t *)smem, *empty = full + STAGES;
     volatile uint32_t *region_ok = (volatile uint32_t *)(smem + BAR_BYTES - 16);  // 1 once the staging region is this launch's own; 2: the claim gave up
     uint8_t *stages = smem + BAR_BYTES;
@@ -199,6 +199,7 @@ qgemv_kq_stream_kernel(const __grid_constant__ Maps<NG> maps, const Head head, G
         if (lane == 0) {
             if (!(early & 1)) {
                 asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations come from the kernel in front
+                asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
                 for (uint32_t i = 0; i < pre; i++) load_a(i, i);
             } else {
                 // Claim the staging region: word 0 is its owner (a launch id, 0 = free). Whoever swaps its id into a free

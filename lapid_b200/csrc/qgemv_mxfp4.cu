@@ -63,8 +63,8 @@ template <int M> __device__ __forceinline__ void block_dot(const uint8_t *b, con
 // KS warps share a row and split its blocks (matrices with few rows and a long K would otherwise leave most warp slots of
 // an SM empty); their partial sums meet in shared memory and are added in warp order.
 template <int M, int KS> __global__ void __launch_bounds__(WARPS * 32) qgemv_mxfp4_kernel(GemvArgs p) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t k = p.k, kg = k / GROUP;
     if (p.ids) {
@@ -121,7 +121,6 @@ template <int M, int KS> __global__ void __launch_bounds__(WARPS * 32) qgemv_mxf
 // through its own double buffer in shared memory. The weights do not depend on the launch before this one, so the
 // first row is requested before that launch's results are waited for.
 template <int M> __global__ void __launch_bounds__(WARPS * 32) qgemv_mxfp4_staged_kernel(GemvArgs p) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t k = p.k, kg = k / GROUP, rowb = kg * MXFP4_BYTES;
@@ -150,6 +149,7 @@ template <int M> __global__ void __launch_bounds__(WARPS * 32) qgemv_mxfp4_stage
     uint32_t row = blockIdx.x * WARPS + warp;
     if (row < p.n) request(row, buf);
     if (!p.ids) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (int cur = 0; row < p.n; row += stride, cur ^= 1) {
         if (row + stride < p.n) {
             request(row + stride, buf + (cur ^ 1) * slot);

@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(Shape<M>::WARPS * 32, Shape<M>::MIN_CTAS) qgem
         }
     };
     if constexpr (MOE) {  // the expert ids come from the kernel before this one: nothing can be fetched ahead of it
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
     issue();
     issue();
@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(Shape<M>::WARPS * 32, Shape<M>::MIN_CTAS) qgem
     };
     if (early) copy_acts();
     if constexpr (!MOE) {
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
     bool waited = !early;
 

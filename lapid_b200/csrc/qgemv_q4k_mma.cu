@@ -197,8 +197,8 @@ qgemv_q4k_mma_kernel(const __grid_constant__ WeightMapsT<NG> maps, GemvGroupT<NG
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (early) copy_acts();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     bool waited = !early;
 
     __shared__ TpPushCtx tp_ctx;  // only the first member of a launch may push (tensor-parallel launches are never grouped)
