@@ -1827,7 +1827,7 @@ lapid_b200_status lapid_b200_from_ggml_blocks(lapid_b200_device *dev, int32_t fo
             fail("out_of_bounds", "from_ggml_blocks: output holds " + std::to_string(dst->bytes) + " < " + std::to_string(l.total));
         std::lock_guard<std::mutex> lock(dev->mu);
         dev->make_current();
-        cuda_check(cudaMemsetAsync(dst->ptr, 0, l.total, dev->stream), "memset");
+        cuda_check(lb::zero_gaps(dst->ptr, l.qs_bytes, l.scales_offset, l.scales_bytes, l.total, dev->stream), "memset");
         if (block_bytes(format)) {
             if (want) cuda_check(cudaMemcpyAsync(dst->ptr, src->ptr, want, cudaMemcpyDeviceToDevice, dev->stream), "copy");
         } else if (format == LAPID_B200_DTYPE_INT4) {

@@ -128,20 +128,8 @@ __device__ __forceinline__ int nearest_int(float f) {
     return (int)(__float_as_uint(v) & 0x007fffffu) - 0x00400000;
 }
 
-// 6-bit scale and min of sub-block j (0..8) from the 12 packed bytes of a Q4_K header
-// (crates/lapid-quant/src/kquant.rs:178-184). `s` points at the 12 bytes.
-__device__ __forceinline__ void scale_min_k4(int j, const uint8_t *s, int &sc, int &mn) {
-    if (j < 4) {
-        sc = s[j] & 63;
-        mn = s[j + 4] & 63;
-    } else {
-        sc = (s[j + 4] & 0xF) | ((s[j - 4] >> 6) << 4);
-        mn = (s[j + 4] >> 4) | ((s[j] >> 6) << 4);
-    }
-}
-
-// The same unpacking from the three 32-bit words that hold the 12 bytes (w0 = bytes 0..3,
-// w1 = 4..7, w2 = 8..11): scales and mins of sub-blocks 2p and 2p+1 for pair p.
+// 6-bit scales and mins (crates/lapid-quant/src/kquant.rs:178-184) from the three 32-bit words of a Q4_K header that hold the 12 packed
+// bytes (w0 = bytes 0..3, w1 = 4..7, w2 = 8..11): scales and mins of sub-blocks 2p and 2p+1 for pair p.
 __device__ __forceinline__ void scale_min_pair(int p, uint32_t w0, uint32_t w1, uint32_t w2, int &sc0, int &mn0,
                                                int &sc1, int &mn1) {
     if (p < 2) {

@@ -87,20 +87,4 @@ template <int FMT> __device__ __forceinline__ float iq_half_scale(const uint8_t 
     return xmul(xmul(d, xadd(0.5f, (float)s)), FMT == FMT_IQ3XXS ? 0.5f : 0.25f);
 }
 
-// Element e (0..256) of the block at b, bit for bit as the reference's dequantizers give it.
-template <int FMT> __device__ __forceinline__ float iq_element(const uint8_t *b, int e, const uint8_t *grid) {
-    uint32_t lo, hi, signs;
-    iq_group8<FMT>(b, e >> 3, grid, lo, hi, signs);
-    const int i = e & 7;
-    const uint32_t g = ((i < 4 ? lo : hi) >> (8 * (i & 3))) & 255u;
-    const float v = xmul(iq_half_scale<FMT>(b, e >> 4), (float)g);
-    return (signs >> i) & 1u ? -v : v;
-}
-
-// Four grid bytes with the signs of bits 0..3 of `s` applied, as four int8 values.
-__device__ __forceinline__ uint32_t iq_apply_signs(uint32_t g, uint32_t s) {
-    const uint32_t m = (((s & 15u) * 0x00204081u) & 0x01010101u) * 0xFFu;  // 0xFF in the bytes whose sign bit is set
-    return __vsub4(g ^ m, m);
-}
-
 }  // namespace lb

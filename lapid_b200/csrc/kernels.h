@@ -37,8 +37,9 @@ cudaError_t launch_q8_0_to_planes(const void *blocks, void *dst, uint64_t scales
 cudaError_t launch_q4_0_to_planes(const void *blocks, void *dst, uint64_t scales_offset, uint64_t n_groups,
                                   int sm_count, cudaStream_t stream);
 
-
 // ---- quantize.cu
+// Zeroes what lies between and behind the two planes of a tensor of `total` bytes (one plane: scales_offset is its end).
+cudaError_t zero_gaps(void *dst, uint64_t payload, uint64_t scales_offset, uint64_t scales_bytes, uint64_t total, cudaStream_t stream);
 cudaError_t launch_quantize(int fmt, const float *src, uint64_t rows, uint64_t cols, uint64_t scales_offset,
                             uint64_t total_bytes, void *dst, int sm_count, cudaStream_t stream);
 

@@ -1512,3 +1512,25 @@ def test_gemv_int4_bulk_copy_kernel(be, oracle):
     finally:
         be.set_option("gemv_mma_rows", "2")
         be.set_option("gemv", "fast")
+
+
+@pytest.mark.parametrize("fmt,name", FMTS)
+def test_quantizers_on_extremes(be, oracle, fmt, name):
+    """Values that send the searches to their rare branches (constant and zero sub-blocks, one outlier, all negative, very small and
+    large magnitudes), in a number of blocks that leaves the last CTA part empty."""
+    n, k = 37, 1024
+    w = O.normal(3200, n * k, 0.05).reshape(n, k).copy()
+    w[0] = 0.0
+    w[1] = 0.25
+    w[2] = -0.125
+    w[3, ::32] = 50.0
+    w[4] = -np.abs(w[4])
+    w[5] = np.abs(w[5])
+    w[6] *= 1e-12
+    w[7] *= 1e30 if fmt == lp.DType.MXFP4 else 1e4
+    w[8, 64:256] = 0.0
+    w[9] = np.round(w[9] * 40) / 40
+    want = oracle.quantize(int(fmt), w.reshape(-1), n, k)
+    assert np.array_equal(quant.quantize(be, fmt, w, n, k), want)
+    bits = oracle.dequantize(int(fmt), want, n, k).reshape(-1).view(np.uint32)
+    assert np.array_equal(quant.dequantize(be, fmt, want, n, k).reshape(-1).view(np.uint32), bits)
