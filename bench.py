@@ -521,12 +521,12 @@ def gemv_kernel_name(fmt: int, m: int, n: int = 0, k: int = 0) -> str:
     if fmt == 7:
         return "qgemv_kq_stream_kernel<q5_k>" if m >= 3 and not small else "qgemv_kq_fast_kernel<q5_k>"
     if fmt == 5:
-        return "qgemv_i4_mma_kernel" if m >= 2 else ("qgemv_i8_fast_kernel<int4>" if k % 512 == 0 else "qgemv_i4_kernel")
+        return "qgemv_i8_mma_kernel<int4>" if m >= 2 or k % 512 else "qgemv_i8_fast_kernel<int4>"
     if fmt == 9:
         return "qgemv_mxfp4_mma_kernel" if m >= 3 and k % 512 == 0 else "qgemv_mxfp4_kernel"
     if fmt >= 10:
         return "qgemv_iq_kernel"
-    return "qgemv_i8_mma_kernel" if m >= 2 else "qgemv_i8_fast_kernel"
+    return "qgemv_i8_mma_kernel" if m >= 2 or k % 512 else "qgemv_i8_fast_kernel"
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch / algorithmic bytes of that launch, from the ncu

@@ -33,7 +33,6 @@ SOURCES = {
     "qgemv_iq.cu": [],
     "iquant.cu": ["-DLAPID_B200_IQ_GRIDS_FILE=" + os.path.join(CSRC, "iq_grids.bin")],
     "qgemv_i8_mma.cu": [],
-    "qgemv_i4_mma.cu": [],
     "qgemm_f32.cu": [],
     "qgemm_tc.cu": [],
     "noalloc.cu": [],

@@ -380,6 +380,10 @@ struct PendingGroup {
             if (r.hits(out)) return false;
         g.item[g.count] = a;
         g.count++;
+        if (f == LAPID_B200_DTYPE_INT8 || f == LAPID_B200_DTYPE_INT4) {  // (one activation operand for the whole launch)
+            g.count--;
+            return a.qa == g.item[0].qa;
+        }
         bool fits = md == 3 ? true  // its shared memory does not depend on the members
                     : md != 2 ? lb::qgemv_kq_group_smem(f, g) <= 227 * 1024 - 256
                               : f == LAPID_B200_DTYPE_Q6_K ? lb::qgemv_q6k_mma_group_fits(g) : lb::qgemv_q4k_mma_group_fits(g);
@@ -406,6 +410,8 @@ struct PendingGroup {
         const bool pdl = dev.pdl_launch();
         const uint64_t before = dev.stream_ws.kernels;
         if (mode == 3) cuda_check(lb::launch_qgemv_kq_stream(fmt, out, dev.stream_ws, dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (fmt == LAPID_B200_DTYPE_INT8 || fmt == LAPID_B200_DTYPE_INT4)
+            cuda_check(lb::launch_qgemv_i8_mma(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (mode == 2 && fmt == LAPID_B200_DTYPE_Q6_K) cuda_check(lb::launch_qgemv_q6k_mma(out, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (mode == 2) cuda_check(lb::launch_qgemv_q4k_mma(out, dev.sm_count, pdl, dev.stream, dev.gemv_stream ? &dev.stream_ws : nullptr), "qgemv launch");
         else cuda_check(lb::launch_qgemv_kq_group(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
@@ -505,8 +511,9 @@ Plan plan_launch(const lapid_b200_device &dev, const lapid_b200_launch &l) {
                 (p.stream ||
                  (l.b_dtype == LAPID_B200_DTYPE_Q4_K && p.rows >= dev.gemv_mma_rows && lb::qgemv_q4k_mma_shape_ok(p.rows, (uint32_t)l.k)) ||
                  (l.b_dtype == LAPID_B200_DTYPE_Q6_K && p.rows > dev.gemv_mma_rows && lb::qgemv_q6k_mma_shape_ok(p.rows, (uint32_t)l.k)) ||
-                 (l.b_dtype == LAPID_B200_DTYPE_INT8 && p.rows >= dev.gemv_mma_rows && lb::qgemv_i8_mma_shape_ok(p.rows, (uint32_t)l.k)) ||
-                 (l.b_dtype == LAPID_B200_DTYPE_INT4 && p.rows >= dev.gemv_mma_rows && lb::qgemv_i4_mma_shape_ok(p.rows, (uint32_t)l.k)) ||
+                 // (one row: the bulk-copy kernel where it takes the shape)
+                 ((l.b_dtype == LAPID_B200_DTYPE_INT8 || l.b_dtype == LAPID_B200_DTYPE_INT4) && (p.rows >= dev.gemv_mma_rows || (p.rows == 1 && !p.fast_i8)) &&
+                  lb::qgemv_i8_mma_shape_ok(l.b_dtype, p.rows, (uint32_t)l.k)) ||
                  (l.b_dtype == LAPID_B200_DTYPE_MXFP4 && dev.mxfp4_mma_rows > 0 && p.rows >= dev.mxfp4_mma_rows &&
                   lb::qgemv_mxfp4_mma_shape_ok(p.rows, (uint32_t)l.k)));
         // Small Q5_K / Q6_K matrices at three and four rows: their tensor-core kernels cost about 5 us whatever the size
@@ -917,8 +924,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
         g.a_bs = q.a_bs;
         g.a_rs = q.a_rs;
         g.status = dev.status_dev;
-        if (pend && slot->records && l.b_dtype != LAPID_B200_DTYPE_INT8 && l.b_dtype != LAPID_B200_DTYPE_INT4 &&
-            l.b_dtype != LAPID_B200_DTYPE_MXFP4) {  // (the Int8 / Int4 / MXFP4 kernels take one launch at a time)
+        if (pend && slot->records && l.b_dtype != LAPID_B200_DTYPE_MXFP4) {  // (the MXFP4 kernels take one launch at a time)
             using Range = PendingGroup::Range;
             const char *ob = (const char *)out->ptr;
             Range wr{ob + 4 * l.out.offset, ob + 4 * last};
@@ -951,15 +957,13 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
         const uint64_t ws_before = dev.stream_ws.kernels;
         if (slot->records == 2 && l.b_dtype == LAPID_B200_DTYPE_MXFP4) {
             cuda_check(lb::launch_qgemv_mxfp4_mma(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        } else if (slot->records == 2 && l.b_dtype == LAPID_B200_DTYPE_INT4) {
-            cuda_check(lb::launch_qgemv_i4_mma(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        } else if (slot->records == 2 && l.b_dtype == LAPID_B200_DTYPE_INT8) {
-            cuda_check(lb::launch_qgemv_i8_mma(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         } else if (slot->records == 2) {
             lb::GemvGroup one{};
             one.count = 1;
             one.item[0] = g;
-            if (p.stream) cuda_check(lb::launch_qgemv_kq_stream(l.b_dtype, one, dev.stream_ws, dev.sm_count, pdl, dev.stream), "qgemv launch");
+            if (l.b_dtype == LAPID_B200_DTYPE_INT8 || l.b_dtype == LAPID_B200_DTYPE_INT4)
+                cuda_check(lb::launch_qgemv_i8_mma(l.b_dtype, one, dev.sm_count, pdl, dev.stream), "qgemv launch");
+            else if (p.stream) cuda_check(lb::launch_qgemv_kq_stream(l.b_dtype, one, dev.stream_ws, dev.sm_count, pdl, dev.stream), "qgemv launch");
             else if (l.b_dtype == LAPID_B200_DTYPE_Q6_K) cuda_check(lb::launch_qgemv_q6k_mma(one, dev.sm_count, pdl, dev.stream), "qgemv launch");
             else cuda_check(lb::launch_qgemv_q4k_mma(one, dev.sm_count, pdl, dev.stream, dev.gemv_stream ? &dev.stream_ws : nullptr), "qgemv launch");
             g.epi.n = one.item[0].epi.n;  // (cleared when the launch evaluated its expression itself)

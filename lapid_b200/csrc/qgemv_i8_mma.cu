@@ -1,19 +1,28 @@
-// Int8 (GGUF Q8_0 in lapid's plane layout) decode GEMV for 2..8 activation rows on the warp-level
-// int8 tensor-core instruction. Arithmetic as in qgemv_i8.cu: exact integer dot products per
+// Int8 planes (GGUF Q8_0 in lapid's plane layout) and Int4 nibble planes: decode GEMV for 1..8 activation rows on the
+// warp-level int8 tensor-core instruction. Arithmetic as in qgemv_i8.cu / qgemv_i4.cu: exact integer dot products per
 // 32-element group, one f32 step per group, f32(dot) * da * db (crates/lapid-cpu/src/matmul/
 // qkernels.rs:60-84; the order of the two scale multiplications and of the f32 sums differs).
 //
-// The weights are plain signed bytes, so they are the MMA's A operand as they lie in memory: one
+// Int8 weights are plain signed bytes, so they are the MMA's A operand as they lie in memory: one
 // `mma.sync.m16n8k32.s8.s8` covers 16 weight rows x one 32-element group x 8 activation rows, and
-// nothing has to be unpacked. Per CTA the warps split K in chunks of 512 (warp w takes chunks w,
-// w + WARPS, ... of the CTA's 16-row tile) and their partial 16x8 tiles are summed in shared memory in
-// warp order. A warp's stage is 16 rows x 512 quants plus their 16 x 16 f16 scales, brought in by
+// nothing has to be unpacked. Int4: a nibble q (weight q - 8) becomes the int8 value 16 (q - 8) with two logic operations
+// per register, the exact factor 1/16 goes into the group scale. Per CTA the warps split K in chunks of 512 (warp w takes
+// chunks w, w + WARPS, ... of the CTA's 16-row tile) and their partial 16x8 tiles are summed in shared memory in
+// warp order. A warp's stage is 16 rows x 512 quants plus their f16 scales, brought in by
 // `cp.async` (16 bytes per lane and instruction) into a layout of the kernel's choosing: 16-byte
-// chunk c of row r sits at chunk position c ^ 2 (r & 3), which makes the fragment loads (64 bits per
-// lane: within a group the k order is free, lane t takes quants 8t..8t+7 of both operands)
-// bank-conflict free. Stages of the next chunks are in flight while one is consumed (two per warp,
-// cp.async groups), and the first ones are issued before the programmatic-dependent-launch wait.
-// Activations: the same shared-memory tiles as the K-quant tensor-core kernels.
+// chunk c of row r sits at chunk position c ^ 2 (r & 3) (Int4: c ^ (r & 7)), which makes the fragment loads (64 bits per
+// lane: within a group the k order is free, lane t takes quants 8t..8t+7 of both operands; Int4: elements 0..15 are
+// the low nibbles of the group's 16 bytes, 16..31 the high ones) bank-conflict free. Stages of the next chunks are in flight
+// while one is consumed (two per warp, cp.async groups), and the first ones are issued before the
+// programmatic-dependent-launch wait. Activations: the same shared-memory tiles as the K-quant tensor-core kernels.
+//
+// RAGGED: K any multiple of 32. The last chunk of a row is partly there (the copies past it are zero-filled, its missing groups
+// skipped), and a row's scales start at any even byte: three aligned 16-byte pieces around a chunk's 32 bytes of scales
+// are staged and read with 16-bit loads. Widths that are no multiple of 512 are common (2880, shards of 7680) and took the
+// generic dp4a kernel before: RAGGED_FIGURES
+//
+// Several projections over the same activations (q, k, v; gate, up) run as one launch over the concatenated tiles. Early
+// mode (GemvArgs::early): activations are read and tiles computed before the dependency wait, which comes before the first store.
 #include "common.cuh"
 #include "kernels.h"
 #include "tp_ll.cuh"
@@ -21,11 +30,12 @@
 namespace lb {
 namespace i8m {
 
-constexpr int KC = 512;                        // quants per row and stage
-constexpr int Q_BYTES = 16 * KC;               // 8192
-constexpr int STAGE = Q_BYTES + 16 * (KC / 16);  // + 16 rows x 32 bytes of f16 scales = 8704
+constexpr int KC = 512;  // quants per row and stage
 constexpr int STAGES = 2;
 constexpr float MAGIC = 12582912.0f;
+__host__ __device__ constexpr uint32_t row_bytes(bool i4) { return i4 ? KC / 2 : KC; }  // of a row's quants in a stage
+__host__ __device__ constexpr uint32_t scale_bytes(bool ragged) { return ragged ? 48 : KC / 16; }
+__host__ __device__ constexpr uint32_t stage_bytes(bool i4, bool ragged) { return 16 * (row_bytes(i4) + scale_bytes(ragged)); }
 
 __device__ __forceinline__ uint32_t s32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -36,44 +46,76 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, ui
         : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
 }
+// 16 bytes; only the first `bytes` (0 or 16) are read, the rest is zero
+__device__ __forceinline__ void copy16(uint8_t *dst, const uint8_t *src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s32(dst)), "l"(src), "r"(bytes) : "memory");
+}
 
 __host__ __device__ constexpr uint32_t act_block_bytes(uint32_t rows) { return 256 * rows + 512; }  // per 256 k, as the K-quant kernels' tiles
 
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvArgs p) {
+template <bool I4, bool RAGGED, int WARPS, int NG>
+__global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvGroupT<NG> grp) {
     constexpr int THREADS = WARPS * 32;
+    constexpr uint32_t ROWB = row_bytes(I4), Q_BYTES = 16 * ROWB, SCB = scale_bytes(RAGGED), STAGE = stage_bytes(I4, RAGGED);
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gq = lane >> 2, t4 = lane & 3;
-    const uint32_t M = p.rows, k = p.k, kg = k / GROUP;
-    const uint32_t iters = k / KC;
+    const uint32_t M = grp.item[0].rows, k = grp.item[0].k, kg = k / GROUP, rowb = I4 ? k / 2 : k;
+    const uint32_t iters = (k + KC - 1) / KC;
     const uint32_t ABLK = act_block_bytes(M);
-    const uint32_t tasks = (p.n + 15) / 16;
+    const uint32_t tasks = grp.task_end[NG == 1 ? 0 : grp.count - 1];
     const uint32_t t_lo = (uint32_t)(((uint64_t)tasks * blockIdx.x) / gridDim.x);
     const uint32_t t_hi = (uint32_t)(((uint64_t)tasks * (blockIdx.x + 1)) / gridDim.x);
-    const uint8_t *wq = p.w;
-    const uint8_t *ws = p.w + p.scales_offset;
+    // the member a 16-row tile belongs to, and the tile's number inside it
+    auto locate = [&](uint32_t t, uint32_t &local) -> int {
+        int i = 0;
+        if constexpr (NG > 1)
+            while (t >= grp.task_end[i]) i++;
+        local = i ? t - grp.task_end[i - 1] : t;
+        return i;
+    };
 
     uint8_t *ring = smem + (size_t)warp * (STAGES * STAGE);
     float *red = (float *)(smem + (size_t)WARPS * STAGES * STAGE);  // [2][WARPS][128]
     uint8_t *acts = (uint8_t *)(red + 2 * WARPS * 128);
 
-    // producer cursor: (tile, chunk, ring slot). One stage = 512 + 32 sixteen-byte copies, 17 per lane.
+    // producer cursor: (tile, chunk, ring slot). One stage = 512 (Int4: 256) + 32 (RAGGED: 48) sixteen-byte copies.
     uint32_t pt = t_lo, pit = warp, pslot = 0;
     auto issue = [&]() {
         if (pt < t_hi && (uint32_t)warp < iters) {
+            uint32_t local;
+            const GemvArgs &p = grp.item[locate(pt, local)];
             uint8_t *dst = ring + (size_t)pslot * STAGE;
-            const uint32_t row0 = pt * 16;
+            const uint32_t row0 = local * 16;
+            // rows past the end repeat the last one; their outputs are dropped
+            if constexpr (I4) {
 #pragma unroll
-            for (int i = 0; i < 16; i++) {  // quants: lane -> 16-byte chunk `lane` of row i
-                const uint32_t row = min(row0 + i, p.n - 1);  // rows past the end repeat the last one; their outputs are dropped
-                const uint8_t *src = wq + (size_t)row * k + (size_t)pit * KC + 16 * lane;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s32(dst + i * KC + 16 * (lane ^ (2 * (i & 3))))), "l"(src) : "memory");
+                for (int i = 0; i < 8; i++) {  // nibbles: lane -> 16-byte chunk (lane & 15) of row 2 i + (lane >> 4)
+                    const uint32_t r = 2 * i + (lane >> 4), c = lane & 15;
+                    const uint8_t *src = p.w + (size_t)min(row0 + r, p.n - 1) * rowb;
+                    const uint32_t at = pit * ROWB + 16 * c;
+                    const bool there = !RAGGED || at < rowb;
+                    copy16(dst + r * ROWB + 16 * (c ^ (r & 7)), src + (there ? at : 0), there ? 16 : 0);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i++) {  // quants: lane -> 16-byte chunk `lane` of row i
+                    const uint8_t *src = p.w + (size_t)min(row0 + i, p.n - 1) * rowb;
+                    const uint32_t at = pit * ROWB + 16 * lane;
+                    const bool there = !RAGGED || at < rowb;
+                    copy16(dst + i * ROWB + 16 * (lane ^ (2 * (i & 3))), src + (there ? at : 0), there ? 16 : 0);
+                }
             }
-            {   // scales: lane -> half (lane & 1) of row lane / 2
+            if constexpr (RAGGED) {  // scales: piece j of row i of the three aligned ones; the readable bytes end with the matrix's last line
+                const uint64_t end = (p.scales_offset + (uint64_t)p.n * kg * 2 + 15) & ~(uint64_t)15;
+                for (uint32_t e = lane; e < 48; e += 32) {
+                    const uint32_t i = e / 3, j = e % 3;
+                    const uint64_t at = ((p.scales_offset + ((uint64_t)min(row0 + i, p.n - 1) * kg + pit * (KC / GROUP)) * 2) & ~(uint64_t)15) + 16 * j;
+                    copy16(dst + Q_BYTES + i * SCB + 16 * j, p.w + (at < end ? at : 0), at < end ? 16 : 0);
+                }
+            } else {  // scales: lane -> half (lane & 1) of row lane / 2
                 const uint32_t row = min(row0 + (lane >> 1), p.n - 1);
-                const uint8_t *src = ws + ((size_t)row * kg + (size_t)pit * (KC / GROUP)) * 2 + 16 * (lane & 1);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s32(dst + Q_BYTES + 16 * lane)), "l"(src) : "memory");
+                copy16(dst + Q_BYTES + 16 * lane, p.w + p.scales_offset + ((size_t)row * kg + (size_t)pit * (KC / GROUP)) * 2 + 16 * (lane & 1), 16);
             }
             pslot ^= 1;
             pit += WARPS;
@@ -87,16 +129,16 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvArgs p)
     issue();
     issue();
 
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    bool waited = grp.item[0].early == 0;
+    if (waited) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    __shared__ TpPushCtx tp_ctx;
-    if (p.tp && threadIdx.x == 0) tp_push_ctx_load(&tp_ctx, p.tp);
+    __shared__ TpPushCtx tp_ctx;  // (a launch that pushes is never early and has one member)
+    if (grp.item[0].tp && threadIdx.x == 0) tp_push_ctx_load(&tp_ctx, grp.item[0].tp);
     {   // the activation tiles, once per CTA (their own cp.async group, waited for with the first stage)
-        const uint32_t chunks = (k / QK) * ABLK / 16;
-        const uint8_t *src = (const uint8_t *)p.qa;
-        for (uint32_t c = threadIdx.x; c < chunks; c += THREADS)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s32(acts + 16 * c)), "l"(src + 16 * (size_t)c) : "memory");
+        const uint32_t chunks = ((k + QK - 1) / QK) * ABLK / 16;
+        const uint8_t *src = (const uint8_t *)grp.item[0].qa;
+        for (uint32_t c = threadIdx.x; c < chunks; c += THREADS) copy16(acts + 16 * c, src + 16 * (size_t)c, 16);
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
@@ -106,30 +148,54 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvArgs p)
     const uint32_t cp = (uint32_t)(2 * t4) < M ? t4 : 0;  // activation row pair of this lane's C fragment
     uint32_t cslot = 0, par = 0;
     for (uint32_t t = t_lo; t < t_hi; t++, par ^= 1) {
+        uint32_t local;
+        const GemvArgs &p = grp.item[locate(t, local)];
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         for (uint32_t it = warp; it < iters; it += WARPS) {
             asm volatile("cp.async.wait_group 1;" ::: "memory");  // all but the newest group: this stage has landed
             __syncwarp();
             const uint8_t *stage = ring + (size_t)cslot * STAGE;
+            const uint16_t *sr0 = nullptr, *sr1 = nullptr;  // RAGGED: the scales of this lane's two weight rows
+            if constexpr (RAGGED) {
+                auto skew = [&](uint32_t r) { return (uint32_t)((min(local * 16 + r, p.n - 1) * kg + it * (KC / GROUP)) * 2) & 15u; };  // (scales_offset is a multiple of 16)
+                sr0 = (const uint16_t *)(stage + Q_BYTES + gq * SCB + skew(gq));
+                sr1 = (const uint16_t *)(stage + Q_BYTES + (gq + 8) * SCB + skew(gq + 8));
+            }
 #pragma unroll
             for (int blk = 0; blk < 2; blk++) {  // the chunk's two 256-wide activation tiles
                 const uint8_t *ab = acts + (size_t)(2 * it + blk) * ABLK;
                 const float2 *dsp = (const float2 *)(ab + 256 * M) + 2 * cp;  // {da[c0], da[c1]} of group s at [8 * (s >> 1) + (s & 1)]
                 // the f16 scales of this lane's two weight rows for the tile's eight groups
-                const uint4 sw0 = *(const uint4 *)(stage + Q_BYTES + gq * 32 + 16 * blk);
-                const uint4 sw1 = *(const uint4 *)(stage + Q_BYTES + (gq + 8) * 32 + 16 * blk);
+                uint4 sw0 = make_uint4(0, 0, 0, 0), sw1 = sw0;
+                if constexpr (!RAGGED) {
+                    sw0 = *(const uint4 *)(stage + Q_BYTES + gq * SCB + 16 * blk);
+                    sw1 = *(const uint4 *)(stage + Q_BYTES + (gq + 8) * SCB + 16 * blk);
+                }
                 const uint32_t s0[4] = {sw0.x, sw0.y, sw0.z, sw0.w}, s1[4] = {sw1.x, sw1.y, sw1.z, sw1.w};
 #pragma unroll
                 for (int s = 0; s < 8; s++) {
-                    const int c16 = 2 * (8 * blk + s) + (t4 >> 1);  // 16-byte chunk of the row that holds quants 8 t4 .. 8 t4 + 7 of the group
-                    const uint2 a_lo = *(const uint2 *)(stage + gq * KC + 16 * (c16 ^ (2 * (gq & 3))) + 8 * (t4 & 1));
-                    const uint2 a_hi = *(const uint2 *)(stage + (gq + 8) * KC + 16 * (c16 ^ (2 * (gq & 3))) + 8 * (t4 & 1));
+                    if (RAGGED && it * (KC / GROUP) + 8 * blk + s >= kg) break;
+                    uint32_t a0, a1, a2, a3;
+                    if constexpr (I4) {
+                        const int c16 = 8 * blk + s;  // the group's 16 bytes are one chunk of the row
+                        const uint2 w_lo = *(const uint2 *)(stage + gq * ROWB + 16 * (c16 ^ (gq & 7)) + 8 * (t4 & 1));
+                        const uint2 w_hi = *(const uint2 *)(stage + (gq + 8) * ROWB + 16 * (c16 ^ (gq & 7)) + 8 * (t4 & 1));
+                        const int sh = t4 < 2 ? 4 : 0;  // low nibbles (elements 0..15 of the group) for t4 < 2, high nibbles above
+                        a0 = ((w_lo.x << sh) & 0xF0F0F0F0u) ^ 0x80808080u, a2 = ((w_lo.y << sh) & 0xF0F0F0F0u) ^ 0x80808080u;
+                        a1 = ((w_hi.x << sh) & 0xF0F0F0F0u) ^ 0x80808080u, a3 = ((w_hi.y << sh) & 0xF0F0F0F0u) ^ 0x80808080u;
+                    } else {
+                        const int c16 = 2 * (8 * blk + s) + (t4 >> 1);  // 16-byte chunk of the row that holds quants 8 t4 .. 8 t4 + 7 of the group
+                        const uint2 w_lo = *(const uint2 *)(stage + gq * ROWB + 16 * (c16 ^ (2 * (gq & 3))) + 8 * (t4 & 1));
+                        const uint2 w_hi = *(const uint2 *)(stage + (gq + 8) * ROWB + 16 * (c16 ^ (2 * (gq & 3))) + 8 * (t4 & 1));
+                        a0 = w_lo.x, a1 = w_hi.x, a2 = w_lo.y, a3 = w_hi.y;
+                    }
                     const uint2 b = *(const uint2 *)(ab + s * (M * 32) + colq * 32 + 8 * t4);
                     int c[4];
-                    mma_s8(c, a_lo.x, a_hi.x, a_lo.y, a_hi.y, b.x, b.y);
+                    mma_s8(c, a0, a1, a2, a3, b.x, b.y);
                     const float2 da = dsp[8 * (s >> 1) + (s & 1)];
-                    const float w0 = half_bits_to_float((s0[s >> 1] >> (16 * (s & 1))) & 0xffff);
-                    const float w1 = half_bits_to_float((s1[s >> 1] >> (16 * (s & 1))) & 0xffff);
+                    const uint32_t h0 = RAGGED ? sr0[8 * blk + s] : (s0[s >> 1] >> (16 * (s & 1))) & 0xffff;
+                    const uint32_t h1 = RAGGED ? sr1[8 * blk + s] : (s1[s >> 1] >> (16 * (s & 1))) & 0xffff;
+                    const float w0 = half_bits_to_float(h0) * (I4 ? 0.0625f : 1.0f), w1 = half_bits_to_float(h1) * (I4 ? 0.0625f : 1.0f);  // (Int4: the dot is 16 times too large)
                     acc[0] = fmaf((__int_as_float(c[0]) - MAGIC) * da.x, w0, acc[0]);
                     acc[1] = fmaf((__int_as_float(c[1]) - MAGIC) * da.y, w0, acc[1]);
                     acc[2] = fmaf((__int_as_float(c[2]) - MAGIC) * da.x, w1, acc[2]);
@@ -147,13 +213,17 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvArgs p)
 #pragma unroll
         for (int i = 0; i < 4; i++) mine[i * 32 + lane] = acc[i];
         __syncthreads();  // the buffer of the other parity is free again once every warp got here
+        if (!waited) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            waited = true;
+        }
         for (uint32_t e = threadIdx.x; e < 128; e += THREADS) {
             const float *src = red + (size_t)par * WARPS * 128 + e;
             float v = src[0];
 #pragma unroll
             for (int w = 1; w < WARPS; w++) v += src[(size_t)w * 128];
             const uint32_t el = e & 31, i = e >> 5;
-            const uint32_t row = t * 16 + (el >> 2) + ((i & 2) ? 8 : 0);
+            const uint32_t row = local * 16 + (el >> 2) + ((i & 2) ? 8 : 0);
             const uint32_t r = 2 * (el & 3) + (i & 1);
             if (row < p.n && r < M) {
                 const uint32_t bt = r / p.m, ri = r % p.m;
@@ -166,20 +236,35 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvArgs p)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-static size_t smem_bytes(int warps, uint32_t rows, uint32_t k) {
-    return (size_t)warps * (STAGES * STAGE + 2 * 128 * 4) + (size_t)(k / QK) * act_block_bytes(rows);
+static bool ragged(uint32_t k) { return k % KC != 0; }
+static size_t smem_bytes(bool i4, int warps, uint32_t rows, uint32_t k) {
+    return (size_t)warps * (STAGES * stage_bytes(i4, ragged(k)) + 2 * 128 * 4) + (size_t)((k + QK - 1) / QK) * act_block_bytes(rows);
 }
 
-template <int WARPS> static cudaError_t launch_w(const GemvArgs &a, int sm_count, bool pdl, cudaStream_t stream) {
-    auto kern = qgemv_i8_mma_kernel<WARPS>;
-    const size_t smem = smem_bytes(WARPS, a.rows, a.k);
+template <bool I4, bool RAGGED, int WARPS, int NG> static cudaError_t launch_w(const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream) {
+    auto kern = qgemv_i8_mma_kernel<I4, RAGGED, WARPS, NG>;
+    GemvGroupT<NG> g{};
+    g.count = group.count;
+    uint32_t tasks = 0;
+    for (int i = 0; i < group.count; i++) {
+        g.item[i] = group.item[i];
+        g.task_end[i] = tasks += (group.item[i].n + 15) / 16;
+    }
+    const size_t smem = smem_bytes(I4, WARPS, g.item[0].rows, g.item[0].k);
     static DynamicSmemOptIn opted;
     if (cudaError_t e = opted.raise((const void *)kern, smem); e != cudaSuccess) return e;
-    const uint32_t tasks = (a.n + 15) / 16;
-    uint32_t per_sm = (uint32_t)((227 * 1024) / (smem + 1024));
-    if (per_sm < 1) per_sm = 1;
-    uint32_t grid = (uint32_t)sm_count * per_sm;
-    if (grid > tasks) grid = tasks;
+    uint32_t fit = (uint32_t)((227 * 1024) / (smem + 1024));
+    if (fit < 1) fit = 1;
+    // CTAs per SM: the count whose equal shares of the 16-row tiles are the most even (896 tiles over 296 CTAs are
+    // rounds of 4 and 3: a quarter of the time half the GPU idles; over 148 they are 7 and 6); more CTAs on a tie
+    uint32_t grid = 1;
+    double best = 0.0;
+    for (uint32_t c = 1; c <= fit && c <= 4; c++) {
+        uint32_t gr = (uint32_t)sm_count * c;
+        if (gr > tasks) gr = tasks;
+        const double eff = (double)tasks / ((double)gr * ((tasks + gr - 1) / gr));
+        if (eff >= best) best = eff, grid = gr;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(WARPS * 32);
@@ -190,21 +275,32 @@ template <int WARPS> static cudaError_t launch_w(const GemvArgs &a, int sm_count
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, a);
+    return cudaLaunchKernelEx(&cfg, kern, g);
+}
+template <bool I4, bool RAGGED> static cudaError_t launch_k(const GemvGroup &g, int sm_count, bool pdl, cudaStream_t stream) {
+    const bool eight = smem_bytes(I4, 8, g.item[0].rows, g.item[0].k) <= 227 * 1024 - 256;
+    if (g.count == 1)
+        return eight ? launch_w<I4, RAGGED, 8, 1>(g, sm_count, pdl, stream) : launch_w<I4, RAGGED, 4, 1>(g, sm_count, pdl, stream);
+    return eight ? launch_w<I4, RAGGED, 8, GEMV_GROUP_MAX>(g, sm_count, pdl, stream) : launch_w<I4, RAGGED, 4, GEMV_GROUP_MAX>(g, sm_count, pdl, stream);
 }
 
 }  // namespace i8m
 
-// K a multiple of 512 (whole stages; also makes every 16-byte copy of quants and scales aligned).
-bool qgemv_i8_mma_shape_ok(uint32_t rows, uint32_t k) {
-    if (rows < 1 || rows > 8 || k < i8m::KC || k % i8m::KC != 0) return false;
-    return i8m::smem_bytes(4, rows, k) <= 227 * 1024 - 256;
+// Any K (a multiple of 32) whose activation tiles leave room for four warps' rings.
+bool qgemv_i8_mma_shape_ok(int fmt, uint32_t rows, uint32_t k) {
+    return rows >= 1 && rows <= 8 && k >= GROUP && k % GROUP == 0 && i8m::smem_bytes(fmt == FMT_INT4, 4, rows, k) <= 227 * 1024 - 256;
 }
 
-cudaError_t launch_qgemv_i8_mma(const GemvArgs &a, int sm_count, bool pdl, cudaStream_t stream) {
-    if (!qgemv_i8_mma_shape_ok(a.rows, a.k) || ((uintptr_t)a.w & 15) != 0 || (a.scales_offset & 15) != 0) return cudaErrorInvalidValue;
-    if (i8m::smem_bytes(8, a.rows, a.k) <= 227 * 1024 - 256) return i8m::launch_w<8>(a, sm_count, pdl, stream);
-    return i8m::launch_w<4>(a, sm_count, pdl, stream);
+cudaError_t launch_qgemv_i8_mma(int fmt, const GemvGroup &g, int sm_count, bool pdl, cudaStream_t stream) {
+    if (g.count < 1 || !qgemv_i8_mma_shape_ok(fmt, g.item[0].rows, g.item[0].k)) return cudaErrorInvalidValue;
+    for (int i = 0; i < g.count; i++) {
+        const GemvArgs &a = g.item[i];
+        if (a.qa != g.item[0].qa || a.k != g.item[0].k || a.rows != g.item[0].rows || ((uintptr_t)a.w & 15) != 0 || (a.scales_offset & 15) != 0)
+            return cudaErrorInvalidValue;
+    }
+    const bool rag = i8m::ragged(g.item[0].k);
+    if (fmt == FMT_INT4) return rag ? i8m::launch_k<true, true>(g, sm_count, pdl, stream) : i8m::launch_k<true, false>(g, sm_count, pdl, stream);
+    return rag ? i8m::launch_k<false, true>(g, sm_count, pdl, stream) : i8m::launch_k<false, false>(g, sm_count, pdl, stream);
 }
 
 }  // namespace lb

@@ -536,7 +536,7 @@ static cudaError_t launch_cfg(GemvGroup &g, int sm_count, bool pdl, cudaStream_t
 
 void qgemv_q4k_mma_set_config(int index) { mm::g_force_config = index < 0 || index > 2 ? -1 : index; }
 
-size_t qgemv_q4k_mma_act_bytes(uint32_t rows, uint32_t k) { return (size_t)(k / QK) * mm::act_block_bytes(rows); }
+size_t qgemv_q4k_mma_act_bytes(uint32_t rows, uint32_t k) { return (size_t)((k + QK - 1) / QK) * mm::act_block_bytes(rows); }
 
 bool qgemv_q4k_mma_shape_ok(uint32_t rows, uint32_t k) {
     if (rows < 1 || rows > 8 || k % QK != 0 || k < QK || !mm::encode_fn()) return false;

@@ -1534,3 +1534,29 @@ def test_quantizers_on_extremes(be, oracle, fmt, name):
     assert np.array_equal(quant.quantize(be, fmt, w, n, k), want)
     bits = oracle.dequantize(int(fmt), want, n, k).reshape(-1).view(np.uint32)
     assert np.array_equal(quant.dequantize(be, fmt, want, n, k).reshape(-1).view(np.uint32), bits)
+
+
+@pytest.mark.parametrize("fmt,ofmt", [(lp.DType.Int8, O.INT8), (lp.DType.Int4, O.INT4)])
+def test_gemv_planes_tensor_core_ragged_k(be, oracle, fmt, ofmt):
+    """K that is no multiple of a stage (512) or of an activation tile (256) on the tensor-core decode kernel: the last stage
+    partly there, scales at every offset from a 16-byte boundary, matrices of one row, one warp with work and
+    several chunks per warp; bias; and three projections of one input as one launch, with tiles of 16 rows that end in each."""
+    for i, (m, n, k) in enumerate([(1, 1, 32), (1, 17, 96), (1, 500, 2880), (2, 16, 480), (3, 77, 544), (4, 33, 736), (5, 100, 1056), (8, 500, 2880),
+                                   (8, 9, 7712), (7, 129, 4064), (1, 40, 14368)]):
+        qb = oracle.quantize(ofmt, O.normal(3000 + i, n * k, 0.05), n, k)
+        a, bv = O.normal(3050 + i, m * k), O.normal(3070 + i, n) if i % 2 else None
+        want, path = oracle.matmul(ofmt, a, qb, n, k, m=m, bias=bv)
+        assert path == "int8_act"
+        got = run_matmul(be, fmt, a, qb, m, n, k, bias=bv)
+        assert max_rel(got, want) <= 2e-5, (m, n, k, max_rel(got, want))
+    for m, k in ((3, 2880), (1, 736), (8, 1024)):
+        ns = (300, 17, 64)
+        x = O.normal(3090 + m, m * k)
+        qbs = [oracle.quantize(ofmt, O.normal(3100 + n, n * k, 0.05), n, k) for n in ns]
+        bufs = [be.upload(x)] + [be.upload(q) for q in qbs] + [be.alloc(m * n * 4) for n in ns]
+        be.take_launch_count()
+        be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1 + i), output=4 + i) for i, n in enumerate(ns)], bufs)
+        assert be.take_launch_count() == 2   # the pre-pass and one kernel
+        for i, n in enumerate(ns):
+            want, _ = oracle.matmul(ofmt, x, qbs[i], n, k, m=m)
+            assert max_rel(bufs[4 + i].download().view(np.float32), want) <= 2e-5, (m, k, n)
