@@ -323,6 +323,7 @@ struct Plan {
     int records() const { return mma ? 2 : fast ? 1 : 0; }  // ActQuantArgs::records
     bool fast_i8 = false;  // specialised Int8 / Int4 GEMV with bulk-copy rings (activations as planes)
     bool tc = false;     // tensor-core GEMM (needs a bf16 copy of the activations in the scratch)
+    size_t tc_copy = 0;  // bytes of that copy, the first of the scratch bytes
 };
 
 // Where the quantized activations of a decode launch live in the scratch, and who makes them.
@@ -335,6 +336,11 @@ struct ActSlot {
     size_t offset = 0;     // into the device scratch
     bool hoisted = false;  // quantized by the batched pre-pass at the head of the call
     bool done = false;
+    // A prefill launch on the tensor cores (records = TC_COPY): `offset` is where its partial sums go, `copy_offset` its bf16 copy of
+    // the operand; launches that read the same operand share the copy of the first (`owner` slots back; -1: its own).
+    static constexpr int TC_COPY = 3;
+    size_t copy_offset = 0, written_before = 0;
+    int owner = -1;
     bool same(const ActSlot &o) const {
         return ptr == o.ptr && off == o.off && bs == o.bs && rs == o.rs && rows == o.rows && m == o.m && k == o.k &&
                records == o.records && a_type == o.a_type;
@@ -531,7 +537,10 @@ Plan plan_launch(const lapid_b200_device &dev, const lapid_b200_launch &l) {
     } else {
         p.tc = !dev.gemm_f32 && l.k % 256 == 0 && l.k >= 256 &&
                (l.b_dtype == LAPID_B200_DTYPE_Q4_K || l.b_dtype == LAPID_B200_DTYPE_Q5_K || l.b_dtype == LAPID_B200_DTYPE_Q6_K);
-        if (p.tc) p.scratch = align_up(lb::qgemm_tc_scratch_bytes(p.rows, (uint32_t)l.n, (uint32_t)l.k, dev.sm_count), 256);
+        if (p.tc) {
+            p.tc_copy = lb::qgemm_tc_copy_bytes(p.rows, (uint32_t)l.k);
+            p.scratch = p.tc_copy + align_up(lb::qgemm_tc_partial_bytes(p.rows, (uint32_t)l.n, (uint32_t)l.k, dev.sm_count), 256);
+        }
     }
     return p;
 }
@@ -759,7 +768,7 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         t.status = dev.status_dev;
         t.tile_expert = route.tile_expert;
         t.row_pair = route.row_pair;
-        cuda_check(lb::launch_qgemm_tc_moe(l.b_dtype, t, (uint32_t)p.e, p.mt, a_bf16, dev.stream), "matmul_id gemm launch");
+        cuda_check(lb::launch_qgemm_tc_moe(l.b_dtype, t, (uint32_t)p.e, p.mt, a_bf16, dev.pdl, dev.stream), "matmul_id gemm launch");
         dev.launches += 2;
         return;
     }
@@ -1002,11 +1011,14 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
         t.k = g.k;
         t.status = dev.status_dev;
         if (lb::qgemm_tc_supported(l.b_dtype, t)) {
-            size_t off = 0;
-            if (slot) off = slot->offset;
+            size_t copy_at = 0, partial_at = p.tc_copy;
+            ActSlot *made = nullptr;  // who knows whether the copy is there
+            if (slot) copy_at = slot->copy_offset, partial_at = slot->offset, made = slot - (slot->owner >= 0 ? slot->owner : 0);
             else dev.ensure_scratch(p.scratch);
             int launched = 0;
-            cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, (char *)dev.scratch + off, dev.sm_count, dev.stream, &launched), "qgemm_tc launch");
+            cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, (char *)dev.scratch + copy_at, !(made && made->done), (char *)dev.scratch + partial_at,
+                                           dev.sm_count, dev.pdl, dev.stream, &launched), "qgemm_tc launch");
+            if (made) made->done = true;
             dev.launches += launched;
             expr_pass();
             return;
@@ -1139,8 +1151,37 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
             }
             if (p.tc) {
                 ActSlot sl;
+                if (ab) {
+                    sl.ptr = ab->ptr;
+                    sl.off = l.a.offset;
+                    sl.bs = l.a.batch_stride;
+                    sl.rs = l.a.row_stride;
+                    sl.rows = p.rows;
+                    sl.m = (uint32_t)l.m;
+                    sl.k = (uint32_t)l.k;
+                    sl.a_type = act_type_of(l.a_dtype);
+                }
+                sl.records = ActSlot::TC_COPY;
+                sl.written_before = written.size();
+                // the copy an earlier launch of the list makes of the same operand (q, k, v; gate, up), as long as nothing since has written
+                // the buffer it comes from
+                for (size_t s2 = slots.size(); s2-- > 0 && ab && dev->act_reuse;) {
+                    if (!slots[s2].same(sl) || slots[s2].owner >= 0) continue;
+                    bool clean = true;
+                    for (size_t w = slots[s2].written_before; w < written.size(); w++)
+                        if ((const char *)ab->ptr < written[w].hi && written[w].lo < (const char *)ab->ptr + ab->bytes) clean = false;
+                    if (clean) {
+                        sl.owner = (int)(slots.size() - s2);
+                        sl.copy_offset = slots[s2].copy_offset;
+                    }
+                    break;
+                }
+                if (sl.owner < 0) {
+                    sl.copy_offset = scratch_total;
+                    scratch_total += p.tc_copy;
+                }
                 sl.offset = scratch_total;
-                scratch_total += p.scratch;
+                scratch_total += p.scratch - p.tc_copy;
                 slots.push_back(sl);
                 slot_of[i] = (int)slots.size() - 1;
             }

@@ -15,7 +15,7 @@
 //              of the bf16 activation tile (`cp.async.bulk.tensor.2d`, each CTA loads its own copy)
 //   warp 18    one lane drives TMA for the weights: per super-block a 2-D tensor-map copy of the
 //              tile rows' packed blocks (144 bytes; Q6_K: 224 bytes around the 2-byte aligned 210),
-//              one super-block ahead of its consumers; Q6_K rows that are not 16-byte multiples
+//              up to five super-blocks ahead of its consumers; Q6_K rows that are not 16-byte multiples
 //              are copied row by row with the plain bulk copy by all lanes of the warp
 //   warp 1     allocates tensor memory; one lane issues `tcgen05.mma` (M=128, N=MT, K=16, four
 //              per k-step and accumulator) on shared-memory descriptors and commits to mbarriers
@@ -70,7 +70,13 @@ template <int FMT, int MT, int NT, bool PAIR = false> struct Cfg {
     static constexpr int ROW_BYTES = FMT == FMT_Q4K ? Q4K_BYTES : FMT == FMT_Q5K ? Q5K_BYTES : Q6K_BOX;  // packed bytes staged per row and super-block
     static constexpr int RAW_BYTES = TN * ROW_BYTES;                         // one 128-row sub-tile: 18432 / 28672
     static constexpr int RAW = NT * RAW_BYTES;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 2 * RAW + 256 /*barriers*/ + 1024 /*alignment slack*/;
+    // Super-blocks of packed weights in flight or in use: as many as the shared memory has room for, at most six. With two, every
+    // refill's latency (about 2 us from HBM for 128 rows of 144 bytes) fell on the few k-steps of one super-block, which is
+    // what bound the tiles with few activation rows.
+    static constexpr int RAW_FIT = (227 * 1024 - 256 - 1024 - STAGES * STAGE_BYTES) / RAW;
+    static constexpr int RAWS = RAW_FIT > 6 ? 6 : RAW_FIT;
+    static_assert(RAWS >= 2, "shared memory");
+    static constexpr int SMEM = STAGES * STAGE_BYTES + RAWS * RAW + 256 /*barriers*/ + 1024 /*alignment slack*/;
 };
 
 __device__ __forceinline__ uint32_t s32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -201,9 +207,9 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *stage0 = smem;
     uint8_t *raw0 = smem + C::STAGES * C::STAGE_BYTES;
-    uint64_t *bars = (uint64_t *)(raw0 + 2 * C::RAW);
+    uint64_t *bars = (uint64_t *)(raw0 + C::RAWS * C::RAW);
     uint64_t *full_a = bars, *full_b = bars + C::STAGES, *empty = bars + 2 * C::STAGES;
-    uint64_t *raw_full = bars + 3 * C::STAGES, *raw_empty = raw_full + 2, *acc_full = raw_full + 4;
+    uint64_t *raw_full = bars + 3 * C::STAGES, *raw_empty = raw_full + C::RAWS, *acc_full = raw_full + 2 * C::RAWS;
     uint32_t *tmem_slot = (uint32_t *)(acc_full + 1);
     uint64_t *peer_ready = acc_full + 2;  // PAIR, leader CTA: the other CTA's operands of a stage are in place
     uint32_t cta_rank = 0;
@@ -216,6 +222,8 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // rows start at expert * n. Tiles past the last used one have no expert.
     uint32_t wrow0 = 0;
     if (p.tile_expert) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // the routing comes from the kernels in front
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         const int32_t e = p.tile_expert[blockIdx.y];
         if (e < 0) return;  // before any barrier or tensor-memory allocation
         wrow0 = (uint32_t)e * p.n;
@@ -231,7 +239,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             mbar_init(full_b + s, NT == 2 ? DEQ_WARPS : GROUP_WARPS);
             mbar_init(empty + s, 1);
         }
-        for (int r = 0; r < 2; r++) {
+        for (int r = 0; r < C::RAWS; r++) {
             mbar_init(raw_full + r, 1);
             mbar_init(raw_empty + r, DEQ_WARPS);
         }
@@ -259,6 +267,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (warp == 0) {
         // ---------------- TMA producer, activation tiles: one 128-byte-swizzled box per k-step
         if (lane == 0) {
+            // Under programmatic dependent launch: barriers, tensor memory and the first packed weights were set up while the kernel in
+            // front (the bf16 copy, or the GEMM before this one) still ran. Whoever follows may start behind this wait.
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             for (uint32_t ks = 0; ks < ksteps && healthy; ks++) {
                 const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
                 if (!mbar_wait(empty + s, (u & 1) ^ 1, 64)) { healthy = false; break; }
@@ -287,7 +299,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             return (uint32_t)min((uint64_t)Q6K_BOX, end16 - src);
         };
         for (uint32_t b = 0; b < nblk && healthy; b++) {
-            const uint32_t r = b & 1, ur = b >> 1;
+            const uint32_t r = b % C::RAWS, ur = b / C::RAWS;
             if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
             if (lane == 0 && rows_valid) {
                 uint64_t src;
@@ -309,7 +321,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // per copy, a whole super-block (four k-steps) ahead of the dequantizing warps
         if (lane == 0) {
             for (uint32_t b = 0; b < nblk && healthy; b++) {
-                const uint32_t r = b & 1, ur = b >> 1;
+                const uint32_t r = b % C::RAWS, ur = b / C::RAWS;
                 if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
                 mbar_expect_tx(raw_full + r, C::RAW);
 #pragma unroll
@@ -392,7 +404,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         float d1[4], m1[4];                       // sub-block scales of this thread's pairs of the current super-block
         for (uint32_t ks = (NT == 2 ? 0 : grp); ks < ksteps && healthy; ks += (NT == 2 ? 1 : 2)) {
             const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
-            const uint32_t b = ks >> 2, pp = ks & 3, r = b & 1, ur = b >> 1;
+            const uint32_t b = ks >> 2, pp = ks & 3, r = b % C::RAWS, ur = b / C::RAWS;
             if constexpr (FMT == FMT_Q6K) {
                 // Q6_K (NT = 1): a super-block is ql[128] | qh[64] | int8 sc[16] | f16 d = 210 bytes, so it
                 // starts on a 2-byte boundary only; the copy starts at the 16-byte boundary below it and
@@ -509,6 +521,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (NT == 1 && grp != 0) {
             // with one accumulator the second group has no epilogue share
         } else if (healthy && mbar_wait(acc_full, 0)) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");  // (long past: the activations waited for it)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int quarter = warp & 3;  // the TMEM lanes this warp may read
             const uint32_t n = n0 + sub * TN + 32 * quarter + lane;
@@ -591,6 +604,8 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
 // split-K second pass: out[m, n] = sum over the splits (in order) of their partial tiles (+ extra)
 __global__ void __launch_bounds__(256) splitk_sum_kernel(GemmTcArgs p, uint32_t splits) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint64_t total = (uint64_t)p.rows * p.n;
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t m = (uint32_t)(e / p.n), n = (uint32_t)(e % p.n);
@@ -606,6 +621,8 @@ __global__ void __launch_bounds__(256) splitk_sum_kernel(GemmTcArgs p, uint32_t 
 // thread, not per element), a thread converts eight consecutive elements (k is a multiple of 256);
 // VEC: the rows are 16-byte aligned, so the loads are 128-bit.
 template <bool VEC> __global__ void __launch_bounds__(256) a_to_bf16_kernel(GemmTcArgs p, __nv_bfloat16 *dst) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (uint32_t r = blockIdx.y; r < p.rows; r += gridDim.y) {
     const void *srow = act_row(p.a, p.a_type, p.a_off, p.a_bs, p.a_rs, r, p.m);
     const float *src = (const float *)srow;  // (VEC: f32 rows only)
@@ -644,29 +661,30 @@ static EncodeTiledFn encode_fn() {
 }
 
 template <int FMT, int MT, int NT, bool PAIR = false>
-static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma, cudaStream_t stream, uint32_t splits = 1) {
+static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma, bool pdl, cudaStream_t stream, uint32_t splits = 1) {
     auto kern = qgemm_tc_kernel<FMT, MT, NT, PAIR>;
     using C = Cfg<FMT, MT, NT, PAIR>;
     static DynamicSmemOptIn opted;
     if (cudaError_t e = opted.raise((const void *)kern, C::SMEM); e != cudaSuccess) return e;
     dim3 grid((a.n + TN * NT - 1) / (TN * NT), (a.rows + MT - 1) / MT, splits);
-    if (!PAIR) {
-        kern<<<grid, THREADS, C::SMEM, stream>>>(mw, ma, a);
-        return cudaGetLastError();
-    }
-    grid.x = (grid.x + 1) & ~1u;  // whole pairs: a CTA past the last weight row works on zero fill and stores nothing
+    if (PAIR) grid.x = (grid.x + 1) & ~1u;  // whole pairs: a CTA past the last weight row works on zero fill and stores nothing
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    if (pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (PAIR) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
     return cudaLaunchKernelEx(&cfg, kern, mw, ma, a);
 }
 
@@ -688,11 +706,11 @@ static uint32_t tc_block_bytes(int fmt) { return fmt == FMT_Q4K ? Q4K_BYTES : fm
 static uint32_t tc_box_bytes(int fmt) { return fmt == FMT_Q6K ? (uint32_t)tc::Q6K_BOX : tc_block_bytes(fmt); }
 // the one-accumulator tile of a format by activation rows per CTA
 template <int FMT> static cudaError_t launch_one_acc(uint32_t mt, const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma,
-                                                     cudaStream_t stream, uint32_t ways = 1) {
+                                                     bool pdl, cudaStream_t stream, uint32_t ways = 1) {
     using namespace tc;
-    return mt == 64 ? launch_mt<FMT, 64, 1>(a, mw, ma, stream, ways)
-                    : mt == 128 ? launch_mt<FMT, 128, 1>(a, mw, ma, stream, ways)
-                                : mt == 256 ? launch_mt<FMT, 256, 1>(a, mw, ma, stream, ways) : cudaErrorInvalidValue;
+    return mt == 64 ? launch_mt<FMT, 64, 1>(a, mw, ma, pdl, stream, ways)
+                    : mt == 128 ? launch_mt<FMT, 128, 1>(a, mw, ma, pdl, stream, ways)
+                                : mt == 256 ? launch_mt<FMT, 256, 1>(a, mw, ma, pdl, stream, ways) : cudaErrorInvalidValue;
 }
 
 // How many ways K is split: only when the tiles would leave more than half of the SMs idle, never
@@ -715,11 +733,11 @@ static uint32_t splitk_ways(uint32_t rows, uint32_t n, uint32_t k, int sm_count)
     return ways < 1 ? 1 : ways;
 }
 
-// bf16 copy of the activations, then (16-byte aligned) the partial sums of a split-K launch
-size_t qgemm_tc_scratch_bytes(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
-    const size_t a_bytes = ((size_t)rows * k * 2 + 255) & ~(size_t)255;
+// the bf16 copy of the activations, and the partial sums of a split-K launch
+size_t qgemm_tc_copy_bytes(uint32_t rows, uint32_t k) { return ((size_t)rows * k * 2 + 255) & ~(size_t)255; }
+size_t qgemm_tc_partial_bytes(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
     const uint32_t ways = splitk_ways(rows, n, k, sm_count);
-    return a_bytes + (ways > 1 ? (size_t)ways * rows * n * 4 : 0);
+    return ways > 1 ? (size_t)ways * rows * n * 4 : 0;
 }
 
 bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, const void *w) {
@@ -730,7 +748,7 @@ bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, c
     return pitch % 16 == 0 && (n * pitch) % 256 == 0 && experts * n < (1ull << 31);
 }
 
-cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, cudaStream_t stream) {
+cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, bool pdl, cudaStream_t stream) {
     using namespace tc;
     if (a.rows == 0 || a.n == 0) return cudaSuccess;
     EncodeTiledFn enc = encode_fn();
@@ -755,28 +773,40 @@ cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, 
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    if (fmt == FMT_Q6K) return launch_one_acc<FMT_Q6K>(mt, a, mw, ma, stream);
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, stream);
-    return launch_one_acc<FMT_Q4K>(mt, a, mw, ma, stream);
+    if (fmt == FMT_Q6K) return launch_one_acc<FMT_Q6K>(mt, a, mw, ma, pdl, stream);
+    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, pdl, stream);
+    return launch_one_acc<FMT_Q4K>(mt, a, mw, ma, pdl, stream);
 }
 
-cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, int sm_count, cudaStream_t stream, int *launched) {
+template <class... P, class... A> static cudaError_t launch_small(void (*kern)(P...), dim3 grid, bool pdl, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, bool copy, void *partial, int sm_count, bool pdl,
+                            cudaStream_t stream, int *launched) {
     using namespace tc;
     *launched = 0;
     if (a.rows == 0 || a.n == 0) return cudaSuccess;
-    *launched = 2;  // the bf16 copy of the activations + the GEMM (+ the split-K sum)
+    *launched = copy ? 2 : 1;  // (the bf16 copy of the activations and) the GEMM (and the split-K sum)
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     const uint32_t mt = a.rows <= 64 ? 64 : (a.rows <= 128 ? 128 : 256);
 
-    {
+    if (copy) {
         const dim3 cgrid((a.k / 8 + 255) / 256, a.rows < 65535u ? a.rows : 65535u);
         const bool vec = a.a_type == ACT_F32 && ((uintptr_t)a.a & 15) == 0 && a.a_off % 4 == 0 && a.a_bs % 4 == 0 && a.a_rs % 4 == 0;
-        if (vec) a_to_bf16_kernel<true><<<cgrid, 256, 0, stream>>>(a, (__nv_bfloat16 *)a_bf16_scratch);
-        else a_to_bf16_kernel<false><<<cgrid, 256, 0, stream>>>(a, (__nv_bfloat16 *)a_bf16_scratch);
+        const cudaError_t e = launch_small(vec ? a_to_bf16_kernel<true> : a_to_bf16_kernel<false>, cgrid, pdl, stream, a, (__nv_bfloat16 *)a_bf16_scratch);
+        if (e != cudaSuccess) return e;
     }
-    cudaError_t ce = cudaGetLastError();
-    if (ce != cudaSuccess) return ce;
 
     // CTA pairs: Q4_K, more than 128 rows (256-row activation tiles), at least two 256-row weight tiles
     const bool pair = g_tc_pair > 0 && fmt == FMT_Q4K && a.rows > 128 && a.n >= 4 * TN;
@@ -809,16 +839,15 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
     const uint32_t ways = splitk_ways(a.rows, a.n, a.k, sm_count);
     if (ways > 1 && !pair) {
         GemmTcArgs b = a;
-        b.partial = (float *)((char *)a_bf16_scratch + (((size_t)a.rows * a.k * 2 + 255) & ~(size_t)255));
+        b.partial = (float *)partial;
         cudaError_t e;
-        e = fmt == FMT_Q6K ? launch_one_acc<FMT_Q6K>(mt, b, mw, ma, stream, ways)
-                           : fmt == FMT_Q5K ? launch_one_acc<FMT_Q5K>(mt, b, mw, ma, stream, ways) : launch_one_acc<FMT_Q4K>(mt, b, mw, ma, stream, ways);
+        e = fmt == FMT_Q6K ? launch_one_acc<FMT_Q6K>(mt, b, mw, ma, pdl, stream, ways)
+                           : fmt == FMT_Q5K ? launch_one_acc<FMT_Q5K>(mt, b, mw, ma, pdl, stream, ways) : launch_one_acc<FMT_Q4K>(mt, b, mw, ma, pdl, stream, ways);
         if (e != cudaSuccess) return e;
         const uint64_t total = (uint64_t)a.rows * a.n;
         const unsigned sgrid = (unsigned)((total + 255) / 256 > (uint64_t)sm_count * 8 ? (uint64_t)sm_count * 8 : (total + 255) / 256);
-        splitk_sum_kernel<<<sgrid, 256, 0, stream>>>(b, ways);
-        *launched = 3;
-        return cudaGetLastError();
+        ++*launched;
+        return launch_small(splitk_sum_kernel, dim3(sgrid), pdl, stream, b, ways);
     }
     // One or two accumulators per CTA at MT = 256: the 256x256 tile halves the activation traffic
     // but there are half as many tiles; take the shape with the shorter modelled time (waves of
@@ -828,7 +857,7 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
     // CTA measured 1.6x the time of a 256-row one, so it pays when it saves more than that in waves
     // of tiles over the SMs. Q6_K only: for Q4_K the two-accumulator 256x256 tile is the better way
     // to the same reuse (it also halves the activation traffic), measured faster in every case.
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, stream);  // (one accumulator tile: no wide or tall variants built)
+    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, pdl, stream);  // (one accumulator tile: no wide or tall variants built)
     bool tall = false;
     if (a.rows > 256 && fmt == FMT_Q6K) {
         const uint64_t nt = (a.n + TN - 1) / TN;
@@ -837,12 +866,12 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         tall = w512 * 16 < w256 * 10;
     }
     if (g_tc_tall >= 0) tall = g_tc_tall != 0 && a.rows > 256;
-    if (tall) return fmt == FMT_Q6K ? launch_mt<FMT_Q6K, 512, 1>(a, mw, ma, stream) : launch_mt<FMT_Q4K, 512, 1>(a, mw, ma, stream);
+    if (tall) return fmt == FMT_Q6K ? launch_mt<FMT_Q6K, 512, 1>(a, mw, ma, pdl, stream) : launch_mt<FMT_Q4K, 512, 1>(a, mw, ma, pdl, stream);
     if (fmt == FMT_Q6K) {  // the larger staged blocks leave room for one accumulator tile only
         switch (mt) {
-            case 64: return launch_mt<FMT_Q6K, 64, 1>(a, mw, ma, stream);
-            case 128: return launch_mt<FMT_Q6K, 128, 1>(a, mw, ma, stream);
-            default: return launch_mt<FMT_Q6K, 256, 1>(a, mw, ma, stream);
+            case 64: return launch_mt<FMT_Q6K, 64, 1>(a, mw, ma, pdl, stream);
+            case 128: return launch_mt<FMT_Q6K, 128, 1>(a, mw, ma, pdl, stream);
+            default: return launch_mt<FMT_Q6K, 256, 1>(a, mw, ma, pdl, stream);
         }
     }
     bool wide = a.rows > 128 && a.n >= 2 * TN;
@@ -853,11 +882,11 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         wide = w2 * 26 <= w1 * 15;
     }
     if (g_tc_wide >= 0) wide = g_tc_wide != 0;
-    if (pair) return launch_mt<FMT_Q4K, 256, 2, true>(a, mw, ma, stream);
+    if (pair) return launch_mt<FMT_Q4K, 256, 2, true>(a, mw, ma, pdl, stream);
     switch (mt) {
-        case 64: return launch_mt<FMT_Q4K, 64, 1>(a, mw, ma, stream);
-        case 128: return launch_mt<FMT_Q4K, 128, 1>(a, mw, ma, stream);
-        default: return wide ? launch_mt<FMT_Q4K, 256, 2>(a, mw, ma, stream) : launch_mt<FMT_Q4K, 256, 1>(a, mw, ma, stream);
+        case 64: return launch_mt<FMT_Q4K, 64, 1>(a, mw, ma, pdl, stream);
+        case 128: return launch_mt<FMT_Q4K, 128, 1>(a, mw, ma, pdl, stream);
+        default: return wide ? launch_mt<FMT_Q4K, 256, 2>(a, mw, ma, pdl, stream) : launch_mt<FMT_Q4K, 256, 1>(a, mw, ma, pdl, stream);
     }
 }
 
