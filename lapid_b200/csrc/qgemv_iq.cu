@@ -36,37 +36,45 @@ __device__ __forceinline__ void signed8(uint32_t glo, uint32_t ghi, uint32_t s8,
     hi = signed4(ghi, s8 >> 4);
 }
 
-// The eight int8-weight registers (w[2l], w[2l + 1] = 8-group l) and the two half scales of sub-block ib.
+// The packed bytes of sub-block ib of the block at b: grid indices, signs, scales, f16 d.
+struct Raw32 {
+    uint32_t a, b, c, d;
+};
+template <int FMT> __device__ __forceinline__ Raw32 load32(const uint8_t *b, int ib) {
+    const uint8_t *p = b + 2 + 8 * ib;
+    if constexpr (FMT == FMT_IQ2XXS) return Raw32{ld32_by16(p), ld32_by16(p + 4), 0u, ld16(b)};
+    else if constexpr (FMT == FMT_IQ2XS) return Raw32{ld32_by16(p), ld32_by16(p + 4), b[66 + ib], ld16(b)};
+    else if constexpr (FMT == FMT_IQ2S) return Raw32{ld32_by16(b + 2 + 4 * ib), ld32_by16(b + 34 + 4 * ib), (uint32_t)b[66 + ib] | ((uint32_t)b[74 + ib] << 8), ld16(b)};
+    else return Raw32{ld32_by16(p), ld32_by16(p + 4), ld32_by16(b + 66 + 4 * ib), ld16(b)};
+}
+// The eight int8-weight registers (w[2l], w[2l + 1] = 8-group l) and the two half scales of a sub-block.
 template <int FMT>
-__device__ __forceinline__ void unpack32(const uint8_t *b, int ib, const uint8_t *grid, uint32_t (&w)[8], float &sc0, float &sc1) {
-    const float d = half_bits_to_float(ld16(b));
+__device__ __forceinline__ void unpack32(const Raw32 &raw, const uint8_t *grid, uint32_t (&w)[8], float &sc0, float &sc1) {
+    const float d = half_bits_to_float(raw.d);
     uint32_t idx[4], sg[4], s0, s1;  // grid entry and sign-table entry of each 8-group; the 4-bit scales
     if constexpr (FMT == FMT_IQ2XXS) {
-        const uint8_t *p = b + 2 + 8 * ib;
-        const uint32_t q = ld32_by16(p), a1 = ld32_by16(p + 4);
+        const uint32_t q = raw.a, a1 = raw.b;
 #pragma unroll
         for (int l = 0; l < 4; l++) idx[l] = (q >> (8 * l)) & 255u, sg[l] = (a1 >> (7 * l)) & 127u;
         s0 = s1 = a1 >> 28;
     } else if constexpr (FMT == FMT_IQ2XS) {
-        const uint8_t *p = b + 2 + 8 * ib;
-        const uint32_t q01 = ld32_by16(p), q23 = ld32_by16(p + 4), sc = b[66 + ib];
+        const uint32_t q01 = raw.a, q23 = raw.b, sc = raw.c;
         idx[0] = q01 & 511u, sg[0] = (q01 >> 9) & 127u, idx[1] = (q01 >> 16) & 511u, sg[1] = q01 >> 25;
         idx[2] = q23 & 511u, sg[2] = (q23 >> 9) & 127u, idx[3] = (q23 >> 16) & 511u, sg[3] = q23 >> 25;
         s0 = sc & 15u, s1 = sc >> 4;
     } else if constexpr (FMT == FMT_IQ2S) {
-        const uint32_t q = ld32_by16(b + 2 + 4 * ib), sn = ld32_by16(b + 34 + 4 * ib), qh = b[66 + ib], sc = b[74 + ib];
+        const uint32_t q = raw.a, sn = raw.b, qh = raw.c & 255u, sc = raw.c >> 8;
 #pragma unroll
         for (int l = 0; l < 4; l++) idx[l] = ((q >> (8 * l)) & 255u) | (((qh >> (2 * l)) & 3u) << 8), sg[l] = (sn >> (8 * l)) & 255u;
         s0 = sc & 15u, s1 = sc >> 4;
     } else {
-        const uint32_t aux = ld32_by16(b + 66 + 4 * ib);
+        const uint32_t aux = raw.c;
 #pragma unroll
         for (int l = 0; l < 4; l++) sg[l] = (aux >> (7 * l)) & 127u;
         s0 = s1 = aux >> 28;
     }
     if constexpr (FMT == FMT_IQ3XXS) {
-        const uint8_t *p = b + 2 + 8 * ib;
-        const uint32_t q0 = ld32_by16(p), q1 = ld32_by16(p + 4);
+        const uint32_t q0 = raw.a, q1 = raw.b;
 #pragma unroll
         for (int l = 0; l < 4; l++) {
             const uint32_t q = l < 2 ? q0 >> (16 * l) : q1 >> (16 * (l - 2));
@@ -94,12 +102,29 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
         uint4 *dst = (uint4 *)grid;
         for (int i = threadIdx.x; i < iq_grid_bytes(FMT) / 16; i += WARPS * 32) dst[i] = __ldg(src + i);
     }
-    __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t k = p.k, kg = k / GROUP, nblk = k / QK;
     constexpr int BB = iq_block_bytes(FMT);
+    const int ib = lane & 7;  // this lane's sub-block
+    constexpr int RPC = WARPS / KS * ROWS;  // rows of a CTA per pass
+    const int wg = warp / KS, ks = warp % KS;
+    // The packed bytes of the step after the one being multiplied are on their way (those of a row's first step since the pass began, or,
+    // for the first pass, since before the dependency wait): a step is some 110 instructions a row, far less than a trip to HBM.
+    // A token through 8 layers (IQ2_XXS, one row): 581 -> 551 us.
+    Raw32 raw[ROWS];
+    auto fetch = [&](uint32_t row0, uint32_t blk) {
+        if (blk >= nblk) return;
+#pragma unroll
+        for (int j = 0; j < ROWS; j++) {
+            const uint32_t row = row0 + j < p.n ? row0 + j : p.n - 1;  // (a row past the end repeats the last one; not stored)
+            raw[j] = load32<FMT>(p.w + ((uint64_t)row * nblk + blk) * BB, ib);
+        }
+    };
+    const uint32_t blk0 = (lane >> 3) + 4 * ks;
+    if (!p.ids && blockIdx.x * RPC < p.n) fetch(blockIdx.x * RPC + wg * ROWS, blk0);
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (p.ids) {
         // Expert-indexed launch (Kernel::MatMulId at decode sizes): grid row y is one (token, slot) pair
         const uint32_t pair = blockIdx.y, token = pair / p.id_r;
@@ -110,10 +135,8 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
         p.qa += (uint64_t)token * k;
         p.da += (uint64_t)token * kg;
         p.out_off += (uint64_t)pair * p.n;
+        if (blockIdx.x * RPC < p.n) fetch(blockIdx.x * RPC + wg * ROWS, blk0);
     }
-    const int ib = lane & 7;  // this lane's sub-block
-    constexpr int RPC = WARPS / KS * ROWS;  // rows of a CTA per pass
-    const int wg = warp / KS, ks = warp % KS;
     __shared__ float part[KS > 1 ? WARPS * ROWS * M : 1];
     for (uint32_t base = blockIdx.x * RPC; base < p.n; base += gridDim.x * RPC) {  // (the same number of passes for every warp of the CTA)
         const uint32_t row0 = base + wg * ROWS;
@@ -122,14 +145,15 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
         for (int j = 0; j < ROWS; j++)
 #pragma unroll
             for (int r = 0; r < M; r++) acc[j][r] = 0.0f;
-        for (uint32_t blk = (lane >> 3) + 4 * ks; blk < nblk; blk += 4 * KS) {
+        for (uint32_t blk = blk0; blk < nblk; blk += 4 * KS) {
+            Raw32 cur[ROWS];
+#pragma unroll
+            for (int j = 0; j < ROWS; j++) cur[j] = raw[j];
+            fetch(row0, blk + 4 * KS);
             uint32_t w[ROWS][8];
             float sc[ROWS][2];
 #pragma unroll
-            for (int j = 0; j < ROWS; j++) {
-                const uint32_t row = row0 + j < p.n ? row0 + j : p.n - 1;  // (a row past the end repeats the last one; not stored)
-                unpack32<FMT>(p.w + ((uint64_t)row * nblk + blk) * BB, ib, grid, w[j], sc[j][0], sc[j][1]);
-            }
+            for (int j = 0; j < ROWS; j++) unpack32<FMT>(cur[j], grid, w[j], sc[j][0], sc[j][1]);
             const uint32_t g = blk * 8 + ib;  // activation group of this sub-block
 #pragma unroll
             for (int r = 0; r < M; r++) {
@@ -151,6 +175,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
                 }
             }
         }
+        if (base + gridDim.x * RPC < p.n) fetch(row0 + gridDim.x * RPC, blk0);  // the next pass
 #pragma unroll
         for (int j = 0; j < ROWS; j++) {
 #pragma unroll
