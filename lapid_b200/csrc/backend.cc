@@ -768,7 +768,7 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         t.status = dev.status_dev;
         t.tile_expert = route.tile_expert;
         t.row_pair = route.row_pair;
-        cuda_check(lb::launch_qgemm_tc_moe(l.b_dtype, t, (uint32_t)p.e, p.mt, a_bf16, dev.pdl, dev.stream), "matmul_id gemm launch");
+        cuda_check(lb::launch_qgemm_tc_moe(l.b_dtype, t, (uint32_t)p.e, p.mt, a_bf16, dev.stream), "matmul_id gemm launch");
         dev.launches += 2;
         return;
     }
@@ -1017,7 +1017,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             else dev.ensure_scratch(p.scratch);
             int launched = 0;
             cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, (char *)dev.scratch + copy_at, !(made && made->done), (char *)dev.scratch + partial_at,
-                                           dev.sm_count, dev.pdl, dev.stream, &launched), "qgemm_tc launch");
+                                           dev.sm_count, dev.stream, &launched), "qgemm_tc launch");
             if (made) made->done = true;
             dev.launches += launched;
             expr_pass();

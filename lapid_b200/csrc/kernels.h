@@ -324,14 +324,13 @@ bool qgemm_tc_supported(int fmt, const GemmTcArgs &args);
 size_t qgemm_tc_copy_bytes(uint32_t rows, uint32_t k);  // bf16 copy of the activations
 size_t qgemm_tc_partial_bytes(uint32_t rows, uint32_t n, uint32_t k, int sm_count);  // split-K partial sums (0: not split)
 void qgemm_tc_set_splitk(int v);  // tuning: -1 choose, 0 / 1 never, n > 1 always n ways
-// copy: make the bf16 copy first (false: an earlier launch of the same call has made it). pdl: launch programmatically; the weights are
-// then read while the kernel in front, one of the same call, still runs.
-cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &args, void *a_bf16_scratch, bool copy, void *partial, int sm_count, bool pdl,
+// copy: make the bf16 copy first (false: an earlier launch of the same call has made it).
+cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &args, void *a_bf16_scratch, bool copy, void *partial, int sm_count,
                             cudaStream_t stream, int *launched);
 // Kernel::MatMulId on the tensor cores: `a_bf16` holds the activation rows in tile-space order (moe.cu), the
 // weights are a dense stack of `experts` matrices [n, k] (no padding between them), mt in {64, 128, 256}.
 bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, const void *w);
-cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &args, uint32_t experts, uint32_t mt, void *a_bf16, bool pdl, cudaStream_t stream);
+cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &args, uint32_t experts, uint32_t mt, void *a_bf16, cudaStream_t stream);
 void qgemm_tc_set_wide(int v);  // tuning: -1 choose, 0 / 1 force one / two accumulators per CTA
 void qgemm_tc_set_pair(int v);  // tuning: 1 = CTA pairs (cta_group::2) for the two-accumulator Q4_K tile
 void qgemm_tc_set_tall(int v);  // tuning: -1 choose, 0 / 1 never / always 512 activation rows per CTA above 256 rows

@@ -222,8 +222,6 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // rows start at expert * n. Tiles past the last used one have no expert.
     uint32_t wrow0 = 0;
     if (p.tile_expert) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // the routing comes from the kernels in front
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         const int32_t e = p.tile_expert[blockIdx.y];
         if (e < 0) return;  // before any barrier or tensor-memory allocation
         wrow0 = (uint32_t)e * p.n;
@@ -267,10 +265,6 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (warp == 0) {
         // ---------------- TMA producer, activation tiles: one 128-byte-swizzled box per k-step
         if (lane == 0) {
-            // Under programmatic dependent launch: barriers, tensor memory and the first packed weights were set up while the kernel in
-            // front (the bf16 copy, or the GEMM before this one) still ran. Whoever follows may start behind this wait.
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             for (uint32_t ks = 0; ks < ksteps && healthy; ks++) {
                 const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
                 if (!mbar_wait(empty + s, (u & 1) ^ 1, 64)) { healthy = false; break; }
@@ -521,7 +515,6 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (NT == 1 && grp != 0) {
             // with one accumulator the second group has no epilogue share
         } else if (healthy && mbar_wait(acc_full, 0)) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");  // (long past: the activations waited for it)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int quarter = warp & 3;  // the TMEM lanes this warp may read
             const uint32_t n = n0 + sub * TN + 32 * quarter + lane;
@@ -604,8 +597,6 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
 // split-K second pass: out[m, n] = sum over the splits (in order) of their partial tiles (+ extra)
 __global__ void __launch_bounds__(256) splitk_sum_kernel(GemmTcArgs p, uint32_t splits) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint64_t total = (uint64_t)p.rows * p.n;
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t m = (uint32_t)(e / p.n), n = (uint32_t)(e % p.n);
@@ -621,8 +612,6 @@ __global__ void __launch_bounds__(256) splitk_sum_kernel(GemmTcArgs p, uint32_t 
 // thread, not per element), a thread converts eight consecutive elements (k is a multiple of 256);
 // VEC: the rows are 16-byte aligned, so the loads are 128-bit.
 template <bool VEC> __global__ void __launch_bounds__(256) a_to_bf16_kernel(GemmTcArgs p, __nv_bfloat16 *dst) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (uint32_t r = blockIdx.y; r < p.rows; r += gridDim.y) {
     const void *srow = act_row(p.a, p.a_type, p.a_off, p.a_bs, p.a_rs, r, p.m);
     const float *src = (const float *)srow;  // (VEC: f32 rows only)
@@ -661,7 +650,7 @@ static EncodeTiledFn encode_fn() {
 }
 
 template <int FMT, int MT, int NT, bool PAIR = false>
-static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma, bool pdl, cudaStream_t stream, uint32_t splits = 1) {
+static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma, cudaStream_t stream, uint32_t splits = 1) {
     auto kern = qgemm_tc_kernel<FMT, MT, NT, PAIR>;
     using C = Cfg<FMT, MT, NT, PAIR>;
     static DynamicSmemOptIn opted;
@@ -673,12 +662,8 @@ static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const C
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     cfg.attrs = attr;
-    if (pdl) {
-        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-    }
     if (PAIR) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
         attr[cfg.numAttrs].val.clusterDim.x = 2;
@@ -706,11 +691,11 @@ static uint32_t tc_block_bytes(int fmt) { return fmt == FMT_Q4K ? Q4K_BYTES : fm
 static uint32_t tc_box_bytes(int fmt) { return fmt == FMT_Q6K ? (uint32_t)tc::Q6K_BOX : tc_block_bytes(fmt); }
 // the one-accumulator tile of a format by activation rows per CTA
 template <int FMT> static cudaError_t launch_one_acc(uint32_t mt, const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma,
-                                                     bool pdl, cudaStream_t stream, uint32_t ways = 1) {
+                                                     cudaStream_t stream, uint32_t ways = 1) {
     using namespace tc;
-    return mt == 64 ? launch_mt<FMT, 64, 1>(a, mw, ma, pdl, stream, ways)
-                    : mt == 128 ? launch_mt<FMT, 128, 1>(a, mw, ma, pdl, stream, ways)
-                                : mt == 256 ? launch_mt<FMT, 256, 1>(a, mw, ma, pdl, stream, ways) : cudaErrorInvalidValue;
+    return mt == 64 ? launch_mt<FMT, 64, 1>(a, mw, ma, stream, ways)
+                    : mt == 128 ? launch_mt<FMT, 128, 1>(a, mw, ma, stream, ways)
+                                : mt == 256 ? launch_mt<FMT, 256, 1>(a, mw, ma, stream, ways) : cudaErrorInvalidValue;
 }
 
 // How many ways K is split: only when the tiles would leave more than half of the SMs idle, never
@@ -748,7 +733,7 @@ bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, c
     return pitch % 16 == 0 && (n * pitch) % 256 == 0 && experts * n < (1ull << 31);
 }
 
-cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, bool pdl, cudaStream_t stream) {
+cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, cudaStream_t stream) {
     using namespace tc;
     if (a.rows == 0 || a.n == 0) return cudaSuccess;
     EncodeTiledFn enc = encode_fn();
@@ -773,25 +758,12 @@ cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, 
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    if (fmt == FMT_Q6K) return launch_one_acc<FMT_Q6K>(mt, a, mw, ma, pdl, stream);
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, pdl, stream);
-    return launch_one_acc<FMT_Q4K>(mt, a, mw, ma, pdl, stream);
+    if (fmt == FMT_Q6K) return launch_one_acc<FMT_Q6K>(mt, a, mw, ma, stream);
+    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, stream);
+    return launch_one_acc<FMT_Q4K>(mt, a, mw, ma, stream);
 }
 
-template <class... P, class... A> static cudaError_t launch_small(void (*kern)(P...), dim3 grid, bool pdl, cudaStream_t stream, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
-cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, bool copy, void *partial, int sm_count, bool pdl,
+cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, bool copy, void *partial, int sm_count,
                             cudaStream_t stream, int *launched) {
     using namespace tc;
     *launched = 0;
@@ -804,8 +776,9 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
     if (copy) {
         const dim3 cgrid((a.k / 8 + 255) / 256, a.rows < 65535u ? a.rows : 65535u);
         const bool vec = a.a_type == ACT_F32 && ((uintptr_t)a.a & 15) == 0 && a.a_off % 4 == 0 && a.a_bs % 4 == 0 && a.a_rs % 4 == 0;
-        const cudaError_t e = launch_small(vec ? a_to_bf16_kernel<true> : a_to_bf16_kernel<false>, cgrid, pdl, stream, a, (__nv_bfloat16 *)a_bf16_scratch);
-        if (e != cudaSuccess) return e;
+        if (vec) a_to_bf16_kernel<true><<<cgrid, 256, 0, stream>>>(a, (__nv_bfloat16 *)a_bf16_scratch);
+        else a_to_bf16_kernel<false><<<cgrid, 256, 0, stream>>>(a, (__nv_bfloat16 *)a_bf16_scratch);
+        if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
     }
 
     // CTA pairs: Q4_K, more than 128 rows (256-row activation tiles), at least two 256-row weight tiles
@@ -841,13 +814,14 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         GemmTcArgs b = a;
         b.partial = (float *)partial;
         cudaError_t e;
-        e = fmt == FMT_Q6K ? launch_one_acc<FMT_Q6K>(mt, b, mw, ma, pdl, stream, ways)
-                           : fmt == FMT_Q5K ? launch_one_acc<FMT_Q5K>(mt, b, mw, ma, pdl, stream, ways) : launch_one_acc<FMT_Q4K>(mt, b, mw, ma, pdl, stream, ways);
+        e = fmt == FMT_Q6K ? launch_one_acc<FMT_Q6K>(mt, b, mw, ma, stream, ways)
+                           : fmt == FMT_Q5K ? launch_one_acc<FMT_Q5K>(mt, b, mw, ma, stream, ways) : launch_one_acc<FMT_Q4K>(mt, b, mw, ma, stream, ways);
         if (e != cudaSuccess) return e;
         const uint64_t total = (uint64_t)a.rows * a.n;
         const unsigned sgrid = (unsigned)((total + 255) / 256 > (uint64_t)sm_count * 8 ? (uint64_t)sm_count * 8 : (total + 255) / 256);
         ++*launched;
-        return launch_small(splitk_sum_kernel, dim3(sgrid), pdl, stream, b, ways);
+        splitk_sum_kernel<<<sgrid, 256, 0, stream>>>(b, ways);
+        return cudaGetLastError();
     }
     // One or two accumulators per CTA at MT = 256: the 256x256 tile halves the activation traffic
     // but there are half as many tiles; take the shape with the shorter modelled time (waves of
@@ -857,7 +831,7 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
     // CTA measured 1.6x the time of a 256-row one, so it pays when it saves more than that in waves
     // of tiles over the SMs. Q6_K only: for Q4_K the two-accumulator 256x256 tile is the better way
     // to the same reuse (it also halves the activation traffic), measured faster in every case.
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, pdl, stream);  // (one accumulator tile: no wide or tall variants built)
+    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, stream);  // (one accumulator tile: no wide or tall variants built)
     bool tall = false;
     if (a.rows > 256 && fmt == FMT_Q6K) {
         const uint64_t nt = (a.n + TN - 1) / TN;
@@ -866,12 +840,12 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         tall = w512 * 16 < w256 * 10;
     }
     if (g_tc_tall >= 0) tall = g_tc_tall != 0 && a.rows > 256;
-    if (tall) return fmt == FMT_Q6K ? launch_mt<FMT_Q6K, 512, 1>(a, mw, ma, pdl, stream) : launch_mt<FMT_Q4K, 512, 1>(a, mw, ma, pdl, stream);
+    if (tall) return fmt == FMT_Q6K ? launch_mt<FMT_Q6K, 512, 1>(a, mw, ma, stream) : launch_mt<FMT_Q4K, 512, 1>(a, mw, ma, stream);
     if (fmt == FMT_Q6K) {  // the larger staged blocks leave room for one accumulator tile only
         switch (mt) {
-            case 64: return launch_mt<FMT_Q6K, 64, 1>(a, mw, ma, pdl, stream);
-            case 128: return launch_mt<FMT_Q6K, 128, 1>(a, mw, ma, pdl, stream);
-            default: return launch_mt<FMT_Q6K, 256, 1>(a, mw, ma, pdl, stream);
+            case 64: return launch_mt<FMT_Q6K, 64, 1>(a, mw, ma, stream);
+            case 128: return launch_mt<FMT_Q6K, 128, 1>(a, mw, ma, stream);
+            default: return launch_mt<FMT_Q6K, 256, 1>(a, mw, ma, stream);
         }
     }
     bool wide = a.rows > 128 && a.n >= 2 * TN;
@@ -882,11 +856,11 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         wide = w2 * 26 <= w1 * 15;
     }
     if (g_tc_wide >= 0) wide = g_tc_wide != 0;
-    if (pair) return launch_mt<FMT_Q4K, 256, 2, true>(a, mw, ma, pdl, stream);
+    if (pair) return launch_mt<FMT_Q4K, 256, 2, true>(a, mw, ma, stream);
     switch (mt) {
-        case 64: return launch_mt<FMT_Q4K, 64, 1>(a, mw, ma, pdl, stream);
-        case 128: return launch_mt<FMT_Q4K, 128, 1>(a, mw, ma, pdl, stream);
-        default: return wide ? launch_mt<FMT_Q4K, 256, 2>(a, mw, ma, pdl, stream) : launch_mt<FMT_Q4K, 256, 1>(a, mw, ma, pdl, stream);
+        case 64: return launch_mt<FMT_Q4K, 64, 1>(a, mw, ma, stream);
+        case 128: return launch_mt<FMT_Q4K, 128, 1>(a, mw, ma, stream);
+        default: return wide ? launch_mt<FMT_Q4K, 256, 2>(a, mw, ma, stream) : launch_mt<FMT_Q4K, 256, 1>(a, mw, ma, stream);
     }
 }
 
