@@ -316,6 +316,7 @@ struct GemmTcArgs {
     uint32_t rows, m, n, k;
     int *status;
     float *partial;  // split-K launches: [splits][rows][n] partial sums in the scratch; nullptr otherwise
+    uint32_t tiles_x, tiles_y, splits;  // set by the launcher
     // Expert-indexed launches (launch_qgemm_tc_moe): rows = the tile space, n = rows of ONE expert's matrix
     const int32_t *tile_expert;  // nullptr for an ordinary launch
     const int32_t *row_pair;
@@ -330,7 +331,7 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &args, void *a_bf16_scratc
 // Kernel::MatMulId on the tensor cores: `a_bf16` holds the activation rows in tile-space order (moe.cu), the
 // weights are a dense stack of `experts` matrices [n, k] (no padding between them), mt in {64, 128, 256}.
 bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, const void *w);
-cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &args, uint32_t experts, uint32_t mt, void *a_bf16, cudaStream_t stream);
+cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &args, uint32_t experts, uint32_t mt, void *a_bf16, int sm_count, cudaStream_t stream);
 void qgemm_tc_set_wide(int v);  // tuning: -1 choose, 0 / 1 force one / two accumulators per CTA
 void qgemm_tc_set_pair(int v);  // tuning: 1 = CTA pairs (cta_group::2) for the two-accumulator Q4_K tile
 void qgemm_tc_set_tall(int v);  // tuning: -1 choose, 0 / 1 never / always 512 activation rows per CTA above 256 rows

@@ -62,7 +62,7 @@ constexpr uint32_t SPIN_LIMIT = 1u << 24;
 // PAIR: two CTAs of a cluster run as one `cta_group::2` tensor-core unit: each dequantizes its own
 // 128*NT weight rows and loads only HALF of the activation tile (the instruction reads both CTAs'
 // halves), which halves the activation traffic from L2 and leaves room for a third stage.
-template <int FMT, int MT, int NT, bool PAIR = false> struct Cfg {
+template <int FMT, int MT, int NT, bool PAIR = false, bool LOOP = false> struct Cfg {
     static constexpr int STAGES = PAIR ? 3 : ((NT == 2 || MT == 512) ? 2 : (MT == 256 ? 3 : 4));
     static constexpr int A_BYTES = (PAIR ? MT / 2 : MT) * 128;
     static constexpr int W_BYTES = NT * B_BYTES;
@@ -76,6 +76,7 @@ template <int FMT, int MT, int NT, bool PAIR = false> struct Cfg {
     static constexpr int RAW_FIT = (227 * 1024 - 256 - 1024 - STAGES * STAGE_BYTES) / RAW;
     static constexpr int RAWS = RAW_FIT > 6 ? 6 : RAW_FIT;
     static_assert(RAWS >= 2, "shared memory");
+    static constexpr int ACCS = LOOP && 2 * MT * NT <= 512 ? 2 : 1;  // accumulator sets: two where the 512 columns of tensor memory hold them
     static constexpr int SMEM = STAGES * STAGE_BYTES + RAWS * RAW + 256 /*barriers*/ + 1024 /*alignment slack*/;
 };
 
@@ -195,13 +196,36 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// N consecutive columns of this warp's 32 lanes of tensor memory
+template <int N> __device__ __forceinline__ void tmem_ld(uint32_t (&r)[N], uint32_t addr) {
+    static_assert(N == 16 || N == 32, "columns");
+    if constexpr (N == 32)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+              "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+              "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+            : "r"(addr)
+            : "memory");
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(addr)
+            : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // f32 bits of (2^23 + byte `sel` of w): the byte planted in the mantissa by one PRMT
 __device__ __forceinline__ float biased(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)); }
 
-template <int FMT, int MT, int NT, bool PAIR>
+template <int FMT, int MT, int NT, bool PAIR, bool LOOP>
 __global__ void __launch_bounds__(THREADS, 1)
 qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, GemmTcArgs p) {
-    using C = Cfg<FMT, MT, NT, PAIR>;
+    using C = Cfg<FMT, MT, NT, PAIR, LOOP>;
     constexpr int RAW_BYTES = C::RAW_BYTES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -210,26 +234,42 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     uint64_t *bars = (uint64_t *)(raw0 + C::RAWS * C::RAW);
     uint64_t *full_a = bars, *full_b = bars + C::STAGES, *empty = bars + 2 * C::STAGES;
     uint64_t *raw_full = bars + 3 * C::STAGES, *raw_empty = raw_full + C::RAWS, *acc_full = raw_full + 2 * C::RAWS;
-    uint32_t *tmem_slot = (uint32_t *)(acc_full + 1);
-    uint64_t *peer_ready = acc_full + 2;  // PAIR, leader CTA: the other CTA's operands of a stage are in place
+    uint64_t *acc_empty = acc_full + 2;
+    uint32_t *tmem_slot = (uint32_t *)(acc_full + 4);
+    uint64_t *peer_ready = acc_full + 5;  // PAIR, leader CTA: the other CTA's operands of a stage are in place
     uint32_t cta_rank = 0;
     if constexpr (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta_rank));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t n0 = blockIdx.x * (TN * NT), m0 = blockIdx.y * MT;
+    // The tiles of the launch: weight tile x (the fast index), activation tile y, split z of K. LOOP: a CTA takes every gridDim.x-th tile: no CTA
+    // start, tensor-memory allocation and first trip to HBM per tile; the producers run ahead into the next tile, and its first
+    // weights are dequantized before the results of the last one are stored. Expert-indexed launches, whose tiles are many and
+    // short, run this way (512 tokens, 8 of 128 experts of 768 x 2048: 130 -> 104 us a launch; a block of two layers 905 -> 754); the others have one tile per CTA (the
+    // loop's bookkeeping costs their dequantizing warps more than it saves: 77 rows on 14336 x 4096 39 us without, 47 with it).
     // Expert-indexed launch (Kernel::MatMulId, moe.cu): the activation tiles are runs of (token, slot)
     // pairs grouped by expert; the weights are the dense stack [experts * n, k], so a tile's weight
-    // rows start at expert * n. Tiles past the last used one have no expert.
-    uint32_t wrow0 = 0;
-    if (p.tile_expert) {
-        const int32_t e = p.tile_expert[blockIdx.y];
-        if (e < 0) return;  // before any barrier or tensor-memory allocation
-        wrow0 = (uint32_t)e * p.n;
-    }
-    // split-K: CTA z of gridDim.z takes the super-blocks [kb0, kb0 + nblk) of K and writes a partial tile
-    const uint32_t nblk_total = p.k / QK, per_split = (nblk_total + gridDim.z - 1) / gridDim.z;
-    const uint32_t kb0 = blockIdx.z * per_split;
-    const uint32_t nblk = min(per_split, nblk_total - kb0), ksteps = nblk * (QK / KS);
+    // rows start at expert * n; tiles past the last used one have no expert.
+    struct Tile {
+        uint32_t n0, m0, wrow0, kb0, nblk, z;
+    };
+    const uint32_t nx = p.tiles_x, ny = p.tiles_y, ntiles = nx * ny * p.splits;
+    const uint32_t nblk_total = p.k / QK, per_split = (nblk_total + p.splits - 1) / p.splits;
+    auto tile_at = [&](uint32_t t, Tile &o) -> bool {
+        const uint32_t c = t / nx, x = t - c * nx;
+        o.z = c / ny;
+        const uint32_t y = c - o.z * ny;
+        o.wrow0 = 0;
+        if (p.tile_expert) {
+            const int32_t e = p.tile_expert[y];
+            if (e < 0) return false;
+            o.wrow0 = (uint32_t)e * p.n;
+        }
+        o.n0 = x * (TN * NT), o.m0 = y * MT;
+        // split-K: this tile takes the super-blocks [kb0, kb0 + nblk) of K and writes partial sums
+        o.kb0 = o.z * per_split;
+        o.nblk = min(per_split, nblk_total - o.kb0);
+        return true;
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; s++) {
@@ -241,17 +281,20 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             mbar_init(raw_full + r, 1);
             mbar_init(raw_empty + r, DEQ_WARPS);
         }
-        mbar_init(acc_full, 1);
+        for (int a = 0; a < 2; a++) {
+            mbar_init(acc_full + a, 1);
+            mbar_init(acc_empty + a, DEQ_WARPS);
+        }
         if constexpr (PAIR)
             for (int s = 0; s < C::STAGES; s++) mbar_init(peer_ready + s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
         if constexpr (PAIR) {  // the same warp of both CTAs: a pair-wide allocation of the same columns
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"((uint32_t)(MT * NT)) : "memory");
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
         } else {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"((uint32_t)(MT * NT)) : "memory");
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
     }
@@ -265,17 +308,22 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (warp == 0) {
         // ---------------- TMA producer, activation tiles: one 128-byte-swizzled box per k-step
         if (lane == 0) {
-            for (uint32_t ks = 0; ks < ksteps && healthy; ks++) {
-                const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
-                if (!mbar_wait(empty + s, (u & 1) ^ 1, 64)) { healthy = false; break; }
-                mbar_expect_tx(full_a + s, C::A_BYTES);
-                if constexpr (PAIR) {  // this CTA's half of the activation tile
-                    tma_load_2d(stage0 + s * C::STAGE_BYTES + C::W_BYTES, &map_a, (int)(kb0 * QK + ks * KS), (int)(m0 + (MT / 2) * cta_rank), full_a + s);
-                } else {
+            uint32_t kc = 0;  // k-steps so far, over all tiles
+            Tile o;
+            for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
+                if (!tile_at(t, o)) continue;
+                for (uint32_t ks = 0; ks < o.nblk * (QK / KS) && healthy; ks++, kc++) {
+                    const uint32_t s = kc % C::STAGES, u = kc / C::STAGES;
+                    if (!mbar_wait(empty + s, (u & 1) ^ 1, 64)) { healthy = false; break; }
+                    mbar_expect_tx(full_a + s, C::A_BYTES);
+                    if constexpr (PAIR) {  // this CTA's half of the activation tile
+                        tma_load_2d(stage0 + s * C::STAGE_BYTES + C::W_BYTES, &map_a, (int)(o.kb0 * QK + ks * KS), (int)(o.m0 + (MT / 2) * cta_rank), full_a + s);
+                    } else {
 #pragma unroll
-                    for (int h = 0; h < (MT + 255) / 256; h++)  // a box holds at most 256 rows
-                        tma_load_2d(stage0 + s * C::STAGE_BYTES + C::W_BYTES + h * 256 * 128, &map_a, (int)(kb0 * QK + ks * KS), (int)(m0 + 256 * h),
-                                    full_a + s);
+                        for (int h = 0; h < (MT + 255) / 256; h++)  // a box holds at most 256 rows
+                            tma_load_2d(stage0 + s * C::STAGE_BYTES + C::W_BYTES + h * 256 * 128, &map_a, (int)(o.kb0 * QK + ks * KS), (int)(o.m0 + 256 * h),
+                                        full_a + s);
+                    }
                 }
             }
             if (!healthy && p.status) atomicOr(p.status, 2);
@@ -285,28 +333,33 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // multiple of 2048, e.g. the K/8 shard of a row-parallel projection): no tensor map can
         // describe them, so every lane copies rows of the tile with the plain bulk copy, each from
         // the 16-byte boundary below its block (the consumers compute the same per-row offset)
-        const uint32_t rows_valid = min((uint32_t)TN, p.n > n0 ? p.n - n0 : 0u);
         const uint64_t pitch = (uint64_t)nblk_total * Q6K_BYTES;
         const uint64_t end16 = ((uint64_t)(uintptr_t)p.w + (uint64_t)p.n * pitch + 15) & ~(uint64_t)15;  // never read past the matrix's last 16-byte line
-        auto copy_of = [&](uint32_t rr, uint32_t b, uint64_t &src) -> uint32_t {
-            src = ((uint64_t)(uintptr_t)p.w + (uint64_t)(n0 + rr) * pitch + (uint64_t)(kb0 + b) * Q6K_BYTES) & ~(uint64_t)15;
-            return (uint32_t)min((uint64_t)Q6K_BOX, end16 - src);
-        };
-        for (uint32_t b = 0; b < nblk && healthy; b++) {
-            const uint32_t r = b % C::RAWS, ur = b / C::RAWS;
-            if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
-            if (lane == 0 && rows_valid) {
-                uint64_t src;
-                mbar_expect_tx(raw_full + r, (rows_valid - 1) * Q6K_BOX + copy_of(rows_valid - 1, b, src));  // only the last row can be short
-            }
-            __syncwarp();
-            for (uint32_t rr = lane; rr < rows_valid; rr += 32) {
-                uint64_t src;
-                const uint32_t bytes = copy_of(rr, b, src);
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                 s32(raw0 + r * C::RAW + rr * Q6K_BOX)),
-                             "l"(src), "r"(bytes), "r"(s32(raw_full + r))
-                             : "memory");
+        uint32_t bc = 0;  // super-blocks so far, over all tiles
+        Tile o;
+        for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
+            if (!tile_at(t, o)) continue;
+            const uint32_t rows_valid = min((uint32_t)TN, p.n > o.n0 ? p.n - o.n0 : 0u);
+            auto copy_of = [&](uint32_t rr, uint32_t b, uint64_t &src) -> uint32_t {
+                src = ((uint64_t)(uintptr_t)p.w + (uint64_t)(o.n0 + rr) * pitch + (uint64_t)(o.kb0 + b) * Q6K_BYTES) & ~(uint64_t)15;
+                return (uint32_t)min((uint64_t)Q6K_BOX, end16 - src);
+            };
+            for (uint32_t b = 0; b < o.nblk && healthy; b++, bc++) {
+                const uint32_t r = bc % C::RAWS, ur = bc / C::RAWS;
+                if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
+                if (lane == 0 && rows_valid) {
+                    uint64_t src;
+                    mbar_expect_tx(raw_full + r, (rows_valid - 1) * Q6K_BOX + copy_of(rows_valid - 1, b, src));  // only the last row can be short
+                }
+                __syncwarp();
+                for (uint32_t rr = lane; rr < rows_valid; rr += 32) {
+                    uint64_t src;
+                    const uint32_t bytes = copy_of(rr, b, src);
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     s32(raw0 + r * C::RAW + rr * Q6K_BOX)),
+                                 "l"(src), "r"(bytes), "r"(s32(raw_full + r))
+                                 : "memory");
+                }
             }
         }
         if (!healthy && lane == 0 && p.status) atomicOr(p.status, 32);
@@ -314,15 +367,20 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // ---------------- TMA producer, packed weights: one super-block of every row of the tile
         // per copy, a whole super-block (four k-steps) ahead of the dequantizing warps
         if (lane == 0) {
-            for (uint32_t b = 0; b < nblk && healthy; b++) {
-                const uint32_t r = b % C::RAWS, ur = b / C::RAWS;
-                if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
-                mbar_expect_tx(raw_full + r, C::RAW);
+            uint32_t bc = 0;
+            Tile o;
+            for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
+                if (!tile_at(t, o)) continue;
+                for (uint32_t b = 0; b < o.nblk && healthy; b++, bc++) {
+                    const uint32_t r = bc % C::RAWS, ur = bc / C::RAWS;
+                    if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
+                    mbar_expect_tx(raw_full + r, C::RAW);
 #pragma unroll
-                for (int t = 0; t < NT; t++)
-                    tma_load_2d(raw0 + r * C::RAW + t * RAW_BYTES, &map_w,
-                                FMT == FMT_Q6K ? (int)(((kb0 + b) * Q6K_BYTES) & ~15u) : (int)((kb0 + b) * C::ROW_BYTES), (int)(wrow0 + n0 + t * TN),
-                                raw_full + r);
+                    for (int q = 0; q < NT; q++)
+                        tma_load_2d(raw0 + r * C::RAW + q * RAW_BYTES, &map_w,
+                                    FMT == FMT_Q6K ? (int)(((o.kb0 + b) * Q6K_BYTES) & ~15u) : (int)((o.kb0 + b) * C::ROW_BYTES), (int)(o.wrow0 + o.n0 + q * TN),
+                                    raw_full + r);
+                }
             }
             if (!healthy && p.status) atomicOr(p.status, 32);
         }
@@ -330,8 +388,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // ---------------- MMA issuer of a CTA pair. The leader (rank 0) issues for both CTAs: M = 256
         // (128 weight rows from each CTA's tile), N = MT (each CTA holds MT / 2 activation rows), the
         // accumulators land in each CTA's own tensor memory. The other CTA's issuer warp only reports
-        // when its operands of a stage are in place. Completion is committed to both CTAs' barriers.
-        if (lane == 0) {
+        // when its operands of a stage are in place. Completion is committed to both CTAs' barriers. (One tile per CTA.)
+        Tile o;
+        if (lane == 0 && tile_at(blockIdx.x, o)) {
+            const uint32_t ksteps = o.nblk * (QK / KS);
             const uint32_t peer = cta_rank ^ 1;
             if (cta_rank == 0) {
                 constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT >> 3) << 17) | ((uint32_t)((2 * TN) >> 4) << 24);
@@ -369,22 +429,31 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             // D f32, A and B bf16, both K-major, M = 128, N = MT
             constexpr int MMA_N = MT > 256 ? 256 : MT;  // an instruction takes at most 256 columns: MT = 512 issues two
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MMA_N >> 3) << 17) | ((uint32_t)(TN >> 4) << 24);
-            for (uint32_t ks = 0; ks < ksteps && healthy; ks++) {
-                const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
-                if (!mbar_wait(full_a + s, u & 1, 32) || !mbar_wait(full_b + s, u & 1, 32)) { healthy = false; break; }
+            uint32_t kc = 0, ti = 0;  // k-steps and tiles so far
+            Tile o;
+            for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
+                if (!tile_at(t, o)) continue;
+                const uint32_t acc = ti % C::ACCS, ua = ti / C::ACCS, tmem_d = tmem_base + acc * (MT * NT);
+                ti++;
+                if (LOOP && !mbar_wait(acc_empty + acc, (ua & 1) ^ 1, 32)) { healthy = false; break; }  // its last results have been read
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t wt = s32(stage0 + s * C::STAGE_BYTES), at = wt + C::W_BYTES;
+                for (uint32_t ks = 0; ks < o.nblk * (QK / KS) && healthy; ks++, kc++) {
+                    const uint32_t s = kc % C::STAGES, u = kc / C::STAGES;
+                    if (!mbar_wait(full_a + s, u & 1, 32) || !mbar_wait(full_b + s, u & 1, 32)) { healthy = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t wt = s32(stage0 + s * C::STAGE_BYTES), at = wt + C::W_BYTES;
 #pragma unroll
-                for (int t = 0; t < NT; t++)
+                    for (int q = 0; q < NT; q++)
 #pragma unroll
-                    for (int kk = 0; kk < KS / 16; kk++)
+                        for (int kk = 0; kk < KS / 16; kk++)
 #pragma unroll
-                        for (int h = 0; h < MT / MMA_N; h++)
-                            mma_bf16(tmem_base + t * MT + h * MMA_N, smem_desc(wt + t * B_BYTES + kk * 32),
-                                     smem_desc(at + h * MMA_N * 128 + kk * 32), idesc, (ks | kk) ? 1u : 0u);
-                mma_commit(empty + s);  // the stage may be refilled once these MMAs have read it
+                            for (int h = 0; h < MT / MMA_N; h++)
+                                mma_bf16(tmem_d + q * MT + h * MMA_N, smem_desc(wt + q * B_BYTES + kk * 32),
+                                         smem_desc(at + h * MMA_N * 128 + kk * 32), idesc, (ks | kk) ? 1u : 0u);
+                    mma_commit(empty + s);  // the stage may be refilled once these MMAs have read it
+                }
+                mma_commit(acc_full + acc);
             }
-            mma_commit(acc_full);
             if (!healthy && p.status) atomicOr(p.status, 4);
         }
     } else {
@@ -396,9 +465,83 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const int row = 32 * (dw & 3) + lane, half = dw >> 2;
         const int sub = NT == 2 ? grp : 0;        // weight sub-tile of this thread
         float d1[4], m1[4];                       // sub-block scales of this thread's pairs of the current super-block
-        for (uint32_t ks = (NT == 2 ? 0 : grp); ks < ksteps && healthy; ks += (NT == 2 ? 1 : 2)) {
-            const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
-            const uint32_t b = ks >> 2, pp = ks & 3, r = b % C::RAWS, ur = b / C::RAWS;
+        uint32_t kc0 = 0, bc0 = 0, ti = 0;        // k-steps, super-blocks and tiles before the current tile
+        Tile o, done;                             // the current tile; the one whose results are to be stored
+
+        // ---------------- epilogue: TMEM lane = weight row, column = activation row
+        auto store_tile = [&](const Tile &o, uint32_t index) {
+            const uint32_t acc = index % C::ACCS;
+            if (!mbar_wait(acc_full + acc, (index / C::ACCS) & 1)) {
+                if (lane == 0 && p.status) atomicOr(p.status, 16);
+                healthy = false;
+                return;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int quarter = warp & 3;  // the TMEM lanes this warp may read
+            const uint32_t n = o.n0 + sub * TN + 32 * quarter + lane;
+            constexpr int COLS = NT == 2 ? MT / 2 : MT / 4, CH = COLS < 32 ? COLS : 32;  // the columns of this warp: a half (NT = 1: a quarter) of them
+            const int cbase = (NT == 2 ? half : (warp - 2) >> 2) * COLS;
+#pragma unroll 1
+            for (int c0 = 0; c0 < COLS; c0 += CH) {
+                uint32_t r[CH];
+                tmem_ld<CH>(r, tmem_base + acc * (MT * NT) + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(sub * MT + cbase + c0));
+                if (LOOP && c0 + CH == COLS) {  // this warp's last read of the accumulators: they may be overwritten
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_empty + acc);
+                }
+                if (p.row_pair) {  // expert-indexed: tile-space row -> (token, slot) pair = output row; padding rows have none
+                    const uint32_t mfirst = o.m0 + cbase + c0;
+                    if (n < p.n) {
+#pragma unroll
+                        for (int j = 0; j < CH; j++) {
+                            const int32_t pair = p.row_pair[mfirst + j];
+                            if (pair >= 0) p.out[p.out_off + (uint64_t)pair * p.n + n] = __uint_as_float(r[j]);
+                        }
+                    }
+                } else if (n < p.n && p.partial) {  // split-K: this CTA's partial sums, [split][row][n]; summed by a second kernel
+                    const uint32_t mfirst = o.m0 + cbase + c0;
+                    float *prow = p.partial + ((size_t)o.z * p.rows + mfirst) * p.n + n;
+#pragma unroll
+                    for (int j = 0; j < CH; j++)
+                        if (mfirst + j < p.rows) prow[(size_t)j * p.n] = __uint_as_float(r[j]);
+                } else if (n < p.n) {
+                    // (batch, row) of the chunk's first activation row by one division, then by stepping
+                    const uint32_t mfirst = o.m0 + cbase + c0;
+                    uint32_t bt = mfirst / p.m, i = mfirst % p.m;
+                    float *orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + n;
+                    const float *erow = p.extra ? p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)n * p.ex_s2 : nullptr;
+                    if (!erow && i + CH <= p.m && mfirst + CH <= p.rows) {  // the common case: 32 whole rows of one batch entry, no epilogue term
+#pragma unroll
+                        for (int j = 0; j < CH; j++) orow[(uint64_t)j * p.out_rs] = __uint_as_float(r[j]);
+                        continue;
+                    }
+#pragma unroll
+                    for (int j = 0; j < CH; j++) {
+                        if (mfirst + j < p.rows) {
+                            float v = __uint_as_float(r[j]);
+                            if (erow) v += *erow;
+                            *orow = v;
+                        }
+                        if (++i == p.m) {  // next batch entry
+                            i = 0;
+                            bt++;
+                            orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + n;
+                            if (erow) erow = p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)n * p.ex_s2;
+                        } else {
+                            orow += p.out_rs;
+                            if (erow) erow += p.ex_s1;
+                        }
+                    }
+                }
+            }
+        };
+        for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
+          if (!tile_at(t, o)) continue;
+          const uint32_t ksteps = o.nblk * (QK / KS), first = NT == 2 ? 0 : grp;
+          for (uint32_t ks = first; ks < ksteps && healthy; ks += (NT == 2 ? 1 : 2)) {
+            const uint32_t s = (kc0 + ks) % C::STAGES, u = (kc0 + ks) / C::STAGES;
+            const uint32_t b = ks >> 2, pp = ks & 3, r = (bc0 + b) % C::RAWS, ur = (bc0 + b) / C::RAWS;
             if constexpr (FMT == FMT_Q6K) {
                 // Q6_K (NT = 1): a super-block is ql[128] | qh[64] | int8 sc[16] | f16 d = 210 bytes, so it
                 // starts on a 2-byte boundary only; the copy starts at the 16-byte boundary below it and
@@ -412,14 +555,14 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (pp < 2 && !mbar_wait(raw_full + r, ur & 1)) { healthy = false; break; }
                 if (!mbar_wait(empty + s, (u & 1) ^ 1)) { healthy = false; break; }
                 const uint32_t j = lane & 15, h = j >> 3, jj = j & 7, nh = pp >> 1, hi = pp & 1;
-                const uint64_t pitch = (uint64_t)nblk_total * Q6K_BYTES, wbase = (uint64_t)(uintptr_t)p.w + (uint64_t)(kb0 + b) * Q6K_BYTES;
+                const uint64_t pitch = (uint64_t)nblk_total * Q6K_BYTES, wbase = (uint64_t)(uintptr_t)p.w + (uint64_t)(o.kb0 + b) * Q6K_BYTES;
                 const uint64_t unbias32 = pack2(-8388640.0f, -8388640.0f);  // -(2^23 + 32)
 #pragma unroll 2
                 for (int pass = 0; pass < 8; pass++) {
                     const int rw = 16 * dw + 2 * pass + (lane >> 4);
                     // where the block starts inside its 224 staged bytes: the distance of its address from
                     // the 16-byte boundary below it (the same for every row when the row pitch is a multiple of 16)
-                    const uint32_t skew = (uint32_t)((wbase + (uint64_t)(n0 + rw) * pitch) & 15u);
+                    const uint32_t skew = (uint32_t)((wbase + (uint64_t)(o.n0 + rw) * pitch) & 15u);
                     const uint8_t *blk = raw0 + r * C::RAW + rw * Q6K_BOX + skew;
                     const uint16_t *ql = (const uint16_t *)(blk + 64 * nh + 32 * h + 4 * jj);
                     const uint16_t *qh = (const uint16_t *)(blk + 128 + 32 * nh + 4 * jj);
@@ -442,146 +585,82 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> tensor-core reads
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full_b + s);
-                continue;
-            }
-            const uint8_t *blk = raw0 + r * C::RAW + sub * RAW_BYTES + row * C::ROW_BYTES;
-            if (NT == 2 ? pp == 0 : pp < 2) {  // first k-step of this thread in the block
-                if (!mbar_wait(raw_full + r, ur & 1)) { healthy = false; break; }
-                const uint4 h = *(const uint4 *)blk;
-                const float d = half_bits_to_float(h.x & 0xffff), dmin = half_bits_to_float(h.x >> 16);
-                const float nd = d * -8388608.0f, ndmin = dmin * -8388608.0f;
-                const uint32_t w0 = h.y, w1 = h.z, w2 = h.w;
-                const uint32_t sc_lo = w0 & 0x3F3F3F3Fu, mn_lo = w1 & 0x3F3F3F3Fu;
-                const uint32_t sc_hi = (w2 & 0x0F0F0F0Fu) | (((w0 >> 6) & 0x03030303u) << 4);
-                const uint32_t mn_hi = ((w2 >> 4) & 0x0F0F0F0Fu) | (((w1 >> 6) & 0x03030303u) << 4);
-                // pair q: sub-block 2q + half = byte 2*(q&1) + half of the lo (q < 2) / hi words
+            } else {
+                const uint8_t *blk = raw0 + r * C::RAW + sub * RAW_BYTES + row * C::ROW_BYTES;
+                if (NT == 2 ? pp == 0 : pp < 2) {  // first k-step of this thread in the block
+                    if (!mbar_wait(raw_full + r, ur & 1)) { healthy = false; break; }
+                    const uint4 h = *(const uint4 *)blk;
+                    const float d = half_bits_to_float(h.x & 0xffff), dmin = half_bits_to_float(h.x >> 16);
+                    const float nd = d * -8388608.0f, ndmin = dmin * -8388608.0f;
+                    const uint32_t w0 = h.y, w1 = h.z, w2 = h.w;
+                    const uint32_t sc_lo = w0 & 0x3F3F3F3Fu, mn_lo = w1 & 0x3F3F3F3Fu;
+                    const uint32_t sc_hi = (w2 & 0x0F0F0F0Fu) | (((w0 >> 6) & 0x03030303u) << 4);
+                    const uint32_t mn_hi = ((w2 >> 4) & 0x0F0F0F0Fu) | (((w1 >> 6) & 0x03030303u) << 4);
+                    // pair q: sub-block 2q + half = byte 2*(q&1) + half of the lo (q < 2) / hi words
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const uint32_t sel = 0x7440u + 2 * (q & 1) + half;
-                    d1[q] = fmaf(d, biased(q < 2 ? sc_lo : sc_hi, sel), nd);        // d * sc, exact (see qgemv_q4k.cu)
-                    m1[q] = fmaf(dmin, biased(q < 2 ? mn_lo : mn_hi, sel), ndmin);  // dmin * m, exact
+                    for (int q = 0; q < 4; q++) {
+                        const uint32_t sel = 0x7440u + 2 * (q & 1) + half;
+                        d1[q] = fmaf(d, biased(q < 2 ? sc_lo : sc_hi, sel), nd);        // d * sc, exact (see qgemv_q4k.cu)
+                        m1[q] = fmaf(dmin, biased(q < 2 ? mn_lo : mn_hi, sel), ndmin);  // dmin * m, exact
+                    }
                 }
-            }
-            // Q5_K: Q4_K's block with the fifth bits qh[32] between the header and the nibbles; bit s of qh[l]
-            // belongs to element 32 s + l (crates/lapid-quant/src/kquant.rs:355-373)
-            constexpr int QS = FMT == FMT_Q5K ? 48 : 16;
-            const uint4 qa = *(const uint4 *)(blk + QS + 32 * pp), qb = *(const uint4 *)(blk + QS + 16 + 32 * pp);
-            uint4 ha = make_uint4(0, 0, 0, 0), hb = ha;
-            if constexpr (FMT == FMT_Q5K) {
-                ha = *(const uint4 *)(blk + 16);
-                hb = *(const uint4 *)(blk + 32);
-            }
-            if (NT == 2 ? pp == 3 : pp >= 2) {  // this thread's last read of the block's packed bytes
+                // Q5_K: Q4_K's block with the fifth bits qh[32] between the header and the nibbles; bit s of qh[l]
+                // belongs to element 32 s + l (crates/lapid-quant/src/kquant.rs:355-373)
+                constexpr int QS = FMT == FMT_Q5K ? 48 : 16;
+                const uint4 qa = *(const uint4 *)(blk + QS + 32 * pp), qb = *(const uint4 *)(blk + QS + 16 + 32 * pp);
+                uint4 ha = make_uint4(0, 0, 0, 0), hb = ha;
+                if constexpr (FMT == FMT_Q5K) {
+                    ha = *(const uint4 *)(blk + 16);
+                    hb = *(const uint4 *)(blk + 32);
+                }
+                if (NT == 2 ? pp == 3 : pp >= 2) {  // this thread's last read of the block's packed bytes
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(raw_empty + r);
+                }
+                const float sd = pp == 0 ? d1[0] : pp == 1 ? d1[1] : pp == 2 ? d1[2] : d1[3];
+                const float nm = -(pp == 0 ? m1[0] : pp == 1 ? m1[1] : pp == 2 ? m1[2] : m1[3]);
+                const uint64_t sd2 = pack2(sd, sd), nm2 = pack2(nm, nm), unbias = pack2(-8388608.0f, -8388608.0f);
+                uint32_t v[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+                if (half) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) v[i] >>= 4;
+                }
+                if constexpr (FMT == FMT_Q5K) {
+                    const uint32_t hq[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+#pragma unroll
+                    for (int i = 0; i < 8; i++) v[i] = (v[i] & 0x0F0F0F0Fu) | (((hq[i] >> (2 * pp + half)) & 0x01010101u) << 4);
+                }
+                if (!mbar_wait(empty + s, (u & 1) ^ 1)) { healthy = false; break; }
+                uint8_t *dst = stage0 + s * C::STAGE_BYTES + sub * B_BYTES + row * 128;
+#pragma unroll
+                for (int c = 0; c < 4; c++) {  // 16-byte chunk = 8 consecutive k = two packed words
+                    uint32_t o[4];
+#pragma unroll
+                    for (int w = 0; w < 2; w++) {
+                        const uint32_t t = v[2 * c + w] & (FMT == FMT_Q5K ? 0x1F1F1F1Fu : 0x0F0F0F0Fu);
+                        // y = sd * q - m1 with one rounding, two elements per instruction
+                        const uint64_t q01 = add2(pack2(biased(t, 0x7440u), biased(t, 0x7441u)), unbias);
+                        const uint64_t q23 = add2(pack2(biased(t, 0x7442u), biased(t, 0x7443u)), unbias);
+                        o[2 * w] = to_bf16x2(fma2(sd2, q01, nm2));
+                        o[2 * w + 1] = to_bf16x2(fma2(sd2, q23, nm2));
+                    }
+                    const int chunk = (4 * half + c) ^ (row & 7);
+                    *(uint4 *)(dst + 16 * chunk) = make_uint4(o[0], o[1], o[2], o[3]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> tensor-core reads
                 __syncwarp();
-                if (lane == 0) mbar_arrive(raw_empty + r);
+                if (lane == 0) mbar_arrive(full_b + s);
             }
-            const float sd = pp == 0 ? d1[0] : pp == 1 ? d1[1] : pp == 2 ? d1[2] : d1[3];
-            const float nm = -(pp == 0 ? m1[0] : pp == 1 ? m1[1] : pp == 2 ? m1[2] : m1[3]);
-            const uint64_t sd2 = pack2(sd, sd), nm2 = pack2(nm, nm), unbias = pack2(-8388608.0f, -8388608.0f);
-            uint32_t v[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-            if (half) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] >>= 4;
-            }
-            if constexpr (FMT == FMT_Q5K) {
-                const uint32_t hq[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = (v[i] & 0x0F0F0F0Fu) | (((hq[i] >> (2 * pp + half)) & 0x01010101u) << 4);
-            }
-            if (!mbar_wait(empty + s, (u & 1) ^ 1)) { healthy = false; break; }
-            uint8_t *dst = stage0 + s * C::STAGE_BYTES + sub * B_BYTES + row * 128;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {  // 16-byte chunk = 8 consecutive k = two packed words
-                uint32_t o[4];
-#pragma unroll
-                for (int w = 0; w < 2; w++) {
-                    const uint32_t t = v[2 * c + w] & (FMT == FMT_Q5K ? 0x1F1F1F1Fu : 0x0F0F0F0Fu);
-                    // y = sd * q - m1 with one rounding, two elements per instruction
-                    const uint64_t q01 = add2(pack2(biased(t, 0x7440u), biased(t, 0x7441u)), unbias);
-                    const uint64_t q23 = add2(pack2(biased(t, 0x7442u), biased(t, 0x7443u)), unbias);
-                    o[2 * w] = to_bf16x2(fma2(sd2, q01, nm2));
-                    o[2 * w + 1] = to_bf16x2(fma2(sd2, q23, nm2));
-                }
-                const int chunk = (4 * half + c) ^ (row & 7);
-                *(uint4 *)(dst + 16 * chunk) = make_uint4(o[0], o[1], o[2], o[3]);
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> tensor-core reads
-            __syncwarp();
-            if (lane == 0) mbar_arrive(full_b + s);
+            // the results of the tile before, behind the first weights of this one: the tensor cores have work meanwhile
+            if (LOOP && ks == first && ti > 0) store_tile(done, ti - 1);
+          }
+          kc0 += ksteps;
+          bc0 += o.nblk;
+          ti++;
+          done = o;
         }
         if (!healthy && lane == 0 && p.status) atomicOr(p.status, 8);
-
-        // ---------------- epilogue: TMEM lane = weight row, column = activation row
-        if (NT == 1 && grp != 0) {
-            // with one accumulator the second group has no epilogue share
-        } else if (healthy && mbar_wait(acc_full, 0)) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int quarter = warp & 3;  // the TMEM lanes this warp may read
-            const uint32_t n = n0 + sub * TN + 32 * quarter + lane;
-            constexpr int COLS = MT / 2;   // each half of the epilogue warps takes half of the columns
-            const int cbase = half * COLS;
-#pragma unroll 1
-            for (int c0 = 0; c0 < COLS; c0 += 32) {
-                uint32_t r[32];
-                const uint32_t taddr = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(sub * MT + cbase + c0);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-                      "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-                      "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (p.row_pair) {  // expert-indexed: tile-space row -> (token, slot) pair = output row; padding rows have none
-                    const uint32_t mfirst = m0 + cbase + c0;
-                    if (n < p.n) {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            const int32_t pair = p.row_pair[mfirst + j];
-                            if (pair >= 0) p.out[p.out_off + (uint64_t)pair * p.n + n] = __uint_as_float(r[j]);
-                        }
-                    }
-                } else if (n < p.n && p.partial) {  // split-K: this CTA's partial sums, [split][row][n]; summed by a second kernel
-                    const uint32_t mfirst = m0 + cbase + c0;
-                    float *prow = p.partial + ((size_t)blockIdx.z * p.rows + mfirst) * p.n + n;
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (mfirst + j < p.rows) prow[(size_t)j * p.n] = __uint_as_float(r[j]);
-                } else if (n < p.n) {
-                    // (batch, row) of the chunk's first activation row by one division, then by stepping
-                    const uint32_t mfirst = m0 + cbase + c0;
-                    uint32_t bt = mfirst / p.m, i = mfirst % p.m;
-                    float *orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + n;
-                    const float *erow = p.extra ? p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)n * p.ex_s2 : nullptr;
-                    if (!erow && i + 32 <= p.m && mfirst + 32 <= p.rows) {  // the common case: 32 whole rows of one batch entry, no epilogue term
-#pragma unroll
-                        for (int j = 0; j < 32; j++) orow[(uint64_t)j * p.out_rs] = __uint_as_float(r[j]);
-                        continue;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        if (mfirst + j < p.rows) {
-                            float v = __uint_as_float(r[j]);
-                            if (erow) v += *erow;
-                            *orow = v;
-                        }
-                        if (++i == p.m) {  // next batch entry
-                            i = 0;
-                            bt++;
-                            orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + n;
-                            if (erow) erow = p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)n * p.ex_s2;
-                        } else {
-                            orow += p.out_rs;
-                            if (erow) erow += p.ex_s1;
-                        }
-                    }
-                }
-            }
-        } else if (lane == 0 && p.status) {
-            atomicOr(p.status, 16);
-        }
+        if (healthy && ti > 0) store_tile(done, ti - 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -589,9 +668,9 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if constexpr (PAIR)
-            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(MT * NT)) : "memory");
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
         else
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(MT * NT)) : "memory");
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
     }
 }
 
@@ -649,14 +728,20 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-template <int FMT, int MT, int NT, bool PAIR = false>
-static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma, cudaStream_t stream, uint32_t splits = 1) {
-    auto kern = qgemm_tc_kernel<FMT, MT, NT, PAIR>;
-    using C = Cfg<FMT, MT, NT, PAIR>;
+template <int FMT, int MT, int NT, bool PAIR = false, bool LOOP = false>
+static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma, int sm_count, cudaStream_t stream, uint32_t splits = 1) {
+    auto kern = qgemm_tc_kernel<FMT, MT, NT, PAIR, LOOP>;
+    using C = Cfg<FMT, MT, NT, PAIR, LOOP>;
     static DynamicSmemOptIn opted;
     if (cudaError_t e = opted.raise((const void *)kern, C::SMEM); e != cudaSuccess) return e;
-    dim3 grid((a.n + TN * NT - 1) / (TN * NT), (a.rows + MT - 1) / MT, splits);
-    if (PAIR) grid.x = (grid.x + 1) & ~1u;  // whole pairs: a CTA past the last weight row works on zero fill and stores nothing
+    GemmTcArgs b = a;
+    b.tiles_x = (a.n + TN * NT - 1) / (TN * NT);
+    if (PAIR) b.tiles_x = (b.tiles_x + 1) & ~1u;  // whole pairs: a CTA past the last weight row works on zero fill and stores nothing
+    b.tiles_y = (a.rows + MT - 1) / MT;
+    b.splits = splits;
+    const uint64_t tiles = (uint64_t)b.tiles_x * b.tiles_y * splits;
+    if (tiles >= (1u << 31)) return cudaErrorInvalidValue;
+    const dim3 grid((unsigned)(!LOOP || tiles < (uint64_t)sm_count ? tiles : (uint64_t)sm_count));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(THREADS);
@@ -670,7 +755,7 @@ static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const C
         attr[cfg.numAttrs].val.clusterDim.y = 1;
         attr[cfg.numAttrs++].val.clusterDim.z = 1;
     }
-    return cudaLaunchKernelEx(&cfg, kern, mw, ma, a);
+    return cudaLaunchKernelEx(&cfg, kern, mw, ma, b);
 }
 
 }  // namespace tc
@@ -690,12 +775,12 @@ bool qgemm_tc_supported(int fmt, const GemmTcArgs &a) {
 static uint32_t tc_block_bytes(int fmt) { return fmt == FMT_Q4K ? Q4K_BYTES : fmt == FMT_Q5K ? Q5K_BYTES : Q6K_BYTES; }
 static uint32_t tc_box_bytes(int fmt) { return fmt == FMT_Q6K ? (uint32_t)tc::Q6K_BOX : tc_block_bytes(fmt); }
 // the one-accumulator tile of a format by activation rows per CTA
-template <int FMT> static cudaError_t launch_one_acc(uint32_t mt, const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma,
-                                                     cudaStream_t stream, uint32_t ways = 1) {
+template <int FMT, bool LOOP = false> static cudaError_t launch_one_acc(uint32_t mt, const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma,
+                                                     int sm_count, cudaStream_t stream, uint32_t ways = 1) {
     using namespace tc;
-    return mt == 64 ? launch_mt<FMT, 64, 1>(a, mw, ma, stream, ways)
-                    : mt == 128 ? launch_mt<FMT, 128, 1>(a, mw, ma, stream, ways)
-                                : mt == 256 ? launch_mt<FMT, 256, 1>(a, mw, ma, stream, ways) : cudaErrorInvalidValue;
+    return mt == 64 ? launch_mt<FMT, 64, 1, false, LOOP>(a, mw, ma, sm_count, stream, ways)
+                    : mt == 128 ? launch_mt<FMT, 128, 1, false, LOOP>(a, mw, ma, sm_count, stream, ways)
+                                : mt == 256 ? launch_mt<FMT, 256, 1, false, LOOP>(a, mw, ma, sm_count, stream, ways) : cudaErrorInvalidValue;
 }
 
 // How many ways K is split: only when the tiles would leave more than half of the SMs idle, never
@@ -733,7 +818,7 @@ bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, c
     return pitch % 16 == 0 && (n * pitch) % 256 == 0 && experts * n < (1ull << 31);
 }
 
-cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, cudaStream_t stream) {
+cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, int sm_count, cudaStream_t stream) {
     using namespace tc;
     if (a.rows == 0 || a.n == 0) return cudaSuccess;
     EncodeTiledFn enc = encode_fn();
@@ -758,9 +843,9 @@ cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, 
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    if (fmt == FMT_Q6K) return launch_one_acc<FMT_Q6K>(mt, a, mw, ma, stream);
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, stream);
-    return launch_one_acc<FMT_Q4K>(mt, a, mw, ma, stream);
+    if (fmt == FMT_Q6K) return launch_one_acc<FMT_Q6K, true>(mt, a, mw, ma, sm_count, stream);
+    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K, true>(mt, a, mw, ma, sm_count, stream);
+    return launch_one_acc<FMT_Q4K, true>(mt, a, mw, ma, sm_count, stream);
 }
 
 cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, bool copy, void *partial, int sm_count,
@@ -814,8 +899,8 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         GemmTcArgs b = a;
         b.partial = (float *)partial;
         cudaError_t e;
-        e = fmt == FMT_Q6K ? launch_one_acc<FMT_Q6K>(mt, b, mw, ma, stream, ways)
-                           : fmt == FMT_Q5K ? launch_one_acc<FMT_Q5K>(mt, b, mw, ma, stream, ways) : launch_one_acc<FMT_Q4K>(mt, b, mw, ma, stream, ways);
+        e = fmt == FMT_Q6K ? launch_one_acc<FMT_Q6K>(mt, b, mw, ma, sm_count, stream, ways)
+                           : fmt == FMT_Q5K ? launch_one_acc<FMT_Q5K>(mt, b, mw, ma, sm_count, stream, ways) : launch_one_acc<FMT_Q4K>(mt, b, mw, ma, sm_count, stream, ways);
         if (e != cudaSuccess) return e;
         const uint64_t total = (uint64_t)a.rows * a.n;
         const unsigned sgrid = (unsigned)((total + 255) / 256 > (uint64_t)sm_count * 8 ? (uint64_t)sm_count * 8 : (total + 255) / 256);
@@ -831,7 +916,7 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
     // CTA measured 1.6x the time of a 256-row one, so it pays when it saves more than that in waves
     // of tiles over the SMs. Q6_K only: for Q4_K the two-accumulator 256x256 tile is the better way
     // to the same reuse (it also halves the activation traffic), measured faster in every case.
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, stream);  // (one accumulator tile: no wide or tall variants built)
+    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, sm_count, stream);  // (one accumulator tile: no wide or tall variants built)
     bool tall = false;
     if (a.rows > 256 && fmt == FMT_Q6K) {
         const uint64_t nt = (a.n + TN - 1) / TN;
@@ -840,12 +925,12 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         tall = w512 * 16 < w256 * 10;
     }
     if (g_tc_tall >= 0) tall = g_tc_tall != 0 && a.rows > 256;
-    if (tall) return fmt == FMT_Q6K ? launch_mt<FMT_Q6K, 512, 1>(a, mw, ma, stream) : launch_mt<FMT_Q4K, 512, 1>(a, mw, ma, stream);
+    if (tall) return fmt == FMT_Q6K ? launch_mt<FMT_Q6K, 512, 1>(a, mw, ma, sm_count, stream) : launch_mt<FMT_Q4K, 512, 1>(a, mw, ma, sm_count, stream);
     if (fmt == FMT_Q6K) {  // the larger staged blocks leave room for one accumulator tile only
         switch (mt) {
-            case 64: return launch_mt<FMT_Q6K, 64, 1>(a, mw, ma, stream);
-            case 128: return launch_mt<FMT_Q6K, 128, 1>(a, mw, ma, stream);
-            default: return launch_mt<FMT_Q6K, 256, 1>(a, mw, ma, stream);
+            case 64: return launch_mt<FMT_Q6K, 64, 1>(a, mw, ma, sm_count, stream);
+            case 128: return launch_mt<FMT_Q6K, 128, 1>(a, mw, ma, sm_count, stream);
+            default: return launch_mt<FMT_Q6K, 256, 1>(a, mw, ma, sm_count, stream);
         }
     }
     bool wide = a.rows > 128 && a.n >= 2 * TN;
@@ -856,11 +941,11 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
         wide = w2 * 26 <= w1 * 15;
     }
     if (g_tc_wide >= 0) wide = g_tc_wide != 0;
-    if (pair) return launch_mt<FMT_Q4K, 256, 2, true>(a, mw, ma, stream);
+    if (pair) return launch_mt<FMT_Q4K, 256, 2, true>(a, mw, ma, sm_count, stream);
     switch (mt) {
-        case 64: return launch_mt<FMT_Q4K, 64, 1>(a, mw, ma, stream);
-        case 128: return launch_mt<FMT_Q4K, 128, 1>(a, mw, ma, stream);
-        default: return wide ? launch_mt<FMT_Q4K, 256, 2>(a, mw, ma, stream) : launch_mt<FMT_Q4K, 256, 1>(a, mw, ma, stream);
+        case 64: return launch_mt<FMT_Q4K, 64, 1>(a, mw, ma, sm_count, stream);
+        case 128: return launch_mt<FMT_Q4K, 128, 1>(a, mw, ma, sm_count, stream);
+        default: return wide ? launch_mt<FMT_Q4K, 256, 2>(a, mw, ma, sm_count, stream) : launch_mt<FMT_Q4K, 256, 1>(a, mw, ma, sm_count, stream);
     }
 }
 

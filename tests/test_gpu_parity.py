@@ -1560,3 +1560,41 @@ def test_gemv_planes_tensor_core_ragged_k(be, oracle, fmt, ofmt):
         for i, n in enumerate(ns):
             want, _ = oracle.matmul(ofmt, x, qbs[i], n, k, m=m)
             assert max_rel(bufs[4 + i].download().view(np.float32), want) <= 2e-5, (m, k, n)
+
+
+@pytest.mark.parametrize("fmt", [lp.DType.Q4K, lp.DType.Q5K, lp.DType.Q6K])
+@pytest.mark.parametrize("m,n,k", [(20, 19333, 512), (100, 19200, 768), (200, 19201, 256), (300, 38500, 256), (600, 19333, 512)])
+def test_gemm_tensor_core_more_tiles_than_sms(be, fmt, m, n, k):
+    """CTAs that take several tiles: both accumulator sets and their reuse, rings that run on from tile to tile, ragged last tiles; every
+    tile height. Bar: the rounding of both operands to bf16, as in test_gemm_tensor_core; the reference is the exact f32 kernel."""
+    w = np.tile(O.normal(3300, 1024 * k, 0.02), (n + 1023) // 1024)[: n * k]
+    w = (w.reshape(n, k) * (1 + 0.001 * (np.arange(n, dtype=np.float32) % 997))[:, None]).astype(np.float32)   # no two row tiles alike
+    qb = quant.quantize(be, fmt, w, n, k)
+    a = O.normal(3301, m * k)
+    got = run_matmul(be, fmt, a, qb, m, n, k)
+    be.set_option("gemm", "f32")
+    want = run_matmul(be, fmt, a, qb, m, n, k)
+    be.set_option("gemm", "tc")
+    assert rel_l2(got, want) <= 4e-3 and max_rel(got, want) <= 3e-2
+
+
+@pytest.mark.parametrize("fmt", [lp.DType.Q4K, lp.DType.Q6K])
+def test_matmul_id_tensor_core_more_tiles_than_sms(be, fmt):
+    """The same for expert-indexed launches, with experts that get no token (tiles to skip) and experts with more than one tile."""
+    from lapid_b200.backend import matmul_id_launch
+    t, r, e, n, k = 400, 4, 48, 1024, 2048
+    rng = np.random.default_rng(9)
+    ids = np.stack([rng.permutation(40)[:r] for _ in range(t)]).astype(np.int32)
+    ids[:150, 0] = 44
+    x = O.normal(3310, t * k)
+    qb = quant.quantize(be, fmt, O.normal(3311, e * n * k, 0.02), e * n, k)
+    outs = []
+    for mode in ("tc", "f32"):
+        be.set_option("gemm", mode)
+        bufs = [be.upload(x), be.upload(qb), be.upload(ids), be.alloc(t * r * n * 4)]
+        l = matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 1, 2), output=3)
+        be.prepare([l])
+        be.execute([l], bufs)
+        outs.append(bufs[3].download().view(np.float32))
+    be.set_option("gemm", "tc")
+    assert rel_l2(outs[0], outs[1]) <= 4e-3 and max_rel(outs[0], outs[1]) <= 3e-2
