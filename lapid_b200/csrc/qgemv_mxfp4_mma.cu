@@ -3,7 +3,7 @@
 // 0, 1, 2, 3, 4, 6, 8, 12 and their negatives; crates/lapid-quant/src/mxfp4.rs:14-25) decode GEMV for 1..8 activation
 // rows on the warp-level int8 tensor-core instruction. Arithmetic as in qgemv_mxfp4.cu (lapid-cpu's,
 // crates/lapid-cpu/src/mxfp4.rs:38-58): the exact integer dot product of KV with the int8 activations per block, one
-// f32 step per block. The sibling of qgemv_i4_mma.cu: same CTA structure (a CTA owns 16-row tiles, its warps split K
+// f32 step per block. The sibling of qgemv_i8_mma.cu: same CTA structure (a CTA owns 16-row tiles, its warps split K
 // in chunks of 512, stages by cp.async, partial 16x8 tiles summed in warp order, the activation tiles of the K-quant
 // kernels).
 //
