@@ -613,7 +613,15 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     ha = *(const uint4 *)(blk + 16);
                     hb = *(const uint4 *)(blk + 32);
                 }
-                if (NT == 2 ? pp == 3 : pp >= 2) {  // this thread's last read of the block's packed bytes
+                if (NT == 2 ? pp == 3 : pp >= 2) {
+                    // This thread's last read of the block's packed bytes: the slot goes back, but only once the loads have returned. Shared
+                    // loads that nothing has waited for yet may be carried out behind the arrival (hundreds of cycles
+                    // behind it while the load / store unit is busy) and then read the first rows of the next block. The vote
+                    // over what they brought waits for them, and nothing hangs on its result. (Giving the slot back behind the
+                    // stores below, which need the values as well: 2048 rows on 11008 x 4096 228 against 225 us, the ring has two slots there.)
+                    uint32_t brought = (qa.x ^ qa.y ^ qa.z ^ qa.w) ^ (qb.x ^ qb.y ^ qb.z ^ qb.w);
+                    if constexpr (FMT == FMT_Q5K) brought ^= (ha.x ^ ha.y ^ ha.z ^ ha.w) ^ (hb.x ^ hb.y ^ hb.z ^ hb.w);
+                    if (__any_sync(0xffffffffu, brought == 0x9E3779B9u)) __nanosleep(1);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(raw_empty + r);
                 }

@@ -1598,3 +1598,28 @@ def test_matmul_id_tensor_core_more_tiles_than_sms(be, fmt):
         outs.append(bufs[3].download().view(np.float32))
     be.set_option("gemm", "tc")
     assert rel_l2(outs[0], outs[1]) <= 4e-3 and max_rel(outs[0], outs[1]) <= 3e-2
+
+
+@pytest.mark.parametrize("fmt", [lp.DType.Q4K, lp.DType.Q5K, lp.DType.Q6K])
+@pytest.mark.parametrize("t", [200, 480, 1200])
+def test_matmul_id_tensor_core_loop_every_tile_height(be, fmt, t):
+    """Expert-indexed launches whose CTAs take several tiles each, so that both accumulator sets are used again, at every tile height:
+    33, 80 and 200 rows per expert on average take tiles of 64, 128 and 256 rows (the last uses all of tensor memory). The order
+    of every sum is fixed, so repeats give the same bits. Bar as above."""
+    from lapid_b200.backend import matmul_id_launch
+    r, e, n, k = 4, 24, 4992, 512   # 39 weight tiles x at least 24 activation tiles
+    ids = np.stack([np.random.default_rng(i).permutation(e)[:r] for i in range(t)]).astype(np.int32)
+    x = O.normal(3320, t * k)
+    w = (O.normal(3321, n * k, 0.02).reshape(1, n, k) * (1 + 0.1 * np.arange(e, dtype=np.float32))[:, None, None]).astype(np.float32)
+    bufs = [be.upload(x), be.upload(quant.quantize(be, fmt, w.reshape(-1), e * n, k)), be.upload(ids), be.alloc(t * r * n * 4)]
+    l = matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 1, 2), output=3)
+    be.set_option("gemm", "f32")
+    be.execute([l], bufs)
+    want = bufs[3].download().view(np.float32).copy()
+    be.set_option("gemm", "tc")
+    be.execute([l], bufs)
+    got = bufs[3].download().view(np.float32).copy()
+    assert rel_l2(got, want) <= 4e-3 and max_rel(got, want) <= 3e-2
+    for _ in range(5):
+        be.execute([l], bufs)
+        assert np.array_equal(bufs[3].download().view(np.float32), got)
