@@ -32,57 +32,94 @@ __device__ __forceinline__ float4 scale4(float4 a, float s) { return make_float4
 __device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 __device__ __forceinline__ float sumsq4(float4 a, float ss) { return fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, ss)))); }
 
-// One CTA per row, VEC float4 per thread in registers. A decode step has one to eight rows, so what counts there is the
+// One CTA per row, its float4s in registers. A decode step has one to eight rows, so what counts there is the
 // chain load -> sum -> store: as many threads as the row has float4s (up to 1024), all loads of a thread issued
-// before the first is used, one barrier. A prompt has enough rows to fill the chip, so memory bandwidth is the bound (x, residual, sum and
+// before the first is used, two barriers. A prompt has enough rows to fill the chip, so memory bandwidth is the bound (x, residual, sum and
 // out: 16 bytes an element). A row split over a cluster of eight CTAs, which this replaces, paid two cluster barriers for
-// every row: 2048 x 8192 took 320 us (0.8 TB/s), now 38 (7.1 TB/s of which part is L2), 77 x 4096 16.5 and 3.0, one row of 4096 inside a
-// decode step 3.5 us less.
-template <int VEC> __global__ void __launch_bounds__(1024) rms_norm_kernel(RmsNormArgs p) {
-    __shared__ float partial[32];
-    const uint32_t row = blockIdx.x, n4 = p.cols / 4, tid = threadIdx.x, step = blockDim.x;
+// every row: 2048 x 8192 took 311 us (0.9 TB/s), now 42 (6.4 TB/s, part of it L2), 77 x 4096 14.2 and 3.1, one
+// row of 4096 in a chain of them 4.4 and 2.2.
+//
+// The order of the sum of squares is that of the row split over `parts` CTAs of 256 threads (tp_rms_norm_kernel, below, which has
+// to split it): a row gives the same bits however many rows there are and in both kernels, so a stack gives the same tokens
+// on one GPU and on a group of one. A slice of 32 float4s of a part is one warp's work (PER = 2: and the 32 float4s 256 behind them), its sum
+// a butterfly; the slices of a part are added in order, then the parts in order. SLICES of them go to each warp.
+template <int SLICES, int PER> __global__ void __launch_bounds__(1024) rms_norm_kernel(RmsNormArgs p, uint32_t parts) {
+    __shared__ __align__(16) float partial[64];  // slice w of part q: [8 q + w]
+    __shared__ float row_rstd;
+    const uint32_t row = blockIdx.x, n4 = p.cols / 4, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const uint32_t per = (n4 + parts - 1) / parts, width = (min(per, 256u) + 31) / 32;  // float4s and slices of a part
     const size_t at = (size_t)row * n4;
     const float4 *x = (const float4 *)p.x + at, *res = (const float4 *)p.residual + at;
+    uint32_t c0[SLICES], c_hi[SLICES], slot[SLICES];
+#pragma unroll
+    for (int s = 0; s < SLICES; s++) {
+        const uint32_t slice = (threadIdx.x >> 5) + s * warps, part = slice / width, w = slice - part * width;
+        slot[s] = 8 * part + w;
+        c0[s] = part * per + 32 * w + lane;
+        c_hi[s] = part < parts ? min(n4, (part + 1) * per) : 0u;
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    float4 v[VEC], r[VEC];
+    float4 v[SLICES][PER], r[SLICES][PER];
 #pragma unroll
-    for (int i = 0; i < VEC; i++) {
-        const uint32_t c = tid + i * step;
-        v[i] = r[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (c < n4) {
-            v[i] = x[c];
-            if (p.residual) r[i] = res[c];
+    for (int s = 0; s < SLICES; s++)
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const uint32_t c = c0[s] + 256 * i;
+            v[s][i] = r[s][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (c < c_hi[s]) {
+                v[s][i] = x[c];
+                if (p.residual) r[s][i] = res[c];
+            }
+        }
+    float ss[SLICES];
+#pragma unroll
+    for (int s = 0; s < SLICES; s++) {
+        ss[s] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            if (p.residual) v[s][i] = add4(v[s][i], r[s][i]);
+            ss[s] = sumsq4(v[s][i], ss[s]);
         }
     }
-    float ss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VEC; i++) {
-        if (p.residual) v[i] = add4(v[i], r[i]);
-        ss = sumsq4(v[i], ss);
-    }
+    for (int o = 16; o; o >>= 1)
 #pragma unroll
-    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((tid & 31) == 0) partial[tid >> 5] = ss;
+        for (int s = 0; s < SLICES; s++) ss[s] += __shfl_xor_sync(0xffffffffu, ss[s], o);
+#pragma unroll
+    for (int s = 0; s < SLICES; s++)
+        if (lane == 0 && slot[s] < 64) partial[slot[s]] = ss[s];
     __syncthreads();
-    float tot = (tid & 31) < step / 32 ? partial[tid & 31] : 0.0f;
+    // one warp for all (thirty of them doing the same would take the issue slots): lane q adds the slices of part q, then the parts
+    // are added (what is past the row counts as 0)
+    if (threadIdx.x < 32) {
+        const float4 lo = *(const float4 *)&partial[8 * (lane & 7)], hi = *(const float4 *)&partial[8 * (lane & 7) + 4];
+        const float sl[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        float mine = 0.0f, tot = 0.0f;
 #pragma unroll
-    for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    const float rstd = 1.0f / sqrtf(tot * (1.0f / (float)p.cols) + p.eps);
+        for (uint32_t w = 0; w < 8; w++) mine += w < width && (lane & 7) < parts ? sl[w] : 0.0f;
 #pragma unroll
-    for (int i = 0; i < VEC; i++) {
-        const uint32_t c = tid + i * step;
-        const bool active = c < n4;
-        float4 a = scale4(v[i], rstd);
-        if (active) {
-            if (p.weight) a = mul4(a, ((const float4 *)p.weight)[c]);
-            ((float4 *)p.out)[at + c] = a;
-            if (p.sum_out) ((float4 *)p.sum_out)[at + c] = v[i];
-        }
-        // the same values as the int8 operand of the GEMVs that read `out` (whole warps of the row take the branch together,
-        // lanes past the row pass active = false)
-        if (p.q.qa && (tid & ~31u) + i * step < n4) act_quant_quad(p.q, active, row, 4 * c, a);
+        for (int q = 0; q < 8; q++) tot += __shfl_sync(0xffffffffu, mine, q);
+        if (lane == 0) row_rstd = 1.0f / sqrtf(tot * (1.0f / (float)p.cols) + p.eps);
     }
+    __syncthreads();
+    const float rstd = row_rstd;
+#pragma unroll
+    for (int s = 0; s < SLICES; s++)
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const uint32_t c = c0[s] + 256 * i;
+            const bool active = c < c_hi[s];
+            float4 a = scale4(v[s][i], rstd);
+            if (active) {
+                if (p.weight) a = mul4(a, ((const float4 *)p.weight)[c]);
+                ((float4 *)p.out)[at + c] = a;
+                if (p.sum_out) ((float4 *)p.sum_out)[at + c] = v[s][i];
+            }
+            // the same values as the int8 operand of the GEMVs that read `out` (a whole warp takes the branch together, lanes
+            // past the part pass active = false)
+            if (p.q.qa && c - lane < c_hi[s]) act_quant_quad(p.q, active, row, 4 * c, a);
+        }
 }
 
 // Tensor-parallel input: x = sum over ranks (in rank order) of the partials they pushed for the call in progress, polled
@@ -232,14 +269,13 @@ cudaError_t launch_rms_norm(const RmsNormArgs &a, bool pdl, cudaStream_t stream)
         pdl_config(cfg, attr, a.rows * parts, pdl, stream, parts);
         return cudaLaunchKernelEx(&cfg, tp_rms_norm_kernel, a);
     }
-    // few rows: the most threads a row can use; many: two float4 per thread, so that several rows share an SM
-    const unsigned n4 = a.cols / 4, per = a.rows <= 64 ? 1 : 2;
-    unsigned threads = (n4 + per - 1) / per;
-    threads = threads >= 1024 ? 1024 : (threads + 31) / 32 * 32;
-    pdl_config(cfg, attr, a.rows, pdl, stream, 1, threads);
-    if (n4 <= threads) return cudaLaunchKernelEx(&cfg, rms_norm_kernel<1>, a);
-    if (n4 <= 2 * threads) return cudaLaunchKernelEx(&cfg, rms_norm_kernel<2>, a);
-    return cudaLaunchKernelEx(&cfg, rms_norm_kernel<4>, a);
+    const uint32_t parts = rms_norm_parts(a.cols), per = (a.cols / 4 + parts - 1) / parts, slices = parts * (((per < 256 ? per : 256) + 31) / 32);
+    // few rows: a warp per slice as far as a CTA goes; many: two slices per warp, so that several rows share an SM
+    const bool one = a.rows <= 64 && slices <= 32;
+    pdl_config(cfg, attr, a.rows, pdl, stream, 1, 32 * (one ? slices : (slices + 1) / 2));
+    if (per > 256) return cudaLaunchKernelEx(&cfg, rms_norm_kernel<2, 2>, a, parts);  // (64 slices)
+    if (one) return cudaLaunchKernelEx(&cfg, rms_norm_kernel<1, 1>, a, parts);
+    return cudaLaunchKernelEx(&cfg, rms_norm_kernel<2, 1>, a, parts);
 }
 
 cudaError_t launch_silu_mul(const float *gate, const float *up, float *out, uint64_t n, uint32_t cols, const ActOut &q, int sm_count,

@@ -554,6 +554,50 @@ def test_glue_kernels_rms_norm_and_silu_mul(be):
     assert e.value.code == "invalid_launch"
 
 
+@pytest.mark.parametrize("cols", [4, 260, 1028, 2880, 4096, 8192, 12292, 16384])
+def test_rms_norm_bits_depend_neither_on_the_rows_nor_on_the_kernel(be, cols):
+    """A row's sum of squares is added up in one order, however many rows there are (one to 64: a thread per float4 where a
+    CTA has them; more: two) and in the tensor-parallel kernel too, which splits the row over CTAs: a group of one rank
+    gives what one GPU gives, bit for bit. Against f64 as above."""
+    import ctypes as C
+    import torch
+    from lapid_b200 import _lib
+    rows, k, n_few = 130, 32, 8
+    rng = np.random.default_rng(cols)
+    qb = quant.quantize(be, lp.DType.Int8, O.normal(cols, cols * k, 0.5), cols, k)
+    ba, bw, bx = be.upload(rng.standard_normal(rows * k, dtype=np.float32)), be.upload(qb), be.alloc(rows * cols * 4)
+    launch = matmul_launch(lp.DType.Int8, n_few, cols, k, inputs=(0, 1), output=2)
+    be.execute([matmul_launch(lp.DType.Int8, rows, cols, k, inputs=(0, 1), output=2)], [ba, bw, bx])
+    be.execute([launch], [ba, bw, bx])          # the first rows as the decode kernel gives them, as the push below does
+    x = bx.download().view(np.float32).reshape(rows, cols)
+    r, w = rng.standard_normal((rows, cols), dtype=np.float32), rng.standard_normal(cols, dtype=np.float32)
+    br, bg, bo, bs = be.upload(r), be.upload(w), be.alloc(rows * cols * 4), be.alloc(rows * cols * 4)
+    be.rms_norm(bx, bo, rows, cols, residual=br, weight=bg, sum_out=bs)
+    be.synchronize()
+    many = bo.download().view(np.float32).reshape(rows, cols)
+    h = (x + r).astype(np.float64)
+    want = h / np.sqrt((h ** 2).mean(axis=1, keepdims=True) + 1e-6) * w
+    assert np.abs(many - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
+    for few in (1, n_few, 64):
+        be.rms_norm(bx, bo, few, cols, residual=br, weight=bg, sum_out=bs)
+        be.synchronize()
+        assert np.array_equal(bo.download().view(np.float32).reshape(rows, cols)[:few], many[:few]), few
+        assert np.array_equal(bs.download().view(np.float32).reshape(rows, cols)[:few], (x + r)[:few])
+    lib = _lib.lib()
+    mem = torch.zeros(int(lib.lapid_b200_tp_comm_bytes(1, n_few * cols)), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    comm = C.c_void_p()
+    _lib.check(lib.lapid_b200_tp_comm_create(be._h, 0, 1, (C.c_void_p * 1)(mem.data_ptr()), n_few * cols, C.byref(comm)))
+    try:
+        arr, packed = be._pack([launch], [ba, bw, bx])
+        _lib.check(lib.lapid_b200_tp_matmul_push(comm, arr, packed, 3))
+        _lib.check(lib.lapid_b200_tp_rms_norm_act(comm, br._h, bg._h, bs._h, bo._h, n_few, cols, 1e-6, None, 0))
+        be.synchronize()
+        assert np.array_equal(bo.download().view(np.float32).reshape(rows, cols)[:n_few], many[:n_few])
+    finally:
+        lib.lapid_b200_tp_comm_free(comm)
+
+
 # ------------------------------------------------------------------ exact-f32 GEMM path
 @pytest.mark.parametrize("fmt,name", FMTS)
 def test_gemm_f32_bit_exact_vs_oracle(be, oracle, fmt, name):
