@@ -22,6 +22,8 @@
 // replaces: 2.71 ms), 1184 rows 48.5 TFLOP/s, where the FMA pipe is busy for about 70 % of the time (ncu: the rest is waits on operands).
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "iquant.cuh"
 #include "kernels.h"
@@ -210,20 +212,16 @@ qgemm_f32_kernel(GemmF32Args p) {
 #pragma unroll
         for (int t = 0; t < WN; t++) {
             const int u = tid + t * THREADS, k = 8 * (u % WP);
+            if (BK == 64 && k0 + (uint32_t)k >= p.k) continue;
             float y[8];
-            if (BK == 16 || k0 + (uint32_t)k < p.k) {
-                expand8<FMT>(wv[t], k0 + (uint32_t)k, y);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; i++) y[i] = 0.0f;
-            }
+            expand8<FMT>(wv[t], k0 + (uint32_t)k, y);
 #pragma unroll
             for (int i = 0; i < 8; i++) Bs[buf][k + i][(u / WP) ^ swz_b(k + i)] = y[i];
         }
     };
 
-    // k is a multiple of 32: the last step of BK = 64 may be half full. The rest is 0 * 0, which leaves every accumulator as it is
-    // (none can be -0: a sum that starts at +0 and rounds to nearest never gets there).
+    // k is a multiple of 32: the last step of BK = 64 may be half full and then ends there (a term 0 * 0 more would turn an accumulator
+    // of -0, which a negative product that underflows leaves, into +0).
     fetch(0);
     stage(0, 0);
     __syncthreads();
@@ -247,17 +245,21 @@ qgemm_f32_kernel(GemmF32Args p) {
                 else *(float2 *)&b[kk & 1][2 * j] = *(const float2 *)src;
             }
         };
-        operands(0);
+        auto multiply = [&](auto steps) {
+            operands(0);
 #pragma unroll 16
-        for (int kk = 0; kk < BK; kk++) {
-            if (kk + 1 < BK) operands(kk + 1);
+            for (int kk = 0; kk < steps.value; kk++) {
+                if (kk + 1 < steps.value) operands(kk + 1);
 #pragma unroll
-            for (int j = 0; j < TN; j++) {
-                const uint64_t b2 = pack2(b[kk & 1][j], b[kk & 1][j]);
+                for (int j = 0; j < TN; j++) {
+                    const uint64_t b2 = pack2(b[kk & 1][j], b[kk & 1][j]);
 #pragma unroll
-                for (int i = 0; i < TM / 2; i++) fma2(acc[i][j], a2[kk & 1][i], b2);
+                    for (int i = 0; i < TM / 2; i++) fma2(acc[i][j], a2[kk & 1][i], b2);
+                }
             }
-        }
+        };
+        if (BK == 64 && p.k - k0 < BK) multiply(std::integral_constant<int, BK / 2>());
+        else multiply(std::integral_constant<int, BK>());
         if (more) {
             stage(buf ^ 1, k0 + BK);  // the other buffer's readers passed the barrier of the step before
             __syncthreads();

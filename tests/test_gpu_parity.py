@@ -1667,3 +1667,18 @@ def test_matmul_id_tensor_core_loop_every_tile_height(be, fmt, t):
     for _ in range(5):
         be.execute([l], bufs)
         assert np.array_equal(bufs[3].download().view(np.float32), got)
+
+
+def test_gemm_f32_negative_zero(be, oracle):
+    """A sum that is left at -0 (a negative product that underflows) keeps its sign: nothing is added behind the last of the k terms, also where
+    k ends in the middle of the kernel's step (16 x 32 tiles: steps of 64)."""
+    for m, n, k in [(12, 40, 96), (12, 40, 64), (9, 33, 32), (16, 32, 160)]:
+        a = np.zeros((m, k), np.float32)
+        a[:, k - 1] = -1e-41
+        w = np.full((n, k), 1e-5, np.float32)
+        qb = oracle.quantize(O.INT8, w.reshape(-1), n, k)
+        want, _ = oracle.matmul(O.INT8, a.reshape(-1), qb, n, k, m=m)
+        want = np.asarray(want, np.float32).reshape(-1)
+        assert (want.view(np.uint32) == 0x80000000).all()
+        got = run_matmul(be, lp.DType.Int8, a.reshape(-1), qb, m, n, k)
+        assert np.array_equal(np.asarray(got, np.float32).reshape(-1).view(np.uint32), want.view(np.uint32)), (m, n, k)
