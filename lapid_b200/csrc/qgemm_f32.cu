@@ -303,9 +303,10 @@ qgemm_f32_kernel(GemmF32Args p) {
     }
 }
 
+constexpr uint32_t GRID_Y_MAX = 65535;
 template <int FMT, int BM, int BN, int BK, int TM, int TN> static cudaError_t launch_tile(const GemmF32Args &a, cudaStream_t stream) {
     const dim3 grid((a.n + BN - 1) / BN, (a.rows + BM - 1) / BM);
-    if (grid.y > 65535) return cudaErrorInvalidValue;
+    if (grid.y > GRID_Y_MAX) return cudaErrorInvalidValue;
     qgemm_f32_kernel<FMT, BM, BN, BK, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, stream>>>(a);
     return cudaGetLastError();
 }
@@ -337,7 +338,9 @@ uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts, uint64_t n, int sm
     const uint64_t used = experts < pairs ? experts : pairs;
     if (!used) return 64;
     const double avg = (double)pairs / (double)used;
-    return F32_TILES[pick_tile(used, avg + (avg > 1 ? sqrt(avg) : 0), n, sm_count)].bm;
+    int i = pick_tile(used, avg + (avg > 1 ? sqrt(avg) : 0), n, sm_count);
+    while (i > 0 && moe_max_tiles(pairs, experts, F32_TILES[i].bm) > GRID_Y_MAX) i--;  // tens of thousands of experts: taller tiles, fewer of them
+    return F32_TILES[i].bm;
 }
 
 template <int FMT> static cudaError_t launch_fmt(const GemmF32Args &a, int sm_count, cudaStream_t stream) {

@@ -1682,3 +1682,31 @@ def test_gemm_f32_negative_zero(be, oracle):
         assert (want.view(np.uint32) == 0x80000000).all()
         got = run_matmul(be, lp.DType.Int8, a.reshape(-1), qb, m, n, k)
         assert np.array_equal(np.asarray(got, np.float32).reshape(-1).view(np.uint32), want.view(np.uint32)), (m, n, k)
+
+
+def test_matmul_id_tens_of_thousands_of_experts(be):
+    """The activation tiles of an expert-indexed launch are one grid dimension (65535): with very many experts of few rows each the tiles are
+    taken taller. Reference: f64 on the dequantized weights."""
+    import torch
+    from lapid_b200.backend import matmul_id_launch
+    t, r, e, n, k = 100000, 4, 50000, 32, 32
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    ids = torch.randint(0, e, (t, r), dtype=torch.int32, device="cuda", generator=g)
+    x = torch.randn(t, k, device="cuda", generator=g)
+    total = 1280   # 1024 quants, 64 bytes of scales, padded to 256
+    w = torch.zeros(e, total, dtype=torch.uint8, device="cuda")
+    q = torch.randint(-127, 128, (e, n, k), dtype=torch.int8, device="cuda", generator=g)
+    d = torch.rand(e, n, device="cuda", generator=g).add_(0.5).half()
+    w[:, :1024] = q.view(torch.uint8).view(e, n * k)
+    w[:, 1024:1088] = d.view(torch.uint8).view(e, 2 * n)
+    out = torch.zeros(t, r, n, device="cuda")
+    torch.cuda.synchronize()
+    bufs = [be.wrap_tensor(v) for v in (x, w.view(-1), ids, out)]
+    be.execute([matmul_id_launch(lp.DType.Int8, t, r, e, n, k, inputs=(0, 1, 2), output=3)], bufs)
+    worst = 0.0
+    for lo in range(0, t, 10000):
+        deq = (q[ids[lo:lo + 10000].long()].double() * d[ids[lo:lo + 10000].long()].double()[..., None])
+        want = (deq * x[lo:lo + 10000].double()[:, None, None, :]).sum(-1)
+        worst = max(worst, float((out[lo:lo + 10000].double() - want).norm() / want.norm()))
+    assert worst <= 1e-6   # 32 f32 terms: about 2e-7
