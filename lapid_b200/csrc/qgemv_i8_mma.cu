@@ -19,7 +19,9 @@
 // RAGGED: K any multiple of 32. The last chunk of a row is partly there (the copies past it are zero-filled, its missing groups
 // skipped), and a row's scales start at any even byte: three aligned 16-byte pieces around a chunk's 32 bytes of scales
 // are staged and read with 16-bit loads. Widths that are no multiple of 512 are common (2880, shards of 7680) and took the
-// generic dp4a kernel before (int8, three rows, 12 layers of 2880 / 7680: a token 922 us, now 593).
+// generic dp4a kernel before (int8, three rows, 12 layers of 2880 / 7680: a token 922 us, now 604). Its lanes' sums were short and met in a
+// butterfly; so that the f32 sums are no further off than its, the even and odd groups of a 256-wide tile are summed apart, the
+// tiles behind that, the warps in pairs (against f64, K 1024..14336: 8.1e-8 as before; one chain per warp 1.2e-7, and 593 us).
 //
 // Several projections over the same activations (q, k, v; gate, up) run as one launch over the concatenated tiles. Early
 // mode (GemvArgs::early): activations are read and tiles computed before the dependency wait, which comes before the first store.
@@ -172,9 +174,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvGroupT<
                     sw1 = *(const uint4 *)(stage + Q_BYTES + (gq + 8) * SCB + 16 * blk);
                 }
                 const uint32_t s0[4] = {sw0.x, sw0.y, sw0.z, sw0.w}, s1[4] = {sw1.x, sw1.y, sw1.z, sw1.w};
+                float part[2][4] = {};  // RAGGED: the tile's even and odd groups
 #pragma unroll
                 for (int s = 0; s < 8; s++) {
                     if (RAGGED && it * (KC / GROUP) + 8 * blk + s >= kg) break;
+                    float (&sum)[4] = RAGGED ? part[s & 1] : acc;
                     uint32_t a0, a1, a2, a3;
                     if constexpr (I4) {
                         const int c16 = 8 * blk + s;  // the group's 16 bytes are one chunk of the row
@@ -196,11 +200,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvGroupT<
                     const uint32_t h0 = RAGGED ? sr0[8 * blk + s] : (s0[s >> 1] >> (16 * (s & 1))) & 0xffff;
                     const uint32_t h1 = RAGGED ? sr1[8 * blk + s] : (s1[s >> 1] >> (16 * (s & 1))) & 0xffff;
                     const float w0 = half_bits_to_float(h0) * (I4 ? 0.0625f : 1.0f), w1 = half_bits_to_float(h1) * (I4 ? 0.0625f : 1.0f);  // (Int4: the dot is 16 times too large)
-                    acc[0] = fmaf((__int_as_float(c[0]) - MAGIC) * da.x, w0, acc[0]);
-                    acc[1] = fmaf((__int_as_float(c[1]) - MAGIC) * da.y, w0, acc[1]);
-                    acc[2] = fmaf((__int_as_float(c[2]) - MAGIC) * da.x, w1, acc[2]);
-                    acc[3] = fmaf((__int_as_float(c[3]) - MAGIC) * da.y, w1, acc[3]);
+                    sum[0] = fmaf((__int_as_float(c[0]) - MAGIC) * da.x, w0, sum[0]);
+                    sum[1] = fmaf((__int_as_float(c[1]) - MAGIC) * da.y, w0, sum[1]);
+                    sum[2] = fmaf((__int_as_float(c[2]) - MAGIC) * da.x, w1, sum[2]);
+                    sum[3] = fmaf((__int_as_float(c[3]) - MAGIC) * da.y, w1, sum[3]);
                 }
+                if constexpr (RAGGED)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) acc[i] += part[0][i] + part[1][i];
             }
             __syncwarp();  // every lane is done reading the slot before it is refilled
             issue();
@@ -219,9 +226,20 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(GemvGroupT<
         }
         for (uint32_t e = threadIdx.x; e < 128; e += THREADS) {
             const float *src = red + (size_t)par * WARPS * 128 + e;
-            float v = src[0];
+            float v;
+            if constexpr (RAGGED) {  // in pairs
+                float half[2];
 #pragma unroll
-            for (int w = 1; w < WARPS; w++) v += src[(size_t)w * 128];
+                for (int h = 0; h < 2; h++) {
+                    const float *q = src + (size_t)h * (WARPS / 2) * 128;
+                    half[h] = WARPS == 8 ? (q[0] + q[128]) + (q[256] + q[384]) : q[0] + q[128];
+                }
+                v = half[0] + half[1];
+            } else {
+                v = src[0];
+#pragma unroll
+                for (int w = 1; w < WARPS; w++) v += src[(size_t)w * 128];
+            }
             const uint32_t el = e & 31, i = e >> 5;
             const uint32_t row = local * 16 + (el >> 2) + ((i & 2) ? 8 : 0);
             const uint32_t r = 2 * (el & 3) + (i & 1);

@@ -1606,6 +1606,34 @@ def test_gemv_planes_tensor_core_ragged_k(be, oracle, fmt, ofmt):
             assert max_rel(bufs[4 + i].download().view(np.float32), want) <= 2e-5, (m, k, n)
 
 
+@pytest.mark.parametrize("fmt", [lp.DType.Int8, lp.DType.Int4])
+def test_gemv_planes_ragged_k_sum_error(be, fmt):
+    """Widths that are no multiple of 512: the f32 sum over the groups against f64 on the same int8 activations. Bar: 2^-23 relative (2-norm). A chain of
+    c additions of equal terms ends with about sqrt(c / 6) units of 2^-24: the kernel's chains of four groups, up to eight tiles
+    and eight warps in pairs give 1.0e-7 at k = 14304, one chain per warp (64 groups) would give 1.9e-7."""
+    import torch
+    n = 600
+    for m, k in ((3, 14304), (1, 13856), (8, 9632), (2, 2880)):
+        w, x = O.normal(3200 + k, n * k, 0.02), O.normal(3201 + k, m * k)
+        qb = quant.quantize(be, fmt, w, n, k)
+        got = run_matmul(be, fmt, x, qb, m, n, k)
+        q = torch.from_numpy(np.ascontiguousarray(qb)).view(torch.uint8)
+        quants = n * k if fmt == lp.DType.Int8 else n * k // 2
+        at = (quants + 255) // 256 * 256
+        scales = q[at:at + n * k // 32 * 2].view(torch.float16).view(n, k // 32).double()
+        if fmt == lp.DType.Int8:
+            wi = q[:quants].view(torch.int8).view(n, k // 32, 32).double()
+        else:
+            nib = q[:quants].view(n, k // 32, 16).int()
+            wi = (torch.cat([nib & 15, nib >> 4], dim=2) - 8).double()
+        groups = torch.from_numpy(x).view(m, k // 32, 32)
+        d = groups.abs().amax(-1) / 127.0                       # as the pre-pass: f32 scale, its f32 reciprocal, round to even
+        act = torch.round(groups * (1.0 / d)[..., None]).clamp(-127, 127).double() * d.double()[..., None]
+        want = act.view(m, k) @ (wi * scales[..., None]).view(n, k).t()
+        err = float((torch.from_numpy(np.asarray(got, np.float32)).view(m, n).double() - want).norm() / want.norm())
+        assert err <= 2.0 ** -23, (m, k, err)
+
+
 @pytest.mark.parametrize("fmt", [lp.DType.Q4K, lp.DType.Q5K, lp.DType.Q6K])
 @pytest.mark.parametrize("m,n,k", [(20, 19333, 512), (100, 19200, 768), (200, 19201, 256), (300, 38500, 256), (600, 19333, 512)])
 def test_gemm_tensor_core_more_tiles_than_sms(be, fmt, m, n, k):
