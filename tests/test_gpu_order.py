@@ -1,15 +1,18 @@
-"""Prompts give the same bits every time: the order of every sum is fixed by the launch, not by timing, so the bar is equality."""
+"""What the order of the kernels on the device must not change: steps captured in a CUDA graph and replayed with new inputs give the bits
+of the same step run kernel by kernel (option ``pdl`` = 0: no kernel starts before the one in front of it has finished), and prompts
+give the same bits every time. The bar is equality throughout: the order of every sum is fixed by the launch, not by timing."""
 import numpy as np
 import pytest
 
 import lapid_b200 as lp
 from lapid_b200 import tp
-from lapid_b200.backend import DType, matmul_id_launch
+from lapid_b200.backend import DType, matmul_id_launch, matmul_launch
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
-MIXES = {"q4_k_m": lambda p, i: tp.q4km_format(p, i, 2), "q5_k": lambda p, i: int(DType.Q5K)}
+MIXES = {"q4_k_m": lambda p, i: tp.q4km_format(p, i, 2), "q5_k": lambda p, i: int(DType.Q5K), "q6_k": lambda p, i: int(DType.Q6K),
+         "int8": lambda p, i: int(DType.Int8), "int4": lambda p, i: int(DType.Int4), "mxfp4": lambda p, i: int(DType.MXFP4)}
 
 
 def _weights(be, fmt, n, k, seed, std=0.04):
@@ -33,12 +36,114 @@ def _device(**options):
     return be, stream
 
 
+def _capture(be, stream, queue):
+    """`queue` once plainly (scratch, kernel attributes), then as a graph on the stream."""
+    import torch
+    with torch.cuda.stream(stream):
+        queue()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        be.set_stream(torch.cuda.current_stream().cuda_stream)
+        queue()
+    be.set_stream(stream.cuda_stream)
+    return graph
+
+
 def _stack(be, shape, m, mix, fuse_act, weights=None):
     formats = [{p: MIXES[mix](p, i) for p in ("q", "k", "v", "o", "gate", "up", "down")} for i in range(2)]
     if weights is None:
         weights = [{p: _weights(be, f[p], n, k, 500 + 10 * i + j) for j, (p, n, k, _) in enumerate(shape.projections())}
                    for i, f in enumerate(formats)]
     return tp.GpuTpLayers(be, shape, 1, 0, m, weights, formats, fuse_act=fuse_act), weights
+
+
+@pytest.mark.parametrize("fuse_act", [False, True])
+@pytest.mark.parametrize("m", [1, 3, 8])
+@pytest.mark.parametrize("mix", list(MIXES))
+def test_captured_decode_step_gives_the_bits_of_the_serial_one(mix, m, fuse_act):
+    """Six layers: rms_norm -> q, k, v -> o -> rms_norm -> gate, up -> silu_mul -> down. Under capture the first kernel of a list
+    requests its weights while the glue kernel or the pre-pass in front of it runs, and the later ones read their quantized activations early."""
+    import torch
+    serial, s0 = _device(pdl="0")
+    be, s1 = _device()
+    shape = tp.LayerShape(1024, 8, 2, 128, 2048) if fuse_act or mix not in ("int8", "int4") else tp.LayerShape(960, 8, 2, 120, 1888)  # (ragged widths)
+    ref, weights = _stack(serial, shape, m, mix, fuse_act)
+    ours, _ = _stack(be, shape, m, mix, fuse_act, weights)
+    assert not fuse_act or any(l is not None for ls in ours.act_layouts for l in ls)
+    inputs = [torch.from_numpy(O.normal(700 + i, m * shape.d_model).reshape(m, -1)).cuda() for i in range(4)]
+    torch.cuda.synchronize()
+    graph = _capture(be, s1, lambda: ours.token(6))
+    wants = []
+    for x in inputs:
+        with torch.cuda.stream(s0):
+            ref.h.copy_(x)
+            wants.append(ref.token(6).clone())
+        s0.synchronize()
+    for rep in range(40):
+        i = rep % len(inputs)
+        with torch.cuda.stream(s1):
+            ours.h.copy_(inputs[i])
+            graph.replay()
+            got = ours.hw.clone()
+        s1.synchronize()
+        assert torch.isfinite(got).all() and torch.equal(got, wants[i]), rep
+    serial.synchronize()
+    be.synchronize()
+
+
+@pytest.mark.parametrize("fmt", [DType.Q4K, DType.Q6K, DType.Int8, DType.Iq3Xxs])
+@pytest.mark.parametrize("m", [1, 4])
+def test_captured_weights_written_between_the_glue_kernel_and_the_list(fmt, m):
+    """A list behind a glue kernel may request weights early only when nothing stands between the two: here a copy (then a kernel) rewrites
+    the weights there, in every replay with other ones."""
+    import torch
+    be, stream = _device()
+    n, k = 2048, 2048
+    if fmt == DType.Iq3Xxs:  # (no quantizer: any bytes are a block)
+        a_set = [torch.randint(0, 256, (n * k // 256, 98), dtype=torch.uint8, device="cuda") for _ in range(2)]
+        for b in a_set:
+            b[:, :2] = torch.full((len(b),), 1e-3, device="cuda").half().view(torch.uint8).view(-1, 2)
+        a_set = [torch.cat([b.reshape(-1), b.new_zeros(tp.layout_total(int(fmt), n, k) - b.numel())]) for b in a_set]
+    else:
+        a_set = [_weights(be, int(fmt), n, k, 800 + i) for i in range(2)]
+    source, w = a_set[0].clone(), torch.zeros_like(a_set[0])
+    x, normed, out = (torch.from_numpy(O.normal(810, m * k).reshape(m, k)).cuda(), torch.zeros(m, k, device="cuda"), torch.zeros(m, n, device="cuda"))
+    layout, nbytes = be.act_layout(matmul_launch(fmt, m, n, k))
+    qact = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    bufs = [be.wrap_tensor(t) for t in (normed, w, out, qact, x)]
+    plain = [matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)]
+    fused = [matmul_launch(fmt, m, n, k, inputs=(3, 1), output=2, a_quantized=True)]
+    wants = []
+    with torch.cuda.stream(stream):
+        be.rms_norm(bufs[4], bufs[0], m, k, qact=bufs[3], layout=layout)
+        for a in a_set:
+            w.copy_(a)
+            be.execute(plain, bufs)
+            wants.append(out.clone())
+    stream.synchronize()
+    assert not torch.equal(wants[0], wants[1])
+    for between in (lambda: w.copy_(source), lambda: torch.add(source, 0, out=w)):
+        for ls in (plain, fused):
+            def queue():
+                be.rms_norm(bufs[4], bufs[0], m, k, qact=bufs[3], layout=layout)
+                between()
+                be.execute_async(ls, bufs)
+            graph = _capture(be, stream, queue)
+            second = _capture(be, stream, lambda: be.execute_async(ls, bufs))  # no glue kernel of its own capture in front
+            for rep in range(20):
+                with torch.cuda.stream(stream):
+                    source.copy_(a_set[rep % 2])
+                    out.zero_()
+                    graph.replay()
+                    got = out.clone()
+                    w.copy_(a_set[(rep + 1) % 2])
+                    second.replay()
+                    other = out.clone()
+                stream.synchronize()
+                assert torch.equal(got, wants[rep % 2]) and torch.equal(other, wants[(rep + 1) % 2]), rep
+    be.synchronize()
 
 
 @pytest.mark.parametrize("m,layers", [(77, 6), (2048, 2)])

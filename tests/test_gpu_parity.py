@@ -374,7 +374,7 @@ def test_gemv_q6k_tensor_core_decode_kernel(be, oracle):
 
 
 def test_gemv_int8_tensor_core_decode_kernel(be, oracle):
-    """The Int8 tensor-core decode kernel (2..8 rows, K a multiple of 512) against the oracle and
+    """The Int8 tensor-core decode kernel (2..8 rows, here K a multiple of 512) against the oracle and
     against the dp4a kernel: ragged n, every row count, bias, K with several chunks per warp."""
     try:
         seed = 1000
@@ -396,7 +396,7 @@ def test_gemv_int8_tensor_core_decode_kernel(be, oracle):
 
 
 def test_gemv_int4_tensor_core_decode_kernel(be, oracle):
-    """The Int4 tensor-core decode kernel (2..8 rows, K a multiple of 512) against the oracle and against the plain
+    """The Int4 tensor-core decode kernel (2..8 rows, here K a multiple of 512) against the oracle and against the plain
     streaming kernel: ragged n, every row count, bias, K with several chunks per warp, weights at both ends of the
     4-bit range (a row of all 0 and all 15 codes)."""
     try:
@@ -1637,8 +1637,8 @@ def test_gemv_planes_ragged_k_sum_error(be, fmt):
 @pytest.mark.parametrize("fmt", [lp.DType.Q4K, lp.DType.Q5K, lp.DType.Q6K])
 @pytest.mark.parametrize("m,n,k", [(20, 19333, 512), (100, 19200, 768), (200, 19201, 256), (300, 38500, 256), (600, 19333, 512)])
 def test_gemm_tensor_core_more_tiles_than_sms(be, fmt, m, n, k):
-    """CTAs that take several tiles: both accumulator sets and their reuse, rings that run on from tile to tile, ragged last tiles; every
-    tile height. Bar: the rounding of both operands to bf16, as in test_gemm_tensor_core; the reference is the exact f32 kernel."""
+    """Launches of more tiles (one per CTA) than SMs, with a ragged last tile; every tile height. Bar: the rounding of both operands to
+    bf16, as in test_gemm_tensor_core; the reference is the exact f32 kernel."""
     w = np.tile(O.normal(3300, 1024 * k, 0.02), (n + 1023) // 1024)[: n * k]
     w = (w.reshape(n, k) * (1 + 0.001 * (np.arange(n, dtype=np.float32) % 997))[:, None]).astype(np.float32)   # no two row tiles alike
     qb = quant.quantize(be, fmt, w, n, k)
@@ -1652,7 +1652,7 @@ def test_gemm_tensor_core_more_tiles_than_sms(be, fmt, m, n, k):
 
 @pytest.mark.parametrize("fmt", [lp.DType.Q4K, lp.DType.Q6K])
 def test_matmul_id_tensor_core_more_tiles_than_sms(be, fmt):
-    """The same for expert-indexed launches, with experts that get no token (tiles to skip) and experts with more than one tile."""
+    """Expert-indexed launches, whose CTAs take many tiles: with experts that get no token (tiles to skip) and experts with more than one tile."""
     from lapid_b200.backend import matmul_id_launch
     t, r, e, n, k = 400, 4, 48, 1024, 2048
     rng = np.random.default_rng(9)
@@ -1695,6 +1695,38 @@ def test_matmul_id_tensor_core_loop_every_tile_height(be, fmt, t):
     for _ in range(5):
         be.execute([l], bufs)
         assert np.array_equal(bufs[3].download().view(np.float32), got)
+
+
+@pytest.mark.parametrize("n", [768, 20000])
+def test_activation_copy_sharing_tensor_core(be, n):
+    """Prefill launches of a list that read the same operand share its bf16 copy (n = 768: split over K too); a launch that overwrites the
+    operand, or another view of the same buffer, gets a copy of its own. Every result has the bits of the launch run by itself."""
+    m, k, fmt = 77, 1024, lp.DType.Q4K
+    w = [quant.quantize(be, fmt, O.normal(3400 + i, rows * k, 0.05), rows, k) for i, rows in enumerate((n, n, k))]
+    x, y = O.normal(3410, (m + 3) * k), O.normal(3411, m * k)
+    # 0 x, 1 y, 2..4 weights, 5.. outputs
+    bufs = [be.upload(x), be.upload(y)] + [be.upload(q) for q in w] + [be.alloc(m * n * 4) for _ in range(5)]
+    view = MatView(3 * k, m * k, k)
+    ls = [matmul_launch(fmt, m, n, k, inputs=(0, 2), output=5),
+          matmul_launch(fmt, m, n, k, inputs=(0, 3), output=6),
+          matmul_launch(fmt, m, n, k, inputs=(0, 2), output=7, a=view),   # rows 3.. of the same buffer
+          matmul_launch(fmt, m, k, k, inputs=(1, 4), output=0),           # overwrites the first 77 rows
+          matmul_launch(fmt, m, n, k, inputs=(0, 3), output=8),           # must see them
+          matmul_launch(fmt, m, n, k, inputs=(0, 2), output=9)]
+    be.prepare(ls)
+    counts, results = [], []
+    for reuse, one_list in (("0", False), ("0", True), ("1", True), ("1", True)):
+        be.set_option("act_reuse", reuse)
+        bufs[0].write(0, x)
+        be.take_launch_count()
+        for part in [ls] if one_list else [[l] for l in ls]:
+            be.execute(part, bufs)
+        counts.append(be.take_launch_count())
+        results.append([bufs[b].download().view(np.float32).copy() for b in (0, 5, 6, 7, 8, 9)])
+    be.set_option("act_reuse", "1")
+    assert all(np.array_equal(a, b) for other in results[1:] for a, b in zip(results[0], other))
+    assert not np.array_equal(results[0][2], results[0][4])   # (the rewritten operand gives something else)
+    assert counts[0] == counts[1] and counts[2] == counts[3] == counts[0] - 2   # launches 2 and 6 make no copy
 
 
 def test_gemm_f32_negative_zero(be, oracle):
