@@ -179,7 +179,9 @@ struct lapid_b200_device {
     uint32_t gemv_max_rows = 8;
     // Inside one execute list: kernels launched since the batched activation pre-pass at its head, -1 when the list
     // has none. Every kernel that waits for its predecessor lets its successor start only after that wait (the glue and
-    // pre-pass kernels and the decode kernels outside early mode issue launch_dependents behind their wait), so every kernel behind
+    // pre-pass kernels and the decode kernels outside early mode issue launch_dependents behind their wait; two more issue it first:
+    // qgemv_kq_finalize_kernel, which like an early kernel starts behind the first kernel of its list itself, and tp_all_reduce_kernel, which is in
+    // no list: behind it come a glue kernel or a pre-pass, which wait, or a first kernel launched fully serialised), so every kernel behind
     // the first of the list starts after the pre-pass has completed and may read its results before its own
     // dependency wait (GemvArgs::early).
     int after_hoist = -1;

@@ -255,7 +255,7 @@ bool rms_norm_shape_ok(uint32_t cols) { return cols >= 4 && cols % 4 == 0 && col
 
 static unsigned rms_norm_parts(uint32_t cols) { return cols >= 4096 ? 8 : cols >= 2048 ? 4 : cols >= 1024 ? 2 : 1; }
 
-// every CTA of the cluster gets whole 32-element groups, in whole blocks of the quantized layouts
+// every part of the row (a CTA of the tensor-parallel kernel) has whole 32-element groups, the row whole blocks of the quantized layouts
 bool rms_norm_quant_ok(uint32_t cols) { return rms_norm_shape_ok(cols) && cols % QK == 0 && (cols / 4) % (8 * rms_norm_parts(cols)) == 0; }
 
 cudaError_t launch_rms_norm(const RmsNormArgs &a, bool pdl, cudaStream_t stream) {

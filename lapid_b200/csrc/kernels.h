@@ -368,7 +368,7 @@ struct RmsNormArgs {
 };
 bool rms_norm_shape_ok(uint32_t cols);  // multiple of 4, at most 16384
 cudaError_t launch_rms_norm(const RmsNormArgs &args, bool pdl, cudaStream_t stream);
-bool rms_norm_quant_ok(uint32_t cols);  // the row splits over the cluster in whole 32-element groups
+bool rms_norm_quant_ok(uint32_t cols);  // the row's parts (CTAs of the tensor-parallel kernel) are whole 32-element groups
 // silu(gate) * up over [rows, cols] (q.qa set: also as a quantized activation operand; cols % 32 == 0)
 cudaError_t launch_silu_mul(const float *gate, const float *up, float *out, uint64_t n, uint32_t cols, const ActOut &q, int sm_count,
                             bool pdl, cudaStream_t stream);

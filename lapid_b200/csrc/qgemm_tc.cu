@@ -22,15 +22,16 @@
 //   warps 2-17 dequantize to bf16 into the 128-byte-swizzled K-major layout the tensor core reads.
 //              Q4_K: thread (row, half) expands one 32-element sub-block per k-step (NT = 1: warps
 //              2-9 the even k-steps, 10-17 the odd ones; NT = 2: the two groups own the two 128-row
-//              sub-tiles). Q6_K: 16 lanes share a row, lane = four weights. Afterwards warps 2-9
-//              (NT = 2: all) are the epilogue: `tcgen05.ld` 32 lanes x 32 columns at a time,
+//              sub-tiles). Q6_K: 16 lanes share a row, lane = four weights. Afterwards they
+//              are the epilogue: `tcgen05.ld` 32 lanes x 16 or 32 columns at a time,
 //              optional `+ extra`, coalesced f32 stores
 // The weight tile is the M side of the MMA and the activations the N side, so 64 prefill rows
 // use a 128x64 instruction at full rate instead of padding to 128 rows.
 // Tile shapes: NT = 2 at MT = 256 (two accumulators, all 512 columns of tensor memory) halves the
 // activation traffic per flop; MT = 512 with NT = 1 halves the dequantization per flop instead
 // (chosen for Q6_K by waves of tiles over the SMs). Launches with too few tiles for the SMs split K
-// over gridDim.z: partial tiles go to a scratch area and a second kernel sums them in order.
+// (the grid is one-dimensional: weight tiles, activation tiles, splits): partial tiles go to a scratch area and a second kernel
+// sums them in order.
 // PAIR (off by default): two CTAs of a cluster as one `cta_group::2` unit, each loading half of the
 // activation tile; measured slower than the single-CTA 256x256 tile.
 // Every mbarrier wait is bounded: a wait that gives up sets a bit in the host-visible status
@@ -365,7 +366,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (!healthy && lane == 0 && p.status) atomicOr(p.status, 32);
     } else if (warp == 18) {
         // ---------------- TMA producer, packed weights: one super-block of every row of the tile
-        // per copy, a whole super-block (four k-steps) ahead of the dequantizing warps
+        // per copy, up to RAWS super-blocks (of four k-steps) ahead of the dequantizing warps
         if (lane == 0) {
             uint32_t bc = 0;
             Tile o;
@@ -901,7 +902,7 @@ cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, 
             return cudaErrorInvalidValue;
     }
     // Too few tiles for the SMs (small n: a tensor-parallel shard, a few prefill rows on a narrow
-    // matrix): split K over gridDim.z, partial tiles into the scratch, summed in order by a second kernel.
+    // matrix): split K, partial tiles into the scratch, summed in order by a second kernel.
     const uint32_t ways = splitk_ways(a.rows, a.n, a.k, sm_count);
     if (ways > 1 && !pair) {
         GemmTcArgs b = a;

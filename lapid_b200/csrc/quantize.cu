@@ -17,7 +17,7 @@
 // (two separately rounded results in one instruction; only the running sums, whose order is fixed, stay scalar), the
 // level of an element as a float that never leaves the 2^23 offset domain (no integer conversions, which run at a quarter of the rate), everything in
 // registers. The levels of the best candidate are not kept: they are rarely needed, and the scale they came from gives them again.
-// 14336 x 4096: 899 us (Q4_K; scalar operations with the levels in local memory: 1336)
+// 14336 x 4096: 880 us (Q4_K; scalar operations with the levels in local memory: 1336)
 #include "common.cuh"
 #include "kernels.h"
 
