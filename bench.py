@@ -18,7 +18,9 @@ weights N(0, 0.02) quantized on the device by the library's own quantizer, activ
                kernel at M = 1 and the int8 tensor-core kernel at M >= 2): algorithmic bytes per
                launch / mean launch time over its cases, against the measured HBM copy bandwidth
   cpu_baseline the oracle's restatement of lapid-cpu's path, timed on this host's cores
-  cases        per (format, shape, M) GB/s, each timed alone over cold weight copies
+
+One more JSON object goes to stderr: ``cases`` (per format, shape and M GB/s, each timed alone over cold weight copies), ``prefill``,
+``matmul_id``, ``stack8b``, ``tp70b``, ``roofline_by_kernel`` and ``check`` in full.
 
 ``--impl reference`` times the CPU restatement of lapid-cpu's path (the reference itself is Rust
 and cannot be built where no Rust toolchain exists) on the same workload.
@@ -462,35 +464,37 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         "clocks": sampler.summary(),
         "e2e": {"value": e2e_val, "unit": "GB/s", "h2d_bytes_per_step": ao * 4, "d2h_bytes_per_step": oo * 4,
                 "ms_per_step": e2e_s * 1e3,
-                "calls_per_step": "one execute_io: 16 writes, 16 launches in " + (f"chunks of {args.e2e_chunk}" if args.e2e_chunk else "three chunks of about equal transfer bytes (the library's choice)") + ", 16 reads (a chunk's adjacent transfers go as one copy; "
-                                  "uploads, launches and downloads of different chunks overlap); waits",
+                "calls_per_step": "one execute_io: 16 writes, 16 launches in " + (f"chunks of {args.e2e_chunk}" if args.e2e_chunk else "chunks the library picks") + ", 16 reads; waits",
                 "three_calls": {"value": world * step_bytes / three_s / 1e9, "ms_per_step": three_s * 1e3,
-                                "calls_per_step": "write + execute(16 launches, waits) + download, one after the other"}},
+                                "calls_per_step": "write + execute + download, one after the other"}},
         "gpu_launches": launches_per_step * args.steps,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": roof_traffic, "peak_kind": peak_kind, "kernel": roof_kernel, "by_kernel": roof_detail,
-                     "what": "Q4_K decode launches of the kernel with the larger time share (act-quant pre-pass included): "
-                             "algorithmic bytes / mean launch time over its cases; traffic is MODELLED, not measured in this run: "
-                             "mean algorithmic bytes per launch x the DRAM-bytes / algorithmic-bytes ratio of the ncu capture "
-                             "summarised under profiles/ (null when that kernel has no capture)"},
+                     "traffic": roof_traffic, "peak_kind": peak_kind, "kernel": roof_kernel,
+                     "what": "algorithmic bytes / mean time of the kernel with the larger time share; traffic modelled from its ncu capture"},
     }
+    # The line has to be read whole by programs that keep only the end of a run's output: what goes beyond the headline is one JSON
+    # object of its own on stderr.
+    # roofline.what in full: Q4_K decode launches of the kernel with the larger time share (act-quant pre-pass included), algorithmic bytes /
+    # mean launch time over its cases; traffic = mean algorithmic bytes per launch x the DRAM-bytes / algorithmic-bytes ratio of
+    # the ncu capture summarised under profiles/ (null when that kernel has no capture), not measured in this run.
+    details = {"roofline_by_kernel": roof_detail}
     if world > 1 and isinstance(tp_obj, dict) and "decode_b1" in tp_obj:
         line["config"]["tp70b"] = {"decode_tok_s": tp_obj["decode_b1"]["tok_s"],
                                    "decode_frac_of_hbm_ceiling": tp_obj["decode_b1"].get("frac_of_hbm_ceiling"),
                                    "prefill_m512_tok_s": tp_obj.get("prefill_m512", {}).get("tok_s"),
                                    "prefill_collective_share": tp_obj.get("prefill_m512", {}).get("collective_share"),
                                    "note": "the headline value is a communication-free replica run; the tensor-parallel stack "
-                                           "with real exchanges is this object (details under tp70b)"}
+                                           "with real exchanges is this object (details under tp70b on stderr)"}
     if case_rows:
-        line["cases"] = case_rows
+        details["cases"] = case_rows
     if prefill_rows:
-        line["prefill"] = prefill_rows
+        details["prefill"] = prefill_rows
     if stack_obj:
-        line["stack8b"] = stack_obj
+        details["stack8b"] = stack_obj
     if moe_rows:
-        line["matmul_id"] = moe_rows
+        details["matmul_id"] = moe_rows
     if tp_obj:
-        line["tp70b"] = tp_obj
+        details["tp70b"] = tp_obj
     if check is not None:
         if prefill_rows:
             check["prefill"] = [r["check"] for r in prefill_rows if "check" in r]
@@ -501,9 +505,11 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         decode = [check[kk]["max_rel"] for kk in ("sweep", "e2e", "stack8b") if isinstance(check.get(kk), dict) and "max_rel" in check[kk]]
         check["decode_worst_max_rel"] = max(decode) if decode else None
         check["prefill_worst_rel_l2"] = max([c["rel_l2"] for c in check.get("prefill", [])], default=None)
-        line["check"] = check
+        details["check"] = check
+        line["check"] = {kk: check[kk] for kk in ("decode_worst_max_rel", "prefill_worst_rel_l2")}
     if world == 1 and not args.no_cpu:
         line["cpu_baseline"] = cpu_baseline(cases, fmt)
+    print(json.dumps(details), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
 
 
