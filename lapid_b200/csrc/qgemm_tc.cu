@@ -245,7 +245,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // The tiles of the launch: weight tile x (the fast index), activation tile y, split z of K. LOOP: a CTA takes every gridDim.x-th tile: no CTA
     // start, tensor-memory allocation and first trip to HBM per tile; the producers run ahead into the next tile, and its first
     // weights are dequantized before the results of the last one are stored. Expert-indexed launches, whose tiles are many and
-    // short, run this way (512 tokens, 8 of 128 experts of 768 x 2048: 130 -> 104 us a launch; a block of two layers 905 -> 754); the others have one tile per CTA (the
+    // short, run this way (512 tokens, 8 of 128 experts of 768 x 2048: 130 -> 104 us a launch; a block of two layers 905 -> 762); the others have one tile per CTA (the
     // loop's bookkeeping costs their dequantizing warps more than it saves: 77 rows on 14336 x 4096 39 us without, 47 with it).
     // Expert-indexed launch (Kernel::MatMulId, moe.cu): the activation tiles are runs of (token, slot)
     // pairs grouped by expert; the weights are the dense stack [experts * n, k], so a tile's weight
