@@ -343,6 +343,7 @@ struct ActSlot {
     static constexpr int TC_COPY = 3;
     size_t copy_offset = 0, written_before = 0;
     int owner = -1;
+    bool w_clean = false;  // no earlier launch of the list writes the launch's weights
     bool same(const ActSlot &o) const {
         return ptr == o.ptr && off == o.off && bs == o.bs && rs == o.rs && rows == o.rows && m == o.m && k == o.k &&
                records == o.records && a_type == o.a_type;
@@ -759,7 +760,7 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
     const uint32_t rows = route.max_tiles * route.mt;
     if (p.tc && lb::qgemm_tc_moe_supported(l.b_dtype, p.e, l.n, l.k, w->ptr) && p.wl.total == p.wl.qs_bytes) {
         void *a_bf16 = base + p.route_bytes;
-        cuda_check(lb::launch_moe_gather_bf16((const float *)x->ptr, route, (uint32_t)p.r, (uint32_t)l.k, a_bf16, dev.stream), "matmul_id gather launch");
+        cuda_check(lb::launch_moe_gather_bf16((const float *)x->ptr, route, (uint32_t)p.r, (uint32_t)l.k, a_bf16, dev.pdl, dev.stream), "matmul_id gather launch");
         lb::GemmTcArgs t{};
         t.w = (const uint8_t *)w->ptr;
         t.out = (float *)out->ptr;
@@ -770,7 +771,7 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         t.status = dev.status_dev;
         t.tile_expert = route.tile_expert;
         t.row_pair = route.row_pair;
-        cuda_check(lb::launch_qgemm_tc_moe(l.b_dtype, t, (uint32_t)p.e, p.mt, a_bf16, dev.sm_count, dev.stream), "matmul_id gemm launch");
+        cuda_check(lb::launch_qgemm_tc_moe(l.b_dtype, t, (uint32_t)p.e, p.mt, a_bf16, dev.sm_count, dev.pdl, dev.stream), "matmul_id gemm launch");
         dev.launches += 2;
         return;
     }
@@ -1018,8 +1019,11 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             if (slot) copy_at = slot->copy_offset, partial_at = slot->offset, made = slot - (slot->owner >= 0 ? slot->owner : 0);
             else dev.ensure_scratch(p.scratch);
             int launched = 0;
+            // Everything older than the kernel in front has completed when a kernel of this chain starts (each lets its successor start
+            // behind its own wait), so the weights may be read at once unless a launch of this list writes them.
+            t.w_early = slot && slot->w_clean;
             cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, (char *)dev.scratch + copy_at, !(made && made->done), (char *)dev.scratch + partial_at,
-                                           dev.sm_count, dev.stream, &launched), "qgemm_tc launch");
+                                           dev.sm_count, dev.pdl, dev.stream, &launched), "qgemm_tc launch");
             if (made) made->done = true;
             dev.launches += launched;
             expr_pass();
@@ -1165,6 +1169,11 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
                 }
                 sl.records = ActSlot::TC_COPY;
                 sl.written_before = written.size();
+                if (lapid_b200_buffer *wb = l.n_inputs > 1 && l.inputs[1] < nbuf ? buffers[l.inputs[1]] : nullptr) {
+                    sl.w_clean = true;
+                    for (const Range &w : written)
+                        if ((const char *)wb->ptr < w.hi && w.lo < (const char *)wb->ptr + wb->bytes) sl.w_clean = false;
+                }
                 // the copy an earlier launch of the list makes of the same operand (q, k, v; gate, up), as long as nothing since has written
                 // the buffer it comes from
                 for (size_t s2 = slots.size(); s2-- > 0 && ab && dev->act_reuse;) {
@@ -1637,14 +1646,12 @@ lapid_b200_status lapid_b200_device_set_option(lapid_b200_device *dev, const cha
             lb::qgemv_iq_set_rows_per_warp(std::atoi(value));
         } else if (k == "gemv_ctas_per_sm") {
             lb::qgemv_q4k_fast_set_cta_cap(std::atoi(value));
-        } else if (k == "gemm_wide") {
-            lb::qgemm_tc_set_wide(std::atoi(value));
+        } else if (k == "gemm_wide" || k == "gemm_tall") {
+            // accepted, without effect: the tile shapes these chose between are one shape now
         } else if (k == "gemm_splitk") {
             lb::qgemm_tc_set_splitk(std::atoi(value));
         } else if (k == "gemm_pair") {
             lb::qgemm_tc_set_pair(std::atoi(value));
-        } else if (k == "gemm_tall") {
-            lb::qgemm_tc_set_tall(std::atoi(value));
         } else if (k == "gemm") {
             if (v == "f32") dev->gemm_f32 = true;
             else if (v == "tc") dev->gemm_f32 = false;

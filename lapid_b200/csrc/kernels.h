@@ -316,7 +316,8 @@ struct GemmTcArgs {
     uint32_t rows, m, n, k;
     int *status;
     float *partial;  // split-K launches: [splits][rows][n] partial sums in the scratch; nullptr otherwise
-    uint32_t tiles_x, tiles_y, splits;  // set by the launcher
+    bool w_early;    // under programmatic dependent launch the weights may be read before the kernel in front has completed
+    uint32_t tiles_x, tiles_y, splits, full, units, mt, group;  // set by the launcher
     // Expert-indexed launches (launch_qgemm_tc_moe): rows = the tile space, n = rows of ONE expert's matrix
     const int32_t *tile_expert;  // nullptr for an ordinary launch
     const int32_t *row_pair;
@@ -327,15 +328,12 @@ size_t qgemm_tc_partial_bytes(uint32_t rows, uint32_t n, uint32_t k, int sm_coun
 void qgemm_tc_set_splitk(int v);  // tuning: -1 choose, 0 / 1 never, n > 1 always n ways
 // copy: make the bf16 copy first (false: an earlier launch of the same call has made it).
 cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &args, void *a_bf16_scratch, bool copy, void *partial, int sm_count,
-                            cudaStream_t stream, int *launched);
+                            bool pdl, cudaStream_t stream, int *launched);
 // Kernel::MatMulId on the tensor cores: `a_bf16` holds the activation rows in tile-space order (moe.cu), the
 // weights are a dense stack of `experts` matrices [n, k] (no padding between them), mt in {64, 128, 256}.
 bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, const void *w);
-cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &args, uint32_t experts, uint32_t mt, void *a_bf16, int sm_count, cudaStream_t stream);
-void qgemm_tc_set_wide(int v);  // tuning: -1 choose, 0 / 1 force one / two accumulators per CTA
-void qgemm_tc_set_pair(int v);  // tuning: 1 = CTA pairs (cta_group::2) for the two-accumulator Q4_K tile
-void qgemm_tc_set_tall(int v);  // tuning: -1 choose, 0 / 1 never / always 512 activation rows per CTA above 256 rows
-
+cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &args, uint32_t experts, uint32_t mt, void *a_bf16, int sm_count, bool pdl, cudaStream_t stream);
+void qgemm_tc_set_pair(int v);  // tuning: -1 choose, 0 never: CTA pairs (cta_group::2)
 
 // ---- moe.cu: device-side grouping of (token, slot) pairs by expert for Kernel::MatMulId
 struct MoeRouteArgs {
@@ -350,7 +348,7 @@ uint32_t moe_max_tiles(uint64_t pairs, uint64_t experts, uint32_t mt);
 size_t moe_route_bytes(uint64_t pairs, uint64_t experts, uint32_t mt);
 void moe_route_layout(void *scratch, uint64_t pairs, uint64_t experts, uint32_t mt, MoeRouteArgs &args);  // fills all but ids and status
 cudaError_t launch_moe_route(const MoeRouteArgs &args, bool pdl, cudaStream_t stream);
-cudaError_t launch_moe_gather_bf16(const float *x, const MoeRouteArgs &route, uint32_t r, uint32_t k, void *dst, cudaStream_t stream);
+cudaError_t launch_moe_gather_bf16(const float *x, const MoeRouteArgs &route, uint32_t r, uint32_t k, void *dst, bool pdl, cudaStream_t stream);
 
 // ---- glue.cu: the row / elementwise steps between the projections of a layer (not on the matmul path)
 struct RmsNormArgs {

@@ -77,12 +77,13 @@ __global__ void __launch_bounds__(ROUTE_THREADS) moe_route_kernel(MoeRouteArgs a
 }
 
 // bf16 copy of the activation rows in tile-space order (the tensor-core kernel's A operand):
-// row i of dst = x[row_pair[i] / r], zeros for a padding row. blockIdx.y walks the rows.
+// row i = x[row_pair[i] / r], zeros for a padding row, laid out [k / 64][rows][64] as qgemm_tc.cu wants it. blockIdx.y walks the rows.
 __global__ void __launch_bounds__(256) moe_gather_bf16_kernel(const float *x, const int32_t *row_pair, uint32_t r, uint32_t k,
                                                               uint32_t rows, __nv_bfloat16 *dst) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (uint32_t row = blockIdx.y; row < rows; row += gridDim.y) {
         const int32_t pair = row_pair[row];
-        uint4 *out = (uint4 *)(dst + (size_t)row * k);
         const float4 *src = pair < 0 ? nullptr : (const float4 *)(x + (size_t)((uint32_t)pair / r) * k);
         for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < k / 8; c8 += gridDim.x * blockDim.x) {
             __nv_bfloat162 o[4];
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(256) moe_gather_bf16_kernel(const float *x, co
             } else {
                 o[0] = o[1] = o[2] = o[3] = __floats2bfloat162_rn(0.0f, 0.0f);
             }
-            out[c8] = *(const uint4 *)o;
+            ((uint4 *)dst)[((size_t)(c8 / 8) * rows + row) * 8 + c8 % 8] = *(const uint4 *)o;
         }
     }
 }
@@ -136,13 +137,20 @@ cudaError_t launch_moe_route(const MoeRouteArgs &a, bool pdl, cudaStream_t strea
     return cudaLaunchKernelEx(&cfg, moe_route_kernel, a);
 }
 
-cudaError_t launch_moe_gather_bf16(const float *x, const MoeRouteArgs &a, uint32_t r, uint32_t k, void *dst, cudaStream_t stream) {
+cudaError_t launch_moe_gather_bf16(const float *x, const MoeRouteArgs &a, uint32_t r, uint32_t k, void *dst, bool pdl, cudaStream_t stream) {
     const uint32_t rows = a.max_tiles * a.mt;
     if (rows == 0) return cudaSuccess;
     if (k % 8 != 0 || ((uintptr_t)x & 15) != 0) return cudaErrorInvalidValue;
-    const dim3 grid((k / 8 + 255) / 256, rows < 65535u ? rows : 65535u);
-    moe_gather_bf16_kernel<<<grid, 256, 0, stream>>>(x, a.row_pair, r, k, rows, (__nv_bfloat16 *)dst);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((k / 8 + 255) / 256, rows < 65535u ? rows : 65535u);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, moe_gather_bf16_kernel, x, (const int32_t *)a.row_pair, r, k, rows, (__nv_bfloat16 *)dst);
 }
 
 }  // namespace lb

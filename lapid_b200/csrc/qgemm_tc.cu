@@ -1,5 +1,5 @@
 // Prefill GEMM on the 5th-generation tensor cores: out[m, n] = sum_k A[m, k] * dequant(W)[n, k] for
-// Q4_K and Q6_K weights, bf16 operands, f32 accumulation in tensor memory.
+// Q4_K, Q5_K and Q6_K weights, bf16 operands, f32 accumulation in tensor memory.
 //
 // Reference semantics: lapid-cpu's path for more than 8 rows multiplies f32 activations by the
 // dequantized f32 weights (crates/lapid-cpu/src/matmul/qdeq.rs:57-123); lapid-cuda's tensor-core
@@ -9,31 +9,35 @@
 // f32, so the result differs from the f32 reference by the operand rounding only (2^-9 relative
 // per operand).
 //
-// One CTA computes a 128*NT (weight rows) x MT (activation rows, 64/128/256/512) output tile, K in
-// steps of 64 (one Q4_K "pair": 32 bytes of quants = two 32-element sub-blocks):
-//   warp 0     one lane drives TMA for the activations: per k-step a 128-byte swizzled 2-D copy
-//              of the bf16 activation tile (`cp.async.bulk.tensor.2d`, each CTA loads its own copy)
-//   warp 18    one lane drives TMA for the weights: per super-block a 2-D tensor-map copy of the
-//              tile rows' packed blocks (144 bytes; Q6_K: 224 bytes around the 2-byte aligned 210),
-//              up to five super-blocks ahead of its consumers; Q6_K rows that are not 16-byte multiples
-//              are copied row by row with the plain bulk copy by all lanes of the warp
-//   warp 1     allocates tensor memory; one lane issues `tcgen05.mma` (M=128, N=MT, K=16, four
-//              per k-step and accumulator) on shared-memory descriptors and commits to mbarriers
-//   warps 2-17 dequantize to bf16 into the 128-byte-swizzled K-major layout the tensor core reads.
-//              Q4_K: thread (row, half) expands one 32-element sub-block per k-step (NT = 1: warps
-//              2-9 the even k-steps, 10-17 the odd ones; NT = 2: the two groups own the two 128-row
-//              sub-tiles). Q6_K: 16 lanes share a row, lane = four weights. Afterwards they
-//              are the epilogue: `tcgen05.ld` 32 lanes x 16 or 32 columns at a time,
-//              optional `+ extra`, coalesced f32 stores
-// The weight tile is the M side of the MMA and the activations the N side, so 64 prefill rows
-// use a 128x64 instruction at full rate instead of padding to 128 rows.
-// Tile shapes: NT = 2 at MT = 256 (two accumulators, all 512 columns of tensor memory) halves the
-// activation traffic per flop; MT = 512 with NT = 1 halves the dequantization per flop instead
-// (chosen for Q6_K by waves of tiles over the SMs). Launches with too few tiles for the SMs split K
-// (the grid is one-dimensional: weight tiles, activation tiles, splits): partial tiles go to a scratch area and a second kernel
-// sums them in order.
-// PAIR (off by default): two CTAs of a cluster as one `cta_group::2` unit, each loading half of the
-// activation tile; measured slower than the single-CTA 256x256 tile.
+// The weights are the M side of the instruction, the activations the N side, so a tile has as many columns as the launch
+// has rows (in steps of 16) and nothing is padded to 128. What bounds the kernel is the expansion of the packed weights
+// (integer instructions, about 1.7 a weight for Q4_K) against the tensor pipe, so:
+//   - an expanded weight goes from registers straight into tensor memory (`tcgen05.st`, the A operand of the instruction may
+//     lie there): lane = weight row, 64 k = 32 columns. Shared memory then only carries the activations and the packed
+//     blocks; as bf16 in shared memory the weights were written and read through the same 128 bytes a cycle that the
+//     activations need.
+//   - a thread owns one row and 64 of a super-block's 256 k: one look at the header's scales for 64 weights, no partner.
+//   - above 128 rows two CTAs of a cluster are one `cta_group::2` unit: 256 weight rows (each CTA expands its own 128) by up
+//     to 256 activation rows, of which each CTA loads half: an expanded weight feeds 256 columns, an activation 256 rows.
+//
+// Roles of a CTA's 19 warps:
+//   warps 0-15 expand: warp (quarter of the rows, j) writes the 64 k at 64 j of every super-block into its half of a stage of tensor
+//              memory. They are also the epilogue: the accumulator is given back once its columns are in registers, and
+//              the stores run beside the next tile's first products.
+//   warp 16    one lane drives TMA for the activations: a 128-byte swizzled copy of the tile's rows for two k-steps of 64 at a time
+//   warp 17    allocates tensor memory; one lane issues `tcgen05.mma` (A in tensor memory, B by shared-memory descriptor; four
+//              K=16 steps per k-step) and commits to mbarriers
+//   warp 18    one lane drives TMA for the weights: per super-block a 2-D tensor-map copy of the 128 rows' packed blocks
+//              (144 / 176 bytes; Q6_K: 240 bytes from the 16-byte boundary below the 2-byte aligned 210); Q6_K rows
+//              that are not 16-byte multiples are copied row by row with the plain bulk copy by all lanes of the warp
+// A CTA (pair) takes every gridDim-th unit of the launch: no CTA start and no first trip to HBM per tile, and the first two
+// super-blocks of a tile are expanded before the results of the one before are stored. Tensor memory: 256 columns of accumulators
+// (one 256-column set for a pair, two of 128 for a single CTA), 4 stages of 64 columns (two k-steps) of weights.
+// Units: whole tiles as long as they fill every CTA, and where the last round would leave SMs idle its tiles are split over K
+// (tc_plan() below); the partial tiles of those go to a scratch area and a second kernel sums them in order.
+//
+// Programmatic dependent launch: barriers, tensor memory and the packed weights come before `griddepcontrol.wait`; only what
+// the kernel in front may have written (activations, expert tables, epilogue terms) and all stores come behind it.
 // Every mbarrier wait is bounded: a wait that gives up sets a bit in the host-visible status
 // word, the roles fall through to the end, tensor memory is released and the kernel returns.
 #include <cuda.h>
@@ -48,37 +52,27 @@ namespace lb {
 
 namespace tc {
 
-constexpr int TN = 128;            // weight rows per tile
-constexpr int KS = 64;             // k per stage
-constexpr int Q6K_BOX = 224;       // Q6_K: bytes staged per row and super-block (210 from a 2-byte aligned start, see below)
-constexpr int B_BYTES = TN * 128;  // bf16 weight tile of one stage
-constexpr int THREADS = 608;       // 19 warps
-constexpr int DEQ_WARPS = 16;      // two groups of eight: even and odd k-steps
-constexpr int GROUP_WARPS = 8;
-constexpr uint32_t SPIN_LIMIT = 1u << 24;
+constexpr int TN = 128;            // weight rows per CTA
+constexpr int KS = 64;             // k per k-step: 128 bytes of bf16, the width of a swizzled row
+constexpr int STAGE_KS = 2;        // k-steps per stage: half a super-block (one k-step per stage: the waits and commits of the issuing warp took as long as the products)
+constexpr int STAGES = 4;          // two super-blocks in flight
+constexpr int Q6K_BOX = 240;       // Q6_K: bytes staged per row and super-block (210 from a 2-byte aligned start; an odd number of 16-byte chunks keeps 128-bit row loads free of bank conflicts)
+constexpr int DEQ_WARPS = 16;
+constexpr int ACT_WARP = DEQ_WARPS, MMA_WARP = DEQ_WARPS + 1, RAW_WARP = DEQ_WARPS + 2;
+constexpr int THREADS = 32 * (DEQ_WARPS + 3);
+constexpr int A_COL = 256;         // tensor-memory column of the first weight stage
+constexpr uint32_t SPIN_LIMIT = 1u << 22;
 
-// MT activation rows x (NT * 128) weight rows per CTA. NT = 2 keeps two accumulators (all 512
-// columns of tensor memory at MT = 256) so that one activation tile feeds twice the weights: the
-// bf16 activation tile is the larger part of what an SM pulls from L2 per k-step.
-// PAIR: two CTAs of a cluster run as one `cta_group::2` tensor-core unit: each dequantizes its own
-// 128*NT weight rows and loads only HALF of the activation tile (the instruction reads both CTAs'
-// halves), which halves the activation traffic from L2 and leaves room for a third stage.
-template <int FMT, int MT, int NT, bool PAIR = false, bool LOOP = false> struct Cfg {
-    static constexpr int STAGES = PAIR ? 3 : ((NT == 2 || MT == 512) ? 2 : (MT == 256 ? 3 : 4));
-    static constexpr int A_BYTES = (PAIR ? MT / 2 : MT) * 128;
-    static constexpr int W_BYTES = NT * B_BYTES;
-    static constexpr int STAGE_BYTES = W_BYTES + A_BYTES;
+template <int FMT, bool PAIR> struct Cfg {
+    static constexpr int MT = PAIR ? 256 : 128;  // most activation rows of a tile
+    static constexpr int ACCS = PAIR ? 1 : 2;    // accumulator sets of MT columns
+    static constexpr int A_BYTES = STAGE_KS * 128 * 128;  // activations of one stage in this CTA: up to 128 rows of 64 bf16, twice
     static constexpr int ROW_BYTES = FMT == FMT_Q4K ? Q4K_BYTES : FMT == FMT_Q5K ? Q5K_BYTES : Q6K_BOX;  // packed bytes staged per row and super-block
-    static constexpr int RAW_BYTES = TN * ROW_BYTES;                         // one 128-row sub-tile: 18432 / 28672
-    static constexpr int RAW = NT * RAW_BYTES;
-    // Super-blocks of packed weights in flight or in use: as many as the shared memory has room for, at most six. With two, a refill from
-    // HBM had only the few k-steps of one super-block to arrive in (together with the shared bf16 copy: a prompt of 77 rows
-    // through 8 layers 1902 -> 1779 us).
-    static constexpr int RAW_FIT = (227 * 1024 - 256 - 1024 - STAGES * STAGE_BYTES) / RAW;
-    static constexpr int RAWS = RAW_FIT > 6 ? 6 : RAW_FIT;
-    static_assert(RAWS >= 2, "shared memory");
-    static constexpr int ACCS = LOOP && 2 * MT * NT <= 512 ? 2 : 1;  // accumulator sets: two where the 512 columns of tensor memory hold them
-    static constexpr int SMEM = STAGES * STAGE_BYTES + RAWS * RAW + 256 /*barriers*/ + 1024 /*alignment slack*/;
+    static constexpr int RAW = TN * ROW_BYTES;
+    // Super-blocks of packed weights in flight or in use: as many as the shared memory has room for (5 / 4 / 3)
+    static constexpr int RAWS = (227 * 1024 - 512 - 1024 - STAGES * A_BYTES) / RAW;
+    static_assert(RAWS >= 3 && 3 * STAGES + 2 * RAWS + 5 <= 64, "shared memory");
+    static constexpr int SMEM = STAGES * A_BYTES + RAWS * RAW + 512 /*barriers*/ + 1024 /*alignment slack*/;
 };
 
 __device__ __forceinline__ uint32_t s32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -92,7 +86,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s32(bar)) : "memory");
 }
 // Bounded wait. A waiter that is not on the critical path sleeps between polls so that it does not
-// take issue slots from the dequantizing warps.
+// take issue slots from the expanding warps.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t sleep_ns = 0) {
     for (uint32_t spin = 0; spin < SPIN_LIMIT; spin++) {
         uint32_t ok;
@@ -106,6 +100,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
     }
     return false;
 }
+
+// A whole warp waits: all lanes or none give up.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
 // Two f32 lanes in one 64-bit register pair: Blackwell's packed f32 pipe halves the instruction
 // count of the dequantization.
@@ -143,31 +140,38 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
                  "l"((uint64_t)map), "r"(x), "r"(y), "r"(s32(bar))
                  : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                     s32(dst)),
+                 "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(s32(bar))
+                 : "memory");
+}
 
 // K-major operand, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
+// D[tmem] (+)= A[tmem] * B[smem]: PAIR: the unit of both CTAs, each holding its own 128 rows of A and D and half the rows of B
+template <bool PAIR> __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar)) : "memory");
-}
-// ---- the same for a pair of CTAs (`cta_group::2`); `cluster_addr` may name a barrier of either CTA
-__device__ __forceinline__ void mma_bf16_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit_pair(uint32_t cluster_addr) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr) : "memory");
+// arrival on the barrier (PAIR: on the barrier at the same place of both CTAs) when the products issued so far are done
+template <bool PAIR> __device__ __forceinline__ void mma_commit(uint64_t *bar) {
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(s32(bar)), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar)) : "memory");
 }
 // the shared::cluster address of `p` in CTA `rank` of this cluster
 __device__ __forceinline__ uint32_t cluster_addr_of(const void *p, uint32_t rank) {
@@ -175,11 +179,14 @@ __device__ __forceinline__ uint32_t cluster_addr_of(const void *p, uint32_t rank
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(s32(p)), "r"(rank));
     return r;
 }
+// Arrival on a barrier of either CTA. What it reports was complete before (tensor-memory stores that `tcgen05.wait::st` has waited for,
+// copies whose barrier has completed), so it carries no cluster-wide release: that one waits for every store of the thread and
+// took 1100 to 1500 cycles an arrival.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// bounded wait with cluster-scope acquire: the arrival comes from the other CTA of the pair
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, uint32_t sleep_ns = 0) {
+// bounded wait with cluster-scope acquire: arrivals may come from the other CTA of the pair
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity) {
     for (uint32_t spin = 0; spin < SPIN_LIMIT; spin++) {
         uint32_t ok;
         asm volatile(
@@ -188,7 +195,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
             : "r"(s32(bar)), "r"(parity)
             : "memory");
         if (ok) return true;
-        if (sleep_ns) __nanosleep(sleep_ns);
     }
     return false;
 }
@@ -196,86 +202,230 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-
-// N consecutive columns of this warp's 32 lanes of tensor memory
-template <int N> __device__ __forceinline__ void tmem_ld(uint32_t (&r)[N], uint32_t addr) {
-    static_assert(N == 16 || N == 32, "columns");
-    if constexpr (N == 32)
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-              "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-              "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(addr)
-            : "memory");
-    else
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(addr)
-            : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
 }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// 16 consecutive columns of this warp's 32 lanes of tensor memory (not waited for: tmem_ld_wait)
+__device__ __forceinline__ void tmem_ld16(uint32_t *r, uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// 16 columns of this warp's 32 lanes (not waited for: tmem_st_wait)
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]), "r"(r[1]),
+        "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+        "r"(r[14]), "r"(r[15]), "r"(addr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // f32 bits of (2^23 + byte `sel` of w): the byte planted in the mantissa by one PRMT
 __device__ __forceinline__ float biased(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)); }
+// 2^23 + (w & mask): a nibble planted where it lies (mask within the 23 bits of the mantissa): 2^p times its value, p = its lowest bit
+// (one three-input logic operation: the exponent comes in a register, since of two constants the instruction encodes one)
+template <uint32_t MASK> __device__ __forceinline__ float planted(uint32_t w, uint32_t exponent) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(exponent));
+    return __uint_as_float(r);
+}
+__device__ __forceinline__ uint32_t planted_exponent() {
+    uint32_t r;
+    asm volatile("mov.b32 %0, 0x4B000000;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint64_t unbias2(float a, float b) { return add2(pack2(a, b), pack2(-8388608.0f, -8388608.0f)); }
+__device__ __forceinline__ uint32_t rot(uint32_t v, uint32_t by) { return __funnelshift_l(v, v, by); }
 
-template <int FMT, int MT, int NT, bool PAIR, bool LOOP>
+// ---- expansion of one thread's share of a super-block: row = its lane, k = 64 j .. 64 j + 63, in two halves of 32 weights (16 registers of
+// two bf16 each, k ascending). The words it needs are loaded a super-block ahead.
+//
+// Q4_K / Q5_K (crates/lapid-quant/src/kquant.rs:337-373): byte l of the 32 bytes at 32 j holds element 64 j + l in its low and 64 j + 32 + l
+// in its high nibble; scales and mins of sub-blocks 2 j and 2 j + 1. Q5_K: bit s of qh[l] belongs to element 32 s + l.
+// Q6_K (:375-396): ql[128] | qh[64] | int8 sc[16] | f16 d. k-step j: half nh = j >> 1 of the 256, nibble hi = j & 1; the first 32 weights from
+// ql[64 nh + l], the second 32 from ql[64 nh + 32 + l]; the two high bits from qh[32 nh + l] >> 2 (2 hi + h); scale
+// sc[8 nh + 2 (2 hi + h) + l / 16].
+template <int FMT> struct Packed {
+    uint4 h;
+    uint32_t w[8], x[FMT == FMT_Q5K ? 8 : 1];
+};
+template <> struct Packed<FMT_Q6K> {
+    uint32_t wl[16], wh[8], sc, d;
+};
+template <int FMT> __device__ __forceinline__ void load_packed(Packed<FMT> &r, const uint8_t *blk, uint32_t j) {
+    constexpr int QS = FMT == FMT_Q5K ? 48 : 16;
+    r.h = *(const uint4 *)blk;
+    *(uint4 *)r.w = *(const uint4 *)(blk + QS + 32 * j);
+    *(uint4 *)(r.w + 4) = *(const uint4 *)(blk + QS + 16 + 32 * j);
+    if constexpr (FMT == FMT_Q5K) {
+        *(uint4 *)r.x = *(const uint4 *)(blk + 16);
+        *(uint4 *)(r.x + 4) = *(const uint4 *)(blk + 32);
+    }
+}
+// 16 + 8 words of a Q6_K block's ql and qh from 128-bit chunks of its staged row; the block starts 4 WS (+ 2: sh = 16) bytes behind a chunk boundary
+template <int WS> __device__ __forceinline__ void q6k_words(const uint8_t *row, uint32_t nh, uint32_t sh, uint32_t (&wl)[16], uint32_t (&wh)[8]) {
+    uint32_t t[20];
+#pragma unroll
+    for (int c = 0; c < 5; c++) *(uint4 *)(t + 4 * c) = *(const uint4 *)(row + 64 * nh + 16 * c);
+#pragma unroll
+    for (int i = 0; i < 16; i++) wl[i] = __funnelshift_r(t[i + WS], t[i + WS + 1], sh);
+#pragma unroll
+    for (int c = 0; c < 3; c++) *(uint4 *)(t + 4 * c) = *(const uint4 *)(row + 128 + 32 * nh + 16 * c);
+#pragma unroll
+    for (int i = 0; i < 8; i++) wh[i] = __funnelshift_r(t[i + WS], t[i + WS + 1], sh);
+}
+// `skew`: where the block starts in its staged row; `uniform`: the same for every row of the matrix
+__device__ __forceinline__ void load_packed_q6(Packed<FMT_Q6K> &r, const uint8_t *row, uint32_t skew, bool uniform, uint32_t j) {
+    const uint32_t nh = j >> 1, hi = j & 1, sh = 8 * (skew & 2);
+    if (uniform) {
+        switch (skew >> 2) {
+            case 0: q6k_words<0>(row, nh, sh, r.wl, r.wh); break;
+            case 1: q6k_words<1>(row, nh, sh, r.wl, r.wh); break;
+            case 2: q6k_words<2>(row, nh, sh, r.wl, r.wh); break;
+            default: q6k_words<3>(row, nh, sh, r.wl, r.wh); break;
+        }
+    } else {
+        const uint32_t *a = (const uint32_t *)(row + (skew & ~3u) + 64 * nh), *c = (const uint32_t *)(row + (skew & ~3u) + 128 + 32 * nh);
+        uint32_t prev = a[0];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const uint32_t next = a[i + 1];
+            r.wl[i] = __funnelshift_r(prev, next, sh);
+            prev = next;
+        }
+        prev = c[0];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t next = c[i + 1];
+            r.wh[i] = __funnelshift_r(prev, next, sh);
+            prev = next;
+        }
+    }
+    const uint16_t *scp = (const uint16_t *)(row + skew + 192 + 8 * nh + 4 * hi);
+    r.sc = (uint32_t)scp[0] | ((uint32_t)scp[1] << 16);
+    r.d = *(const uint16_t *)(row + skew + 208);
+}
+// d * byte `sel` of w, exactly: d (2^23 + b) - d 2^23 has one rounding, and d b (11 x 8 bits) needs none
+__device__ __forceinline__ float scaled(float d, uint32_t w, uint32_t sel, float neg_d23) { return fmaf(d, biased(w, sel), neg_d23); }
+// half H (0: the first 32 weights) of the share
+template <int FMT, int H> __device__ __forceinline__ void expand(const Packed<FMT> &r, uint32_t j, uint32_t e23, uint32_t (&o)[16]) {
+    if constexpr (FMT == FMT_Q6K) {
+        const float d = half_bits_to_float(r.d);
+        const uint32_t hi = j & 1, up = (4 - 4 * hi - 2 * H) & 31;  // rotation that brings the two high bits of every byte to bits 4 and 5
+        const uint32_t sb = r.sc ^ 0x80808080u;                      // scales + 128
+        const float nd = d * -8388608.0f;
+        // d * sc (11 x 8 bits) and d * sc * (q - 32) are exact in f32
+        const float sd[2] = {fmaf(-128.0f, d, scaled(d, sb, 0x7440u + 2 * H, nd)), fmaf(-128.0f, d, scaled(d, sb, 0x7441u + 2 * H, nd))};
+        const uint64_t unbias32 = pack2(-8388640.0f, -8388640.0f);   // -(2^23 + 32)
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t q = ((r.wl[8 * H + i] >> (4 * hi)) & 0x0F0F0F0Fu) | (rot(r.wh[i], up) & 0x30303030u);
+            const uint64_t s2 = pack2(sd[i >> 2], sd[i >> 2]);
+            o[2 * i] = to_bf16x2(mul2(s2, add2(pack2(biased(q, 0x7440u), biased(q, 0x7441u)), unbias32)));
+            o[2 * i + 1] = to_bf16x2(mul2(s2, add2(pack2(biased(q, 0x7442u), biased(q, 0x7443u)), unbias32)));
+        }
+    } else {
+        // the two 6-bit scales in bytes 0 and 1 of sc, the mins in mn (scale_min_pair's layout)
+        const uint32_t sh = 16 * (j & 1);
+        const uint32_t w0 = r.h.y >> sh, w1 = r.h.z >> sh, w2 = r.h.w >> sh;
+        const uint32_t sc = j < 2 ? w0 & 0x3F3Fu : (w2 & 0x0F0Fu) | ((w0 >> 2) & 0x3030u);
+        const uint32_t mn = j < 2 ? w1 & 0x3F3Fu : ((w2 >> 4) & 0x0F0Fu) | ((w1 >> 2) & 0x3030u);
+        const float d = half_bits_to_float(r.h.x & 0xffff), dmin = half_bits_to_float(r.h.x >> 16);
+        const float s = scaled(d, sc, 0x7440u + H, d * -8388608.0f), m = -scaled(dmin, mn, 0x7440u + H, dmin * -8388608.0f);
+        const uint64_t nm = pack2(m, m);
+        if constexpr (FMT == FMT_Q4K) {
+            // Each nibble is planted where it lies, which costs one logic operation a weight and one shift for four; its power of two
+            // goes into the multiplier, so y = sc q - m still has one rounding and the bits of the plain form.
+            constexpr float P4 = 0x1p-4f, P8 = 0x1p-8f, P12 = 0x1p-12f, P16 = 0x1p-16f;
+            const uint64_t s01 = H ? pack2(s * P4, s * P12) : pack2(s, s * P8), s23 = H ? pack2(s * P8, s * P16) : pack2(s * P16, s * P12);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t v = r.w[i] >> 12;  // byte 2's high nibble at bit 8, byte 3's at 12 and 16
+                o[2 * i] = to_bf16x2(fma2(s01, unbias2(planted<H ? 0xF0u : 0xFu>(r.w[i], e23), planted<H ? 0xF000u : 0xF00u>(r.w[i], e23)), nm));
+                o[2 * i + 1] = to_bf16x2(fma2(s23, unbias2(planted<H ? 0xF00u : 0xF0000u>(H ? v : r.w[i], e23), planted<H ? 0xF0000u : 0xF000u>(v, e23)), nm));
+            }
+        } else {
+            const uint64_t s2 = pack2(s, s);
+            const uint32_t up = (4 - 2 * j - H) & 31;  // rotation that brings bit 2 j + H of every byte to bit 4
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t a = ((H ? r.w[i] >> 4 : r.w[i]) & 0x0F0F0F0Fu) | (rot(r.x[i], up) & 0x10101010u);
+                o[2 * i] = to_bf16x2(fma2(s2, unbias2(biased(a, 0x7440u), biased(a, 0x7441u)), nm));
+                o[2 * i + 1] = to_bf16x2(fma2(s2, unbias2(biased(a, 0x7442u), biased(a, 0x7443u)), nm));
+            }
+        }
+    }
+}
+
+// One unit of work: a tile of 128 (PAIR: 256) weight rows x mt activation rows and the super-blocks [kb0, kb0 + nblk) of K.
+struct Tile {
+    uint32_t n0, m0, wrow0, kb0, nblk;
+    int32_t part;  // -1: the tile's results; else which partial tile
+};
+
+template <int FMT, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, GemmTcArgs p) {
-    using C = Cfg<FMT, MT, NT, PAIR, LOOP>;
-    constexpr int RAW_BYTES = C::RAW_BYTES;
+    using C = Cfg<FMT, PAIR>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *stage0 = smem;
-    uint8_t *raw0 = smem + C::STAGES * C::STAGE_BYTES;
+    uint8_t *raw0 = smem + STAGES * C::A_BYTES;
     uint64_t *bars = (uint64_t *)(raw0 + C::RAWS * C::RAW);
-    uint64_t *full_a = bars, *full_b = bars + C::STAGES, *empty = bars + 2 * C::STAGES;
-    uint64_t *raw_full = bars + 3 * C::STAGES, *raw_empty = raw_full + C::RAWS, *acc_full = raw_full + 2 * C::RAWS;
-    uint64_t *acc_empty = acc_full + 2;
-    uint32_t *tmem_slot = (uint32_t *)(acc_full + 4);
-    uint64_t *peer_ready = acc_full + 5;  // PAIR, leader CTA: the other CTA's operands of a stage are in place
-    uint32_t cta_rank = 0;
-    if constexpr (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta_rank));
+    uint64_t *full_a = bars, *full_w = bars + STAGES, *empty = bars + 2 * STAGES;  // activations, weights in place; stage read by the tensor cores
+    uint64_t *raw_full = bars + 3 * STAGES, *raw_empty = raw_full + C::RAWS;
+    uint64_t *acc_full = raw_empty + C::RAWS, *acc_empty = acc_full + 2;
+    uint32_t *tmem_slot = (uint32_t *)(acc_empty + 2);
+    uint32_t rank = 0;
+    if constexpr (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // The tiles of the launch: weight tile x (the fast index), activation tile y, split z of K. LOOP: a CTA takes every gridDim.x-th tile: no CTA
-    // start, tensor-memory allocation and first trip to HBM per tile; the producers run ahead into the next tile, and its first
-    // weights are dequantized before the results of the last one are stored. Expert-indexed launches, whose tiles are many and
-    // short, run this way (512 tokens, 8 of 128 experts of 768 x 2048: 130 -> 104 us a launch; a block of two layers 905 -> 762); the others have one tile per CTA (the
-    // loop's bookkeeping costs their dequantizing warps more than it saves: 77 rows on 14336 x 4096 39 us without, 47 with it).
-    // Expert-indexed launch (Kernel::MatMulId, moe.cu): the activation tiles are runs of (token, slot)
-    // pairs grouped by expert; the weights are the dense stack [experts * n, k], so a tile's weight
-    // rows start at expert * n; tiles past the last used one have no expert.
-    struct Tile {
-        uint32_t n0, m0, wrow0, kb0, nblk, z;
-    };
-    const uint32_t nx = p.tiles_x, ny = p.tiles_y, ntiles = nx * ny * p.splits;
-    const uint32_t nblk_total = p.k / QK, per_split = (nblk_total + p.splits - 1) / p.splits;
-    auto tile_at = [&](uint32_t t, Tile &o) -> bool {
-        const uint32_t c = t / nx, x = t - c * nx;
-        o.z = c / ny;
-        const uint32_t y = c - o.z * ny;
+    // Units [0, full) are whole tiles, those behind are `splits` to a tile. Within `group` activation tiles the tile order
+    // walks the activation tiles first, so that the CTAs that run side by side share packed weights in L2.
+    const uint32_t nx = p.tiles_x, ny = p.tiles_y, units = p.units, step = PAIR ? gridDim.x >> 1 : gridDim.x, first = PAIR ? blockIdx.x >> 1 : blockIdx.x;
+    const uint32_t nblk_total = p.k / QK;
+    auto tile_at = [&](uint32_t u, Tile &o) -> bool {
+        uint32_t t = u, z = 0;
+        o.part = -1;
+        o.kb0 = 0, o.nblk = nblk_total;
+        if (u >= p.full) {
+            const uint32_t v = u - p.full, per = (nblk_total + p.splits - 1) / p.splits;
+            t = v / p.splits, z = v - t * p.splits;
+            o.part = (int32_t)v;
+            t += p.full;
+            o.kb0 = z * per;
+            o.nblk = min(per, nblk_total - o.kb0);
+        }
+        const uint32_t g = t / (nx * p.group), r = t - g * nx * p.group, gy = min(p.group, ny - g * p.group);
+        const uint32_t x = r / gy, y = g * p.group + (r - x * gy);
         o.wrow0 = 0;
         if (p.tile_expert) {
+            // Expert-indexed launch (Kernel::MatMulId, moe.cu): the activation tiles are runs of (token, slot)
+            // pairs grouped by expert; the weights are the dense stack [experts * n, k], so a tile's weight
+            // rows start at expert * n; tiles past the last used one have no expert.
             const int32_t e = p.tile_expert[y];
             if (e < 0) return false;
             o.wrow0 = (uint32_t)e * p.n;
         }
-        o.n0 = x * (TN * NT), o.m0 = y * MT;
-        // split-K: this tile takes the super-blocks [kb0, kb0 + nblk) of K and writes partial sums
-        o.kb0 = o.z * per_split;
-        o.nblk = min(per_split, nblk_total - o.kb0);
+        o.n0 = x * (PAIR ? 2 * TN : TN) + rank * TN;
+        o.m0 = y * p.mt;
         return true;
     };
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::STAGES; s++) {
+        for (int s = 0; s < STAGES; s++) {
             mbar_init(full_a + s, 1);
-            mbar_init(full_b + s, NT == 2 ? DEQ_WARPS : GROUP_WARPS);
+            mbar_init(full_w + s, PAIR ? 17 : 8);  // the eight warps of a stage; PAIR: of both CTAs, and the other CTA's activations
             mbar_init(empty + s, 1);
         }
         for (int r = 0; r < C::RAWS; r++) {
@@ -284,18 +434,16 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(acc_full + a, 1);
-            mbar_init(acc_empty + a, DEQ_WARPS);
+            mbar_init(acc_empty + a, PAIR ? 2 * DEQ_WARPS : DEQ_WARPS);
         }
-        if constexpr (PAIR)
-            for (int s = 0; s < C::STAGES; s++) mbar_init(peer_ready + s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == MMA_WARP) {
         if constexpr (PAIR) {  // the same warp of both CTAs: a pair-wide allocation of the same columns
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(512u) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
         } else {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(512u) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
     }
@@ -305,52 +453,49 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     bool healthy = true;
+    if (p.tile_expert || !p.w_early) grid_dep_wait();  // every role looks the tiles' experts up; weights the kernel in front may write
 
-    if (warp == 0) {
-        // ---------------- TMA producer, activation tiles: one 128-byte-swizzled box per k-step
+    if (warp == ACT_WARP) {
+        // ---------------- TMA producer, activations: two k-steps of 128-byte-swizzled rows per copy (PAIR: this CTA's half of the rows)
         if (lane == 0) {
-            uint32_t kc = 0;  // k-steps so far, over all tiles
+            grid_dep_wait();
+            grid_dep_launch();
+            const uint32_t rows = PAIR ? p.mt / 2 : p.mt;
+            uint32_t s = 0, ph = 1;
             Tile o;
-            for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
-                if (!tile_at(t, o)) continue;
-                for (uint32_t ks = 0; ks < o.nblk * (QK / KS) && healthy; ks++, kc++) {
-                    const uint32_t s = kc % C::STAGES, u = kc / C::STAGES;
-                    if (!mbar_wait(empty + s, (u & 1) ^ 1, 64)) { healthy = false; break; }
-                    mbar_expect_tx(full_a + s, C::A_BYTES);
-                    if constexpr (PAIR) {  // this CTA's half of the activation tile
-                        tma_load_2d(stage0 + s * C::STAGE_BYTES + C::W_BYTES, &map_a, (int)(o.kb0 * QK + ks * KS), (int)(o.m0 + (MT / 2) * cta_rank), full_a + s);
-                    } else {
-#pragma unroll
-                        for (int h = 0; h < (MT + 255) / 256; h++)  // a box holds at most 256 rows
-                            tma_load_2d(stage0 + s * C::STAGE_BYTES + C::W_BYTES + h * 256 * 128, &map_a, (int)(o.kb0 * QK + ks * KS), (int)(o.m0 + 256 * h),
-                                        full_a + s);
-                    }
+            for (uint32_t u = first; u < units && healthy; u += step) {
+                if (!tile_at(u, o)) continue;
+                for (uint32_t h = 0; h < 2 * o.nblk; h++) {  // halves of super-blocks
+                    if (!mbar_wait(empty + s, ph, 32)) { healthy = false; break; }
+                    mbar_expect_tx(full_a + s, rows * 128 * STAGE_KS);
+                    tma_load_3d(stage0 + s * C::A_BYTES, &map_a, 0, (int)(o.m0 + rows * rank), (int)(o.kb0 * (QK / KS) + h * STAGE_KS), full_a + s);
+                    if (++s == STAGES) s = 0, ph ^= 1;
                 }
             }
             if (!healthy && p.status) atomicOr(p.status, 2);
         }
-    } else if (warp == 18 && FMT == FMT_Q6K && ((nblk_total * Q6K_BYTES) & 15u) != 0) {
+    } else if (warp == RAW_WARP && FMT == FMT_Q6K && ((nblk_total * Q6K_BYTES) & 15u) != 0) {
         // ---------------- packed Q6_K weights whose rows are not a multiple of 16 bytes (K not a
         // multiple of 2048, e.g. the K/8 shard of a row-parallel projection): no tensor map can
         // describe them, so every lane copies rows of the tile with the plain bulk copy, each from
         // the 16-byte boundary below its block (the consumers compute the same per-row offset)
         const uint64_t pitch = (uint64_t)nblk_total * Q6K_BYTES;
         const uint64_t end16 = ((uint64_t)(uintptr_t)p.w + (uint64_t)p.n * pitch + 15) & ~(uint64_t)15;  // never read past the matrix's last 16-byte line
-        uint32_t bc = 0;  // super-blocks so far, over all tiles
+        uint32_t r = 0, ph = 1;
         Tile o;
-        for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
-            if (!tile_at(t, o)) continue;
+        for (uint32_t u = first; u < units && healthy; u += step) {
+            if (!tile_at(u, o)) continue;
             const uint32_t rows_valid = min((uint32_t)TN, p.n > o.n0 ? p.n - o.n0 : 0u);
             auto copy_of = [&](uint32_t rr, uint32_t b, uint64_t &src) -> uint32_t {
                 src = ((uint64_t)(uintptr_t)p.w + (uint64_t)(o.n0 + rr) * pitch + (uint64_t)(o.kb0 + b) * Q6K_BYTES) & ~(uint64_t)15;
-                return (uint32_t)min((uint64_t)Q6K_BOX, end16 - src);
+                return (uint32_t)min((uint64_t)224, end16 - src);
             };
-            for (uint32_t b = 0; b < o.nblk && healthy; b++, bc++) {
-                const uint32_t r = bc % C::RAWS, ur = bc / C::RAWS;
-                if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
-                if (lane == 0 && rows_valid) {
+            for (uint32_t b = 0; b < o.nblk; b++) {
+                if (!warp_wait(raw_empty + r, ph)) { healthy = false; break; }
+                if (lane == 0) {
                     uint64_t src;
-                    mbar_expect_tx(raw_full + r, (rows_valid - 1) * Q6K_BOX + copy_of(rows_valid - 1, b, src));  // only the last row can be short
+                    if (rows_valid) mbar_expect_tx(raw_full + r, (rows_valid - 1) * 224 + copy_of(rows_valid - 1, b, src));  // only the last row can be short
+                    else mbar_arrive(raw_full + r);  // (the second CTA of a pair past the last row)
                 }
                 __syncwarp();
                 for (uint32_t rr = lane; rr < rows_valid; rr += 32) {
@@ -361,364 +506,309 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                                  "l"(src), "r"(bytes), "r"(s32(raw_full + r))
                                  : "memory");
                 }
+                if (++r == C::RAWS) r = 0, ph ^= 1;
             }
         }
         if (!healthy && lane == 0 && p.status) atomicOr(p.status, 32);
-    } else if (warp == 18) {
+    } else if (warp == RAW_WARP) {
         // ---------------- TMA producer, packed weights: one super-block of every row of the tile
-        // per copy, up to RAWS super-blocks (of four k-steps) ahead of the dequantizing warps
+        // per copy, up to RAWS super-blocks (of four k-steps) ahead of the expanding warps
         if (lane == 0) {
-            uint32_t bc = 0;
+            uint32_t r = 0, ph = 1;
             Tile o;
-            for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
-                if (!tile_at(t, o)) continue;
-                for (uint32_t b = 0; b < o.nblk && healthy; b++, bc++) {
-                    const uint32_t r = bc % C::RAWS, ur = bc / C::RAWS;
-                    if (!mbar_wait(raw_empty + r, (ur & 1) ^ 1, 64)) { healthy = false; break; }
+            for (uint32_t u = first; u < units && healthy; u += step) {
+                if (!tile_at(u, o)) continue;
+                for (uint32_t b = 0; b < o.nblk; b++) {
+                    if (!mbar_wait(raw_empty + r, ph, 32)) { healthy = false; break; }
                     mbar_expect_tx(raw_full + r, C::RAW);
-#pragma unroll
-                    for (int q = 0; q < NT; q++)
-                        tma_load_2d(raw0 + r * C::RAW + q * RAW_BYTES, &map_w,
-                                    FMT == FMT_Q6K ? (int)(((o.kb0 + b) * Q6K_BYTES) & ~15u) : (int)((o.kb0 + b) * C::ROW_BYTES), (int)(o.wrow0 + o.n0 + q * TN),
-                                    raw_full + r);
+                    tma_load_2d(raw0 + r * C::RAW, &map_w, FMT == FMT_Q6K ? (int)(((o.kb0 + b) * Q6K_BYTES) & ~15u) : (int)((o.kb0 + b) * C::ROW_BYTES),
+                                (int)(o.wrow0 + o.n0), raw_full + r);
+                    if (++r == C::RAWS) r = 0, ph ^= 1;
                 }
             }
             if (!healthy && p.status) atomicOr(p.status, 32);
         }
-    } else if (warp == 1 && PAIR) {
-        // ---------------- MMA issuer of a CTA pair. The leader (rank 0) issues for both CTAs: M = 256
-        // (128 weight rows from each CTA's tile), N = MT (each CTA holds MT / 2 activation rows), the
-        // accumulators land in each CTA's own tensor memory. The other CTA's issuer warp only reports
-        // when its operands of a stage are in place. Completion is committed to both CTAs' barriers. (One tile per CTA.)
-        Tile o;
-        if (lane == 0 && tile_at(blockIdx.x, o)) {
-            const uint32_t ksteps = o.nblk * (QK / KS);
-            const uint32_t peer = cta_rank ^ 1;
-            if (cta_rank == 0) {
-                constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT >> 3) << 17) | ((uint32_t)((2 * TN) >> 4) << 24);
-                for (uint32_t ks = 0; ks < ksteps && healthy; ks++) {
-                    const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
-                    if (!mbar_wait(full_a + s, u & 1, 32) || !mbar_wait(full_b + s, u & 1, 32) || !mbar_wait_cluster(peer_ready + s, u & 1, 32)) {
-                        healthy = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t wt = s32(stage0 + s * C::STAGE_BYTES), at = wt + C::W_BYTES;
-#pragma unroll
-                    for (int t = 0; t < NT; t++)
-#pragma unroll
-                        for (int kk = 0; kk < KS / 16; kk++)
-                            mma_bf16_pair(tmem_base + t * MT, smem_desc(wt + t * B_BYTES + kk * 32), smem_desc(at + kk * 32), idesc, (ks | kk) ? 1u : 0u);
-                    mma_commit_pair(s32(empty + s));
-                    mma_commit_pair(cluster_addr_of(empty + s, peer));
-                }
-                mma_commit_pair(s32(acc_full));
-                mma_commit_pair(cluster_addr_of(acc_full, peer));
-                if (!healthy && p.status) atomicOr(p.status, 4);
-            } else {
-                for (uint32_t ks = 0; ks < ksteps && healthy; ks++) {
-                    const uint32_t s = ks % C::STAGES, u = ks / C::STAGES;
-                    if (!mbar_wait(full_a + s, u & 1, 32) || !mbar_wait(full_b + s, u & 1, 32)) { healthy = false; break; }
-                    mbar_arrive_cluster(cluster_addr_of(peer_ready + s, peer));
-                }
-                if (!healthy && p.status) atomicOr(p.status, 4);
-            }
-        }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer
+    } else if (warp == MMA_WARP && PAIR && rank == 1) {
+        // ---------------- the pair's second CTA: its activations of a stage are in place
         if (lane == 0) {
-            // D f32, A and B bf16, both K-major, M = 128, N = MT
-            constexpr int MMA_N = MT > 256 ? 256 : MT;  // an instruction takes at most 256 columns: MT = 512 issues two
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MMA_N >> 3) << 17) | ((uint32_t)(TN >> 4) << 24);
-            uint32_t kc = 0, ti = 0;  // k-steps and tiles so far
+            const uint32_t to = cluster_addr_of(full_w, 0);
+            uint32_t s = 0, ph = 0;
             Tile o;
-            for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
-                if (!tile_at(t, o)) continue;
-                const uint32_t acc = ti % C::ACCS, ua = ti / C::ACCS, tmem_d = tmem_base + acc * (MT * NT);
-                ti++;
-                if (LOOP && !mbar_wait(acc_empty + acc, (ua & 1) ^ 1, 32)) { healthy = false; break; }  // its last results have been read
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (uint32_t ks = 0; ks < o.nblk * (QK / KS) && healthy; ks++, kc++) {
-                    const uint32_t s = kc % C::STAGES, u = kc / C::STAGES;
-                    if (!mbar_wait(full_a + s, u & 1, 32) || !mbar_wait(full_b + s, u & 1, 32)) { healthy = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t wt = s32(stage0 + s * C::STAGE_BYTES), at = wt + C::W_BYTES;
-#pragma unroll
-                    for (int q = 0; q < NT; q++)
-#pragma unroll
-                        for (int kk = 0; kk < KS / 16; kk++)
-#pragma unroll
-                            for (int h = 0; h < MT / MMA_N; h++)
-                                mma_bf16(tmem_d + q * MT + h * MMA_N, smem_desc(wt + q * B_BYTES + kk * 32),
-                                         smem_desc(at + h * MMA_N * 128 + kk * 32), idesc, (ks | kk) ? 1u : 0u);
-                    mma_commit(empty + s);  // the stage may be refilled once these MMAs have read it
+            for (uint32_t u = first; u < units && healthy; u += step) {
+                if (!tile_at(u, o)) continue;
+                for (uint32_t h = 0; h < 2 * o.nblk; h++) {
+                    if (!mbar_wait(full_a + s, ph)) { healthy = false; break; }
+                    mbar_arrive_cluster(to + 8 * s);
+                    if (++s == STAGES) s = 0, ph ^= 1;
                 }
-                mma_commit(acc_full + acc);
             }
             if (!healthy && p.status) atomicOr(p.status, 4);
         }
+    } else if (warp == MMA_WARP) {
+        // ---------------- MMA issuer (PAIR: the first CTA's, for both). The whole warp walks the loop and one elected lane issues, so that the
+        // operands stay in uniform registers (issued by one lane of a diverged warp: 80 cycles a product instead of 28).
+        // D f32, A and B bf16, both K-major, M = 128 (PAIR: 256), N = mt
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((p.mt >> 3) << 17) | ((uint32_t)((PAIR ? 2 * TN : TN) >> 4) << 24);
+        const uint32_t half_rows = (PAIR ? p.mt / 2 : p.mt) * 8;  // rows * 128 bytes between a stage's two k-steps, in the descriptor's units of 16
+        uint32_t s = 0, ph = 0, ti = 0;  // stage, its phase, tiles so far
+        Tile o;
+        for (uint32_t u = first; u < units && healthy; u += step) {
+            if (!tile_at(u, o)) continue;
+            const uint32_t acc = ti % C::ACCS, tmem_d = tmem_base + acc * C::MT, halves = 2 * o.nblk;
+            if (!__all_sync(0xffffffffu, mbar_wait_cluster(acc_empty + acc, ((ti / C::ACCS) & 1) ^ 1))) { healthy = false; break; }  // its last results have been read
+            ti++;
+            for (uint32_t h = 0; h < halves; h++) {
+                if (!__all_sync(0xffffffffu, mbar_wait(full_a + s, ph) && mbar_wait_cluster(full_w + s, ph))) { healthy = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t wt = tmem_base + A_COL + s * (STAGE_KS * KS / 2);
+                const uint64_t at = smem_desc(s32(stage0) + s * C::A_BYTES);
+                if (elect_one()) {
+#pragma unroll
+                    for (int q = 0; q < STAGE_KS; q++)
+#pragma unroll
+                        for (int kk = 0; kk < KS / 16; kk++)
+                            mma_bf16<PAIR>(tmem_d, wt + q * (KS / 2) + 8 * kk, at + q * half_rows + 2 * kk, idesc, (h | q | kk) ? 1u : 0u);
+                    mma_commit<PAIR>(empty + s);  // the stage may be refilled once these have read it
+                    if (h + 1 == halves) mma_commit<PAIR>(acc_full + acc);
+                }
+                __syncwarp();
+                if (++s == STAGES) s = 0, ph ^= 1;
+            }
+        }
+        if (!healthy && lane == 0 && p.status) atomicOr(p.status, 4);
     } else {
-        // ---------------- dequantize: thread = (weight row of the tile, which 32 of the 64 k); the
-        // first eight warps take the even k-steps, the other eight the odd ones, so that a warp
-        // has two MMA periods for one k-step and the groups' waits overlap
-        // (NT = 2: the two groups own the two 128-row sub-tiles instead and every warp does every k-step)
-        const int dw = (warp - 2) & 7, grp = (warp - 2) >> 3;
-        const int row = 32 * (dw & 3) + lane, half = dw >> 2;
-        const int sub = NT == 2 ? grp : 0;        // weight sub-tile of this thread
-        float d1[4], m1[4];                       // sub-block scales of this thread's pairs of the current super-block
-        uint32_t kc0 = 0, bc0 = 0, ti = 0;        // k-steps, super-blocks and tiles before the current tile
-        Tile o, done;                             // the current tile; the one whose results are to be stored
+        // ---------------- expand and store
+        const uint32_t quarter = warp & 3, j = (uint32_t)warp >> 2;  // the tensor-memory lanes this warp may touch; which 64 k of a super-block
+        const uint32_t row = 32 * quarter + lane;
+        const uint32_t lanes = (32 * quarter) << 16;
+        Tile o, nt, done;                // the current tile; the one behind it; the one whose results are to be stored
+        const uint32_t e23 = planted_exponent();
+        uint32_t sb = 0, ti = 0;         // super-blocks and tiles so far
+        uint32_t r = 0, rph = 0;         // ring slot and phase
 
-        // ---------------- epilogue: TMEM lane = weight row, column = activation row
-        auto store_tile = [&](const Tile &o, uint32_t index) {
+        // ---------------- epilogue: tensor-memory lane = weight row, column = activation row
+        auto store_tile = [&](const Tile &t, uint32_t index) {
+            constexpr int ROUNDS = C::MT / 128;  // rounds of two chunks of 16 columns: this warp has every fourth chunk
             const uint32_t acc = index % C::ACCS;
-            if (!mbar_wait(acc_full + acc, (index / C::ACCS) & 1)) {
+            if (!warp_wait(acc_full + acc, (index / C::ACCS) & 1)) {
                 if (lane == 0 && p.status) atomicOr(p.status, 16);
                 healthy = false;
                 return;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int quarter = warp & 3;  // the TMEM lanes this warp may read
-            const uint32_t n = o.n0 + sub * TN + 32 * quarter + lane;
-            constexpr int COLS = NT == 2 ? MT / 2 : MT / 4, CH = COLS < 32 ? COLS : 32;  // the columns of this warp: a half (NT = 1: a quarter) of them
-            const int cbase = (NT == 2 ? half : (warp - 2) >> 2) * COLS;
+            grid_dep_wait();  // (returns at once after the first time)
+            const uint32_t n = t.n0 + row;
 #pragma unroll 1
-            for (int c0 = 0; c0 < COLS; c0 += CH) {
-                uint32_t r[CH];
-                tmem_ld<CH>(r, tmem_base + acc * (MT * NT) + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(sub * MT + cbase + c0));
-                if (LOOP && c0 + CH == COLS) {  // this warp's last read of the accumulators: they may be overwritten
+            for (int round = 0; round < ROUNDS; round++) {
+                uint32_t v[32];
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    if (16 * (j + 4 * (2 * round + i)) < p.mt) tmem_ld16(v + 16 * i, tmem_base + acc * C::MT + lanes + 16 * (j + 4 * (2 * round + i)));
+                tmem_ld_wait();
+                if (round == ROUNDS - 1) {  // the accumulator may be overwritten
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty + acc);
+                    if (lane == 0) {
+                        if constexpr (PAIR) mbar_arrive_cluster(cluster_addr_of(acc_empty + acc, 0));
+                        else mbar_arrive(acc_empty + acc);
+                    }
                 }
-                if (p.row_pair) {  // expert-indexed: tile-space row -> (token, slot) pair = output row; padding rows have none
-                    const uint32_t mfirst = o.m0 + cbase + c0;
-                    if (n < p.n) {
 #pragma unroll
-                        for (int j = 0; j < CH; j++) {
-                            const int32_t pair = p.row_pair[mfirst + j];
-                            if (pair >= 0) p.out[p.out_off + (uint64_t)pair * p.n + n] = __uint_as_float(r[j]);
+                for (int i = 0; i < 2; i++) {
+                    const uint32_t col = 16 * (j + 4 * (2 * round + i)), mfirst = t.m0 + col;
+                    if (col >= p.mt) break;
+                    if (t.part >= 0) {  // partial sums, [unit][activation row][weight row]; summed by a second kernel
+                        constexpr uint32_t W = PAIR ? 2 * TN : TN;
+                        float *prow = p.partial + ((size_t)t.part * p.mt + col) * W + rank * TN + row;
+#pragma unroll
+                        for (int c = 0; c < 16; c++) prow[(size_t)c * W] = __uint_as_float(v[16 * i + c]);
+                    } else if (p.row_pair) {  // expert-indexed: tile-space row -> (token, slot) pair = output row; padding rows have none
+                        if (n < p.n) {
+#pragma unroll
+                            for (int c = 0; c < 16; c++) {
+                                const int32_t pair = p.row_pair[mfirst + c];
+                                if (pair >= 0) p.out[p.out_off + (uint64_t)pair * p.n + n] = __uint_as_float(v[16 * i + c]);
+                            }
                         }
-                    }
-                } else if (n < p.n && p.partial) {  // split-K: this CTA's partial sums, [split][row][n]; summed by a second kernel
-                    const uint32_t mfirst = o.m0 + cbase + c0;
-                    float *prow = p.partial + ((size_t)o.z * p.rows + mfirst) * p.n + n;
+                    } else if (n < p.n && mfirst < p.rows) {
+                        // (batch, row) of the chunk's first activation row by one division, then by stepping
+                        uint32_t bt = mfirst / p.m, ir = mfirst % p.m;
+                        float *orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)ir * p.out_rs + n;
+                        const float *erow = p.extra ? p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)ir * p.ex_s1 + (int64_t)n * p.ex_s2 : nullptr;
+                        const uint32_t cnt = min(16u, p.rows - mfirst);
+                        if (!erow && ir + cnt <= p.m) {  // the common case: rows of one batch entry, no epilogue term
 #pragma unroll
-                    for (int j = 0; j < CH; j++)
-                        if (mfirst + j < p.rows) prow[(size_t)j * p.n] = __uint_as_float(r[j]);
-                } else if (n < p.n) {
-                    // (batch, row) of the chunk's first activation row by one division, then by stepping
-                    const uint32_t mfirst = o.m0 + cbase + c0;
-                    uint32_t bt = mfirst / p.m, i = mfirst % p.m;
-                    float *orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + n;
-                    const float *erow = p.extra ? p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)n * p.ex_s2 : nullptr;
-                    if (!erow && i + CH <= p.m && mfirst + CH <= p.rows) {  // the common case: 32 whole rows of one batch entry, no epilogue term
-#pragma unroll
-                        for (int j = 0; j < CH; j++) orow[(uint64_t)j * p.out_rs] = __uint_as_float(r[j]);
-                        continue;
-                    }
-#pragma unroll
-                    for (int j = 0; j < CH; j++) {
-                        if (mfirst + j < p.rows) {
-                            float v = __uint_as_float(r[j]);
-                            if (erow) v += *erow;
-                            *orow = v;
-                        }
-                        if (++i == p.m) {  // next batch entry
-                            i = 0;
-                            bt++;
-                            orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + n;
-                            if (erow) erow = p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)n * p.ex_s2;
+                            for (uint32_t c = 0; c < 16; c++)
+                                if (c < cnt) orow[(uint64_t)c * p.out_rs] = __uint_as_float(v[16 * i + c]);
                         } else {
-                            orow += p.out_rs;
-                            if (erow) erow += p.ex_s1;
+#pragma unroll
+                            for (int c = 0; c < 16; c++) {
+                                if (mfirst + c < p.rows) {
+                                    float x = __uint_as_float(v[16 * i + c]);
+                                    if (erow) x += *erow;
+                                    *orow = x;
+                                }
+                                if (++ir == p.m) {  // next batch entry
+                                    ir = 0;
+                                    bt++;
+                                    orow = p.out + p.out_off + (uint64_t)bt * p.out_bs + n;
+                                    if (erow) erow = p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)n * p.ex_s2;
+                                } else {
+                                    orow += p.out_rs;
+                                    if (erow) erow += p.ex_s1;
+                                }
+                            }
                         }
                     }
                 }
             }
         };
-        for (uint32_t t = blockIdx.x; t < ntiles && healthy; t = LOOP ? t + gridDim.x : ntiles) {
-          if (!tile_at(t, o)) continue;
-          const uint32_t ksteps = o.nblk * (QK / KS), first = NT == 2 ? 0 : grp;
-          for (uint32_t ks = first; ks < ksteps && healthy; ks += (NT == 2 ? 1 : 2)) {
-            const uint32_t s = (kc0 + ks) % C::STAGES, u = (kc0 + ks) / C::STAGES;
-            const uint32_t b = ks >> 2, pp = ks & 3, r = (bc0 + b) % C::RAWS, ur = (bc0 + b) / C::RAWS;
-            if constexpr (FMT == FMT_Q6K) {
-                // Q6_K (NT = 1): a super-block is ql[128] | qh[64] | int8 sc[16] | f16 d = 210 bytes, so it
-                // starts on a 2-byte boundary only; the copy starts at the 16-byte boundary below it and
-                // takes 224 bytes per row. 16 lanes share one weight row of the k-step: lane j expands the
-                // four weights 4j..4j+3 of its 64 (16-bit shared loads, conflict-free along the row), a
-                // warp does two rows per pass and 16 rows per k-step.
-                //   k-step pp of the block: half nh = pp >> 1 of the 256, nibble hi = pp & 1; the first 32
-                //   weights come from ql[64 nh + l], the second 32 from ql[64 nh + 32 + l]; the two high
-                //   bits from qh[32 nh + l] >> 2 * (2 hi + h); scale sc[8 nh + 2 (2 hi + h) + l / 16]
-                //   (crates/lapid-quant/src/kquant.rs:375-396). d * sc * (q - 32) is exact in f32.
-                if (pp < 2 && !mbar_wait(raw_full + r, ur & 1)) { healthy = false; break; }
-                if (!mbar_wait(empty + s, (u & 1) ^ 1)) { healthy = false; break; }
-                const uint32_t j = lane & 15, h = j >> 3, jj = j & 7, nh = pp >> 1, hi = pp & 1;
-                const uint64_t pitch = (uint64_t)nblk_total * Q6K_BYTES, wbase = (uint64_t)(uintptr_t)p.w + (uint64_t)(o.kb0 + b) * Q6K_BYTES;
-                const uint64_t unbias32 = pack2(-8388640.0f, -8388640.0f);  // -(2^23 + 32)
-#pragma unroll 2
-                for (int pass = 0; pass < 8; pass++) {
-                    const int rw = 16 * dw + 2 * pass + (lane >> 4);
-                    // where the block starts inside its 224 staged bytes: the distance of its address from
-                    // the 16-byte boundary below it (the same for every row when the row pitch is a multiple of 16)
-                    const uint32_t skew = (uint32_t)((wbase + (uint64_t)(o.n0 + rw) * pitch) & 15u);
-                    const uint8_t *blk = raw0 + r * C::RAW + rw * Q6K_BOX + skew;
-                    const uint16_t *ql = (const uint16_t *)(blk + 64 * nh + 32 * h + 4 * jj);
-                    const uint16_t *qh = (const uint16_t *)(blk + 128 + 32 * nh + 4 * jj);
-                    const uint32_t wl = (uint32_t)ql[0] | ((uint32_t)ql[1] << 16), wh = (uint32_t)qh[0] | ((uint32_t)qh[1] << 16);
-                    const uint32_t q = ((wl >> (4 * hi)) & 0x0F0F0F0Fu) | (((wh >> (2 * (2 * hi + h))) & 0x03030303u) << 4);
-                    const float sc = (float)(int)*(const int8_t *)(blk + 192 + 8 * nh + 2 * (2 * hi + h) + (jj >> 2));
-                    const float sd = half_bits_to_float(*(const uint16_t *)(blk + 208)) * sc;
-                    const uint64_t sd2 = pack2(sd, sd);
-                    const uint64_t q01 = add2(pack2(biased(q, 0x7440u), biased(q, 0x7441u)), unbias32);
-                    const uint64_t q23 = add2(pack2(biased(q, 0x7442u), biased(q, 0x7443u)), unbias32);
-                    const uint32_t o0 = to_bf16x2(mul2(sd2, q01)), o1 = to_bf16x2(mul2(sd2, q23));
-                    uint8_t *dst = stage0 + s * C::STAGE_BYTES + rw * 128;
-                    const int chunk = (int)(j >> 1) ^ (rw & 7);
-                    *(uint2 *)(dst + 16 * chunk + 8 * (j & 1)) = make_uint2(o0, o1);
-                }
-                if (pp >= 2) {  // this warp's last read of the block's packed bytes
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(raw_empty + r);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> tensor-core reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full_b + s);
-            } else {
-                const uint8_t *blk = raw0 + r * C::RAW + sub * RAW_BYTES + row * C::ROW_BYTES;
-                if (NT == 2 ? pp == 0 : pp < 2) {  // first k-step of this thread in the block
-                    if (!mbar_wait(raw_full + r, ur & 1)) { healthy = false; break; }
-                    const uint4 h = *(const uint4 *)blk;
-                    const float d = half_bits_to_float(h.x & 0xffff), dmin = half_bits_to_float(h.x >> 16);
-                    const float nd = d * -8388608.0f, ndmin = dmin * -8388608.0f;
-                    const uint32_t w0 = h.y, w1 = h.z, w2 = h.w;
-                    const uint32_t sc_lo = w0 & 0x3F3F3F3Fu, mn_lo = w1 & 0x3F3F3F3Fu;
-                    const uint32_t sc_hi = (w2 & 0x0F0F0F0Fu) | (((w0 >> 6) & 0x03030303u) << 4);
-                    const uint32_t mn_hi = ((w2 >> 4) & 0x0F0F0F0Fu) | (((w1 >> 6) & 0x03030303u) << 4);
-                    // pair q: sub-block 2q + half = byte 2*(q&1) + half of the lo (q < 2) / hi words
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const uint32_t sel = 0x7440u + 2 * (q & 1) + half;
-                        d1[q] = fmaf(d, biased(q < 2 ? sc_lo : sc_hi, sel), nd);        // d * sc, exact (see qgemv_q4k.cu)
-                        m1[q] = fmaf(dmin, biased(q < 2 ? mn_lo : mn_hi, sel), ndmin);  // dmin * m, exact
-                    }
-                }
-                // Q5_K: Q4_K's block with the fifth bits qh[32] between the header and the nibbles; bit s of qh[l]
-                // belongs to element 32 s + l (crates/lapid-quant/src/kquant.rs:355-373)
-                constexpr int QS = FMT == FMT_Q5K ? 48 : 16;
-                const uint4 qa = *(const uint4 *)(blk + QS + 32 * pp), qb = *(const uint4 *)(blk + QS + 16 + 32 * pp);
-                uint4 ha = make_uint4(0, 0, 0, 0), hb = ha;
-                if constexpr (FMT == FMT_Q5K) {
-                    ha = *(const uint4 *)(blk + 16);
-                    hb = *(const uint4 *)(blk + 32);
-                }
-                if (NT == 2 ? pp == 3 : pp >= 2) {
-                    // This thread's last read of the block's packed bytes: the slot goes back, but only once the loads have returned. Shared
-                    // loads that nothing has waited for yet may be carried out behind the arrival (hundreds of cycles
-                    // behind it while the load / store unit is busy) and then read the first rows of the next block. The vote
-                    // over what they brought waits for them, and nothing hangs on its result. (Giving the slot back behind the
-                    // stores below, which need the values as well: 2048 rows on 11008 x 4096 228 against 225 us, the ring has two slots there.)
-                    uint32_t brought = (qa.x ^ qa.y ^ qa.z ^ qa.w) ^ (qb.x ^ qb.y ^ qb.z ^ qb.w);
-                    if constexpr (FMT == FMT_Q5K) brought ^= (ha.x ^ ha.y ^ ha.z ^ ha.w) ^ (hb.x ^ hb.y ^ hb.z ^ hb.w);
-                    if (__any_sync(0xffffffffu, brought == 0x9E3779B9u)) __nanosleep(1);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(raw_empty + r);
-                }
-                const float sd = pp == 0 ? d1[0] : pp == 1 ? d1[1] : pp == 2 ? d1[2] : d1[3];
-                const float nm = -(pp == 0 ? m1[0] : pp == 1 ? m1[1] : pp == 2 ? m1[2] : m1[3]);
-                const uint64_t sd2 = pack2(sd, sd), nm2 = pack2(nm, nm), unbias = pack2(-8388608.0f, -8388608.0f);
-                uint32_t v[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-                if (half) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) v[i] >>= 4;
-                }
-                if constexpr (FMT == FMT_Q5K) {
-                    const uint32_t hq[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
-#pragma unroll
-                    for (int i = 0; i < 8; i++) v[i] = (v[i] & 0x0F0F0F0Fu) | (((hq[i] >> (2 * pp + half)) & 0x01010101u) << 4);
-                }
-                if (!mbar_wait(empty + s, (u & 1) ^ 1)) { healthy = false; break; }
-                uint8_t *dst = stage0 + s * C::STAGE_BYTES + sub * B_BYTES + row * 128;
-#pragma unroll
-                for (int c = 0; c < 4; c++) {  // 16-byte chunk = 8 consecutive k = two packed words
-                    uint32_t o[4];
-#pragma unroll
-                    for (int w = 0; w < 2; w++) {
-                        const uint32_t t = v[2 * c + w] & (FMT == FMT_Q5K ? 0x1F1F1F1Fu : 0x0F0F0F0Fu);
-                        // y = sd * q - m1 with one rounding, two elements per instruction
-                        const uint64_t q01 = add2(pack2(biased(t, 0x7440u), biased(t, 0x7441u)), unbias);
-                        const uint64_t q23 = add2(pack2(biased(t, 0x7442u), biased(t, 0x7443u)), unbias);
-                        o[2 * w] = to_bf16x2(fma2(sd2, q01, nm2));
-                        o[2 * w + 1] = to_bf16x2(fma2(sd2, q23, nm2));
-                    }
-                    const int chunk = (4 * half + c) ^ (row & 7);
-                    *(uint4 *)(dst + 16 * chunk) = make_uint4(o[0], o[1], o[2], o[3]);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> tensor-core reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full_b + s);
+        // The packed words of the next super-block are loaded before this one's are expanded. A ring slot goes back behind the tensor-memory
+        // stores of what was expanded from it: not behind the loads, which may be carried out late (hundreds of cycles behind an
+        // arrival while the load / store unit is busy) and would then read the first rows of the block that follows.
+        uint32_t u = first;                       // the unit whose super-blocks are being loaded
+        const uint32_t to_mma = PAIR ? cluster_addr_of(full_w, 0) : 0;
+        auto next_tile = [&](Tile &t) -> bool {
+            while (u < units && !tile_at(u, t)) u += step;
+            const bool any = u < units;
+            u += step;
+            return any;
+        };
+        auto load = [&](Packed<FMT> &w, const Tile &t, uint32_t b) {
+            if (!warp_wait(raw_full + r, rph)) {
+                healthy = false;
+                return;
             }
-            // the results of the tile before, behind the first weights of this one: the tensor cores have work meanwhile
-            if (LOOP && ks == first && ti > 0) store_tile(done, ti - 1);
-          }
-          kc0 += ksteps;
-          bc0 += o.nblk;
-          ti++;
-          done = o;
+            const uint8_t *blk = raw0 + r * C::RAW + row * C::ROW_BYTES;
+            if constexpr (FMT == FMT_Q6K) {
+                // where the block starts inside its staged bytes: the distance of its address from the 16-byte boundary below it
+                const uint32_t pitch = nblk_total * Q6K_BYTES;
+                const uint32_t skew = ((t.kb0 + b) * Q6K_BYTES + (t.n0 + row) * pitch) & 15u;  // (p.w is 16-byte aligned; only the low bits matter)
+                load_packed_q6(w, blk, skew, (pitch & 15u) == 0, j);
+            } else {
+                load_packed<FMT>(w, blk, j);
+            }
+        };
+        constexpr bool AHEAD = FMT == FMT_Q4K;    // (Q5_K, Q6_K: 20 and 26 words a share, not twice in the registers)
+        bool more = next_tile(o);
+        Packed<FMT> cur;
+        if (AHEAD && more) load(cur, o, 0);
+        while (healthy) {
+            // Results of the tile before are stored behind the super-blocks that fit the stages: one more would wait for products
+            // that wait for the accumulator.
+            const uint32_t nblk = more ? o.nblk : 0, store_behind = min(nblk, (uint32_t)(STAGES / 2));
+            for (uint32_t b = 0;; b++) {
+                if (b == store_behind && ti > 0) store_tile(done, ti - 1);
+                if (b == nblk || !healthy) break;
+                if constexpr (!AHEAD) load(cur, o, b);
+                const uint32_t slot = r;
+                if (++r == C::RAWS) r = 0, rph ^= 1;
+                Packed<FMT> next;
+                if (b + 1 < nblk) {
+                    if constexpr (AHEAD) load(next, o, b + 1);
+                } else if ((more = next_tile(nt))) {
+                    if constexpr (AHEAD) load(next, nt, 0);
+                }
+                const uint32_t s = 2 * (sb & 1) + (j >> 1), col = tmem_base + A_COL + lanes + s * (STAGE_KS * KS / 2) + (j & 1) * (KS / 2);
+                uint32_t w[16];
+                expand<FMT, 0>(cur, j, e23, w);
+                if (!healthy || !warp_wait(empty + s, ((sb >> 1) & 1) ^ 1)) { healthy = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                tmem_st16(col, w);
+                expand<FMT, 1>(cur, j, e23, w);
+                tmem_st16(col + 16, w);
+                tmem_st_wait();
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    if constexpr (PAIR) mbar_arrive_cluster(to_mma + 8 * s);
+                    else mbar_arrive(full_w + s);
+                    mbar_arrive(raw_empty + slot);
+                }
+                sb++;
+                if constexpr (AHEAD) cur = next;
+            }
+            if (nblk == 0) break;
+            ti++;
+            done = o;
+            o = nt;
         }
         if (!healthy && lane == 0 && p.status) atomicOr(p.status, 8);
-        if (healthy && ti > 0) store_tile(done, ti - 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if constexpr (PAIR) cluster_sync_all();  // neither CTA releases the pair's tensor memory (or exits) while the other still uses it
-    if (warp == 1) {
+    if (warp == MMA_WARP) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if constexpr (PAIR)
-            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
         else
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(MT * NT * C::ACCS)) : "memory");
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }
 
-// split-K second pass: out[m, n] = sum over the splits (in order) of their partial tiles (+ extra)
-__global__ void __launch_bounds__(256) splitk_sum_kernel(GemmTcArgs p, uint32_t splits) {
-    const uint64_t total = (uint64_t)p.rows * p.n;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t m = (uint32_t)(e / p.n), n = (uint32_t)(e % p.n);
-        float v = p.partial[e];
-        for (uint32_t z = 1; z < splits; z++) v += p.partial[(size_t)z * total + e];
+// Second pass of the tiles split over K: out[m, n] = sum over the splits (in order) of their partial tiles (+ extra). A thread takes
+// four consecutive weight rows of one activation row.
+template <int W> __global__ void __launch_bounds__(256) splitk_sum_kernel(GemmTcArgs p) {
+    grid_dep_wait();
+    grid_dep_launch();
+    const uint32_t tiles = (p.units - p.full) / p.splits, per_tile = p.mt * (W / 4);
+    const size_t part = (size_t)p.mt * W;
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (uint64_t)tiles * per_tile; e += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t ts = (uint32_t)(e / per_tile), q = (uint32_t)(e - (uint64_t)ts * per_tile), col = q / (W / 4), w4 = q % (W / 4);
+        const uint32_t t = p.full + ts, g = t / (p.tiles_x * p.group), rr = t - g * p.tiles_x * p.group, gy = min(p.group, p.tiles_y - g * p.group);
+        const uint32_t x = rr / gy, y = g * p.group + (rr - x * gy);
+        const uint32_t m = y * p.mt + col, n = x * W + 4 * w4;
+        if (m >= p.rows || n >= p.n) continue;
+        const float4 *src = (const float4 *)(p.partial + ts * (size_t)p.splits * part + (size_t)col * W) + w4;
+        float4 v = *src;
+        for (uint32_t z = 1; z < p.splits; z++) {
+            const float4 a = src[z * (part / 4)];
+            v.x += a.x, v.y += a.y, v.z += a.z, v.w += a.w;
+        }
         const uint32_t bt = m / p.m, i = m % p.m;
-        if (p.extra) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)n * p.ex_s2];
-        p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + n] = v;
-    }
-}
-
-// f32 activation rows (any row stride) -> contiguous bf16 [rows, k]: blockIdx.y = row (one division per
-// thread, not per element), a thread converts eight consecutive elements (k is a multiple of 256);
-// VEC: the rows are 16-byte aligned, so the loads are 128-bit.
-template <bool VEC> __global__ void __launch_bounds__(256) a_to_bf16_kernel(GemmTcArgs p, __nv_bfloat16 *dst) {
-  for (uint32_t r = blockIdx.y; r < p.rows; r += gridDim.y) {
-    const void *srow = act_row(p.a, p.a_type, p.a_off, p.a_bs, p.a_rs, r, p.m);
-    const float *src = (const float *)srow;  // (VEC: f32 rows only)
-    uint4 *out = (uint4 *)(dst + (size_t)r * p.k);
-    for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < p.k / 8; c8 += gridDim.x * blockDim.x) {
-        float v[8];
-        if constexpr (VEC) {
-            const float4 lo = ((const float4 *)src)[2 * c8], hi = ((const float4 *)src)[2 * c8 + 1];
-            v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+        float r[4] = {v.x, v.y, v.z, v.w};
+        float *out = p.out + p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + n;
+        if (p.extra) {
+            const float *ex = p.extra + p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1;
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                if (n + c < p.n) r[c] += ex[(int64_t)(n + c) * p.ex_s2];
+        }
+        if (n + 4 <= p.n && ((uintptr_t)out & 15) == 0) {
+            *(float4 *)out = make_float4(r[0], r[1], r[2], r[3]);
         } else {
 #pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = load_act(srow, 8 * c8 + i, p.a_type);
+            for (int c = 0; c < 4; c++)
+                if (n + c < p.n) out[c] = r[c];
         }
-        __nv_bfloat162 o[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) o[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-        out[c8] = *(const uint4 *)o;
     }
-  }
+}
+
+// Activation rows (any row stride) -> bf16 [k / 64][rows][64]: what a k-step of the GEMM loads is one contiguous piece instead of a line from
+// every row. blockIdx.y = row (one division per thread, not per element), a thread converts eight consecutive elements (k is a multiple of 256);
+// VEC: the rows are 16-byte aligned, so the loads are 128-bit.
+template <bool VEC> __global__ void __launch_bounds__(256) a_to_bf16_kernel(GemmTcArgs p, __nv_bfloat16 *dst) {
+    grid_dep_wait();
+    grid_dep_launch();
+    for (uint32_t r = blockIdx.y; r < p.rows; r += gridDim.y) {
+        const void *srow = act_row(p.a, p.a_type, p.a_off, p.a_bs, p.a_rs, r, p.m);
+        const float *src = (const float *)srow;  // (VEC: f32 rows only)
+        for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < p.k / 8; c8 += gridDim.x * blockDim.x) {
+            float v[8];
+            if constexpr (VEC) {
+                const float4 lo = ((const float4 *)src)[2 * c8], hi = ((const float4 *)src)[2 * c8 + 1];
+                v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] = load_act(srow, 8 * c8 + i, p.a_type);
+            }
+            __nv_bfloat162 o[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) o[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            ((uint4 *)dst)[((size_t)(c8 / 8) * p.rows + r) * 8 + c8 % 8] = *(const uint4 *)o;
+        }
+    }
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
@@ -737,44 +827,59 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-template <int FMT, int MT, int NT, bool PAIR = false, bool LOOP = false>
-static cudaError_t launch_mt(const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma, int sm_count, cudaStream_t stream, uint32_t splits = 1) {
-    auto kern = qgemm_tc_kernel<FMT, MT, NT, PAIR, LOOP>;
-    using C = Cfg<FMT, MT, NT, PAIR, LOOP>;
+// A launch with (optionally) the programmatic-dependent and the pair attribute.
+struct LaunchCfg {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    LaunchCfg(dim3 grid, unsigned threads, size_t smem, bool pdl, bool pair, cudaStream_t stream) {
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        if (pdl) {
+            attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+        }
+        if (pair) {
+            attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+            attr[cfg.numAttrs].val.clusterDim.x = 2;
+            attr[cfg.numAttrs].val.clusterDim.y = 1;
+            attr[cfg.numAttrs++].val.clusterDim.z = 1;
+        }
+    }
+};
+
+// How a launch is cut: tiles of 128 (pair: 256) weight rows x mt activation rows, the last ones split over K.
+struct Plan {
+    bool pair;
+    uint32_t mt, nx, ny, full, splits, units;
+    uint32_t split_units() const { return units - full; }
+};
+
+template <int FMT, bool PAIR>
+static cudaError_t launch_tiles(const GemmTcArgs &a, const Plan &pl, const CUtensorMap &mw, const CUtensorMap &ma, int sm_count, bool pdl, cudaStream_t stream) {
+    auto kern = qgemm_tc_kernel<FMT, PAIR>;
+    using C = Cfg<FMT, PAIR>;
     static DynamicSmemOptIn opted;
     if (cudaError_t e = opted.raise((const void *)kern, C::SMEM); e != cudaSuccess) return e;
-    GemmTcArgs b = a;
-    b.tiles_x = (a.n + TN * NT - 1) / (TN * NT);
-    if (PAIR) b.tiles_x = (b.tiles_x + 1) & ~1u;  // whole pairs: a CTA past the last weight row works on zero fill and stores nothing
-    b.tiles_y = (a.rows + MT - 1) / MT;
-    b.splits = splits;
-    const uint64_t tiles = (uint64_t)b.tiles_x * b.tiles_y * splits;
-    if (tiles >= (1u << 31)) return cudaErrorInvalidValue;
-    const dim3 grid((unsigned)(!LOOP || tiles < (uint64_t)sm_count ? tiles : (uint64_t)sm_count));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = C::SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    cfg.attrs = attr;
-    if (PAIR) {
-        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-        attr[cfg.numAttrs].val.clusterDim.x = 2;
-        attr[cfg.numAttrs].val.clusterDim.y = 1;
-        attr[cfg.numAttrs++].val.clusterDim.z = 1;
-    }
-    return cudaLaunchKernelEx(&cfg, kern, mw, ma, b);
+    const uint32_t workers = PAIR ? (uint32_t)sm_count / 2 : (uint32_t)sm_count;
+    const uint32_t n = pl.units < workers ? pl.units : workers;
+    LaunchCfg l(dim3(PAIR ? 2 * n : n), THREADS, C::SMEM, pdl, PAIR, stream);
+    return cudaLaunchKernelEx(&l.cfg, kern, mw, ma, a);
+}
+static cudaError_t launch_plan(int fmt, const GemmTcArgs &a, const Plan &pl, const CUtensorMap &mw, const CUtensorMap &ma, int sm_count, bool pdl, cudaStream_t stream) {
+    if (pl.pair)
+        return fmt == FMT_Q4K ? launch_tiles<FMT_Q4K, true>(a, pl, mw, ma, sm_count, pdl, stream)
+             : fmt == FMT_Q5K ? launch_tiles<FMT_Q5K, true>(a, pl, mw, ma, sm_count, pdl, stream) : launch_tiles<FMT_Q6K, true>(a, pl, mw, ma, sm_count, pdl, stream);
+    return fmt == FMT_Q4K ? launch_tiles<FMT_Q4K, false>(a, pl, mw, ma, sm_count, pdl, stream)
+         : fmt == FMT_Q5K ? launch_tiles<FMT_Q5K, false>(a, pl, mw, ma, sm_count, pdl, stream) : launch_tiles<FMT_Q6K, false>(a, pl, mw, ma, sm_count, pdl, stream);
 }
 
 }  // namespace tc
 
-static int g_tc_wide = -1;  // tuning: -1 choose, 0 never, 1 always use two accumulators at MT = 256
-static int g_tc_tall = -1;  // tuning: -1 choose, 0 never, 1 always use 512-row activation tiles above 256 rows
-static int g_tc_pair = 0;   // tuning: 1 = CTA pairs (cta_group::2) for the two-accumulator Q4_K tile
+static int g_tc_pair = -1;  // tuning: -1 choose, 0 never: CTA pairs (cta_group::2)
 void qgemm_tc_set_pair(int v) { g_tc_pair = v; }
-void qgemm_tc_set_wide(int v) { g_tc_wide = v; }
-void qgemm_tc_set_tall(int v) { g_tc_tall = v; }
 
 bool qgemm_tc_supported(int fmt, const GemmTcArgs &a) {
     if (a.k % QK != 0 || a.k < QK || a.rows < 1 || ((uintptr_t)a.w & 15) != 0 || tc::encode_fn() == nullptr) return false;
@@ -783,40 +888,50 @@ bool qgemm_tc_supported(int fmt, const GemmTcArgs &a) {
 
 static uint32_t tc_block_bytes(int fmt) { return fmt == FMT_Q4K ? Q4K_BYTES : fmt == FMT_Q5K ? Q5K_BYTES : Q6K_BYTES; }
 static uint32_t tc_box_bytes(int fmt) { return fmt == FMT_Q6K ? (uint32_t)tc::Q6K_BOX : tc_block_bytes(fmt); }
-// the one-accumulator tile of a format by activation rows per CTA
-template <int FMT, bool LOOP = false> static cudaError_t launch_one_acc(uint32_t mt, const GemmTcArgs &a, const CUtensorMap &mw, const CUtensorMap &ma,
-                                                     int sm_count, cudaStream_t stream, uint32_t ways = 1) {
-    using namespace tc;
-    return mt == 64 ? launch_mt<FMT, 64, 1, false, LOOP>(a, mw, ma, sm_count, stream, ways)
-                    : mt == 128 ? launch_mt<FMT, 128, 1, false, LOOP>(a, mw, ma, sm_count, stream, ways)
-                                : mt == 256 ? launch_mt<FMT, 256, 1, false, LOOP>(a, mw, ma, sm_count, stream, ways) : cudaErrorInvalidValue;
-}
 
-// How many ways K is split: only when the tiles would leave more than half of the SMs idle, never
-// below two super-blocks per split, never more partial-sum scratch than SPLITK_SCRATCH_MAX.
+// Tiles and K splits of a launch. Above 128 rows pairs of CTAs; the activation rows are divided evenly over as few tiles as hold them.
+// Whole tiles run in rounds over the CTAs (pairs); K is split for the tiles of the last round when that round would be less than
+// half full: `ways` units to a tile, as many as fit the round, never below two super-blocks each, never more than
+// SPLITK_SCRATCH_MAX of partial sums.
 constexpr size_t SPLITK_SCRATCH_MAX = (size_t)256 << 20;
-static int g_tc_splitk = -1;  // tuning: -1 choose, 0/1 never, n > 1 always n (where K allows)
+static int g_tc_splitk = -1;  // tuning: -1 choose, 0/1 never, n > 1 every tile n ways (where K allows)
 void qgemm_tc_set_splitk(int v) { g_tc_splitk = v; }
-static uint32_t splitk_ways(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
-    const uint32_t mt = rows <= 64 ? 64 : (rows <= 128 ? 128 : 256);
-    const uint64_t tiles = (uint64_t)((n + tc::TN - 1) / tc::TN) * ((rows + mt - 1) / mt);
-    const uint32_t nblk = k / QK;
+static tc::Plan tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
+    tc::Plan p{};
+    p.pair = rows > 128 && g_tc_pair != 0;
+    const uint32_t cap = p.pair ? 256 : 128, gran = p.pair ? 32 : 16, width = p.pair ? 2 * tc::TN : tc::TN;
+    p.ny = (rows + cap - 1) / cap;
+    p.mt = ((rows + p.ny - 1) / p.ny + gran - 1) / gran * gran;
+    p.nx = (n + width - 1) / width;
+    const uint64_t tiles = (uint64_t)p.nx * p.ny;
+    const uint32_t workers = (uint32_t)(p.pair ? sm_count / 2 : sm_count), nblk = k / QK;
+    uint64_t tail = 0;
     uint32_t ways = 1;
-    if (g_tc_splitk > 1) ways = (uint32_t)g_tc_splitk;
-    else if (g_tc_splitk < 0 && sm_count > 0 && tiles * 2 <= (uint64_t)sm_count) ways = (uint32_t)((uint64_t)sm_count / tiles);
+    if (g_tc_splitk > 1) {
+        tail = tiles;
+        ways = (uint32_t)g_tc_splitk;
+    } else if (g_tc_splitk < 0 && workers > 0) {
+        tail = tiles % workers;
+        if (tail * 2 > workers) tail = 0;
+        if (tail) ways = (uint32_t)(workers / tail);
+    }
     if (ways > nblk / 2) ways = nblk / 2;
     if (ways > 16) ways = 16;
-    while (ways > 1 && (size_t)ways * rows * n * 4 > SPLITK_SCRATCH_MAX) ways--;
+    while (ways > 1 && tail * ways * p.mt * width * 4 > SPLITK_SCRATCH_MAX) ways--;
     // every split must own at least one super-block
     while (ways > 1 && (uint64_t)(ways - 1) * ((nblk + ways - 1) / ways) >= nblk) ways--;
-    return ways < 1 ? 1 : ways;
+    if (ways <= 1) ways = 1, tail = 0;
+    p.splits = ways;
+    p.full = (uint32_t)(tiles - tail);
+    p.units = (uint32_t)(tiles - tail + tail * ways);
+    return p;
 }
 
 // the bf16 copy of the activations, and the partial sums of a split-K launch
 size_t qgemm_tc_copy_bytes(uint32_t rows, uint32_t k) { return ((size_t)rows * k * 2 + 255) & ~(size_t)255; }
 size_t qgemm_tc_partial_bytes(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
-    const uint32_t ways = splitk_ways(rows, n, k, sm_count);
-    return ways > 1 ? (size_t)ways * rows * n * 4 : 0;
+    const tc::Plan p = tc_plan(rows, n, k, sm_count);
+    return (size_t)p.split_units() * p.mt * (p.pair ? 2 * tc::TN : tc::TN) * 4;
 }
 
 bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, const void *w) {
@@ -827,135 +942,85 @@ bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, c
     return pitch % 16 == 0 && (n * pitch) % 256 == 0 && experts * n < (1ull << 31);
 }
 
-cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, int sm_count, cudaStream_t stream) {
-    using namespace tc;
-    if (a.rows == 0 || a.n == 0) return cudaSuccess;
-    EncodeTiledFn enc = encode_fn();
-    if (!enc || !a.tile_expert || !a.row_pair || a.rows % mt != 0) return cudaErrorInvalidValue;
-    CUtensorMap mw, ma;
+// Tensor maps: packed weights as bytes [weight rows][row bytes], box = one block (Q6_K: the 240 bytes around one) of 128 rows; bf16 activations
+// [k / 64][rows][64], box = 64 k (128 bytes, swizzled) x the rows a CTA loads x the k-steps of a stage.
+static cudaError_t tc_maps(int fmt, const GemmTcArgs &a, uint64_t weight_rows, const tc::Plan &pl, void *a_bf16, CUtensorMap &mw, CUtensorMap &ma) {
+    const tc::EncodeTiledFn enc = tc::encode_fn();
+    if (!enc) return cudaErrorNotSupported;
+    const uint32_t blk_bytes = tc_block_bytes(fmt);
+    cuuint32_t es[3] = {1, 1, 1};
     {
-        const uint32_t blk_bytes = tc_block_bytes(fmt);
-        cuuint64_t dims[2] = {(cuuint64_t)(a.k / QK) * blk_bytes, (cuuint64_t)experts * a.n};
+        cuuint64_t dims[2] = {(cuuint64_t)(a.k / QK) * blk_bytes, weight_rows};
         cuuint64_t strides[1] = {(cuuint64_t)(a.k / QK) * blk_bytes};
-        cuuint32_t box[2] = {(cuuint32_t)tc_box_bytes(fmt), TN};
-        cuuint32_t es[2] = {1, 1};
-        if (enc(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)a.w, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        cuuint32_t box[2] = {(cuuint32_t)tc_box_bytes(fmt), tc::TN};
+        if (strides[0] % 16 != 0) std::memset(&mw, 0, sizeof(mw));  // Q6_K with K not a multiple of 2048: the kernel copies rows itself
+        else if (enc(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)a.w, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
     {
-        cuuint64_t dims[2] = {a.k, a.rows};
-        cuuint64_t strides[1] = {(cuuint64_t)a.k * 2};
-        cuuint32_t box[2] = {KS, mt};
-        cuuint32_t es[2] = {1, 1};
-        if (enc(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a_bf16, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        cuuint64_t dims[3] = {tc::KS, a.rows, a.k / tc::KS};
+        cuuint64_t strides[2] = {tc::KS * 2, (cuuint64_t)a.rows * tc::KS * 2};
+        cuuint32_t box[3] = {tc::KS, pl.pair ? pl.mt / 2 : pl.mt, tc::STAGE_KS};
+        if (enc(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, a_bf16, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    if (fmt == FMT_Q6K) return launch_one_acc<FMT_Q6K, true>(mt, a, mw, ma, sm_count, stream);
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K, true>(mt, a, mw, ma, sm_count, stream);
-    return launch_one_acc<FMT_Q4K, true>(mt, a, mw, ma, sm_count, stream);
+    return cudaSuccess;
+}
+static void tc_fill(GemmTcArgs &a, const tc::Plan &pl, uint32_t group) {
+    a.tiles_x = pl.nx, a.tiles_y = pl.ny, a.splits = pl.splits, a.full = pl.full, a.units = pl.units, a.mt = pl.mt, a.group = group;
 }
 
-cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, bool copy, void *partial, int sm_count,
+cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, uint32_t mt, void *a_bf16, int sm_count, bool pdl, cudaStream_t stream) {
+    if (a.rows == 0 || a.n == 0) return cudaSuccess;
+    if (!a.tile_expert || !a.row_pair || a.rows % mt != 0 || mt % 32 != 0 || mt > 256) return cudaErrorInvalidValue;
+    tc::Plan pl{};
+    pl.pair = mt > 128;
+    pl.mt = mt;
+    pl.nx = (a.n + (pl.pair ? 2 : 1) * tc::TN - 1) / ((pl.pair ? 2 : 1) * tc::TN);
+    pl.ny = a.rows / mt;
+    if ((uint64_t)pl.nx * pl.ny >= (1u << 31)) return cudaErrorInvalidValue;
+    pl.splits = 1;
+    pl.full = pl.units = pl.nx * pl.ny;
+    CUtensorMap mw, ma;
+    if (cudaError_t e = tc_maps(fmt, a, (uint64_t)experts * a.n, pl, a_bf16, mw, ma); e != cudaSuccess) return e;
+    GemmTcArgs b = a;
+    tc_fill(b, pl, 1);
+    return tc::launch_plan(fmt, b, pl, mw, ma, sm_count, pdl, stream);
+}
+
+cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, bool copy, void *partial, int sm_count, bool pdl,
                             cudaStream_t stream, int *launched) {
     using namespace tc;
     *launched = 0;
     if (a.rows == 0 || a.n == 0) return cudaSuccess;
-    *launched = copy ? 2 : 1;  // (the bf16 copy of the activations and) the GEMM (and the split-K sum)
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return cudaErrorNotSupported;
-    const uint32_t mt = a.rows <= 64 ? 64 : (a.rows <= 128 ? 128 : 256);
+    const tc::Plan pl = tc_plan(a.rows, a.n, a.k, sm_count);
+    if ((uint64_t)pl.nx * pl.ny * pl.splits >= (1u << 31)) return cudaErrorInvalidValue;
+    CUtensorMap mw, ma;
+    if (cudaError_t e = tc_maps(fmt, a, a.n, pl, a_bf16_scratch, mw, ma); e != cudaSuccess) return e;
 
     if (copy) {
         const dim3 cgrid((a.k / 8 + 255) / 256, a.rows < 65535u ? a.rows : 65535u);
         const bool vec = a.a_type == ACT_F32 && ((uintptr_t)a.a & 15) == 0 && a.a_off % 4 == 0 && a.a_bs % 4 == 0 && a.a_rs % 4 == 0;
-        if (vec) a_to_bf16_kernel<true><<<cgrid, 256, 0, stream>>>(a, (__nv_bfloat16 *)a_bf16_scratch);
-        else a_to_bf16_kernel<false><<<cgrid, 256, 0, stream>>>(a, (__nv_bfloat16 *)a_bf16_scratch);
-        if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
-    }
-
-    // CTA pairs: Q4_K, more than 128 rows (256-row activation tiles), at least two 256-row weight tiles
-    const bool pair = g_tc_pair > 0 && fmt == FMT_Q4K && a.rows > 128 && a.n >= 4 * TN;
-    CUtensorMap mw, ma;
-    {   // packed weights as bytes: [n rows][row_bytes], box = one 144-byte block (Q6_K: 224 bytes around one) of 128 rows
-        const uint32_t blk_bytes = tc_block_bytes(fmt);
-        cuuint64_t dims[2] = {(cuuint64_t)(a.k / QK) * blk_bytes, a.n};
-        cuuint64_t strides[1] = {(cuuint64_t)(a.k / QK) * blk_bytes};
-        cuuint32_t box[2] = {(cuuint32_t)tc_box_bytes(fmt), TN};
-        cuuint32_t es[2] = {1, 1};
-        if (strides[0] % 16 != 0) {
-            // Q6_K with K not a multiple of 2048: no tensor map for the weights (the kernel copies rows itself)
-            std::memset(&mw, 0, sizeof(mw));
-        } else if (enc(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)a.w, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-            return cudaErrorInvalidValue;
-        }
-    }
-    {   // bf16 activations [rows][k], box = 64 k (128 bytes, swizzled) x MT rows
-        cuuint64_t dims[2] = {a.k, a.rows};
-        cuuint64_t strides[1] = {(cuuint64_t)a.k * 2};
-        cuuint32_t box[2] = {KS, pair ? 128u : (mt > 256 ? 256u : mt)};
-        cuuint32_t es[2] = {1, 1};
-        if (enc(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a_bf16_scratch, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return cudaErrorInvalidValue;
-    }
-    // Too few tiles for the SMs (small n: a tensor-parallel shard, a few prefill rows on a narrow
-    // matrix): split K, partial tiles into the scratch, summed in order by a second kernel.
-    const uint32_t ways = splitk_ways(a.rows, a.n, a.k, sm_count);
-    if (ways > 1 && !pair) {
-        GemmTcArgs b = a;
-        b.partial = (float *)partial;
-        cudaError_t e;
-        e = fmt == FMT_Q6K ? launch_one_acc<FMT_Q6K>(mt, b, mw, ma, sm_count, stream, ways)
-                           : fmt == FMT_Q5K ? launch_one_acc<FMT_Q5K>(mt, b, mw, ma, sm_count, stream, ways) : launch_one_acc<FMT_Q4K>(mt, b, mw, ma, sm_count, stream, ways);
-        if (e != cudaSuccess) return e;
-        const uint64_t total = (uint64_t)a.rows * a.n;
-        const unsigned sgrid = (unsigned)((total + 255) / 256 > (uint64_t)sm_count * 8 ? (uint64_t)sm_count * 8 : (total + 255) / 256);
+        LaunchCfg l(cgrid, 256, 0, pdl, false, stream);
+        if (cudaError_t e = cudaLaunchKernelEx(&l.cfg, vec ? a_to_bf16_kernel<true> : a_to_bf16_kernel<false>, a, (__nv_bfloat16 *)a_bf16_scratch);
+            e != cudaSuccess)
+            return e;
         ++*launched;
-        splitk_sum_kernel<<<sgrid, 256, 0, stream>>>(b, ways);
-        return cudaGetLastError();
     }
-    // One or two accumulators per CTA at MT = 256: the 256x256 tile halves the activation traffic
-    // but there are half as many tiles; take the shape with the shorter modelled time (waves of
-    // tiles over the SMs times the measured cost of a k-step of each shape).
-    // 512 activation rows per CTA (all 512 columns of tensor memory for one 128-row weight tile): every
-    // dequantized weight feeds twice the tensor-core work of the 256-row tiles. A k-step of such a
-    // CTA measured 1.6x the time of a 256-row one, so it pays when it saves more than that in waves
-    // of tiles over the SMs. Q6_K only: for Q4_K the two-accumulator 256x256 tile is the better way
-    // to the same reuse (it also halves the activation traffic), measured faster in every case.
-    if (fmt == FMT_Q5K) return launch_one_acc<FMT_Q5K>(mt, a, mw, ma, sm_count, stream);  // (one accumulator tile: no wide or tall variants built)
-    bool tall = false;
-    if (a.rows > 256 && fmt == FMT_Q6K) {
-        const uint64_t nt = (a.n + TN - 1) / TN;
-        const uint64_t w256 = (nt * ((a.rows + 255) / 256) + sm_count - 1) / sm_count;
-        const uint64_t w512 = (nt * ((a.rows + 511) / 512) + sm_count - 1) / sm_count;
-        tall = w512 * 16 < w256 * 10;
+    GemmTcArgs b = a;
+    b.partial = (float *)partial;
+    tc_fill(b, pl, 8);
+    if (cudaError_t e = launch_plan(fmt, b, pl, mw, ma, sm_count, pdl, stream); e != cudaSuccess) return e;
+    ++*launched;
+    if (pl.split_units()) {
+        const uint64_t threads = (uint64_t)(pl.split_units() / pl.splits) * pl.mt * (pl.pair ? 64 : 32), blocks = (threads + 255) / 256;
+        LaunchCfg l(dim3((unsigned)(blocks > (uint64_t)sm_count * 8 ? (uint64_t)sm_count * 8 : blocks)), 256, 0, pdl, false, stream);
+        if (cudaError_t e = pl.pair ? cudaLaunchKernelEx(&l.cfg, splitk_sum_kernel<256>, b) : cudaLaunchKernelEx(&l.cfg, splitk_sum_kernel<128>, b); e != cudaSuccess) return e;
+        ++*launched;
     }
-    if (g_tc_tall >= 0) tall = g_tc_tall != 0 && a.rows > 256;
-    if (tall) return fmt == FMT_Q6K ? launch_mt<FMT_Q6K, 512, 1>(a, mw, ma, sm_count, stream) : launch_mt<FMT_Q4K, 512, 1>(a, mw, ma, sm_count, stream);
-    if (fmt == FMT_Q6K) {  // the larger staged blocks leave room for one accumulator tile only
-        switch (mt) {
-            case 64: return launch_mt<FMT_Q6K, 64, 1>(a, mw, ma, sm_count, stream);
-            case 128: return launch_mt<FMT_Q6K, 128, 1>(a, mw, ma, sm_count, stream);
-            default: return launch_mt<FMT_Q6K, 256, 1>(a, mw, ma, sm_count, stream);
-        }
-    }
-    bool wide = a.rows > 128 && a.n >= 2 * TN;
-    if (wide) {
-        const uint64_t mt_tiles = (a.rows + 255) / 256;
-        const uint64_t t1 = ((a.n + TN - 1) / TN) * mt_tiles, t2 = ((a.n + 2 * TN - 1) / (2 * TN)) * mt_tiles;
-        const uint64_t w1 = (t1 + sm_count - 1) / sm_count, w2 = (t2 + sm_count - 1) / sm_count;
-        wide = w2 * 26 <= w1 * 15;
-    }
-    if (g_tc_wide >= 0) wide = g_tc_wide != 0;
-    if (pair) return launch_mt<FMT_Q4K, 256, 2, true>(a, mw, ma, sm_count, stream);
-    switch (mt) {
-        case 64: return launch_mt<FMT_Q4K, 64, 1>(a, mw, ma, sm_count, stream);
-        case 128: return launch_mt<FMT_Q4K, 128, 1>(a, mw, ma, sm_count, stream);
-        default: return wide ? launch_mt<FMT_Q4K, 256, 2>(a, mw, ma, sm_count, stream) : launch_mt<FMT_Q4K, 256, 1>(a, mw, ma, sm_count, stream);
-    }
+    return cudaSuccess;
 }
 
 }  // namespace lb
