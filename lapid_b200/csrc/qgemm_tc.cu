@@ -61,7 +61,7 @@ constexpr int DEQ_WARPS = 16;
 constexpr int ACT_WARP = DEQ_WARPS, MMA_WARP = DEQ_WARPS + 1, RAW_WARP = DEQ_WARPS + 2;
 constexpr int THREADS = 32 * (DEQ_WARPS + 3);
 constexpr int A_COL = 256;         // tensor-memory column of the first weight stage
-constexpr uint32_t SPIN_LIMIT = 1u << 22;
+constexpr uint32_t WAIT_NS = 1000000, SPIN_LIMIT = 1u << 12;  // about four seconds in all
 
 template <int FMT, bool PAIR> struct Cfg {
     static constexpr int MT = PAIR ? 256 : 128;  // most activation rows of a tile
@@ -85,22 +85,20 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s32(bar)) : "memory");
 }
-// Bounded wait. A waiter that is not on the critical path sleeps between polls so that it does not
-// take issue slots from the expanding warps.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t sleep_ns = 0) {
+// Bounded wait. A failed attempt may sleep in hardware until the phase completes or WAIT_NS have passed: waiters that come back at once
+// took as many issue slots as the expansion.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     for (uint32_t spin = 0; spin < SPIN_LIMIT; spin++) {
         uint32_t ok;
         asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(ok)
-            : "r"(s32(bar)), "r"(parity)
+            : "r"(s32(bar)), "r"(parity), "r"(WAIT_NS)
             : "memory");
         if (ok) return true;
-        if (sleep_ns) __nanosleep(sleep_ns);
     }
     return false;
 }
-
 // A whole warp waits: all lanes or none give up.
 __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
@@ -181,22 +179,9 @@ __device__ __forceinline__ uint32_t cluster_addr_of(const void *p, uint32_t rank
 }
 // Arrival on a barrier of either CTA. What it reports was complete before (tensor-memory stores that `tcgen05.wait::st` has waited for,
 // copies whose barrier has completed), so it carries no cluster-wide release: that one waits for every store of the thread and
-// took 1100 to 1500 cycles an arrival.
+// took 1100 to 1500 cycles an arrival. Likewise the waits acquire at CTA scope: at cluster scope each one drops the SM's L1.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// bounded wait with cluster-scope acquire: arrivals may come from the other CTA of the pair
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity) {
-    for (uint32_t spin = 0; spin < SPIN_LIMIT; spin++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(s32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
 }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -378,7 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, GemmTcArgs p) {
     using C = Cfg<FMT, PAIR>;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = smem_raw + ((0u - s32(smem_raw)) & 1023u);  // (an offset, not a cast: the loads below stay shared-memory loads)
     uint8_t *stage0 = smem;
     uint8_t *raw0 = smem + STAGES * C::A_BYTES;
     uint64_t *bars = (uint64_t *)(raw0 + C::RAWS * C::RAW);
@@ -466,7 +451,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             for (uint32_t u = first; u < units && healthy; u += step) {
                 if (!tile_at(u, o)) continue;
                 for (uint32_t h = 0; h < 2 * o.nblk; h++) {  // halves of super-blocks
-                    if (!mbar_wait(empty + s, ph, 32)) { healthy = false; break; }
+                    if (!mbar_wait(empty + s, ph)) { healthy = false; break; }
                     mbar_expect_tx(full_a + s, rows * 128 * STAGE_KS);
                     tma_load_3d(stage0 + s * C::A_BYTES, &map_a, 0, (int)(o.m0 + rows * rank), (int)(o.kb0 * (QK / KS) + h * STAGE_KS), full_a + s);
                     if (++s == STAGES) s = 0, ph ^= 1;
@@ -519,7 +504,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             for (uint32_t u = first; u < units && healthy; u += step) {
                 if (!tile_at(u, o)) continue;
                 for (uint32_t b = 0; b < o.nblk; b++) {
-                    if (!mbar_wait(raw_empty + r, ph, 32)) { healthy = false; break; }
+                    if (!mbar_wait(raw_empty + r, ph)) { healthy = false; break; }
                     mbar_expect_tx(raw_full + r, C::RAW);
                     tma_load_2d(raw0 + r * C::RAW, &map_w, FMT == FMT_Q6K ? (int)(((o.kb0 + b) * Q6K_BYTES) & ~15u) : (int)((o.kb0 + b) * C::ROW_BYTES),
                                 (int)(o.wrow0 + o.n0), raw_full + r);
@@ -555,10 +540,10 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         for (uint32_t u = first; u < units && healthy; u += step) {
             if (!tile_at(u, o)) continue;
             const uint32_t acc = ti % C::ACCS, tmem_d = tmem_base + acc * C::MT, halves = 2 * o.nblk;
-            if (!__all_sync(0xffffffffu, mbar_wait_cluster(acc_empty + acc, ((ti / C::ACCS) & 1) ^ 1))) { healthy = false; break; }  // its last results have been read
+            if (!__all_sync(0xffffffffu, mbar_wait(acc_empty + acc, ((ti / C::ACCS) & 1) ^ 1))) { healthy = false; break; }  // its last results have been read
             ti++;
             for (uint32_t h = 0; h < halves; h++) {
-                if (!__all_sync(0xffffffffu, mbar_wait(full_a + s, ph) && mbar_wait_cluster(full_w + s, ph))) { healthy = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(full_a + s, ph) && mbar_wait(full_w + s, ph))) { healthy = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t wt = tmem_base + A_COL + s * (STAGE_KS * KS / 2);
                 const uint64_t at = smem_desc(s32(stage0) + s * C::A_BYTES);
@@ -581,13 +566,12 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const uint32_t quarter = warp & 3, j = (uint32_t)warp >> 2;  // the tensor-memory lanes this warp may touch; which 64 k of a super-block
         const uint32_t row = 32 * quarter + lane;
         const uint32_t lanes = (32 * quarter) << 16;
-        Tile o, nt, done;                // the current tile; the one behind it; the one whose results are to be stored
         const uint32_t e23 = planted_exponent();
         uint32_t sb = 0, ti = 0;         // super-blocks and tiles so far
         uint32_t r = 0, rph = 0;         // ring slot and phase
 
         // ---------------- epilogue: tensor-memory lane = weight row, column = activation row
-        auto store_tile = [&](const Tile &t, uint32_t index) {
+        auto store_tile = [&](uint32_t unit, uint32_t index) {
             constexpr int ROUNDS = C::MT / 128;  // rounds of two chunks of 16 columns: this warp has every fourth chunk
             const uint32_t acc = index % C::ACCS;
             if (!warp_wait(acc_full + acc, (index / C::ACCS) & 1)) {
@@ -597,6 +581,8 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             grid_dep_wait();  // (returns at once after the first time)
+            Tile t;
+            tile_at(unit, t);
             const uint32_t n = t.n0 + row;
 #pragma unroll 1
             for (int round = 0; round < ROUNDS; round++) {
@@ -666,15 +652,13 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // The packed words of the next super-block are loaded before this one's are expanded. A ring slot goes back behind the tensor-memory
         // stores of what was expanded from it: not behind the loads, which may be carried out late (hundreds of cycles behind an
         // arrival while the load / store unit is busy) and would then read the first rows of the block that follows.
-        uint32_t u = first;                       // the unit whose super-blocks are being loaded
         const uint32_t to_mma = PAIR ? cluster_addr_of(full_w, 0) : 0;
-        auto next_tile = [&](Tile &t) -> bool {
-            while (u < units && !tile_at(u, t)) u += step;
-            const bool any = u < units;
-            u += step;
-            return any;
+        Tile o;
+        auto valid = [&](uint32_t u) -> uint32_t {  // the first unit from u on that has work
+            while (u < units && !tile_at(u, o)) u += step;
+            return u;
         };
-        auto load = [&](Packed<FMT> &w, const Tile &t, uint32_t b) {
+        auto load = [&](Packed<FMT> &w, uint32_t kb, uint32_t first_row) {  // (the place of the block matters for Q6_K only)
             if (!warp_wait(raw_full + r, rph)) {
                 healthy = false;
                 return;
@@ -683,32 +667,34 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             if constexpr (FMT == FMT_Q6K) {
                 // where the block starts inside its staged bytes: the distance of its address from the 16-byte boundary below it
                 const uint32_t pitch = nblk_total * Q6K_BYTES;
-                const uint32_t skew = ((t.kb0 + b) * Q6K_BYTES + (t.n0 + row) * pitch) & 15u;  // (p.w is 16-byte aligned; only the low bits matter)
+                const uint32_t skew = (kb * Q6K_BYTES + (first_row + row) * pitch) & 15u;  // (p.w is 16-byte aligned; only the low bits matter)
                 load_packed_q6(w, blk, skew, (pitch & 15u) == 0, j);
             } else {
                 load_packed<FMT>(w, blk, j);
             }
         };
         constexpr bool AHEAD = FMT == FMT_Q4K;    // (Q5_K, Q6_K: 20 and 26 words a share, not twice in the registers)
-        bool more = next_tile(o);
+        uint32_t u = valid(first), done = 0;      // the current unit; the one whose results are to be stored
+        uint32_t kb0 = 0, n0 = 0, nblk = 0;
+        auto enter = [&]() { nblk = u < units ? o.nblk : 0, kb0 = o.kb0, n0 = o.n0; };
+        enter();
         Packed<FMT> cur;
-        if (AHEAD && more) load(cur, o, 0);
+        if (AHEAD && nblk) load(cur, 0, 0);
         while (healthy) {
             // Results of the tile before are stored behind the super-blocks that fit the stages: one more would wait for products
             // that wait for the accumulator.
-            const uint32_t nblk = more ? o.nblk : 0, store_behind = min(nblk, (uint32_t)(STAGES / 2));
+            const uint32_t store_behind = min(nblk, (uint32_t)(STAGES / 2));
+            uint32_t un = u;
             for (uint32_t b = 0;; b++) {
                 if (b == store_behind && ti > 0) store_tile(done, ti - 1);
                 if (b == nblk || !healthy) break;
-                if constexpr (!AHEAD) load(cur, o, b);
+                if constexpr (!AHEAD) load(cur, kb0 + b, n0);
                 const uint32_t slot = r;
                 if (++r == C::RAWS) r = 0, rph ^= 1;
                 Packed<FMT> next;
-                if (b + 1 < nblk) {
-                    if constexpr (AHEAD) load(next, o, b + 1);
-                } else if ((more = next_tile(nt))) {
-                    if constexpr (AHEAD) load(next, nt, 0);
-                }
+                if (b + 1 == nblk) un = valid(u + step);
+                if constexpr (AHEAD)
+                    if (un < units) load(next, 0, 0);
                 const uint32_t s = 2 * (sb & 1) + (j >> 1), col = tmem_base + A_COL + lanes + s * (STAGE_KS * KS / 2) + (j & 1) * (KS / 2);
                 uint32_t w[16];
                 expand<FMT, 0>(cur, j, e23, w);
@@ -730,8 +716,9 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             }
             if (nblk == 0) break;
             ti++;
-            done = o;
-            o = nt;
+            done = u;
+            u = un;
+            enter();
         }
         if (!healthy && lane == 0 && p.status) atomicOr(p.status, 8);
     }
