@@ -245,7 +245,7 @@ template <int FMT> struct Packed {
     uint32_t w[8], x[FMT == FMT_Q5K ? 8 : 1];
 };
 template <> struct Packed<FMT_Q6K> {
-    uint32_t wl[16], wh[8], sc, d;
+    uint32_t wl[8], wh[8], sc, d;  // (wl: of one half at a time)
 };
 template <int FMT> __device__ __forceinline__ void load_packed(Packed<FMT> &r, const uint8_t *blk, uint32_t j) {
     constexpr int QS = FMT == FMT_Q5K ? 48 : 16;
@@ -257,48 +257,45 @@ template <int FMT> __device__ __forceinline__ void load_packed(Packed<FMT> &r, c
         *(uint4 *)(r.x + 4) = *(const uint4 *)(blk + 32);
     }
 }
-// 16 + 8 words of a Q6_K block's ql and qh from 128-bit chunks of its staged row; the block starts 4 WS (+ 2: sh = 16) bytes behind a chunk boundary
-template <int WS> __device__ __forceinline__ void q6k_words(const uint8_t *row, uint32_t nh, uint32_t sh, uint32_t (&wl)[16], uint32_t (&wh)[8]) {
-    uint32_t t[20];
+// Eight words at byte `at` (a multiple of 16) of a Q6_K block, from 128-bit chunks of its staged row; the block starts 4 WS (+ 2: sh = 16) bytes behind
+// a chunk boundary
+template <int WS> __device__ __forceinline__ void q6k_words(const uint8_t *row, uint32_t at, uint32_t sh, uint32_t (&w)[8]) {
+    uint32_t t[12];
 #pragma unroll
-    for (int c = 0; c < 5; c++) *(uint4 *)(t + 4 * c) = *(const uint4 *)(row + 64 * nh + 16 * c);
+    for (int c = 0; c < 3; c++) *(uint4 *)(t + 4 * c) = *(const uint4 *)(row + at + 16 * c);
 #pragma unroll
-    for (int i = 0; i < 16; i++) wl[i] = __funnelshift_r(t[i + WS], t[i + WS + 1], sh);
-#pragma unroll
-    for (int c = 0; c < 3; c++) *(uint4 *)(t + 4 * c) = *(const uint4 *)(row + 128 + 32 * nh + 16 * c);
-#pragma unroll
-    for (int i = 0; i < 8; i++) wh[i] = __funnelshift_r(t[i + WS], t[i + WS + 1], sh);
+    for (int i = 0; i < 8; i++) w[i] = __funnelshift_r(t[i + WS], t[i + WS + 1], sh);
 }
 // `skew`: where the block starts in its staged row; `uniform`: the same for every row of the matrix
-__device__ __forceinline__ void load_packed_q6(Packed<FMT_Q6K> &r, const uint8_t *row, uint32_t skew, bool uniform, uint32_t j) {
-    const uint32_t nh = j >> 1, hi = j & 1, sh = 8 * (skew & 2);
+__device__ __forceinline__ void q6k_run(const uint8_t *row, uint32_t skew, bool uniform, uint32_t at, uint32_t (&w)[8]) {
+    const uint32_t sh = 8 * (skew & 2);
     if (uniform) {
         switch (skew >> 2) {
-            case 0: q6k_words<0>(row, nh, sh, r.wl, r.wh); break;
-            case 1: q6k_words<1>(row, nh, sh, r.wl, r.wh); break;
-            case 2: q6k_words<2>(row, nh, sh, r.wl, r.wh); break;
-            default: q6k_words<3>(row, nh, sh, r.wl, r.wh); break;
+            case 0: q6k_words<0>(row, at, sh, w); break;
+            case 1: q6k_words<1>(row, at, sh, w); break;
+            case 2: q6k_words<2>(row, at, sh, w); break;
+            default: q6k_words<3>(row, at, sh, w); break;
         }
     } else {
-        const uint32_t *a = (const uint32_t *)(row + (skew & ~3u) + 64 * nh), *c = (const uint32_t *)(row + (skew & ~3u) + 128 + 32 * nh);
+        const uint32_t *a = (const uint32_t *)(row + (skew & ~3u) + at);
         uint32_t prev = a[0];
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const uint32_t next = a[i + 1];
-            r.wl[i] = __funnelshift_r(prev, next, sh);
-            prev = next;
-        }
-        prev = c[0];
-#pragma unroll
         for (int i = 0; i < 8; i++) {
-            const uint32_t next = c[i + 1];
-            r.wh[i] = __funnelshift_r(prev, next, sh);
+            const uint32_t next = a[i + 1];
+            w[i] = __funnelshift_r(prev, next, sh);
             prev = next;
         }
     }
-    const uint16_t *scp = (const uint16_t *)(row + skew + 192 + 8 * nh + 4 * hi);
-    r.sc = (uint32_t)scp[0] | ((uint32_t)scp[1] << 16);
-    r.d = *(const uint16_t *)(row + skew + 208);
+}
+template <int H> __device__ __forceinline__ void load_packed_q6(Packed<FMT_Q6K> &r, const uint8_t *row, uint32_t skew, bool uniform, uint32_t j) {
+    const uint32_t nh = j >> 1, hi = j & 1;
+    q6k_run(row, skew, uniform, 64 * nh + 32 * H, r.wl);
+    if (H == 0) {
+        q6k_run(row, skew, uniform, 128 + 32 * nh, r.wh);
+        const uint16_t *scp = (const uint16_t *)(row + skew + 192 + 8 * nh + 4 * hi);
+        r.sc = (uint32_t)scp[0] | ((uint32_t)scp[1] << 16);
+        r.d = *(const uint16_t *)(row + skew + 208);
+    }
 }
 // d * byte `sel` of w, exactly: d (2^23 + b) - d 2^23 has one rounding, and d b (11 x 8 bits) needs none
 __device__ __forceinline__ float scaled(float d, uint32_t w, uint32_t sel, float neg_d23) { return fmaf(d, biased(w, sel), neg_d23); }
@@ -314,7 +311,7 @@ template <int FMT, int H> __device__ __forceinline__ void expand(const Packed<FM
         const uint64_t unbias32 = pack2(-8388640.0f, -8388640.0f);   // -(2^23 + 32)
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const uint32_t q = ((r.wl[8 * H + i] >> (4 * hi)) & 0x0F0F0F0Fu) | (rot(r.wh[i], up) & 0x30303030u);
+            const uint32_t q = ((r.wl[i] >> (4 * hi)) & 0x0F0F0F0Fu) | (rot(r.wh[i], up) & 0x30303030u);
             const uint64_t s2 = pack2(sd[i >> 2], sd[i >> 2]);
             o[2 * i] = to_bf16x2(mul2(s2, add2(pack2(biased(q, 0x7440u), biased(q, 0x7441u)), unbias32)));
             o[2 * i + 1] = to_bf16x2(mul2(s2, add2(pack2(biased(q, 0x7442u), biased(q, 0x7443u)), unbias32)));
@@ -540,7 +537,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         for (uint32_t u = first; u < units && healthy; u += step) {
             if (!tile_at(u, o)) continue;
             const uint32_t acc = ti % C::ACCS, tmem_d = tmem_base + acc * C::MT, halves = 2 * o.nblk;
-            if (!__all_sync(0xffffffffu, mbar_wait(acc_empty + acc, ((ti / C::ACCS) & 1) ^ 1))) { healthy = false; break; }  // its last results have been read
+            if (!warp_wait(acc_empty + acc, ((ti / C::ACCS) & 1) ^ 1)) { healthy = false; break; }  // its last results have been read
             ti++;
             for (uint32_t h = 0; h < halves; h++) {
                 if (!__all_sync(0xffffffffu, mbar_wait(full_a + s, ph) && mbar_wait(full_w + s, ph))) { healthy = false; break; }
@@ -658,22 +655,20 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             while (u < units && !tile_at(u, o)) u += step;
             return u;
         };
+        // Q6_K: where a block starts inside its staged bytes: the distance of its address from the 16-byte boundary below it
+        const uint32_t pitch = nblk_total * Q6K_BYTES;
+        const bool uniform = (pitch & 15u) == 0;
+        auto skew_of = [&](uint32_t kb, uint32_t first_row) { return (kb * Q6K_BYTES + (first_row + row) * pitch) & 15u; };  // (p.w is 16-byte aligned; only the low bits matter)
         auto load = [&](Packed<FMT> &w, uint32_t kb, uint32_t first_row) {  // (the place of the block matters for Q6_K only)
             if (!warp_wait(raw_full + r, rph)) {
                 healthy = false;
                 return;
             }
             const uint8_t *blk = raw0 + r * C::RAW + row * C::ROW_BYTES;
-            if constexpr (FMT == FMT_Q6K) {
-                // where the block starts inside its staged bytes: the distance of its address from the 16-byte boundary below it
-                const uint32_t pitch = nblk_total * Q6K_BYTES;
-                const uint32_t skew = (kb * Q6K_BYTES + (first_row + row) * pitch) & 15u;  // (p.w is 16-byte aligned; only the low bits matter)
-                load_packed_q6(w, blk, skew, (pitch & 15u) == 0, j);
-            } else {
-                load_packed<FMT>(w, blk, j);
-            }
+            if constexpr (FMT == FMT_Q6K) load_packed_q6<0>(w, blk, skew_of(kb, first_row), uniform, j);
+            else load_packed<FMT>(w, blk, j);
         };
-        constexpr bool AHEAD = FMT == FMT_Q4K;    // (Q5_K, Q6_K: 20 and 26 words a share, not twice in the registers)
+        constexpr bool AHEAD = FMT == FMT_Q4K;    // (Q5_K, Q6_K: too many words a share to hold twice)
         uint32_t u = valid(first), done = 0;      // the current unit; the one whose results are to be stored
         uint32_t kb0 = 0, n0 = 0, nblk = 0;
         auto enter = [&]() { nblk = u < units ? o.nblk : 0, kb0 = o.kb0, n0 = o.n0; };
@@ -701,6 +696,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (!healthy || !warp_wait(empty + s, ((sb >> 1) & 1) ^ 1)) { healthy = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 tmem_st16(col, w);
+                if constexpr (FMT == FMT_Q6K) load_packed_q6<1>(cur, raw0 + slot * C::RAW + row * C::ROW_BYTES, skew_of(kb0 + b, n0), uniform, j);
                 expand<FMT, 1>(cur, j, e23, w);
                 tmem_st16(col + 16, w);
                 tmem_st_wait();
