@@ -341,6 +341,10 @@ struct ActSlot {
     // A prefill launch on the tensor cores (records = TC_COPY): `offset` is where its partial sums go, `copy_offset` its bf16 copy of
     // the operand; launches that read the same operand share the copy of the first (`owner` slots back; -1: its own).
     static constexpr int TC_COPY = 3;
+    // An expert-indexed launch on the tensor cores: its key is tokens, slots, experts (off), tile height (rs) and the two buffers; `offset` is where
+    // its routing tables and gathered rows lie, those of the first launch (`owner`) where it shares them.
+    static constexpr int MOE_COPY = 4;
+    const void *ids = nullptr;
     size_t copy_offset = 0, written_before = 0;
     int owner = -1;
     bool w_clean = false;  // no earlier launch of the list writes the launch's weights
@@ -683,7 +687,7 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
 }
 
 void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_buffer *const *buffers, size_t n_buffers,
-                   const ActSlot *slot) {
+                   ActSlot *slot) {
     MoePlan p = plan_matmul_id(dev, l);
     auto get = [&](uint32_t id) -> lapid_b200_buffer * {
         if (id >= n_buffers || !buffers[id])
@@ -755,12 +759,16 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
     lb::moe_route_layout(base, pairs, p.e, p.mt, route);
     route.ids = (const int32_t *)ids->ptr;
     route.status = dev.status_dev;
-    cuda_check(lb::launch_moe_route(route, dev.pdl_launch(), dev.stream), "matmul_id route launch");
-    dev.launches++;
+    ActSlot *made = slot && slot->records == ActSlot::MOE_COPY ? slot - (slot->owner >= 0 ? slot->owner : 0) : nullptr;  // who knows whether the tables are there
+    const bool route_done = made && made->done;
+    if (!route_done) {
+        cuda_check(lb::launch_moe_route(route, dev.pdl_launch(), dev.stream), "matmul_id route launch");
+        dev.launches++;
+    }
     const uint32_t rows = route.max_tiles * route.mt;
     if (p.tc && lb::qgemm_tc_moe_supported(l.b_dtype, p.e, l.n, l.k, w->ptr) && p.wl.total == p.wl.qs_bytes) {
         void *a_bf16 = base + p.route_bytes;
-        cuda_check(lb::launch_moe_gather_bf16((const float *)x->ptr, route, (uint32_t)p.r, (uint32_t)l.k, a_bf16, dev.pdl, dev.stream), "matmul_id gather launch");
+        if (!route_done) cuda_check(lb::launch_moe_gather_bf16((const float *)x->ptr, route, (uint32_t)p.r, (uint32_t)l.k, a_bf16, dev.pdl, dev.stream), "matmul_id gather launch");
         lb::GemmTcArgs t{};
         t.w = (const uint8_t *)w->ptr;
         t.out = (float *)out->ptr;
@@ -772,7 +780,8 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         t.tile_expert = route.tile_expert;
         t.row_pair = route.row_pair;
         cuda_check(lb::launch_qgemm_tc_moe(l.b_dtype, t, (uint32_t)p.e, p.mt, a_bf16, dev.sm_count, dev.pdl, dev.stream), "matmul_id gemm launch");
-        dev.launches += 2;
+        dev.launches += route_done ? 1 : 2;
+        if (made) made->done = true;
         return;
     }
     lb::GemmF32Args f{};
@@ -1099,8 +1108,36 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
             }
             if (l.kind == LAPID_B200_KERNEL_MATMUL_ID && is_quant(l.b_dtype)) {  // a scratch slot of its own; its output counts as written
                 ActSlot sl;
+                const MoePlan p = plan_matmul_id(*dev, l);
+                lapid_b200_buffer *xb = l.n_inputs > 2 && l.inputs[0] < nbuf ? buffers[l.inputs[0]] : nullptr;
+                lapid_b200_buffer *ib = l.n_inputs > 2 && l.inputs[2] < nbuf ? buffers[l.inputs[2]] : nullptr;
                 sl.offset = scratch_total;
-                scratch_total += plan_matmul_id(*dev, l).scratch;
+                // the routing tables and the gathered rows of an earlier launch with the same tokens and ids (gate and up), as long as nothing
+                // since has written either buffer
+                if (p.tc && xb && ib) {
+                    sl.records = ActSlot::MOE_COPY;
+                    sl.ptr = xb->ptr;
+                    sl.ids = ib->ptr;
+                    sl.rows = (uint32_t)p.t;
+                    sl.m = (uint32_t)p.r;
+                    sl.k = (uint32_t)l.k;
+                    sl.off = p.e;
+                    sl.rs = p.mt;
+                    sl.written_before = written.size();
+                    for (size_t s2 = slots.size(); s2-- > 0 && dev->act_reuse;) {
+                        if (!slots[s2].same(sl) || slots[s2].ids != sl.ids || slots[s2].owner >= 0) continue;
+                        bool clean = true;
+                        for (size_t w = slots[s2].written_before; w < written.size(); w++)
+                            for (const lapid_b200_buffer *b : {xb, ib})
+                                if ((const char *)b->ptr < written[w].hi && written[w].lo < (const char *)b->ptr + b->bytes) clean = false;
+                        if (clean) {
+                            sl.owner = (int)(slots.size() - s2);
+                            sl.offset = slots[s2].offset;
+                        }
+                        break;
+                    }
+                }
+                if (sl.owner < 0) scratch_total += p.scratch;
                 slots.push_back(sl);
                 slot_of[i] = (int)slots.size() - 1;
                 lapid_b200_buffer *gb = l.output < nbuf ? buffers[l.output] : nullptr;

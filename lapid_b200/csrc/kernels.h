@@ -339,7 +339,7 @@ void qgemm_tc_set_pair(int v);  // tuning: -1 choose, 0 never: CTA pairs (cta_gr
 struct MoeRouteArgs {
     const int32_t *ids;  // [pairs]
     uint32_t pairs, experts, mt, max_tiles;
-    int32_t *counts, *cursor, *offsets;  // [experts] each
+    int32_t *counts;                     // [experts]
     int32_t *tile_expert;                // [max_tiles]
     int32_t *row_pair;                   // [max_tiles * mt]
     int *status;
