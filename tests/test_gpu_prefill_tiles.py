@@ -1,0 +1,111 @@
+"""Tensor-core prefill (csrc/qgemm_tc.cu) at the edges of its tiles: activation rows around the step from one CTA to a pair and between tiles,
+weight rows that leave the second CTA of a pair without work, whole tiles beside tiles split over K, and the routing tables that
+expert-indexed launches of a list share.
+
+Bar: both operands are rounded to bf16 (2^-9 each) and the sums are f32, so against the exact f32 kernel rel_l2 <= 4e-3 and max_rel <= 3e-2, as
+for the other tests of this kernel."""
+import numpy as np
+import pytest
+
+import lapid_b200 as lp
+from lapid_b200 import quant
+from lapid_b200.backend import MatView, matmul_id_launch, matmul_launch
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+FORMATS = [lp.DType.Q4K, lp.DType.Q5K, lp.DType.Q6K]
+
+
+@pytest.fixture(scope="module")
+def be():
+    return lp.Backend(0)
+
+
+def _close(got, want):
+    got, want = got.astype(np.float64), want.astype(np.float64)
+    rms = np.sqrt((want ** 2).mean())
+    assert np.sqrt(((got - want) ** 2).mean()) / rms <= 4e-3
+    assert (np.abs(got - want) / np.maximum(np.abs(want), rms)).max() <= 3e-2
+
+
+def _both(be, launches, bufs, out):
+    """The output buffer's contents from the tensor cores and from the exact f32 kernel."""
+    res = []
+    for mode in ("tc", "f32"):
+        be.set_option("gemm", mode)
+        try:
+            bufs[out].write(0, np.full(bufs[out].nbytes // 4, -7.0, np.float32))
+            be.execute(launches, bufs)
+        finally:
+            be.set_option("gemm", "tc")
+        res.append(bufs[out].download().view(np.float32).copy())
+    return res
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("m,n,k", [(9, 1, 256), (16, 127, 512), (17, 129, 768), (112, 130, 2048), (128, 300, 1024), (129, 100, 256), (129, 257, 1280),
+                                   (161, 255, 2048), (256, 513, 512), (257, 384, 768), (600, 200, 512)])
+@pytest.mark.parametrize("ways", ["-1", "0", "3"])
+def test_rows_columns_and_splits(be, fmt, m, n, k, ways):
+    x, w = O.normal(5000 + m, m * k), O.normal(5001 + n, n * k, 0.05)
+    bufs = [be.upload(x), be.upload(quant.quantize(be, fmt, w, n, k)), be.alloc(m * n * 4), be.upload(O.normal(5002, n))]
+    for extra in ({}, {"bias_input": 3}):
+        be.set_option("gemm_splitk", ways)
+        try:
+            got, want = _both(be, [matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, **extra)], bufs, 2)
+        finally:
+            be.set_option("gemm_splitk", "-1")
+        _close(got, want)
+
+
+@pytest.mark.parametrize("m,n", [(40, 152 * 128), (300, 38 * 256)])
+def test_whole_tiles_beside_split_ones(be, m, n):
+    """A last round of a few tiles (split over K) behind a full one; the launch by itself and again give the same bits."""
+    fmt, k = lp.DType.Q4K, 1024
+    x, w = O.normal(5100, m * k), np.tile(O.normal(5101, 512 * k, 0.05), n // 512 + 1)[: n * k]
+    w = (w.reshape(n, k) * (1 + 0.001 * (np.arange(n, dtype=np.float32) % 991))[:, None]).astype(np.float32)
+    bufs = [be.upload(x), be.upload(quant.quantize(be, fmt, w, n, k)), be.alloc(m * n * 4)]
+    ls = [matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)]
+    got, want = _both(be, ls, bufs, 2)
+    _close(got, want)
+    be.execute(ls, bufs)
+    assert np.array_equal(bufs[2].download().view(np.float32), got)
+
+
+def test_rows_of_several_batch_entries_in_one_tile(be):
+    """A tile's columns cross batch entries whose outputs are strided; nothing outside the views is written."""
+    fmt, batch, m, n, k = lp.DType.Q4K, 5, 37, 70, 512
+    total = 3 + batch * m * n * 2
+    x = O.normal(5200, batch * m * k)
+    bufs = [be.upload(x), be.upload(quant.quantize(be, fmt, O.normal(5201, n * k, 0.05), n, k)), be.alloc(total * 4)]
+    ls = [matmul_launch(fmt, m, n, k, batch=batch, inputs=(0, 1), output=2, out=MatView(3, n, batch * n))]
+    got, want = _both(be, ls, bufs, 2)
+    _close(got, want)
+    assert np.array_equal(got == -7.0, want == -7.0)
+
+
+@pytest.mark.parametrize("rewrite", [False, True])
+def test_expert_indexed_launches_share_their_tables(be, rewrite):
+    """Gate and up of one list use the same routing tables and gathered rows; a launch that rewrites the tokens in between ends that.
+    Every result has the bits of the launch run by itself."""
+    fmt, t, r, e, n, k = lp.DType.Q4K, 70, 2, 6, 256, 512
+    ids = np.stack([np.random.default_rng(i).permutation(e)[:r] for i in range(t)]).astype(np.int32)
+    ids[:, 0] = np.where(ids[:, 0] == 3, ids[:, 1] ^ 1, ids[:, 0])
+    stacks = [quant.quantize(be, fmt, O.normal(5300 + i, e * n * k, 0.05), e * n, k) for i in range(2)]
+    x, y = O.normal(5310, t * k), O.normal(5311, t * k)
+    # 0 tokens, 1 ids, 2, 3 stacks, 4, 5 outputs, 6 another operand, 7 the matrix that makes new tokens of it
+    bufs = [be.upload(x), be.upload(ids)] + [be.upload(s) for s in stacks] + [be.alloc(t * r * n * 4) for _ in range(2)]
+    bufs += [be.upload(y), be.upload(quant.quantize(be, fmt, O.normal(5312, k * k, 0.05), k, k))]
+    ls = [matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 2, 1), output=4), matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 3, 1), output=5)]
+    if rewrite:
+        ls.insert(1, matmul_launch(fmt, t, k, k, inputs=(6, 7), output=0))
+    res, counts = [], []
+    for one_list in (False, True):
+        bufs[0].write(0, x)
+        be.take_launch_count()
+        for part in [ls] if one_list else [[l] for l in ls]:
+            be.execute(part, bufs)
+        counts.append(be.take_launch_count())
+        res.append([bufs[i].download().view(np.float32).copy() for i in (4, 5)])
+    assert all(np.array_equal(a, b) for a, b in zip(*res))
+    assert counts[1] == counts[0] - (0 if rewrite else 2)   # no second route and gather
