@@ -347,7 +347,6 @@ struct ActSlot {
     const void *ids = nullptr;
     size_t copy_offset = 0, written_before = 0;
     int owner = -1;
-    bool w_clean = false;  // no earlier launch of the list writes the launch's weights
     bool same(const ActSlot &o) const {
         return ptr == o.ptr && off == o.off && bs == o.bs && rs == o.rs && rows == o.rows && m == o.m && k == o.k &&
                records == o.records && a_type == o.a_type;
@@ -374,6 +373,7 @@ struct PendingGroup {
     int fmt = 0, mode = 0;  // kernel of the members: 1 = dp4a kernel, 2 = tensor-core kernel, 3 = balanced-stream tensor-core kernel
     lb::GemvGroup g{};
     bool split_early = false;  // see accepts()
+    bool serial = false;       // an earlier launch of the list writes what a member fetches early (run_launch: src_written)
     std::vector<Range> writes, reads;
 
     bool accepts(int f, int md, const lb::GemvArgs &a, const Range &out, const Range *in, int n_in) {
@@ -418,9 +418,10 @@ struct PendingGroup {
         reads.clear();
         lb::GemvGroup out = g;
         out.count = count;
-        const bool early = dev.early_ok(true);  // members carry early = 1 when their activations came from the pre-pass at the head
+        const bool early = dev.early_ok(true) && !serial;  // members carry early = 1 when their activations came from the pre-pass at the head
         for (int i = 0; i < count; i++) out.item[i].early = early ? out.item[i].early : 0;
-        const bool pdl = dev.pdl_launch();
+        const bool pdl = dev.pdl_launch() && !serial;
+        serial = false;
         const uint64_t before = dev.stream_ws.kernels;
         if (mode == 3) cuda_check(lb::launch_qgemv_kq_stream(fmt, out, dev.stream_ws, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (fmt == LAPID_B200_DTYPE_INT8 || fmt == LAPID_B200_DTYPE_INT4)
@@ -579,8 +580,6 @@ lb::ActOut act_out_checked(lapid_b200_device *dev, lapid_b200_buffer *qact, int3
     return act_out_at(qact->ptr, layout, (uint32_t)rows, (uint32_t)cols);
 }
 
-// `tp` not null: a launch that takes one of the K-quant fast decode kernels hands its result to the
-// tensor-parallel group from its epilogue instead of storing it (`*pushed` says whether it did).
 // Kernel::Gather: out[i, :] = dequant(table[ids[i], :]).
 void check_gather(const lapid_b200_launch &l) {
     const bool quant = is_quant(l.b_dtype);
@@ -803,8 +802,12 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
     dev.launches++;
 }
 
+// `tp` not null: a launch that takes one of the K-quant fast decode kernels hands its result to the
+// tensor-parallel group from its epilogue instead of storing it (`*pushed` says whether it did).
+// `src_written`: an earlier launch of the list writes the weights (or the quantized activation operand). The decode kernels fetch
+// weights before their dependency wait, and the kernel in front may let them start before it has stored, so such a launch is fully serialised.
 void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_buffer *const *buffers, size_t n_buffers,
-                ActSlot *slot, PendingGroup *pend = nullptr, const lb::TpPushTable *tp = nullptr, bool *pushed = nullptr) {
+                ActSlot *slot, PendingGroup *pend = nullptr, const lb::TpPushTable *tp = nullptr, bool *pushed = nullptr, bool src_written = false) {
     if (l.kind == LAPID_B200_KERNEL_GATHER) {
         if (pend) pend->flush(dev);
         run_gather(dev, l, buffers, n_buffers);
@@ -961,6 +964,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
                 slot->done = true;
             }
             pend->add(l.b_dtype, mode, g, wr, in, n_in);
+            pend->serial = pend->serial || src_written;
             return;
         }
         if (pend) pend->flush(dev);
@@ -973,8 +977,8 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             g.tp = tp;
             *pushed = true;
         }
-        g.early = dev.early_ok(slot->hoisted) ? 1 : 0;
-        const bool pdl = dev.pdl_launch();
+        g.early = dev.early_ok(slot->hoisted) && !src_written ? 1 : 0;
+        const bool pdl = dev.pdl_launch() && !src_written;
         const uint64_t ws_before = dev.stream_ws.kernels;
         if (slot->records == 2 && l.b_dtype == LAPID_B200_DTYPE_MXFP4) {
             cuda_check(lb::launch_qgemv_mxfp4_mma(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
@@ -1030,7 +1034,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             int launched = 0;
             // Everything older than the kernel in front has completed when a kernel of this chain starts (each lets its successor start
             // behind its own wait), so the weights may be read at once unless a launch of this list writes them.
-            t.w_early = slot && slot->w_clean;
+            t.w_early = slot && !src_written;
             cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, (char *)dev.scratch + copy_at, !(made && made->done), (char *)dev.scratch + partial_at,
                                            dev.sm_count, dev.pdl, dev.stream, &launched), "qgemm_tc launch");
             if (made) made->done = true;
@@ -1089,6 +1093,7 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
     //    and the GEMVs then follow each other directly.
     std::vector<ActSlot> slots;
     std::vector<int> slot_of(n, -1);
+    std::vector<char> src_written(n, 0);  // an earlier launch of the list writes the launch's weights (or its quantized activation operand)
     size_t scratch_total = 0;
     {
         struct Range { const char *lo, *hi; };
@@ -1153,6 +1158,10 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
             Plan p = plan_launch(*dev, l);
             lapid_b200_buffer *ab = l.n_inputs > 0 && l.inputs[0] < nbuf ? buffers[l.inputs[0]] : nullptr;
             lapid_b200_buffer *ob = l.output < nbuf ? buffers[l.output] : nullptr;
+            lapid_b200_buffer *wb = l.n_inputs > 1 && l.inputs[1] < nbuf ? buffers[l.inputs[1]] : nullptr;
+            for (const lapid_b200_buffer *b : {wb, l.a_dtype == LAPID_B200_DTYPE_ACT_Q8 ? ab : nullptr})
+                for (const Range &w : written)
+                    if (b && (const char *)b->ptr < w.hi && w.lo < (const char *)b->ptr + b->bytes) src_written[i] = 1;
             if (p.gemv && ab && l.a_dtype != LAPID_B200_DTYPE_ACT_Q8) {
                 ActSlot key;
                 key.ptr = ab->ptr;
@@ -1206,11 +1215,6 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
                 }
                 sl.records = ActSlot::TC_COPY;
                 sl.written_before = written.size();
-                if (lapid_b200_buffer *wb = l.n_inputs > 1 && l.inputs[1] < nbuf ? buffers[l.inputs[1]] : nullptr) {
-                    sl.w_clean = true;
-                    for (const Range &w : written)
-                        if ((const char *)wb->ptr < w.hi && w.lo < (const char *)wb->ptr + wb->bytes) sl.w_clean = false;
-                }
                 // the copy an earlier launch of the list makes of the same operand (q, k, v; gate, up), as long as nothing since has written
                 // the buffer it comes from
                 for (size_t s2 = slots.size(); s2-- > 0 && ab && dev->act_reuse;) {
@@ -1307,7 +1311,7 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
     try {
         for (size_t i = 0; i < n; i++) {
             if (profiling) cuda_check(cudaEventRecord(dev->profile_events[2 * i], dev->stream), "cudaEventRecord");
-            run_launch(*dev, launches[i], buffers, nbuf, slot_of[i] >= 0 ? &slots[slot_of[i]] : nullptr, pp);
+            run_launch(*dev, launches[i], buffers, nbuf, slot_of[i] >= 0 ? &slots[slot_of[i]] : nullptr, pp, nullptr, nullptr, src_written[i] != 0);
             if (profiling) cuda_check(cudaEventRecord(dev->profile_events[2 * i + 1], dev->stream), "cudaEventRecord");
         }
     } catch (...) {

@@ -6,7 +6,7 @@ import pytest
 
 import lapid_b200 as lp
 from lapid_b200 import tp
-from lapid_b200.backend import DType, matmul_id_launch, matmul_launch
+from lapid_b200.backend import DType, MatView, matmul_id_launch, matmul_launch
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -200,3 +200,56 @@ def test_expert_prompt_repeats_bit_for_bit():
     stream.synchronize()
     be.synchronize()
     assert torch.isfinite(want).all() and not any(bool(v) for v in differ), differ
+
+
+@pytest.mark.parametrize("writer_rows", [8, 40, 300])
+@pytest.mark.parametrize("fmt", [DType.Int8, DType.Int4, DType.Q4K, DType.Q5K])
+@pytest.mark.parametrize("m", [1, 2, 8])
+def test_weights_written_by_an_earlier_launch_of_the_list(fmt, m, writer_rows):
+    """A launch of the list (decode or prefill on the tensor cores) stores into the packed bytes of a later decode launch's weights; the f32
+    results are taken as the bytes they are, the scales stay. The later launch's activations are clean, so nothing stands between the
+    two kernels; its weights must be the written ones, plain and captured."""
+    import torch
+    per_block = {DType.Int8: 8, DType.Int4: 4, DType.Q4K: 32, DType.Q5K: 32}[fmt]     # floats that a block's packed values take
+    first, pitch = {DType.Q4K: (4, 36), DType.Q5K: (12, 44)}.get(fmt, (0, per_block))  # where they lie: floats before them, from block to block
+    k = 1024
+    blocks = k // (256 if pitch > per_block else 32)
+    n = 4096 if fmt in (DType.Int8, DType.Int4) else 2048
+    wn = per_block if pitch > per_block else 1024           # the writer's columns
+    rows = n * blocks * per_block // wn                      # ... and the rows that fill every block
+    launches = []
+    serial, s0 = _device(pdl="0")
+    be, s1 = _device()
+    w0 = _weights(be, int(fmt), n, k, 990)
+    writer = [_weights(be, int(DType.Q4K), wn, 512, 991 + i) for i in range(2)]
+    xs = torch.from_numpy(O.normal(992, rows * 512).reshape(rows, 512)).cuda()
+    x = torch.from_numpy(O.normal(993, m * k).reshape(m, k)).cuda()
+    w, out = w0.clone(), torch.zeros(m, n, device="cuda")
+    torch.cuda.synchronize()
+    chunk = min(rows, writer_rows)
+    # (two blocks of rows are enough: the first fetches of every warp of the later launch lie in them or not)
+    for r0 in (0, max(0, rows - chunk)):
+        launches.append(matmul_launch(DType.Q4K, chunk, wn, 512, inputs=(0, 1), output=2, a=MatView(r0 * 512, chunk * 512, 512),
+                                      out=MatView(first + r0 * wn // per_block * pitch, 0, pitch if pitch > per_block else wn)))
+    launches.append(matmul_launch(fmt, m, n, k, inputs=(3, 2), output=4))
+    wants = []
+    bufs0 = [[serial.wrap_tensor(t) for t in (xs, wr, w, x, out)] for wr in writer]
+    for b in bufs0:
+        for l in launches:
+            serial.execute([l], b)
+        wants.append(out.view(torch.int32).clone())
+        torch.cuda.synchronize()
+    assert not torch.equal(*wants)
+    bufs = [[be.wrap_tensor(t) for t in (xs, wr, w, x, out)] for wr in writer]
+    graphs = [_capture(be, s1, lambda b=b: be.execute_async(launches, b)) for b in bufs]
+    for rep in range(20):
+        for run in (lambda: be.execute_async(launches, bufs[rep % 2]), graphs[rep % 2].replay):
+            with torch.cuda.stream(s1):
+                w.copy_(w0)
+                out.zero_()
+                run()
+                got = out.view(torch.int32).clone()
+            s1.synchronize()
+            assert torch.equal(got, wants[rep % 2]), rep
+    serial.synchronize()
+    be.synchronize()
