@@ -309,9 +309,8 @@ template <int FMT, int H> __device__ __forceinline__ void expand(const Packed<FM
         const float d = half_bits_to_float(r.d);
         const uint32_t hi = j & 1, up = (4 - 4 * hi - 2 * H) & 31;  // rotation that brings the two high bits of every byte to bits 4 and 5
         const uint32_t sb = r.sc ^ 0x80808080u;                      // scales + 128
-        const float nd = d * -8388608.0f;
-        // d * sc (11 x 8 bits) and d * sc * (q - 32) are exact in f32
-        const float sd[2] = {fmaf(-128.0f, d, scaled(d, sb, 0x7440u + 2 * H, nd)), fmaf(-128.0f, d, scaled(d, sb, 0x7441u + 2 * H, nd))};
+        // d * sc (11 x 8 bits) and d * sc * (q - 32) are exact in f32; d = inf stays inf (removed behind the product, the bias would make it NaN)
+        const float sd[2] = {d * (biased(sb, 0x7440u + 2 * H) - 8388736.0f), d * (biased(sb, 0x7441u + 2 * H) - 8388736.0f)};  // 2^23 + 128
         const uint64_t unbias32 = pack2(-8388640.0f, -8388640.0f);   // -(2^23 + 32)
 #pragma unroll
         for (int i = 0; i < 8; i++) {

@@ -109,3 +109,23 @@ def test_expert_indexed_launches_share_their_tables(be, rewrite):
         res.append([bufs[i].download().view(np.float32).copy() for i in (4, 5)])
     assert all(np.array_equal(a, b) for a, b in zip(*res))
     assert counts[1] == counts[0] - (0 if rewrite else 2)   # no second route and gather
+
+
+@pytest.mark.parametrize("m", [9, 130])
+@pytest.mark.parametrize("k", [512, 2048])
+def test_q6k_infinite_scale_stays_infinite(be, m, k):
+    """A Q6_K row whose block scale is infinite gives infinities of the sign of scale times weight, as the exact f32 kernel does (no NaN of its own)."""
+    n = 130
+    q = quant.quantize(be, lp.DType.Q6K, O.normal(5400, n * k, 0.05), n, k).copy()
+    rows = q[: n * k // 256 * 210].reshape(n, k // 256, 210)
+    for row, scale, d in ((0, 1, 0x7C00), (1, -3, 0x7C00), (129, 5, 0xFC00)):
+        rows[row, :, :192] = 0xFF                    # every value 63 - 32
+        rows[row, :, 192:208] = np.uint8(scale & 0xFF)
+        rows[row, 0, 208:] = np.frombuffer(np.uint16(d).tobytes(), np.uint8)
+    x = np.abs(O.normal(5401, m * k)) + np.float32(0.5)
+    bufs = [be.upload(x.astype(np.float32)), be.upload(q), be.alloc(m * n * 4)]
+    got, want = _both(be, [matmul_launch(lp.DType.Q6K, m, n, k, inputs=(0, 1), output=2)], bufs, 2)
+    got, want = got.reshape(m, n), want.reshape(m, n)
+    assert np.isposinf(want[:, 0]).all() and np.isneginf(want[:, [1, 129]]).all()
+    assert np.array_equal(got[:, [0, 1, 129]], want[:, [0, 1, 129]])
+    _close(got[:, 2:129], want[:, 2:129])
