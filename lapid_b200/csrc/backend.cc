@@ -234,6 +234,7 @@ struct lapid_b200_device {
     bool small_dp4a = true;  // small Q5_K / Q6_K matrices at 3 and 4 rows on the dp4a kernel (see plan_launch)
     bool two_row_dp4a = false;    // two early Q4_K rows on the dp4a kernel (see execute_impl)
     lb::StreamWs stream_ws{};    // workspace of that kernel: partial sums in flight between CTAs (all zero between launches)
+    lb::GemmTcTuning gemm_tc;  // options "gemm_splitk", "gemm_pair"
     bool gemm_f32 = false;  // true: rows > gemv_max_rows always take the exact-f32 GEMM instead of the tensor cores
     // option "profile": every launch of an execute list is bracketed by events (launches run one by one then: nothing is
     // grouped) and its GPU time added to its kernel kind; lapid_b200_take_profile drains the totals
@@ -326,6 +327,7 @@ struct Plan {
     bool fast_i8 = false;  // specialised Int8 / Int4 GEMV with bulk-copy rings (activations as planes)
     bool tc = false;     // tensor-core GEMM (needs a bf16 copy of the activations in the scratch)
     size_t tc_copy = 0;  // bytes of that copy, the first of the scratch bytes
+    lb::GemmTcPlan tc_plan{};
 };
 
 // Where the quantized activations of a decode launch live in the scratch, and who makes them.
@@ -547,7 +549,8 @@ Plan plan_launch(const lapid_b200_device &dev, const lapid_b200_launch &l) {
                (l.b_dtype == LAPID_B200_DTYPE_Q4_K || l.b_dtype == LAPID_B200_DTYPE_Q5_K || l.b_dtype == LAPID_B200_DTYPE_Q6_K);
         if (p.tc) {
             p.tc_copy = lb::qgemm_tc_copy_bytes(p.rows, (uint32_t)l.k);
-            p.scratch = p.tc_copy + align_up(lb::qgemm_tc_partial_bytes(p.rows, (uint32_t)l.n, (uint32_t)l.k, dev.sm_count), 256);
+            p.tc_plan = lb::qgemm_tc_plan(p.rows, (uint32_t)l.n, (uint32_t)l.k, dev.sm_count, dev.gemm_tc);
+            p.scratch = p.tc_copy + align_up(lb::qgemm_tc_partial_bytes(p.tc_plan), 256);
         }
     }
     return p;
@@ -1035,7 +1038,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             // Everything older than the kernel in front has completed when a kernel of this chain starts (each lets its successor start
             // behind its own wait), so the weights may be read at once unless a launch of this list writes them.
             t.w_early = slot && !src_written;
-            cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, (char *)dev.scratch + copy_at, !(made && made->done), (char *)dev.scratch + partial_at,
+            cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, p.tc_plan, (char *)dev.scratch + copy_at, !(made && made->done), (char *)dev.scratch + partial_at,
                                            dev.sm_count, dev.pdl, dev.stream, &launched), "qgemm_tc launch");
             if (made) made->done = true;
             dev.launches += launched;
@@ -1690,9 +1693,9 @@ lapid_b200_status lapid_b200_device_set_option(lapid_b200_device *dev, const cha
         } else if (k == "gemm_wide" || k == "gemm_tall") {
             // accepted, without effect: the tile shapes these chose between are one shape now
         } else if (k == "gemm_splitk") {
-            lb::qgemm_tc_set_splitk(std::atoi(value));
+            dev->gemm_tc.splitk = std::atoi(value);
         } else if (k == "gemm_pair") {
-            lb::qgemm_tc_set_pair(std::atoi(value));
+            dev->gemm_tc.pair = std::atoi(value);
         } else if (k == "gemm") {
             if (v == "f32") dev->gemm_f32 = true;
             else if (v == "tc") dev->gemm_f32 = false;

@@ -315,7 +315,7 @@ struct GemmTcArgs {
     int64_t ex_s0, ex_s1, ex_s2;
     uint32_t rows, m, n, k;
     int *status;
-    float *partial;  // split-K launches: [splits][rows][n] partial sums in the scratch; nullptr otherwise
+    float *partial;  // in the scratch: partial sums of the units that are split over K, [unit][mt][128, pairs of CTAs 256]
     bool w_early;    // under programmatic dependent launch the weights may be read before the kernel in front has completed
     uint32_t tiles_x, tiles_y, splits, full, units, mt, group;  // set by the launcher
     // Expert-indexed launches (launch_qgemm_tc_moe): rows = the tile space, n = rows of ONE expert's matrix
@@ -324,16 +324,26 @@ struct GemmTcArgs {
 };
 bool qgemm_tc_supported(int fmt, const GemmTcArgs &args);
 size_t qgemm_tc_copy_bytes(uint32_t rows, uint32_t k);  // bf16 copy of the activations
-size_t qgemm_tc_partial_bytes(uint32_t rows, uint32_t n, uint32_t k, int sm_count);  // split-K partial sums (0: not split)
-void qgemm_tc_set_splitk(int v);  // tuning: -1 choose, 0 / 1 never, n > 1 always n ways
+// Tuning options of a device: `splitk` -1 choose, 0 / 1 never, n > 1 every tile n ways (where K allows); `pair` -1 choose, 0 never: CTA pairs (cta_group::2)
+struct GemmTcTuning {
+    int splitk = -1, pair = -1;
+};
+// How a launch is cut: tiles of 128 (pair: 256) weight rows x mt activation rows, the last ones split over K. Made once per launch: what it needs of the
+// scratch and what the kernels are given come from the same plan.
+struct GemmTcPlan {
+    bool pair;
+    uint32_t mt, nx, ny, full, splits, units;
+    uint32_t split_units() const { return units - full; }
+};
+GemmTcPlan qgemm_tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count, const GemmTcTuning &tuning);
+size_t qgemm_tc_partial_bytes(const GemmTcPlan &plan);  // split-K partial sums (0: not split)
 // copy: make the bf16 copy first (false: an earlier launch of the same call has made it).
-cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &args, void *a_bf16_scratch, bool copy, void *partial, int sm_count,
+cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &args, const GemmTcPlan &plan, void *a_bf16_scratch, bool copy, void *partial, int sm_count,
                             bool pdl, cudaStream_t stream, int *launched);
 // Kernel::MatMulId on the tensor cores: `a_bf16` holds the activation rows in tile-space order (moe.cu), the
 // weights are a dense stack of `experts` matrices [n, k] (no padding between them), mt in {64, 128, 256}.
 bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, const void *w);
 cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &args, uint32_t experts, uint32_t mt, void *a_bf16, int sm_count, bool pdl, cudaStream_t stream);
-void qgemm_tc_set_pair(int v);  // tuning: -1 choose, 0 never: CTA pairs (cta_group::2)
 
 // ---- moe.cu: device-side grouping of (token, slot) pairs by expert for Kernel::MatMulId
 struct MoeRouteArgs {

@@ -836,12 +836,7 @@ struct LaunchCfg {
     }
 };
 
-// How a launch is cut: tiles of 128 (pair: 256) weight rows x mt activation rows, the last ones split over K.
-struct Plan {
-    bool pair;
-    uint32_t mt, nx, ny, full, splits, units;
-    uint32_t split_units() const { return units - full; }
-};
+using Plan = GemmTcPlan;
 
 template <int FMT, bool PAIR>
 static cudaError_t launch_tiles(const GemmTcArgs &a, const Plan &pl, const CUtensorMap &mw, const CUtensorMap &ma, int sm_count, bool pdl, cudaStream_t stream) {
@@ -864,9 +859,6 @@ static cudaError_t launch_plan(int fmt, const GemmTcArgs &a, const Plan &pl, con
 
 }  // namespace tc
 
-static int g_tc_pair = -1;  // tuning: -1 choose, 0 never: CTA pairs (cta_group::2)
-void qgemm_tc_set_pair(int v) { g_tc_pair = v; }
-
 bool qgemm_tc_supported(int fmt, const GemmTcArgs &a) {
     if (a.k % QK != 0 || a.k < QK || a.rows < 1 || ((uintptr_t)a.w & 15) != 0 || tc::encode_fn() == nullptr) return false;
     return fmt == FMT_Q4K || fmt == FMT_Q5K || fmt == FMT_Q6K;
@@ -880,11 +872,9 @@ static uint32_t tc_box_bytes(int fmt) { return fmt == FMT_Q6K ? (uint32_t)tc::Q6
 // half full: `ways` units to a tile, as many as fit the round, never below two super-blocks each, never more than
 // SPLITK_SCRATCH_MAX of partial sums.
 constexpr size_t SPLITK_SCRATCH_MAX = (size_t)256 << 20;
-static int g_tc_splitk = -1;  // tuning: -1 choose, 0/1 never, n > 1 every tile n ways (where K allows)
-void qgemm_tc_set_splitk(int v) { g_tc_splitk = v; }
-static tc::Plan tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
+GemmTcPlan qgemm_tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count, const GemmTcTuning &tuning) {
     tc::Plan p{};
-    p.pair = rows > 128 && g_tc_pair != 0;
+    p.pair = rows > 128 && tuning.pair != 0;
     const uint32_t cap = p.pair ? 256 : 128, gran = p.pair ? 32 : 16, width = p.pair ? 2 * tc::TN : tc::TN;
     p.ny = (rows + cap - 1) / cap;
     p.mt = ((rows + p.ny - 1) / p.ny + gran - 1) / gran * gran;
@@ -893,10 +883,10 @@ static tc::Plan tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
     const uint32_t workers = (uint32_t)(p.pair ? sm_count / 2 : sm_count), nblk = k / QK;
     uint64_t tail = 0;
     uint32_t ways = 1;
-    if (g_tc_splitk > 1) {
+    if (tuning.splitk > 1) {
         tail = tiles;
-        ways = (uint32_t)g_tc_splitk;
-    } else if (g_tc_splitk < 0 && workers > 0) {
+        ways = (uint32_t)tuning.splitk;
+    } else if (tuning.splitk < 0 && workers > 0) {
         tail = tiles % workers;
         if (tail * 2 > workers) tail = 0;
         if (tail) ways = (uint32_t)(workers / tail);
@@ -915,10 +905,7 @@ static tc::Plan tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
 
 // the bf16 copy of the activations, and the partial sums of a split-K launch
 size_t qgemm_tc_copy_bytes(uint32_t rows, uint32_t k) { return ((size_t)rows * k * 2 + 255) & ~(size_t)255; }
-size_t qgemm_tc_partial_bytes(uint32_t rows, uint32_t n, uint32_t k, int sm_count) {
-    const tc::Plan p = tc_plan(rows, n, k, sm_count);
-    return (size_t)p.split_units() * p.mt * (p.pair ? 2 * tc::TN : tc::TN) * 4;
-}
+size_t qgemm_tc_partial_bytes(const GemmTcPlan &p) { return (size_t)p.split_units() * p.mt * (p.pair ? 2 * tc::TN : tc::TN) * 4; }
 
 bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, const void *w) {
     if (fmt != FMT_Q4K && fmt != FMT_Q5K && fmt != FMT_Q6K) return false;
@@ -976,12 +963,11 @@ cudaError_t launch_qgemm_tc_moe(int fmt, const GemmTcArgs &a, uint32_t experts, 
     return tc::launch_plan(fmt, b, pl, mw, ma, sm_count, pdl, stream);
 }
 
-cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, void *a_bf16_scratch, bool copy, void *partial, int sm_count, bool pdl,
+cudaError_t launch_qgemm_tc(int fmt, const GemmTcArgs &a, const GemmTcPlan &pl, void *a_bf16_scratch, bool copy, void *partial, int sm_count, bool pdl,
                             cudaStream_t stream, int *launched) {
     using namespace tc;
     *launched = 0;
     if (a.rows == 0 || a.n == 0) return cudaSuccess;
-    const tc::Plan pl = tc_plan(a.rows, a.n, a.k, sm_count);
     if ((uint64_t)pl.nx * pl.ny * pl.splits >= (1u << 31)) return cudaErrorInvalidValue;
     CUtensorMap mw, ma;
     if (cudaError_t e = tc_maps(fmt, a, a.n, pl, a_bf16_scratch, mw, ma); e != cudaSuccess) return e;

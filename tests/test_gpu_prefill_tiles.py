@@ -129,3 +129,28 @@ def test_q6k_infinite_scale_stays_infinite(be, m, k):
     assert np.isposinf(want[:, 0]).all() and np.isneginf(want[:, [1, 129]]).all()
     assert np.array_equal(got[:, [0, 1, 129]], want[:, [0, 1, 129]])
     _close(got[:, 2:129], want[:, 2:129])
+
+
+@pytest.mark.parametrize("option,value", [("gemm_splitk", "0"), ("gemm_pair", "0")])
+def test_tile_options_belong_to_the_device(be, option, value):
+    """An option set on one device leaves the launches of another as they are (the plan of a launch, and with it its part of the scratch, depends on both)."""
+    fmt, m, n, k = lp.DType.Q4K, 300, 1024, 4096  # (K split 8 ways in pairs, 6 ways without)
+    x, w = O.normal(5500, m * k), O.normal(5501, n * k, 0.05)
+    other = lp.Backend(0)
+    ls = [matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)]
+
+    def run(dev):
+        bufs = [dev.upload(x), dev.upload(quant.quantize(dev, fmt, w, n, k)), dev.alloc(m * n * 4)]
+        dev.take_launch_count()
+        dev.execute(ls, bufs)
+        return dev.take_launch_count(), bufs[2].download().view(np.float32).copy()
+
+    before = run(be)
+    other.set_option(option, value)
+    try:
+        theirs, after = run(other), run(be)
+    finally:
+        other.set_option(option, "-1")
+    assert before[0] == 3 and after[0] == 3 and np.array_equal(after[1], before[1])
+    assert theirs[0] == 2 if option == "gemm_splitk" else not np.array_equal(theirs[1], before[1])  # (the option is not without effect)
+    _close(theirs[1], before[1])
