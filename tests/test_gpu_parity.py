@@ -655,17 +655,17 @@ def bf16_round(x):
     return u.astype(np.uint32).view(np.float32)
 
 
-@pytest.mark.parametrize("tall", ["-1", "1"])
+@pytest.mark.parametrize("pair", ["-1", "0"])
 @pytest.mark.parametrize("fmt,ofmt", [(lp.DType.Q4K, O.Q4_K), (lp.DType.Q5K, O.Q5_K), (lp.DType.Q6K, O.Q6_K)])
-def test_gemm_tensor_core(be, oracle, fmt, ofmt, tall):
-    be.set_option("gemm_tall", tall)   # "1": 512 activation rows per CTA wherever a launch has more than 256 rows
+def test_gemm_tensor_core(be, oracle, fmt, ofmt, pair):
+    be.set_option("gemm_pair", pair)   # "0": single CTAs also above 128 rows
     try:
-        _gemm_tensor_core_cases(be, oracle, fmt, ofmt, tall == "1")
+        _gemm_tensor_core_cases(be, oracle, fmt, ofmt, pair == "0")
     finally:
-        be.set_option("gemm_tall", "-1")
+        be.set_option("gemm_pair", "-1")
 
 
-def _gemm_tensor_core_cases(be, oracle, fmt, ofmt, tall_only):
+def _gemm_tensor_core_cases(be, oracle, fmt, ofmt, above_128_only):
     """bf16 tensor-core prefill (Q4_K; Q6_K when K is a multiple of 2048): stated bounds vs lapid-cpu's
     f32 path are rel_l2 <= 4e-3 and max_rel <= 2e-2 (both operands rounded to bf16, 2^-9 each; the
     reference allows 2e-3 for its f16 tensor-core kernel, crates/lapid-cuda/src/kquant_tests.rs:191-192).
@@ -682,7 +682,7 @@ def _gemm_tensor_core_cases(be, oracle, fmt, ofmt, tall_only):
           (1, 64, 256, 512, 0, False), (1, 33, 300, 1024, 0, True), (1, 140, 131, 3584, 0, False), (1, 9, 5, 256, 0, False)]
     for (batch, m, n, k, pad, epi) in (q4 if fmt == lp.DType.Q4K else q6):
         seed += 1
-        if tall_only and batch * m <= 256:
+        if above_128_only and batch * m <= 128:
             continue
         big = n * k > 200000
         w = O.normal(seed, n * k, 0.02) if big else rnd(n * k, seed)
@@ -709,26 +709,27 @@ def _gemm_tensor_core_cases(be, oracle, fmt, ofmt, tall_only):
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
-def test_gemm_tensor_core_cta_pairs(be, oracle):
-    """Q4_K prefill with two CTAs per tensor-core unit (`cta_group::2`): the same bounds as the
+@pytest.mark.parametrize("fmt,ofmt", [(lp.DType.Q4K, O.Q4_K), (lp.DType.Q5K, O.Q5_K), (lp.DType.Q6K, O.Q6_K)])
+def test_gemm_tensor_core_cta_pairs(be, oracle, fmt, ofmt):
+    """Prefill with two CTAs per tensor-core unit (`cta_group::2`): the same bounds as the
     single-CTA kernel and, since the products and the f32 accumulation order per output are the same,
     the same bits."""
     seed = 400
     for (m, n, k, epi) in [(512, 1024, 4096, False), (300, 1000, 1024, True), (260, 700, 512, False), (1000, 512, 2048, False)]:
         seed += 1
-        qb = oracle.quantize(O.Q4_K, O.normal(seed, n * k, 0.02), n, k)
+        qb = oracle.quantize(ofmt, O.normal(seed, n * k, 0.02), n, k)
         a = O.normal(seed + 7, m * k)
         bias = rnd(n, seed + 9) if epi else None
         be.set_option("gemm_splitk", "0")   # same k order in both runs
         be.set_option("gemm_pair", "1")
         try:
-            got = run_matmul(be, lp.DType.Q4K, a, qb, m, n, k, bias=bias).reshape(m, n)
+            got = run_matmul(be, fmt, a, qb, m, n, k, bias=bias).reshape(m, n)
             be.set_option("gemm_pair", "0")
-            ref = run_matmul(be, lp.DType.Q4K, a, qb, m, n, k, bias=bias).reshape(m, n)
+            ref = run_matmul(be, fmt, a, qb, m, n, k, bias=bias).reshape(m, n)
         finally:
-            be.set_option("gemm_pair", "0")
+            be.set_option("gemm_pair", "-1")
             be.set_option("gemm_splitk", "-1")
-        deq = oracle.dequantize(O.Q4_K, qb, n, k)
+        deq = oracle.dequantize(ofmt, qb, n, k)
         rounded = bf16_round(a.reshape(m, k)).astype(np.float64) @ bf16_round(deq).astype(np.float64).T + (bias.astype(np.float64) if epi else 0.0)
         assert rel_l2(got, rounded) <= 2e-5, (m, n, k, rel_l2(got, rounded))
         assert np.array_equal(got, ref), (m, n, k)

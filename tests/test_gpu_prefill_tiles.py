@@ -9,7 +9,7 @@ import pytest
 
 import lapid_b200 as lp
 from lapid_b200 import quant
-from lapid_b200.backend import MatView, matmul_id_launch, matmul_launch
+from lapid_b200.backend import MatView, gather_launch, matmul_id_launch, matmul_launch
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -43,32 +43,40 @@ def _both(be, launches, bufs, out):
 
 
 @pytest.mark.parametrize("fmt", FORMATS)
-@pytest.mark.parametrize("m,n,k", [(9, 1, 256), (16, 127, 512), (17, 129, 768), (112, 130, 2048), (128, 300, 1024), (129, 100, 256), (129, 257, 1280),
-                                   (161, 255, 2048), (256, 513, 512), (257, 384, 768), (600, 200, 512)])
+@pytest.mark.parametrize("m,n,k,pair", [(m, n, k, pair) for pair in ("-1", "0") for m, n, k in [
+    (9, 1, 256), (16, 127, 512), (17, 129, 768), (112, 130, 2048), (128, 300, 1024), (129, 100, 256), (129, 257, 1280), (161, 255, 2048), (256, 513, 512),
+    (257, 384, 768), (600, 200, 512)] if pair == "-1" or m > 128])
 @pytest.mark.parametrize("ways", ["-1", "0", "3"])
-def test_rows_columns_and_splits(be, fmt, m, n, k, ways):
+def test_rows_columns_and_splits(be, fmt, m, n, k, ways, pair):
     x, w = O.normal(5000 + m, m * k), O.normal(5001 + n, n * k, 0.05)
     bufs = [be.upload(x), be.upload(quant.quantize(be, fmt, w, n, k)), be.alloc(m * n * 4), be.upload(O.normal(5002, n))]
     for extra in ({}, {"bias_input": 3}):
         be.set_option("gemm_splitk", ways)
+        be.set_option("gemm_pair", pair)
         try:
             got, want = _both(be, [matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, **extra)], bufs, 2)
         finally:
             be.set_option("gemm_splitk", "-1")
+            be.set_option("gemm_pair", "-1")
         _close(got, want)
 
 
-@pytest.mark.parametrize("m,n", [(40, 152 * 128), (300, 38 * 256)])
-def test_whole_tiles_beside_split_ones(be, m, n):
-    """A last round of a few tiles (split over K) behind a full one; the launch by itself and again give the same bits."""
-    fmt, k = lp.DType.Q4K, 1024
+@pytest.mark.parametrize("m", [40, 300])
+@pytest.mark.parametrize("fmt", FORMATS)
+def test_whole_tiles_beside_split_ones(be, fmt, m):
+    """A last round of two tiles of a pair (four of a CTA), split over K, behind a full one; the launch by itself and again give the same bits."""
+    import torch
+    sms, k = torch.cuda.get_device_properties(0).multi_processor_count, 1024
+    n = (sms + 4) * 128 if m <= 128 else (sms // 2 + 2) // 2 * 256   # 300 rows: two activation tiles
     x, w = O.normal(5100, m * k), np.tile(O.normal(5101, 512 * k, 0.05), n // 512 + 1)[: n * k]
     w = (w.reshape(n, k) * (1 + 0.001 * (np.arange(n, dtype=np.float32) % 991))[:, None]).astype(np.float32)
     bufs = [be.upload(x), be.upload(quant.quantize(be, fmt, w, n, k)), be.alloc(m * n * 4)]
     ls = [matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)]
     got, want = _both(be, ls, bufs, 2)
     _close(got, want)
+    be.take_launch_count()
     be.execute(ls, bufs)
+    assert be.take_launch_count() == 3   # the copy, the products, the sum of the split tiles
     assert np.array_equal(bufs[2].download().view(np.float32), got)
 
 
@@ -84,9 +92,9 @@ def test_rows_of_several_batch_entries_in_one_tile(be):
     assert np.array_equal(got == -7.0, want == -7.0)
 
 
-@pytest.mark.parametrize("rewrite", [False, True])
+@pytest.mark.parametrize("rewrite", [None, "tokens", "ids"])
 def test_expert_indexed_launches_share_their_tables(be, rewrite):
-    """Gate and up of one list use the same routing tables and gathered rows; a launch that rewrites the tokens in between ends that.
+    """Gate and up of one list use the same routing tables and gathered rows; a launch that rewrites the tokens or the ids in between ends that.
     Every result has the bits of the launch run by itself."""
     fmt, t, r, e, n, k = lp.DType.Q4K, 70, 2, 6, 256, 512
     ids = np.stack([np.random.default_rng(i).permutation(e)[:r] for i in range(t)]).astype(np.int32)
@@ -97,11 +105,16 @@ def test_expert_indexed_launches_share_their_tables(be, rewrite):
     bufs = [be.upload(x), be.upload(ids)] + [be.upload(s) for s in stacks] + [be.alloc(t * r * n * 4) for _ in range(2)]
     bufs += [be.upload(y), be.upload(quant.quantize(be, fmt, O.normal(5312, k * k, 0.05), k, k))]
     ls = [matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 2, 1), output=4), matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 3, 1), output=5)]
-    if rewrite:
+    if rewrite == "tokens":
         ls.insert(1, matmul_launch(fmt, t, k, k, inputs=(6, 7), output=0))
+    elif rewrite == "ids":  # a gather of the table's one row: other ids, bit for bit
+        other = ids[::-1].copy()
+        bufs += [be.upload(other.view(np.float32).reshape(1, -1)), be.upload(np.zeros(1, np.int32))]
+        ls.insert(1, gather_launch(lp.DType.F32, 1, t * r, 1, inputs=(8, 9), output=1))
     res, counts = [], []
     for one_list in (False, True):
         bufs[0].write(0, x)
+        bufs[1].write(0, ids)
         be.take_launch_count()
         for part in [ls] if one_list else [[l] for l in ls]:
             be.execute(part, bufs)
