@@ -1035,8 +1035,10 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             if (slot) copy_at = slot->copy_offset, partial_at = slot->offset, made = slot - (slot->owner >= 0 ? slot->owner : 0);
             else dev.ensure_scratch(p.scratch);
             int launched = 0;
-            // Everything older than the kernel in front has completed when a kernel of this chain starts (each lets its successor start
-            // behind its own wait), so the weights may be read at once unless a launch of this list writes them.
+            // The weights may be read before the dependency wait unless a launch of this list writes them: the copy of the operand, this
+            // launch's or the one it shares, was made in this list by a kernel that waits before it lets anything behind it start, so all that
+            // is older than the list has completed. That holds as well behind kernels that let their successor start before their own
+            // wait (early decode kernels, qgemv_kq_finalize_kernel): in this list they come behind that copy.
             t.w_early = slot && !src_written;
             cuda_check(lb::launch_qgemm_tc(l.b_dtype, t, p.tc_plan, (char *)dev.scratch + copy_at, !(made && made->done), (char *)dev.scratch + partial_at,
                                            dev.sm_count, dev.pdl, dev.stream, &launched), "qgemm_tc launch");

@@ -6,7 +6,7 @@ import pytest
 
 import lapid_b200 as lp
 from lapid_b200 import tp
-from lapid_b200.backend import DType, MatView, matmul_id_launch, matmul_launch
+from lapid_b200.backend import DType, MatView, gather_launch, matmul_id_launch, matmul_launch
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -204,11 +204,11 @@ def test_expert_prompt_repeats_bit_for_bit():
 
 @pytest.mark.parametrize("writer_rows", [8, 40, 300])
 @pytest.mark.parametrize("fmt", [DType.Int8, DType.Int4, DType.Q4K, DType.Q5K])
-@pytest.mark.parametrize("m", [1, 2, 8])
+@pytest.mark.parametrize("m", [1, 2, 8, 77, 300])
 def test_weights_written_by_an_earlier_launch_of_the_list(fmt, m, writer_rows):
-    """A launch of the list (decode or prefill on the tensor cores) stores into the packed bytes of a later decode launch's weights; the f32
+    """A launch of the list (decode or prefill on the tensor cores) stores into the packed bytes of a later launch's weights; the f32
     results are taken as the bytes they are, the scales stay. The later launch's activations are clean, so nothing stands between the
-    two kernels; its weights must be the written ones, plain and captured."""
+    two kernels of a decode launch; its weights must be the written ones, plain and captured."""
     import torch
     per_block = {DType.Int8: 8, DType.Int4: 4, DType.Q4K: 32, DType.Q5K: 32}[fmt]     # floats that a block's packed values take
     first, pitch = {DType.Q4K: (4, 36), DType.Q5K: (12, 44)}.get(fmt, (0, per_block))  # where they lie: floats before them, from block to block
@@ -251,5 +251,92 @@ def test_weights_written_by_an_earlier_launch_of_the_list(fmt, m, writer_rows):
                 got = out.view(torch.int32).clone()
             s1.synchronize()
             assert torch.equal(got, wants[rep % 2]), rep
+    serial.synchronize()
+    be.synchronize()
+
+
+@pytest.mark.parametrize("how", ["copy", "kernel", "gather"])
+@pytest.mark.parametrize("fmt", [DType.Q4K, DType.Q6K])
+@pytest.mark.parametrize("m", [77, 300])
+def test_prefill_weights_rewritten_right_before_the_launch(fmt, m, how):
+    """Weights that a copy or a kernel in front of the list, or a Gather (which copies bytes) in front of the launch, has just rewritten: the tensor-core
+    kernel requests packed weights before its dependency wait, and must get the new ones."""
+    import torch
+    serial, s0 = _device(pdl="0")
+    be, s1 = _device()
+    n, k = 1024, 2048
+    sets = [_weights(be, int(fmt), n, k, 1000 + i) for i in range(2)]
+    source, w = sets[0].clone(), torch.zeros_like(sets[0])
+    x, out = torch.from_numpy(O.normal(1010, m * k).reshape(m, k)).cuda(), torch.zeros(m, n, device="cuda")
+    row = torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    launch = matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)
+    ls = [gather_launch(DType.F32, 1, w.numel() // 4, 1, inputs=(3, 4), output=1), launch] if how == "gather" else [launch]
+    wants = []
+    for a in sets:
+        serial.execute([launch], [serial.wrap_tensor(t) for t in (x, a, out)])
+        wants.append(out.clone())
+        torch.cuda.synchronize()
+    assert not torch.equal(*wants)
+    bufs = [be.wrap_tensor(t) for t in (x, w, out, source, row)]
+
+    def queue():
+        if how == "copy":
+            w.copy_(source)
+        elif how == "kernel":
+            torch.add(source, 0, out=w)
+        be.execute_async(ls, bufs)
+
+    graph = _capture(be, s1, queue)
+    for rep in range(20):
+        for run in (queue, graph.replay):
+            with torch.cuda.stream(s1):
+                source.copy_(sets[rep % 2])
+                w.copy_(sets[(rep + 1) % 2])
+                out.zero_()
+                run()
+                got = out.clone()
+            s1.synchronize()
+            assert torch.equal(got, wants[rep % 2]), rep
+    serial.synchronize()
+    be.synchronize()
+
+
+@pytest.mark.parametrize("m", [77, 300])
+def test_prefill_with_a_shared_copy_behind_an_early_decode_launch(m):
+    """Two prefill launches of one operand share its bf16 copy; a decode launch between them lets the second start before it has waited itself.
+    The copy and both results have the bits of the serial order."""
+    import torch
+    serial, s0 = _device(pdl="0")
+    be, s1 = _device()
+    n, k = 1024, 2048
+    w1, w2, wd = (_weights(be, int(DType.Q4K), n, k, 1020 + i) for i in range(3))
+    inputs = [torch.from_numpy(O.normal(1030 + i, m * k).reshape(m, k)).cuda() for i in range(2)]
+    x, xd = torch.zeros(m, k, device="cuda"), torch.from_numpy(O.normal(1040, k).reshape(1, k)).cuda()
+    outs = [torch.zeros(r, n, device="cuda") for r in (m, m, 1)]
+    torch.cuda.synchronize()
+    ls = [matmul_launch(DType.Q4K, m, n, k, inputs=(0, 1), output=5), matmul_launch(DType.Q4K, 1, n, k, inputs=(4, 3), output=7),
+          matmul_launch(DType.Q4K, m, n, k, inputs=(0, 2), output=6)]
+    tensors = (x, w1, w2, wd, xd, *outs)
+    wants = []
+    for a in inputs:
+        x.copy_(a)
+        torch.cuda.synchronize()
+        for l in ls:
+            serial.execute([l], [serial.wrap_tensor(t) for t in tensors])
+        wants.append([o.clone() for o in outs])
+        torch.cuda.synchronize()
+    bufs = [be.wrap_tensor(t) for t in tensors]
+    graph = _capture(be, s1, lambda: be.execute_async(ls, bufs))
+    for rep in range(20):
+        for run in (lambda: be.execute_async(ls, bufs), graph.replay):
+            with torch.cuda.stream(s1):
+                x.copy_(inputs[rep % 2])
+                for o in outs:
+                    o.zero_()
+                run()
+                got = [o.clone() for o in outs]
+            s1.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(got, wants[rep % 2])), rep
     serial.synchronize()
     be.synchronize()
