@@ -103,6 +103,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     }
     return false;
 }
+// A producer's last waits: for the copies it has issued into a ring of COUNT slots; (slot, phase) are its next ones, so the slots below were last filled
+// in this lap and the others in the lap before (in the first lap: never, and the wait returns at once).
+template <int COUNT> __device__ __forceinline__ void wait_for_copies(uint64_t *full, uint32_t slot, uint32_t phase) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < COUNT; i++) mbar_wait(full + i, i < slot ? phase ^ 1 : phase);
+}
 // A whole warp waits: all lanes or none give up.
 __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
@@ -457,7 +463,17 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     if (++s == STAGES) s = 0, ph ^= 1;
                 }
             }
-            if (!healthy && p.status) atomicOr(p.status, 2);
+            // Nothing may arrive in this CTA's shared memory or use its tensor memory once it leaves: the products have read every stage that was
+            // filled (a pair's second CTA hears that from the first), and when a role gave up, the copies into the others are done.
+            const uint32_t s_next = s, ph_next = ph;
+            for (int i = 0; i < STAGES && healthy; i++) {
+                healthy = mbar_wait(empty + s, ph);
+                if (++s == STAGES) s = 0, ph ^= 1;
+            }
+            if (!healthy) {
+                wait_for_copies<STAGES>(full_a, s_next, ph_next);
+                if (p.status) atomicOr(p.status, 2);
+            }
         }
     } else if (warp == RAW_WARP && FMT == FMT_Q6K && ((nblk_total * Q6K_BYTES) & 15u) != 0) {
         // ---------------- packed Q6_K weights whose rows are not a multiple of 16 bytes (K not a
@@ -494,6 +510,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (++r == C::RAWS) r = 0, ph ^= 1;
             }
         }
+        if (lane == 0) wait_for_copies<C::RAWS>(raw_full, r, ph);  // (done already unless the expanding warps gave up)
         if (!healthy && lane == 0 && p.status) atomicOr(p.status, 32);
     } else if (warp == RAW_WARP) {
         // ---------------- TMA producer, packed weights: one super-block of every row of the tile
@@ -511,6 +528,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     if (++r == C::RAWS) r = 0, ph ^= 1;
                 }
             }
+            wait_for_copies<C::RAWS>(raw_full, r, ph);  // (done already unless the expanding warps gave up)
             if (!healthy && p.status) atomicOr(p.status, 32);
         }
     } else if (warp == MMA_WARP && PAIR && rank == 1) {
