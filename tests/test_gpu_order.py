@@ -340,3 +340,27 @@ def test_prefill_with_a_shared_copy_behind_an_early_decode_launch(m):
             assert all(torch.equal(a, b) for a, b in zip(got, wants[rep % 2])), rep
     serial.synchronize()
     be.synchronize()
+
+
+def test_prefill_behind_a_launch_that_takes_long():
+    """Two launches share their operand's copy, and the first keeps one SM busy for tens of milliseconds (one tile, K not split): the second, which
+    starts beside it, must wait that long for its activations and not give up."""
+    import torch
+    be, stream = _device(gemm_splitk="0")
+    m, n, k = 9, 128, 1 << 24
+    w = torch.randint(0, 256, (n * k // 256, 144), dtype=torch.uint8, device="cuda")
+    w[:, :4] = torch.full((len(w), 2), 1e-4, device="cuda").half().view(torch.uint8)
+    x = torch.randn(m, k, device="cuda")
+    outs = [torch.zeros(m, n, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    bufs = [be.wrap_tensor(t) for t in (x, w.reshape(-1), *outs)]
+    ls = [matmul_launch(DType.Q4K, m, n, k, inputs=(0, 1), output=2 + i) for i in range(2)]
+    be.execute(ls, bufs)
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    with torch.cuda.stream(stream):
+        start.record()
+        be.execute_async(ls[:1], bufs)
+        end.record()
+    be.execute(ls, bufs)
+    assert start.elapsed_time(end) > 20
+    assert torch.isfinite(outs[0]).all() and outs[0].any() and torch.equal(*outs)
