@@ -29,7 +29,7 @@
 //              K=16 steps per k-step) and commits to mbarriers
 //   warp 18    one lane drives TMA for the weights: per super-block a 2-D tensor-map copy of the 128 rows' packed blocks
 //              (144 / 176 bytes; Q6_K: 240 bytes from the 16-byte boundary below the 2-byte aligned 210); Q6_K rows
-//              that are not 16-byte multiples are copied row by row with the plain bulk copy by all lanes of the warp
+//              that are not 16-byte multiples come in eight copies of every eighth row
 // A CTA (pair) takes every gridDim-th unit of the launch: no CTA start and no first trip to HBM per tile, and the first two
 // super-blocks of a tile are expanded before the results of the one before are stored. Tensor memory: 256 columns of accumulators
 // (one 256-column set for a pair, two of 128 for a single CTA), 4 stages of 64 columns (two k-steps) of weights.
@@ -72,7 +72,7 @@ template <int FMT, bool PAIR> struct Cfg {
     static constexpr int ACCS = PAIR ? 1 : 2;    // accumulator sets of MT columns
     static constexpr int A_BYTES = STAGE_KS * 128 * 128;  // activations of one stage in this CTA: up to 128 rows of 64 bf16, twice
     static constexpr int ROW_BYTES = FMT == FMT_Q4K ? Q4K_BYTES : FMT == FMT_Q5K ? Q5K_BYTES : Q6K_BOX;  // packed bytes staged per row and super-block
-    static constexpr int RAW = TN * ROW_BYTES;
+    static constexpr int RAW = (TN + (FMT == FMT_Q6K ? 8 : 0)) * ROW_BYTES;  // (Q6_K: and room for rows copied one by one)
     // Super-blocks of packed weights in flight or in use: as many as the shared memory has room for (5 / 4 / 3)
     static constexpr int RAWS = (227 * 1024 - 512 - 1024 - STAGES * A_BYTES) / RAW;
     static_assert(RAWS >= 3 && 3 * STAGES + 2 * RAWS + 5 <= 64, "shared memory");
@@ -477,42 +477,48 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             }
         }
     } else if (warp == RAW_WARP && FMT == FMT_Q6K && ((nblk_total * Q6K_BYTES) & 15u) != 0) {
-        // ---------------- packed Q6_K weights whose rows are not a multiple of 16 bytes (K not a
-        // multiple of 2048, e.g. the K/8 shard of a row-parallel projection): no tensor map can
-        // describe them, so every lane copies rows of the tile with the plain bulk copy, each from
-        // the 16-byte boundary below its block (the consumers compute the same per-row offset)
-        const uint64_t pitch = (uint64_t)nblk_total * Q6K_BYTES;
-        const uint64_t end16 = ((uint64_t)(uintptr_t)p.w + (uint64_t)p.n * pitch + 15) & ~(uint64_t)15;  // never read past the matrix's last 16-byte line
-        uint32_t r = 0, ph = 1;
-        Tile o;
-        for (uint32_t u = first; u < units && healthy; u += step) {
-            if (!tile_at(u, o)) continue;
-            const uint32_t rows_valid = min((uint32_t)TN, p.n > o.n0 ? p.n - o.n0 : 0u);
-            auto copy_of = [&](uint32_t rr, uint32_t b, uint64_t &src) -> uint32_t {
-                src = ((uint64_t)(uintptr_t)p.w + (uint64_t)(o.n0 + rr) * pitch + (uint64_t)(o.kb0 + b) * Q6K_BYTES) & ~(uint64_t)15;
-                return (uint32_t)min((uint64_t)224, end16 - src);
-            };
-            for (uint32_t b = 0; b < o.nblk; b++) {
-                if (!warp_wait(raw_empty + r, ph)) { healthy = false; break; }
-                if (lane == 0) {
+        // ---------------- TMA producer, packed Q6_K weights whose rows are not a multiple of 16 bytes (K not a multiple of 2048, e.g. the K/8 shard of a
+        // row-parallel projection). Eight rows are: a row of the tensor map is a group of eight, and copy number g brings row g of the
+        // tile's 16 groups, from the 16-byte boundary below its block (the consumers compute the same offset), to the 16 places from 16 g on.
+        // Rows behind the last whole group are copied one by one, to the places behind the tile's.
+        // What bounds it is the number of copies: with one of each row (128 in place of 8) a super-block took 6 us, 2048 rows on 8192 x 3584 275 us (now
+        // 118), 77 rows 45 (21).
+        if (lane == 0) {
+            const uint64_t pitch = (uint64_t)nblk_total * Q6K_BYTES;
+            const uint64_t end16 = ((uint64_t)(uintptr_t)p.w + (uint64_t)p.n * pitch + 15) & ~(uint64_t)15;  // never read past the matrix's last 16-byte line
+            const uint32_t grouped = p.n & ~7u;
+            uint32_t r = 0, ph = 1;
+            Tile o;
+            for (uint32_t u = first; u < units && healthy; u += step) {
+                if (!tile_at(u, o)) continue;
+                const uint32_t single = grouped >= o.n0 && grouped < o.n0 + TN ? p.n - grouped : 0;
+                auto copy_of = [&](uint32_t i, uint32_t b, uint64_t &src) -> uint32_t {
+                    src = ((uint64_t)(uintptr_t)p.w + (uint64_t)(grouped + i) * pitch + (uint64_t)(o.kb0 + b) * Q6K_BYTES) & ~(uint64_t)15;
+                    return (uint32_t)min((uint64_t)224, end16 - src);
+                };
+                for (uint32_t b = 0; b < o.nblk; b++) {
+                    if (!mbar_wait(raw_empty + r, ph)) { healthy = false; break; }
+                    uint8_t *dst = raw0 + r * C::RAW;
                     uint64_t src;
-                    if (rows_valid) mbar_expect_tx(raw_full + r, (rows_valid - 1) * 224 + copy_of(rows_valid - 1, b, src));  // only the last row can be short
-                    else mbar_arrive(raw_full + r);  // (the second CTA of a pair past the last row)
+                    uint32_t bytes = grouped ? TN * Q6K_BOX : 0;
+                    for (uint32_t i = 0; i < single; i++) bytes += copy_of(i, b, src);
+                    if (bytes) mbar_expect_tx(raw_full + r, bytes);
+                    else mbar_arrive(raw_full + r);  // (fewer than eight rows: the second CTA of a pair has none)
+                    if (grouped)
+                        for (uint32_t g = 0; g < 8; g++)
+                            tma_load_2d(dst + g * (TN / 8) * Q6K_BOX, &map_w, (int)((g * pitch + (uint64_t)(o.kb0 + b) * Q6K_BYTES) & ~(uint64_t)15), (int)(o.n0 / 8), raw_full + r);
+                    for (uint32_t i = 0; i < single; i++) {
+                        const uint32_t n = copy_of(i, b, src);
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s32(dst + (TN + i) * Q6K_BOX)),
+                                     "l"(src), "r"(n), "r"(s32(raw_full + r))
+                                     : "memory");
+                    }
+                    if (++r == C::RAWS) r = 0, ph ^= 1;
                 }
-                __syncwarp();
-                for (uint32_t rr = lane; rr < rows_valid; rr += 32) {
-                    uint64_t src;
-                    const uint32_t bytes = copy_of(rr, b, src);
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                     s32(raw0 + r * C::RAW + rr * Q6K_BOX)),
-                                 "l"(src), "r"(bytes), "r"(s32(raw_full + r))
-                                 : "memory");
-                }
-                if (++r == C::RAWS) r = 0, ph ^= 1;
             }
+            wait_for_copies<C::RAWS>(raw_full, r, ph);  // (done already unless the expanding warps gave up)
+            if (!healthy && p.status) atomicOr(p.status, 32);
         }
-        if (lane == 0) wait_for_copies<C::RAWS>(raw_full, r, ph);  // (done already unless the expanding warps gave up)
-        if (!healthy && lane == 0 && p.status) atomicOr(p.status, 32);
     } else if (warp == RAW_WARP) {
         // ---------------- TMA producer, packed weights: one super-block of every row of the tile
         // per copy, up to RAWS super-blocks (of four k-steps) ahead of the expanding warps
@@ -523,7 +529,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (!tile_at(u, o)) continue;
                 for (uint32_t b = 0; b < o.nblk; b++) {
                     if (!mbar_wait(raw_empty + r, ph)) { healthy = false; break; }
-                    mbar_expect_tx(raw_full + r, C::RAW);
+                    mbar_expect_tx(raw_full + r, TN * C::ROW_BYTES);
                     tma_load_2d(raw0 + r * C::RAW, &map_w, FMT == FMT_Q6K ? (int)(((o.kb0 + b) * Q6K_BYTES) & ~15u) : (int)((o.kb0 + b) * C::ROW_BYTES),
                                 (int)(o.wrow0 + o.n0), raw_full + r);
                     if (++r == C::RAWS) r = 0, ph ^= 1;
@@ -681,19 +687,23 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const uint32_t pitch = nblk_total * Q6K_BYTES;
         const bool uniform = (pitch & 15u) == 0;
         auto skew_of = [&](uint32_t kb, uint32_t first_row) { return (kb * Q6K_BYTES + (first_row + row) * pitch) & 15u; };  // (p.w is 16-byte aligned; only the low bits matter)
+        uint32_t place = row;  // which staged row is this thread's (of the current tile; see the producer)
         auto load = [&](Packed<FMT> &w, uint32_t kb, uint32_t first_row) {  // (the place of the block matters for Q6_K only)
             if (!warp_wait(raw_full + r, rph)) {
                 healthy = false;
                 return;
             }
-            const uint8_t *blk = raw0 + r * C::RAW + row * C::ROW_BYTES;
+            const uint8_t *blk = raw0 + r * C::RAW + place * C::ROW_BYTES;
             if constexpr (FMT == FMT_Q6K) load_packed_q6<0>(w, blk, skew_of(kb, first_row), uniform, j);
             else load_packed<FMT>(w, blk, j);
         };
         constexpr bool AHEAD = FMT == FMT_Q4K;    // (Q5_K, Q6_K: too many words a share to hold twice)
         uint32_t u = valid(first), done = 0;      // the current unit; the one whose results are to be stored
         uint32_t kb0 = 0, n0 = 0, nblk = 0;
-        auto enter = [&]() { nblk = u < units ? o.nblk : 0, kb0 = o.kb0, n0 = o.n0; };
+        auto enter = [&]() {
+            nblk = u < units ? o.nblk : 0, kb0 = o.kb0, n0 = o.n0;
+            if (FMT == FMT_Q6K && !uniform) place = n0 + row < (p.n & ~7u) ? (row & 7) * (TN / 8) + (row >> 3) : TN + (row & 7);
+        };
         enter();
         Packed<FMT> cur;
         if (AHEAD && nblk) load(cur, 0, 0);
@@ -718,7 +728,7 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (!healthy || !warp_wait(empty + s, ((sb >> 1) & 1) ^ 1)) { healthy = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 tmem_st16(col, w);
-                if constexpr (FMT == FMT_Q6K) load_packed_q6<1>(cur, raw0 + slot * C::RAW + row * C::ROW_BYTES, skew_of(kb0 + b, n0), uniform, j);
+                if constexpr (FMT == FMT_Q6K) load_packed_q6<1>(cur, raw0 + slot * C::RAW + place * C::ROW_BYTES, skew_of(kb0 + b, n0), uniform, j);
                 expand<FMT, 1>(cur, j, e23, w);
                 tmem_st16(col + 16, w);
                 tmem_st_wait();
@@ -880,6 +890,8 @@ static cudaError_t launch_plan(int fmt, const GemmTcArgs &a, const Plan &pl, con
 
 bool qgemm_tc_supported(int fmt, const GemmTcArgs &a) {
     if (a.k % QK != 0 || a.k < QK || a.rows < 1 || ((uintptr_t)a.w & 15) != 0 || tc::encode_fn() == nullptr) return false;
+    // (Q6_K rows that are not 16-byte multiples are copied by byte offsets inside groups of eight: a 32-bit coordinate)
+    if (fmt == FMT_Q6K && a.k / QK * Q6K_BYTES % 16 != 0 && 8 * (uint64_t)(a.k / QK) * Q6K_BYTES >= (1ull << 31)) return false;
     return fmt == FMT_Q4K || fmt == FMT_Q5K || fmt == FMT_Q6K;
 }
 
@@ -934,7 +946,8 @@ bool qgemm_tc_moe_supported(int fmt, uint64_t experts, uint64_t n, uint64_t k, c
     return pitch % 16 == 0 && (n * pitch) % 256 == 0 && experts * n < (1ull << 31);
 }
 
-// Tensor maps: packed weights as bytes [weight rows][row bytes], box = one block (Q6_K: the 240 bytes around one) of 128 rows; bf16 activations
+// Tensor maps: packed weights as bytes [weight rows][row bytes], box = one block (Q6_K: the 240 bytes around one) of 128 rows (Q6_K rows that are not
+// 16-byte multiples: [groups of eight rows][their bytes], box = 240 bytes of 16 groups); bf16 activations
 // [k / 64][rows][64], box = 64 k (128 bytes, swizzled) x the rows a CTA loads x the k-steps of a stage.
 static cudaError_t tc_maps(int fmt, const GemmTcArgs &a, uint64_t weight_rows, const tc::Plan &pl, void *a_bf16, CUtensorMap &mw, CUtensorMap &ma) {
     const tc::EncodeTiledFn enc = tc::encode_fn();
@@ -945,7 +958,11 @@ static cudaError_t tc_maps(int fmt, const GemmTcArgs &a, uint64_t weight_rows, c
         cuuint64_t dims[2] = {(cuuint64_t)(a.k / QK) * blk_bytes, weight_rows};
         cuuint64_t strides[1] = {(cuuint64_t)(a.k / QK) * blk_bytes};
         cuuint32_t box[2] = {(cuuint32_t)tc_box_bytes(fmt), tc::TN};
-        if (strides[0] % 16 != 0) std::memset(&mw, 0, sizeof(mw));  // Q6_K with K not a multiple of 2048: the kernel copies rows itself
+        if (strides[0] % 16 != 0) {  // Q6_K with K not a multiple of 2048: a row of the map is a group of eight, a copy takes one row of 16 groups
+            dims[0] *= 8, strides[0] *= 8, dims[1] /= 8;
+            box[1] = tc::TN / 8;
+        }
+        if (dims[1] == 0) std::memset(&mw, 0, sizeof(mw));  // (no whole group: not used)
         else if (enc(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)a.w, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;

@@ -167,3 +167,14 @@ def test_tile_options_belong_to_the_device(be, option, value):
     assert before[0] == 3 and after[0] == 3 and np.array_equal(after[1], before[1])
     assert theirs[0] == 2 if option == "gemm_splitk" else not np.array_equal(theirs[1], before[1])  # (the option is not without effect)
     _close(theirs[1], before[1])
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 128, 131, 136, 263])
+@pytest.mark.parametrize("m,k", [(9, 256), (140, 1792), (300, 2304), (20, 3584)])
+def test_q6k_rows_that_are_no_16_byte_multiples(be, m, n, k):
+    """Rows come in groups of eight (the second CTA of a pair: of none) and one by one behind the last whole group; every block's place in its
+    line differs from row to row."""
+    x, w = O.normal(5600 + m, m * k), O.normal(5601 + n, n * k, 0.05)
+    bufs = [be.upload(x), be.upload(quant.quantize(be, lp.DType.Q6K, w, n, k)), be.alloc(m * n * 4)]
+    got, want = _both(be, [matmul_launch(lp.DType.Q6K, m, n, k, inputs=(0, 1), output=2)], bufs, 2)
+    _close(got, want)
