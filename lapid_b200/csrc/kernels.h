@@ -324,7 +324,8 @@ struct GemmTcArgs {
 };
 bool qgemm_tc_supported(int fmt, const GemmTcArgs &args);
 size_t qgemm_tc_copy_bytes(uint32_t rows, uint32_t k);  // bf16 copy of the activations
-// Tuning options of a device: `splitk` -1 choose, 0 / 1 never, n > 1 every tile n ways (where K allows); `pair` -1 choose, 0 never: CTA pairs (cta_group::2)
+// Tuning options of a device: `splitk` -1 choose, 0 / 1 never, n > 1 every tile n ways (where K allows); `pair` CTA pairs
+// (cta_group::2) above 128 rows: -1 choose, 0 never, 1 always
 struct GemmTcTuning {
     int splitk = -1, pair = -1;
 };

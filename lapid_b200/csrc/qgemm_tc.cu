@@ -898,14 +898,13 @@ bool qgemm_tc_supported(int fmt, const GemmTcArgs &a) {
 static uint32_t tc_block_bytes(int fmt) { return fmt == FMT_Q4K ? Q4K_BYTES : fmt == FMT_Q5K ? Q5K_BYTES : Q6K_BYTES; }
 static uint32_t tc_box_bytes(int fmt) { return fmt == FMT_Q6K ? (uint32_t)tc::Q6K_BOX : tc_block_bytes(fmt); }
 
-// Tiles and K splits of a launch. Above 128 rows pairs of CTAs; the activation rows are divided evenly over as few tiles as hold them.
-// Whole tiles run in rounds over the CTAs (pairs); K is split for the tiles of the last round when that round would be less than
+// Tiles and K splits of a launch on single CTAs or on pairs. The activation rows are divided evenly over as few tiles as hold them. Whole tiles run in rounds over the CTAs (pairs); K is split for the tiles of the last round when that round would be less than
 // half full: `ways` units to a tile, as many as fit the round, never below two super-blocks each, never more than
 // SPLITK_SCRATCH_MAX of partial sums.
 constexpr size_t SPLITK_SCRATCH_MAX = (size_t)256 << 20;
-GemmTcPlan qgemm_tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count, const GemmTcTuning &tuning) {
+static GemmTcPlan cut(bool pair, uint32_t rows, uint32_t n, uint32_t k, int sm_count, int splitk, uint64_t &walk) {
     tc::Plan p{};
-    p.pair = rows > 128 && tuning.pair != 0;
+    p.pair = pair;
     const uint32_t cap = p.pair ? 256 : 128, gran = p.pair ? 32 : 16, width = p.pair ? 2 * tc::TN : tc::TN;
     p.ny = (rows + cap - 1) / cap;
     p.mt = ((rows + p.ny - 1) / p.ny + gran - 1) / gran * gran;
@@ -914,10 +913,10 @@ GemmTcPlan qgemm_tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count, co
     const uint32_t workers = (uint32_t)(p.pair ? sm_count / 2 : sm_count), nblk = k / QK;
     uint64_t tail = 0;
     uint32_t ways = 1;
-    if (tuning.splitk > 1) {
+    if (splitk > 1) {
         tail = tiles;
-        ways = (uint32_t)tuning.splitk;
-    } else if (tuning.splitk < 0 && workers > 0) {
+        ways = (uint32_t)splitk;
+    } else if (splitk < 0 && workers > 0) {
         tail = tiles % workers;
         if (tail * 2 > workers) tail = 0;
         if (tail) ways = (uint32_t)(workers / tail);
@@ -931,7 +930,20 @@ GemmTcPlan qgemm_tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count, co
     p.splits = ways;
     p.full = (uint32_t)(tiles - tail);
     p.units = (uint32_t)(tiles - tail + tail * ways);
+    // the super-blocks that the CTA (pair) with the most to do walks
+    walk = workers ? (tiles - tail + workers - 1) / workers * nblk + (tail * ways + workers - 1) / workers * ((nblk + ways - 1) / ways) : 0;
     return p;
+}
+// Above 128 rows pairs of CTAs: an expanded weight feeds twice the activation rows. A pair takes some 2 us longer to start and end, though, so launches
+// whose tiles fit the single CTAs as well (no CTA walks more super-blocks) stay on those: few rows of weights, or K too short to be split. Single CTAs
+// against pairs: 2048 rows on 300 x 256 Q4_K 10.3 / 12.9 us (the kernel before pairs 11.4), 1024 rows on 768 x 512 10.4 / 12.8 (12.1), 4096 rows on
+// 128 x 2048 17.9 / 21.5 (19.9); where they walk more: 4096 rows on 1024 x 1024 (8 super-blocks against 4) 24.6 / 20.2.
+GemmTcPlan qgemm_tc_plan(uint32_t rows, uint32_t n, uint32_t k, int sm_count, const GemmTcTuning &tuning) {
+    uint64_t single, pairs;
+    const GemmTcPlan one = cut(false, rows, n, k, sm_count, tuning.splitk, single);
+    if (rows <= 128 || tuning.pair == 0) return one;
+    const GemmTcPlan two = cut(true, rows, n, k, sm_count, tuning.splitk, pairs);
+    return tuning.pair < 0 && single <= pairs ? one : two;
 }
 
 // the bf16 copy of the activations, and the partial sums of a split-K launch

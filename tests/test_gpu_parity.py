@@ -655,12 +655,12 @@ def bf16_round(x):
     return u.astype(np.uint32).view(np.float32)
 
 
-@pytest.mark.parametrize("pair", ["-1", "0"])
+@pytest.mark.parametrize("pair", ["-1", "0", "1"])
 @pytest.mark.parametrize("fmt,ofmt", [(lp.DType.Q4K, O.Q4_K), (lp.DType.Q5K, O.Q5_K), (lp.DType.Q6K, O.Q6_K)])
 def test_gemm_tensor_core(be, oracle, fmt, ofmt, pair):
-    be.set_option("gemm_pair", pair)   # "0": single CTAs also above 128 rows
+    be.set_option("gemm_pair", pair)   # above 128 rows: chosen by the launch, single CTAs, pairs
     try:
-        _gemm_tensor_core_cases(be, oracle, fmt, ofmt, pair == "0")
+        _gemm_tensor_core_cases(be, oracle, fmt, ofmt, pair != "-1")
     finally:
         be.set_option("gemm_pair", "-1")
 

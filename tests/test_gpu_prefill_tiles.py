@@ -43,7 +43,7 @@ def _both(be, launches, bufs, out):
 
 
 @pytest.mark.parametrize("fmt", FORMATS)
-@pytest.mark.parametrize("m,n,k,pair", [(m, n, k, pair) for pair in ("-1", "0") for m, n, k in [
+@pytest.mark.parametrize("m,n,k,pair", [(m, n, k, pair) for pair in ("-1", "0", "1") for m, n, k in [
     (9, 1, 256), (16, 127, 512), (17, 129, 768), (112, 130, 2048), (128, 300, 1024), (129, 100, 256), (129, 257, 1280), (161, 255, 2048), (256, 513, 512),
     (257, 384, 768), (600, 200, 512)] if pair == "-1" or m > 128])
 @pytest.mark.parametrize("ways", ["-1", "0", "3"])
