@@ -17,8 +17,9 @@
 //     blocks; as bf16 in shared memory the weights were written and read through the same 128 bytes a cycle that the
 //     activations need.
 //   - a thread owns one row and 64 of a super-block's 256 k: one look at the header's scales for 64 weights, no partner.
-//   - above 128 rows two CTAs of a cluster are one `cta_group::2` unit: 256 weight rows (each CTA expands its own 128) by up
-//     to 256 activation rows, of which each CTA loads half: an expanded weight feeds 256 columns, an activation 256 rows.
+//   - above 128 rows two CTAs of a cluster are one `cta_group::2` unit (where single CTAs do not hold the tiles as well, qgemm_tc_plan()): 256
+//     weight rows (each CTA expands its own 128) by up to 256 activation rows, of which each CTA loads half: an expanded weight
+//     feeds 256 columns, an activation 256 rows.
 //
 // Roles of a CTA's 19 warps:
 //   warps 0-15 expand: warp (quarter of the rows, j) writes the 64 k at 64 j of every super-block into its half of a stage of tensor
@@ -34,11 +35,12 @@
 // super-blocks of a tile are expanded before the results of the one before are stored. Tensor memory: 256 columns of accumulators
 // (one 256-column set for a pair, two of 128 for a single CTA), 4 stages of 64 columns (two k-steps) of weights.
 // Units: whole tiles as long as they fill every CTA, and where the last round would leave SMs idle its tiles are split over K
-// (tc_plan() below); the partial tiles of those go to a scratch area and a second kernel sums them in order.
+// (cut() below); the partial tiles of those go to a scratch area and a second kernel sums them in order.
 //
-// Measured (B200, before: weights through shared memory, one CTA per tile): 77 rows on 14336 x 4096 Q4_K 42.0 -> 25.8 us (instruction issue: 474
-// warp instructions for 64 weights of 32 rows); 2048 rows on 28672 x 8192 Q4_K 936 -> 679 us (1417 TFLOP/s, the sustained rate of cuBLAS under the
-// power cap), on 8192 x 28672 Q6_K 1121 -> 846. Without pairs above 128 rows each CTA would expand every weight for half as many columns.
+// Measured (B200, before: weights through shared memory, one CTA per tile): 77 rows on 14336 x 4096 Q4_K 42.0 -> 25.8 us (1 % more since, the waits at a
+// CTA's end; instruction issue: 474 warp instructions for 64 weights of 32 rows); 2048 rows on 28672 x 8192 Q4_K 936 -> 681 us (1400 TFLOP/s, above the sustained rate of
+// cuBLAS under the power cap), on 8192 x 28672 Q6_K 1121 -> 800, on 8192 x 3584 Q6_K 172 -> 114. All instantiations sit at the cap of 96
+// registers and spill 24 to 80 bytes. Without pairs above 128 rows each CTA would expand every weight for half as many columns.
 //
 // Programmatic dependent launch: barriers, tensor memory and the packed weights come before `griddepcontrol.wait`; only what
 // the kernel in front may have written (activations, expert tables, epilogue terms) and all stores come behind it.
@@ -900,7 +902,9 @@ static uint32_t tc_box_bytes(int fmt) { return fmt == FMT_Q6K ? (uint32_t)tc::Q6
 
 // Tiles and K splits of a launch on single CTAs or on pairs. The activation rows are divided evenly over as few tiles as hold them. Whole tiles run in rounds over the CTAs (pairs); K is split for the tiles of the last round when that round would be less than
 // half full: `ways` units to a tile, as many as fit the round, never below two super-blocks each, never more than
-// SPLITK_SCRATCH_MAX of partial sums.
+// SPLITK_SCRATCH_MAX of partial sums. Half full is where two ways stop fitting one round, and then they cost more than they give (77 rows of
+// Q4_K, K = 4096, on 148 SMs, not split / two / three ways: 64 tiles 27.3 / 20.2 / 26.1 us, 74 tiles 27.2 / 20.7 / 26.3, 75 tiles 27.3 / 30.7 / 26.4,
+// 112 tiles 27.5 / 32.2 / 33.8; 256 rows in pairs, 43 tiles on 74 pairs: 32.0 / 41.5 / 37.5).
 constexpr size_t SPLITK_SCRATCH_MAX = (size_t)256 << 20;
 static GemmTcPlan cut(bool pair, uint32_t rows, uint32_t n, uint32_t k, int sm_count, int splitk, uint64_t &walk) {
     tc::Plan p{};
