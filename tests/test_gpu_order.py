@@ -364,3 +364,38 @@ def test_prefill_behind_a_launch_that_takes_long():
     be.execute(ls, bufs)
     assert start.elapsed_time(end) > 20
     assert torch.isfinite(outs[0]).all() and outs[0].any() and torch.equal(*outs)
+
+
+@pytest.mark.parametrize("chunk", [0, 1, 2])
+@pytest.mark.parametrize("m", [77, 300])
+def test_prefill_with_uploads_between_the_launches(m, chunk):
+    """A prefill step with host buffers: activations and packed weights come up on the copy stream while launches of earlier chunks run; the weights
+    that a launch requests before its dependency wait must be the uploaded ones."""
+    import torch
+    serial, s0 = _device(pdl="0")
+    be, s1 = _device()
+    n, k = 1024, 2048
+    sets = [[_weights(be, int(DType.Q4K), n, k, 1050 + 2 * i + j) for j in range(2)] for i in range(2)]
+    xs = [[torch.from_numpy(O.normal(1060 + 2 * i + j, m * k).reshape(m, k)).cuda() for j in range(2)] for i in range(2)]
+    dev = [torch.zeros_like(t) for t in (*xs[0], *sets[0])] + [torch.zeros(m, n, device="cuda") for _ in range(3)]
+    host = [[t.cpu().pin_memory() for t in (*xs[i], *sets[i])] for i in range(2)]
+    outs = [torch.zeros(m, n).pin_memory() for _ in range(3)]
+    torch.cuda.synchronize()
+    ls = [matmul_launch(DType.Q4K, m, n, k, inputs=(0, 2), output=4), matmul_launch(DType.Q4K, m, n, k, inputs=(0, 3), output=5),
+          matmul_launch(DType.Q4K, m, n, k, inputs=(1, 2), output=6)]
+    wants = []
+    for i in range(2):
+        bufs = [serial.wrap_tensor(t) for t in (*xs[i], *sets[i], *dev[4:])]
+        for l in ls:
+            serial.execute([l], bufs)
+        wants.append([t.cpu() for t in dev[4:]])
+    bufs = [be.wrap_tensor(t) for t in dev]
+    size = [t.numel() * t.element_size() for t in dev]
+    for rep in range(20):
+        h = host[rep % 2]
+        writes = [(b, 0, h[b].data_ptr(), size[b], first) for b, first in ((0, 0), (2, 0), (3, 1), (1, 2))]
+        reads = [(4 + i, 0, outs[i].data_ptr(), size[4 + i], i) for i in range(3)]
+        be.execute_io(ls, bufs, writes, reads, chunk)
+        assert all(torch.equal(a, b) for a, b in zip(outs, wants[rep % 2])), rep
+    serial.synchronize()
+    be.synchronize()
