@@ -801,6 +801,7 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
     f.id_stride = p.wl.total;
     f.id_r = (uint32_t)p.r;
     f.mt = p.mt;
+    f.status = dev.status_dev;
     cuda_check(lb::launch_qgemm_f32(l.b_dtype, f, dev.sm_count, dev.stream), "matmul_id gemm launch");
     dev.launches++;
 }
@@ -1069,6 +1070,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
     f.m = g.m;
     f.n = g.n;
     f.k = g.k;
+    f.status = dev.status_dev;
     cuda_check(lb::launch_qgemm_f32(l.b_dtype, f, dev.sm_count, dev.stream), "qgemm_f32 launch");
     dev.launches++;
     expr_pass();

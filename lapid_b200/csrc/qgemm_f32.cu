@@ -14,12 +14,12 @@
 // CUDA-core kernel: the order of the sum is fixed (one chain of fused multiply-adds over k per output), so neither the tensor
 // cores nor a split of K can be used; what bounds it is FMA issue (128 a clock and SM: 74 TFLOP/s at 1.96 GHz). Two neighbouring
 // activation rows share one packed fma.rn.f32x2 (two independent, separately rounded FMAs in one instruction): half the issue
-// slots of scalar FMAs, which leaves room for the shared-memory loads and for expanding the weights (scalar: 33.4 against
+// slots of scalar FMAs, which leaves room for the shared-memory loads and for expanding the weights (64 x 64 tiles, scalar: 33.4 against
 // 40.6 TFLOP/s at 512 rows on 14336 x 4096). k runs in steps of BK; while a step is multiplied the next one's activations and packed
 // weights are on their way into registers, and two shared-memory buffers leave one barrier per step. Both operands
 // lie as [k][row] in shared memory with an XOR on the row that keeps the transposing stores and the wide reads of a warp free of bank
-// conflicts. int8 weights, 14336 x 4096: 512 rows 1.43 ms (42 TFLOP/s; the 64 x 64 tiles of scalar FMAs without prefetch that this
-// replaces: 2.71 ms), 1184 rows 48.5 TFLOP/s, where the FMA pipe is busy for about 70 % of the time (ncu: the rest is waits on operands).
+// conflicts. Tiles of 64 x 64, 32 x 128 and 16 x 32 outputs; launches with work for 128 rows x 64 columns or more on every SM take the
+// producer / consumer kernel further down.
 #include <math.h>
 
 #include <type_traits>
@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "iquant.cuh"
 #include "kernels.h"
+#include "pipe.cuh"
 
 namespace lb {
 
@@ -130,7 +131,7 @@ __device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) { asm(
 
 // TM x TN outputs per thread, TM in pairs of rows; both in runs of four (16-byte shared loads), the runs of a thread BM / 2 (BN / 2) apart
 // when there are two of them.
-template <int FMT, int BM, int BN, int BK, int TM, int TN> __global__ void __launch_bounds__((BM / TM) * (BN / TN), (TM == 16 ? 256 : 512) / ((BM / TM) * (BN / TN)))
+template <int FMT, int BM, int BN, int BK, int TM, int TN> __global__ void __launch_bounds__((BM / TM) * (BN / TN), 512 / ((BM / TM) * (BN / TN)))
 qgemm_f32_kernel(GemmF32Args p) {
     constexpr int THREADS = (BM / TM) * (BN / TN), TX = BN / TN, TR = TN % 4 ? 2 : 4;  // TR: columns per run
     constexpr int AU = BM * BK / 4, WU = BN * BK / 8, WP = BK / 8;  // loads per step: four activations, eight weights each
@@ -303,6 +304,235 @@ qgemm_f32_kernel(GemmF32Args p) {
     }
 }
 
+// ---- many outputs: producer and consumer warps ------------------------------------------------------------------
+// The same sums with the roles of a CTA's warps split: four producer warps fetch activations and packed weights and write both operands
+// into a ring of shared-memory stages, eight consumer warps do nothing but shared loads and packed FMAs, 8 rows x W columns each thread,
+// and never wait for a barrier of the whole CTA. A tile is 128 rows x 16 W columns, W = 4..8 chosen per tile: a launch's columns are cut
+// into nearly equal tiles so that every SM gets the same number of them, where tiles of a fixed width leave the last round mostly empty
+// (512 rows on 4096 columns: 128 x 128 tiles use 128 of 148 SMs, tiles of 112 columns all of them). One CTA per SM walks its tiles; the
+// producers run ahead into the next one. int8 weights, us, 128 x 128 or 64 x 64 tiles of the kernel above -> this one: 512 rows on 14336 x 4096
+// 1432 -> 1191 (50.5 TFLOP/s), on 4096 x 4096 424 -> 353, 128 rows on 14336 x 4096 425 -> 353, 2048 rows on 9600 x 2880 2203 -> 2140 (52.9).
+// FMA pipe busy 70 %, shared loads 56 % (a load of 16 bytes a lane takes the 128-byte return path four cycles whoever shares it); the rest
+// is latency of two consumer warps a scheduler, and the producers (without their stores and expansion: 56 TFLOP/s). Measured and not better:
+// one consumer warp a scheduler with 16 x 8 outputs a thread (44 TFLOP/s), two with 16 x 8 (48.5), columns up to 12 a thread (49.8),
+// operands fetched over the edge of a stage (46), pairs of rows turned round instead of columns written twice (46).
+namespace ws {
+
+constexpr int BK = 16, STAGES = 4, CONSUMERS = 256, PRODUCERS = 128, W_MIN = 4, W_MAX = 8;
+constexpr int BM = 128, TX = 16, BN = W_MAX * TX;  // BN: the widest tile
+constexpr int A_FLOATS = BK * BM, STAGE_FLOATS = A_FLOATS + BK * BN;
+constexpr size_t SMEM = (size_t)STAGES * STAGE_FLOATS * 4 + 2 * STAGES * 8;
+constexpr uint32_t WAIT_LIMIT = 1u << 19;  // a failed attempt sleeps some 4 us: two seconds
+
+struct Cut {  // how the launch is cut: `per_block` tiles for each block of BM rows, each of whole units of TX columns
+    uint32_t row_blocks, per_block, units, turn;
+    uint64_t tiles;
+};
+struct Tile {
+    uint32_t rb, col0, w;  // w: units of TX columns (0: nothing to do)
+};
+__device__ __forceinline__ Tile tile_at(const GemmF32Args &p, const Cut &c, uint64_t t) {
+    // every block of rows starts at another tile: the wider ones do not all meet on the same CTAs
+    const uint32_t rb = (uint32_t)(t / c.per_block), i = (uint32_t)((t % c.per_block + (uint64_t)rb * c.turn) % c.per_block);
+    const uint32_t u0 = (uint32_t)((uint64_t)i * c.units / c.per_block), u1 = (uint32_t)((uint64_t)(i + 1) * c.units / c.per_block);
+    return Tile{rb, u0 * TX, (p.tile_expert && p.tile_expert[rb] < 0) ? 0u : u1 - u0};
+}
+
+// 8 rows x W columns of a thread: rows 4 ty + 0..3 and BM / 2 further, columns in runs of four, two and one (16-, 8- and 4-byte shared loads).
+template <int W>
+__device__ __forceinline__ bool consume(const GemmF32Args &p, const Tile &tile, const float *ring, uint64_t *full, uint64_t *empty, uint32_t &stage, uint32_t &phase) {
+    constexpr int NQ = W / 4, NP = (W % 4) / 2, N1 = W % 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ty = (lane & 3) + 4 * (warp & 3), tx = (lane >> 2) + 8 * (warp >> 2);
+    uint64_t acc[4][W];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < W; j++) acc[i][j] = 0;
+    for (uint32_t k0 = 0; k0 < p.k; k0 += BK) {
+        if (!pipe::mbar_wait(full + stage, phase, WAIT_LIMIT)) return false;
+        const float *As = ring + stage * STAGE_FLOATS, *Bs = As + A_FLOATS;
+        uint64_t a2[2][4];
+        float b[2][W];
+        auto operands = [&](int kk) {
+            const int q = 8 * (kk >> 2);  // (the XOR of the producers' transposing stores)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const ulonglong2 v = *(const ulonglong2 *)(As + kk * BM + ((4 * ty) ^ q) + i * (BM / 2));
+                a2[kk & 1][2 * i] = v.x, a2[kk & 1][2 * i + 1] = v.y;
+            }
+            const float *row = Bs + kk * BN;
+#pragma unroll
+            for (int j = 0; j < NQ; j++) *(float4 *)&b[kk & 1][4 * j] = *(const float4 *)(row + 4 * TX * j + ((4 * tx) ^ q));
+            if constexpr (NP) {
+                const float2 v = *(const float2 *)(row + 4 * TX * NQ + ((2 * tx) ^ q));
+                b[kk & 1][4 * NQ] = v.x, b[kk & 1][4 * NQ + 1] = v.y;
+            }
+            if constexpr (N1) b[kk & 1][W - 1] = row[TX * (W - 1) + (tx ^ q)];
+        };
+        operands(0);
+#pragma unroll
+        for (int kk = 0; kk < BK; kk++) {  // the operands of the next step are on their way
+            if (kk + 1 < BK) operands(kk + 1);
+#pragma unroll
+            for (int j = 0; j < W; j++) {
+                const uint64_t b2 = pack2(b[kk & 1][j], b[kk & 1][j]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) fma2(acc[i][j], a2[kk & 1][i], b2);
+            }
+        }
+        __syncwarp();
+        if (lane == 0) pipe::mbar_arrive(empty + stage);  // (behind the last products: what was read has been used)
+        if (++stage == STAGES) stage = 0, phase ^= 1;
+    }
+    const uint32_t row0 = tile.rb * BM, end = min(p.n, tile.col0 + tile.w * TX);  // (columns past a narrow tile belong to the next one)
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t r = row0 + 4 * ty + (i >> 2) * (BM / 2) + (i & 3);
+        if (r >= p.rows) continue;
+        float *o;
+        const float *ex = nullptr;
+        if (p.tile_expert) {
+            const int32_t pair = p.row_pair[r];
+            if (pair < 0) continue;
+            o = p.out + p.out_off + (uint64_t)pair * p.n;
+        } else {
+            const uint32_t bt = r / p.m, ii = r % p.m;
+            o = p.out + p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)ii * p.out_rs;
+            if (p.extra) ex = p.extra + (p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)ii * p.ex_s1);
+        }
+        float v[W];
+#pragma unroll
+        for (int j = 0; j < W; j++) v[j] = __uint_as_float((uint32_t)((i & 1) ? acc[i >> 1][j] >> 32 : acc[i >> 1][j]));
+#pragma unroll
+        for (int j = 0; j < NQ; j++) {
+            const uint32_t col = tile.col0 + 4 * TX * j + 4 * tx;
+            if (!ex && col + 3 < end && ((uintptr_t)(o + col) & 15) == 0) {
+                *(float4 *)(o + col) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                continue;
+            }
+#pragma unroll
+            for (int l = 0; l < 4; l++)
+                if (col + l < end) o[col + l] = ex ? v[4 * j + l] + ex[(int64_t)(col + l) * p.ex_s2] : v[4 * j + l];
+        }
+#pragma unroll
+        for (int j = 4 * NQ; j < W; j++) {
+            const uint32_t col = tile.col0 + (j < 4 * NQ + 2 * NP ? 4 * TX * NQ + 2 * tx + (j & 1) : TX * (W - 1) + tx);
+            if (col < end) o[col] = ex ? v[j] + ex[(int64_t)col * p.ex_s2] : v[j];
+        }
+    }
+    return true;
+}
+
+template <int FMT> __global__ void __launch_bounds__(CONSUMERS + PRODUCERS, 1) qgemm_f32_ws_kernel(GemmF32Args p, Cut cut) {
+    extern __shared__ __align__(16) float ring[];
+    uint64_t *full = (uint64_t *)(ring + STAGES * STAGE_FLOATS), *empty = full + STAGES;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; i++) pipe::mbar_init(full + i, PRODUCERS / 32), pipe::mbar_init(empty + i, CONSUMERS / 32);
+        pipe::mbar_fence_init();
+    }
+    __syncthreads();
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    if (threadIdx.x < CONSUMERS) {
+        for (uint64_t t = blockIdx.x; t < cut.tiles && ok; t += gridDim.x) {
+            const Tile tile = tile_at(p, cut, t);
+            switch (tile.w) {
+                case 0: break;
+                case 8: ok = consume<8>(p, tile, ring, full, empty, stage, phase); break;
+                case 7: ok = consume<7>(p, tile, ring, full, empty, stage, phase); break;
+                case 6: ok = consume<6>(p, tile, ring, full, empty, stage, phase); break;
+                case 5: ok = consume<5>(p, tile, ring, full, empty, stage, phase); break;
+                default: ok = consume<4>(p, tile, ring, full, empty, stage, phase); break;
+            }
+        }
+    } else {
+        constexpr int AN = BM * BK / 4 / PRODUCERS, WN = W_MAX * TX * 2 / PRODUCERS;  // loads per step: four activations, eight weights each
+        static_assert(BM * BK / 4 % PRODUCERS == 0 && W_MAX * TX * 2 % PRODUCERS == 0, "producers");
+        const int tid = threadIdx.x - CONSUMERS;
+        const uint8_t *stack = p.w;
+        for (uint64_t t = blockIdx.x; t < cut.tiles && ok; t += gridDim.x) {
+            const Tile tile = tile_at(p, cut, t);
+            if (tile.w == 0) continue;
+            const uint32_t row0 = tile.rb * BM, cols = max(tile.w, (uint32_t)W_MIN) * TX;
+            if (p.tile_expert) p.w = stack + (uint64_t)p.tile_expert[tile.rb] * p.id_stride;
+            const void *aptr[AN];
+#pragma unroll
+            for (int i = 0; i < AN; i++) {
+                const uint32_t arow = row0 + (uint32_t)((tid + i * PRODUCERS) >> 2);
+                aptr[i] = nullptr;
+                if (p.tile_expert) {
+                    const int32_t pair = p.row_pair[arow];
+                    if (pair >= 0) aptr[i] = (const char *)p.a + (p.a_off + (uint64_t)((uint32_t)pair / p.id_r) * p.a_rs) * act_elem_bytes(p.a_type);
+                } else if (arow < p.rows) {
+                    aptr[i] = act_row(p.a, p.a_type, p.a_off, p.a_bs, p.a_rs, arow, p.m);
+                }
+            }
+            const int ak = 4 * (tid & 3), arow = tid >> 2, wk = 8 * (tid & 1), wcol = tid >> 1;
+            float av[2][AN][4];
+            Raw8<FMT> wv[2][WN];
+            auto fetch = [&](int set, uint32_t k0) {
+#pragma unroll
+                for (int i = 0; i < AN; i++) {
+                    const uint32_t k = k0 + ak;
+                    if (!aptr[i]) {
+#pragma unroll
+                        for (int l = 0; l < 4; l++) av[set][i][l] = 0.0f;
+                    } else if (p.a_vec && p.a_type == ACT_F32) {
+                        const float4 v = *(const float4 *)((const float *)aptr[i] + k);
+                        av[set][i][0] = v.x, av[set][i][1] = v.y, av[set][i][2] = v.z, av[set][i][3] = v.w;
+                    } else if (p.a_vec) {
+                        const uint2 v = *(const uint2 *)((const uint16_t *)aptr[i] + k);
+#pragma unroll
+                        for (int l = 0; l < 4; l++) av[set][i][l] = widen_act(((l < 2 ? v.x : v.y) >> (16 * (l & 1))) & 0xffffu, p.a_type);
+                    } else {
+#pragma unroll
+                        for (int l = 0; l < 4; l++) av[set][i][l] = load_act(aptr[i], k + l, p.a_type);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < WN; i++) {
+                    const uint32_t c = (uint32_t)wcol + i * (PRODUCERS / 2), row = tile.col0 + c;
+                    if (c < cols) load_raw8<FMT>(p, row < p.n ? row : p.n - 1, k0 + wk, wv[set][i]);  // columns past the matrix are not stored
+                }
+            };
+            auto put = [&](int set, uint32_t k0) {
+                if (!pipe::mbar_wait(empty + stage, phase ^ 1, WAIT_LIMIT)) return false;
+                float *As = ring + stage * STAGE_FLOATS, *Bs = As + A_FLOATS;
+#pragma unroll
+                for (int i = 0; i < AN; i++)
+#pragma unroll
+                    for (int l = 0; l < 4; l++) As[(ak + l) * BM + ((arow + i * (PRODUCERS / 4)) ^ (2 * ak))] = av[set][i][l];
+#pragma unroll
+                for (int i = 0; i < WN; i++) {
+                    const uint32_t c = (uint32_t)wcol + i * (PRODUCERS / 2);
+                    if (c >= cols) continue;
+                    float y[8];
+                    expand8<FMT>(wv[set][i], k0 + wk, y);
+#pragma unroll
+                    for (int l = 0; l < 8; l++) Bs[(wk + l) * BN + (c ^ (2 * wk + 8 * (l >> 2)))] = y[l];
+                }
+                __syncwarp();
+                if ((tid & 31) == 0) pipe::mbar_arrive(full + stage);
+                if (++stage == STAGES) stage = 0, phase ^= 1;
+                return true;
+            };
+            // the operands of the step after the one being written are on their way (k is a multiple of 32: steps come in pairs)
+            fetch(0, 0);
+            for (uint32_t k0 = 0; k0 < p.k && ok; k0 += 2 * BK) {
+                fetch(1, k0 + BK);
+                ok = put(0, k0);
+                if (!ok) break;
+                if (k0 + 2 * BK < p.k) fetch(0, k0 + 2 * BK);
+                ok = put(1, k0 + BK);
+            }
+        }
+    }
+    if (!ok && p.status) atomicOr(p.status, 8);
+}
+
+}  // namespace ws
+
 constexpr uint32_t GRID_Y_MAX = 65535;
 template <int FMT, int BM, int BN, int BK, int TM, int TN> static cudaError_t launch_tile(const GemmF32Args &a, cudaStream_t stream) {
     const dim3 grid((a.n + BN - 1) / BN, (a.rows + BM - 1) / BM);
@@ -311,24 +541,63 @@ template <int FMT, int BM, int BN, int BK, int TM, int TN> static cudaError_t la
     return cudaGetLastError();
 }
 
+// Tiles per block of 128 rows: of the numbers that fill whole rounds of CTAs, the one whose tiles cost least. A CTA takes about 92 + 35 W us
+// for a tile of W units of 16 columns (k = 4096; W below 4 costs what 4 costs), so few rounds of wide tiles win until a round more
+// makes them fit: 512 rows on 4096 columns, one round of 7 units 353 us, two of 4 466; on 14336, four rounds of 6 1191 us, five of 5 1310.
+static ws::Cut ws_cut(uint64_t row_blocks, uint64_t n, int sm_count, double &cost) {
+    ws::Cut c{};
+    c.row_blocks = (uint32_t)row_blocks;
+    c.units = (uint32_t)((n + ws::TX - 1) / ws::TX);
+    cost = 1e30;
+    for (int w = ws::W_MAX; w >= 1; w--) {
+        uint64_t per = (c.units + w - 1) / w;
+        const uint64_t rounds = (row_blocks * per + sm_count - 1) / sm_count;
+        if (rounds * sm_count / row_blocks > per) per = rounds * sm_count / row_blocks;  // more tiles in as many rounds
+        if (per > c.units) per = c.units;
+        const double widest = ceil((double)c.units / (double)per), mean = (double)c.units / (double)per;
+        // (with several rounds the wider tiles spread over the CTAs)
+        const double wide = rounds == 1 ? widest : mean + (widest - mean) / (double)rounds, us = 15 + (double)rounds * (92 + 35 * (wide < 4 ? 4 : wide));
+        if (us < cost) cost = us, c.per_block = (uint32_t)per;
+    }
+    c.tiles = (uint64_t)c.per_block * row_blocks;
+    c.turn = c.per_block / 3 + 1;
+    return c;
+}
+template <int FMT> static cudaError_t launch_ws(const GemmF32Args &a, int sm_count, cudaStream_t stream) {
+    const uint64_t row_blocks = ((uint64_t)a.rows + ws::BM - 1) / ws::BM;
+    if (row_blocks > GRID_Y_MAX) return cudaErrorInvalidValue;
+    double cost;
+    const ws::Cut c = ws_cut(row_blocks, a.n, sm_count, cost);
+    static DynamicSmemOptIn optin;
+    cudaError_t e = optin.raise((const void *)ws::qgemm_f32_ws_kernel<FMT>, ws::SMEM);
+    if (e != cudaSuccess) return e;
+    ws::qgemm_f32_ws_kernel<FMT><<<c.tiles < (uint64_t)sm_count ? (uint32_t)c.tiles : sm_count, ws::CONSUMERS + ws::PRODUCERS, ws::SMEM, stream>>>(a, c);
+    return cudaGetLastError();
+}
+
 // The tiles, and what one costs: an SM with `per` tiles takes about fixed + per * each (us for k = 4096 on a launch that gives every SM
-// that many; measured with int8 weights, the other formats within a tenth). Large tiles multiply faster (fewer shared loads
-// and less weight expansion per FMA: 46, 38, 34 and 15 outputs a us), small ones fill the chip and waste less on a ragged last tile: 512 rows
-// on 14336 x 4096 weights take 1.43 ms on 64 x 64 and 1.47 on 128 x 128 tiles (3.03 of those per SM), 1024 rows 2.72 and 2.52; on
-// 1024 x 4096 weights 16 rows take 84 us on 16 x 32 tiles and 146 on 64 x 64 (the 16 x 32 tile has become a tenth faster since its constants
+// that many; measured with int8 weights, the other formats within a tenth). The producer / consumer kernel (bm 128) multiplies fastest, small
+// tiles fill the chip and waste less on a ragged last tile: 128 rows on 1024 x 4096 weights take 94 us on 16 x 32 tiles, 157 on 64 x 64 and 250
+// on 128 rows; 64 rows on 14336 x 4096 245 us on 64 x 64 and 343 on 128 rows (the 16 x 32 tile has become a tenth faster since its constants
 // were measured: 12 rows on 2048 x 4096 74 us).
 struct F32Tile {
     uint32_t bm, bn;
     double fixed, each, least;
 };
-static const F32Tile F32_TILES[] = {{128, 128, 60, 360, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 122, 0}, {16, 32, 15, 35, 84}};
+static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 122, 0}, {16, 32, 15, 35, 84}};
 static int pick_tile(uint64_t matrices, double rows, uint64_t n, int sm_count) {  // `matrices` products of `rows` rows each
     int best = 0;
     double cost = 1e30;
     for (int i = 0; i < 4; i++) {
         const F32Tile &t = F32_TILES[i];
-        const uint64_t tiles = matrices * (uint64_t)ceil(rows / t.bm) * ((n + t.bn - 1) / t.bn), per = (tiles + sm_count - 1) / sm_count;
-        double c = t.fixed + t.each * (double)per;
+        const uint64_t blocks = matrices * (uint64_t)ceil(rows / t.bm);
+        double c;
+        if (t.bn) {
+            const uint64_t tiles = blocks * ((n + t.bn - 1) / t.bn), per = (tiles + sm_count - 1) / sm_count;
+            c = t.fixed + t.each * (double)per;
+        } else {
+            ws_cut(blocks, n, sm_count, c);
+        }
         if (c < t.least) c = t.least;
         if (c < cost) cost = c, best = i;
     }
@@ -346,7 +615,7 @@ uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts, uint64_t n, int sm
 
 template <int FMT> static cudaError_t launch_fmt(const GemmF32Args &a, int sm_count, cudaStream_t stream) {
     switch (a.tile_expert ? a.mt : F32_TILES[pick_tile(1, a.rows, a.n, sm_count)].bm) {
-        case 128: return launch_tile<FMT, 128, 128, 16, 16, 8>(a, stream);
+        case 128: return launch_ws<FMT>(a, sm_count, stream);
         case 64: return launch_tile<FMT, 64, 64, 16, 8, 4>(a, stream);
         case 32: return launch_tile<FMT, 32, 128, 16, 8, 4>(a, stream);
         case 16: return launch_tile<FMT, 16, 32, 64, 4, 2>(a, stream);
