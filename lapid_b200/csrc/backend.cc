@@ -372,7 +372,7 @@ struct PendingGroup {
         const char *lo, *hi;
         bool hits(const Range &o) const { return lo < o.hi && o.lo < hi; }
     };
-    int fmt = 0, mode = 0;  // kernel of the members: 1 = dp4a kernel, 2 = tensor-core kernel, 3 = balanced-stream tensor-core kernel
+    int fmt = 0, mode = 0;  // kernel of the members: 1 = dp4a kernel, 2 = tensor-core kernel, 3 = balanced-stream tensor-core kernel, 4 = i-quant kernel
     lb::GemvGroup g{};
     bool split_early = false;  // see accepts()
     bool serial = false;       // an earlier launch of the list writes what a member fetches early (run_launch: src_written)
@@ -395,7 +395,7 @@ struct PendingGroup {
             if (r.hits(out)) return false;
         g.item[g.count] = a;
         g.count++;
-        if (f == LAPID_B200_DTYPE_INT8 || f == LAPID_B200_DTYPE_INT4) {  // (one activation operand for the whole launch)
+        if (md == 4 || f == LAPID_B200_DTYPE_INT8 || f == LAPID_B200_DTYPE_INT4) {  // (one activation operand for the whole launch)
             g.count--;
             return a.qa == g.item[0].qa;
         }
@@ -426,6 +426,7 @@ struct PendingGroup {
         serial = false;
         const uint64_t before = dev.stream_ws.kernels;
         if (mode == 3) cuda_check(lb::launch_qgemv_kq_stream(fmt, out, dev.stream_ws, dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (mode == 4) cuda_check(lb::launch_qgemv_iq(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (fmt == LAPID_B200_DTYPE_INT8 || fmt == LAPID_B200_DTYPE_INT4)
             cuda_check(lb::launch_qgemv_i8_mma(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (mode == 2 && fmt == LAPID_B200_DTYPE_Q6_K) cuda_check(lb::launch_qgemv_q6k_mma(out, dev.sm_count, pdl, dev.stream), "qgemv launch");
@@ -751,7 +752,12 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         const bool pdl = dev.pdl_launch();
         if (l.b_dtype == LAPID_B200_DTYPE_INT4) cuda_check(lb::launch_qgemv_i4(g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
-        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
+        else if (is_iquant(l.b_dtype)) {
+            lb::GemvGroup one{};
+            one.count = 1;
+            one.item[0] = g;
+            cuda_check(lb::launch_qgemv_iq(l.b_dtype, one, dev.sm_count, pdl, dev.stream), "matmul_id launch");
+        }
         else if (p.fast) cuda_check(lb::launch_qgemv_kq_moe(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         else cuda_check(lb::launch_qgemv_moe(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         dev.launches += 2;
@@ -952,14 +958,14 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
         g.a_bs = q.a_bs;
         g.a_rs = q.a_rs;
         g.status = dev.status_dev;
-        if (pend && slot->records && l.b_dtype != LAPID_B200_DTYPE_MXFP4) {  // (the MXFP4 kernels take one launch at a time)
+        if (pend && (is_iquant(l.b_dtype) || (slot->records && l.b_dtype != LAPID_B200_DTYPE_MXFP4))) {  // (the MXFP4 kernels take one launch at a time)
             using Range = PendingGroup::Range;
             const char *ob = (const char *)out->ptr;
             Range wr{ob + 4 * l.out.offset, ob + 4 * last};
             Range in[3];
             int n_in = 0;
             for (int i = 0; i < l.n_inputs; i++) in[n_in++] = Range{(const char *)ins[i]->ptr, (const char *)ins[i]->ptr + ins[i]->bytes};
-            const int mode = slot->records == 2 && p.stream ? 3 : slot->records;
+            const int mode = is_iquant(l.b_dtype) ? 4 : slot->records == 2 && p.stream ? 3 : slot->records;
             g.early = slot->hoisted ? 1 : 0;  // gated again when the group goes out
             if (!pend->accepts(l.b_dtype, mode, g, wr, in, n_in)) pend->flush(dev);
             if (!slot->done) {  // its input is not written by a pending launch (checked above), so it may run first
@@ -1001,7 +1007,12 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             cuda_check(lb::launch_qgemv_i4_fast(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (l.b_dtype == LAPID_B200_DTYPE_INT4) cuda_check(lb::launch_qgemv_i4(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (is_iquant(l.b_dtype)) {
+            lb::GemvGroup one{};
+            one.count = 1;
+            one.item[0] = g;
+            cuda_check(lb::launch_qgemv_iq(l.b_dtype, one, dev.sm_count, pdl, dev.stream), "qgemv launch");
+        }
         else if (p.fast_i8 && ((uintptr_t)g.w & 15) == 0) cuda_check(lb::launch_qgemv_i8_fast(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else cuda_check(lb::launch_qgemv(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         dev.launches += dev.stream_ws.kernels > ws_before ? dev.stream_ws.kernels - ws_before : 1;  // (the stream kernel may take two)

@@ -143,7 +143,6 @@ void qgemv_mxfp4_set_staged(int on);  // 1 (default): rows staged through shared
 
 // ---- qgemv_iq.cu: the grid-based i-quants (IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS), 1..8 rows (and the expert-indexed form);
 // reads the activation planes, the codebooks from the per-device table of iquant.cu
-cudaError_t launch_qgemv_iq(int fmt, const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream);
 void qgemv_iq_set_rows_per_warp(int rows);  // 0: per launch (default); 1, 2: forced
 void qgemv_iq_set_k_split(int ways);        // warps per row at one row per warp: 0: per launch (default); 1, 2, 4: forced
 // iquant.cu: uploads the codebooks to the current device (once; outside stream captures)
@@ -215,6 +214,7 @@ template <int N> struct GemvGroupT {
 };
 using GemvGroup = GemvGroupT<GEMV_GROUP_MAX>;
 using GemvSingle = GemvGroupT<1>;  // what a lone launch passes to the kernel: a sixth of the parameter bytes
+cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);  // members read the same activations
 size_t qgemv_kq_group_smem(int fmt, GemvGroup &group);  // dynamic shared memory the group would need
 cudaError_t launch_qgemv_kq_group(int fmt, GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);
 // Q4_K decode on the warp-level int8 tensor-core instruction (2..8 rows pay off); activations as

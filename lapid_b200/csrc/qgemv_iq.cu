@@ -94,8 +94,23 @@ __device__ __forceinline__ void unpack32(const Raw32 &raw, const uint8_t *grid, 
 
 // KS warps share the rows of a warp group and split their blocks (matrices with few rows and a long K would otherwise
 // leave most warp slots of an SM empty); their partial sums meet in shared memory and are added in warp order.
-template <int FMT, int M, int ROWS, int WARPS, int KS>
-__global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const uint8_t *__restrict__ grid_global) {
+// A grouped launch (projections that read the same activations: q and k, gate and up) gives each member a range of CTAs (task_end counts CTAs).
+template <int FMT, int M, int ROWS, int WARPS, int KS, int NG>
+__global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__restrict__ grid_global) {
+    uint32_t cta = blockIdx.x, ctas = gridDim.x;
+    int it = 0;
+    if constexpr (NG > 1) {
+#pragma unroll
+        for (int i = 1; i < NG; i++)
+            if (i < grp.count && blockIdx.x >= grp.task_end[i - 1]) it = i;
+        ctas = grp.task_end[it];
+        if (it) cta -= grp.task_end[it - 1], ctas -= grp.task_end[it - 1];
+    }
+    const GemvArgs &p = grp.item[it];
+    const uint8_t *w_base = p.w;
+    const int8_t *qa = p.qa;
+    const float *da_base = p.da;
+    float *out = p.out + p.out_off;
     __shared__ __align__(16) uint8_t grid[iq_grid_bytes(FMT)];
     {  // the codebook never changes: it may be read before the launch this one depends on has finished
         const uint4 *src = (const uint4 *)grid_global;
@@ -117,11 +132,11 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
 #pragma unroll
         for (int j = 0; j < ROWS; j++) {
             const uint32_t row = row0 + j < p.n ? row0 + j : p.n - 1;  // (a row past the end repeats the last one; not stored)
-            raw[j] = load32<FMT>(p.w + ((uint64_t)row * nblk + blk) * BB, ib);
+            raw[j] = load32<FMT>(w_base + ((uint64_t)row * nblk + blk) * BB, ib);
         }
     };
     const uint32_t blk0 = (lane >> 3) + 4 * ks;
-    if (!p.ids && blockIdx.x * RPC < p.n) fetch(blockIdx.x * RPC + wg * ROWS, blk0);
+    if (!p.ids && cta * RPC < p.n) fetch(cta * RPC + wg * ROWS, blk0);
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -131,14 +146,14 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
         const int32_t id = p.ids[pair];
         const bool bad = id < 0 || (uint32_t)id >= p.id_e;
         if (bad && p.status && threadIdx.x == 0) atomicOr(p.status, 128);
-        p.w += bad ? 0 : (uint64_t)id * p.id_stride;
-        p.qa += (uint64_t)token * k;
-        p.da += (uint64_t)token * kg;
-        p.out_off += (uint64_t)pair * p.n;
-        if (blockIdx.x * RPC < p.n) fetch(blockIdx.x * RPC + wg * ROWS, blk0);
+        w_base += bad ? 0 : (uint64_t)id * p.id_stride;
+        qa += (uint64_t)token * k;
+        da_base += (uint64_t)token * kg;
+        out += (uint64_t)pair * p.n;
+        if (cta * RPC < p.n) fetch(cta * RPC + wg * ROWS, blk0);
     }
     __shared__ float part[KS > 1 ? WARPS * ROWS * M : 1];
-    for (uint32_t base = blockIdx.x * RPC; base < p.n; base += gridDim.x * RPC) {  // (the same number of passes for every warp of the CTA)
+    for (uint32_t base = cta * RPC; base < p.n; base += ctas * RPC) {  // (the same number of passes for every warp of the CTA)
         const uint32_t row0 = base + wg * ROWS;
         float acc[ROWS][M];
 #pragma unroll
@@ -157,9 +172,9 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
             const uint32_t g = blk * 8 + ib;  // activation group of this sub-block
 #pragma unroll
             for (int r = 0; r < M; r++) {
-                const uint4 *ap = (const uint4 *)(p.qa + (uint64_t)r * k + (uint64_t)g * GROUP);
+                const uint4 *ap = (const uint4 *)(qa + (uint64_t)r * k + (uint64_t)g * GROUP);
                 const uint4 a0 = __ldg(ap), a1 = __ldg(ap + 1);
-                const float da = __ldg(p.da + (uint64_t)r * kg + g);
+                const float da = __ldg(da_base + (uint64_t)r * kg + g);
 #pragma unroll
                 for (int j = 0; j < ROWS; j++) {
                     int d0 = __dp4a((int)w[j][0], (int)a0.x, 0);
@@ -175,7 +190,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
                 }
             }
         }
-        if (base + gridDim.x * RPC < p.n) fetch(row0 + gridDim.x * RPC, blk0);  // the next pass
+        if (base + ctas * RPC < p.n) fetch(row0 + ctas * RPC, blk0);  // the next pass
 #pragma unroll
         for (int j = 0; j < ROWS; j++) {
 #pragma unroll
@@ -189,7 +204,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
                 } else if (lane == 0 && row < p.n) {
                     const uint32_t bt = r / p.m, i = r % p.m;
                     if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)row * p.ex_s2];
-                    p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
+                    out[(uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
                 }
             }
         }
@@ -204,7 +219,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
                 if (row < p.n) {
                     const uint32_t bt = r / p.m, i = r % p.m;
                     if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)row * p.ex_s2];
-                    p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
+                    out[(uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
                 }
             }
             __syncthreads();  // the partial sums are read: the next pass may overwrite them
@@ -212,13 +227,23 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(GemvArgs p, const 
     }
 }
 
-template <int FMT, int M, int ROWS, int WARPS, int KS = 1> static cudaError_t launch_r(const GemvArgs &a, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
+template <int FMT, int M, int ROWS, int WARPS, int KS, int NG> static cudaError_t launch_g(const GemvGroup &all, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
     constexpr uint32_t RPC = WARPS / KS * ROWS;
-    const uint32_t want = (a.n + RPC - 1) / RPC;
+    uint64_t want = 0;
+    for (int i = 0; i < all.count; i++) want += (all.item[i].n + RPC - 1) / RPC;
     uint32_t cap = (uint32_t)sm_count * 8 * (8 / WARPS);
     if (pairs > 1) cap = cap / pairs > 0 ? cap / pairs : 1;
+    GemvGroupT<NG> g{};
+    g.count = all.count;
+    uint32_t end = 0;
+    for (int i = 0; i < all.count; i++) {  // each member as many CTAs as it has tiles, or its share of the cap
+        g.item[i] = all.item[i];
+        const uint64_t tiles = (all.item[i].n + RPC - 1) / RPC;
+        uint64_t c = want <= cap ? tiles : (tiles * cap + want - 1) / want;
+        g.task_end[i] = end += (uint32_t)(c ? c : 1);
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(want < cap ? want : cap, pairs);
+    cfg.gridDim = dim3(end, pairs);
     cfg.blockDim = dim3(WARPS * 32);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -226,7 +251,11 @@ template <int FMT, int M, int ROWS, int WARPS, int KS = 1> static cudaError_t la
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, qgemv_iq_kernel<FMT, M, ROWS, WARPS, KS>, a, grid);
+    return cudaLaunchKernelEx(&cfg, qgemv_iq_kernel<FMT, M, ROWS, WARPS, KS, NG>, g, grid);
+}
+template <int FMT, int M, int ROWS, int WARPS, int KS = 1> static cudaError_t launch_r(const GemvGroup &g, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
+    if (g.count == 1) return launch_g<FMT, M, ROWS, WARPS, KS, 1>(g, grid, pairs, sm_count, pdl, stream);
+    return launch_g<FMT, M, ROWS, WARPS, KS, GEMV_GROUP_MAX>(g, grid, pairs, sm_count, pdl, stream);
 }
 
 // Two weight rows per warp share the activation loads and give the scheduler two independent decode chains: the
@@ -236,9 +265,11 @@ template <int FMT, int M, int ROWS, int WARPS, int KS = 1> static cudaError_t la
 // activation row: 24.2 us with two rows per warp, 19.8 with one).
 static int g_rows_per_warp = 0;  // 0: chosen per launch; 1, 2: forced (tests, sweeps)
 static int g_k_split = 0;        // 0: chosen per launch; 1, 2, 4: forced
-template <int FMT, int M> static cudaError_t launch_m(const GemvArgs &a, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
+template <int FMT, int M> static cudaError_t launch_m(const GemvGroup &a, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
     const uint64_t slots = (uint64_t)sm_count * 32;  // warps that keep the SMs' schedulers busy
-    const uint64_t rows = (uint64_t)a.n * pairs, steps = a.k / QK / 4;  // steps: passes of a warp over a row at four blocks per pass
+    uint64_t n = 0;
+    for (int i = 0; i < a.count; i++) n += a.item[i].n;
+    const uint64_t rows = n * pairs, steps = a.item[0].k / QK / 4;  // steps: passes of a warp over a row at four blocks per pass
     int rpw = g_rows_per_warp ? g_rows_per_warp : ((rows + 1) / 2 >= slots ? 2 : 1);
     int ksp = 1;
     if (g_k_split) ksp = g_k_split;
@@ -250,16 +281,17 @@ template <int FMT, int M> static cudaError_t launch_m(const GemvArgs &a, const u
     return launch_r<FMT, M, 1, 8>(a, grid, pairs, sm_count, pdl, stream);
 }
 
-template <int FMT> static cudaError_t launch_fmt(const GemvArgs &args, const uint8_t *grid, int sm_count, bool pdl, cudaStream_t stream) {
-    if (args.ids) {  // one-row GEMV per (token, slot) pair
-        if (args.id_r == 0 || args.id_e == 0 || args.rows > 8 || (uint64_t)args.rows * args.id_r > 65535 || (args.id_stride & 1))
+template <int FMT> static cudaError_t launch_fmt(const GemvGroup &args, const uint8_t *grid, int sm_count, bool pdl, cudaStream_t stream) {
+    const GemvArgs &a = args.item[0];
+    if (a.ids) {  // one-row GEMV per (token, slot) pair
+        if (args.count != 1 || a.id_r == 0 || a.id_e == 0 || a.rows > 8 || (uint64_t)a.rows * a.id_r > 65535 || (a.id_stride & 1))
             return cudaErrorInvalidValue;
-        GemvArgs one = args;
-        one.rows = 1;
-        one.m = 1;
-        return launch_m<FMT, 1>(one, grid, args.rows * args.id_r, sm_count, pdl, stream);
+        GemvGroup one = args;
+        one.item[0].rows = 1;
+        one.item[0].m = 1;
+        return launch_m<FMT, 1>(one, grid, a.rows * a.id_r, sm_count, pdl, stream);
     }
-    switch (args.rows) {
+    switch (a.rows) {
         case 1: return launch_m<FMT, 1>(args, grid, 1, sm_count, pdl, stream);
         case 2: return launch_m<FMT, 2>(args, grid, 1, sm_count, pdl, stream);
         case 3: return launch_m<FMT, 3>(args, grid, 1, sm_count, pdl, stream);
@@ -277,9 +309,13 @@ template <int FMT> static cudaError_t launch_fmt(const GemvArgs &args, const uin
 void qgemv_iq_set_rows_per_warp(int rows) { iq::g_rows_per_warp = rows == 1 || rows == 2 ? rows : 0; }
 void qgemv_iq_set_k_split(int ways) { iq::g_k_split = ways == 1 || ways == 2 || ways == 4 ? ways : 0; }
 
-cudaError_t launch_qgemv_iq(int fmt, const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream) {
-    if (args.n == 0 || args.rows == 0) return cudaSuccess;
-    if (!is_iq(fmt) || args.k % QK != 0 || ((uintptr_t)args.w & 1) != 0 || ((uintptr_t)args.qa & 15) != 0) return cudaErrorInvalidValue;
+cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &args, int sm_count, bool pdl, cudaStream_t stream) {
+    if (args.count < 1 || args.count > GEMV_GROUP_MAX) return cudaErrorInvalidValue;
+    for (int i = 0; i < args.count; i++) {  // members: same rows, k and activations, none of them empty
+        const GemvArgs &a = args.item[i];
+        if (args.count == 1 && (a.n == 0 || a.rows == 0)) return cudaSuccess;
+        if (!is_iq(fmt) || a.n == 0 || a.k % QK != 0 || ((uintptr_t)a.w & 1) != 0 || ((uintptr_t)a.qa & 15) != 0) return cudaErrorInvalidValue;
+    }
     const uint8_t *grids = iq_grids();
     if (!grids) return cudaErrorNotReady;
     const uint8_t *grid = grids + iq_grid_offset(fmt);
