@@ -346,6 +346,8 @@ struct ActSlot {
     // An expert-indexed launch on the tensor cores: its key is tokens, slots, experts (off), tile height (rs) and the two buffers; `offset` is where
     // its routing tables and gathered rows lie, those of the first launch (`owner`) where it shares them.
     static constexpr int MOE_COPY = 4;
+    // An expert-indexed decode launch: its key is the tokens and the layout (off) they are quantized in; `offset` is where, shared like the above.
+    static constexpr int MOE_ACT = 5;
     const void *ids = nullptr;
     size_t copy_offset = 0, written_before = 0;
     int owner = -1;
@@ -367,12 +369,21 @@ void finish_expr(lapid_b200_device &dev, const lb::GemvArgs &it) {
     dev.launches++;
 }
 
+// A launch of one.
+lb::GemvGroup one_of(const lb::GemvArgs &a) {
+    lb::GemvGroup g{};
+    g.count = 1;
+    g.item[0] = a;
+    return g;
+}
+
 struct PendingGroup {
     struct Range {
         const char *lo, *hi;
         bool hits(const Range &o) const { return lo < o.hi && o.lo < hi; }
     };
-    int fmt = 0, mode = 0;  // kernel of the members: 1 = dp4a kernel, 2 = tensor-core kernel, 3 = balanced-stream tensor-core kernel, 4 = i-quant kernel
+    int fmt = 0, mode = 0;  // kernel of the members: 1 = dp4a kernel, 2 = tensor-core kernel, 3 = balanced-stream tensor-core kernel, 4 = row kernels of MXFP4 and
+                            // the i-quants, 5 = the same, expert-indexed
     lb::GemvGroup g{};
     bool split_early = false;  // see accepts()
     bool serial = false;       // an earlier launch of the list writes what a member fetches early (run_launch: src_written)
@@ -395,9 +406,9 @@ struct PendingGroup {
             if (r.hits(out)) return false;
         g.item[g.count] = a;
         g.count++;
-        if (md == 4 || f == LAPID_B200_DTYPE_INT8 || f == LAPID_B200_DTYPE_INT4) {  // (one activation operand for the whole launch)
+        if (md >= 4 || f == LAPID_B200_DTYPE_INT8 || f == LAPID_B200_DTYPE_INT4) {  // (one activation operand for the whole launch)
             g.count--;
-            return a.qa == g.item[0].qa;
+            return a.qa == g.item[0].qa && a.ids == g.item[0].ids && a.id_r == g.item[0].id_r;
         }
         bool fits = md == 3 ? true  // its shared memory does not depend on the members
                     : md != 2 ? lb::qgemv_kq_group_smem(f, g) <= 227 * 1024 - 256
@@ -426,7 +437,8 @@ struct PendingGroup {
         serial = false;
         const uint64_t before = dev.stream_ws.kernels;
         if (mode == 3) cuda_check(lb::launch_qgemv_kq_stream(fmt, out, dev.stream_ws, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        else if (mode == 4) cuda_check(lb::launch_qgemv_iq(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (mode >= 4 && fmt == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(out, dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (mode >= 4) cuda_check(lb::launch_qgemv_iq(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (fmt == LAPID_B200_DTYPE_INT8 || fmt == LAPID_B200_DTYPE_INT4)
             cuda_check(lb::launch_qgemv_i8_mma(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (mode == 2 && fmt == LAPID_B200_DTYPE_Q6_K) cuda_check(lb::launch_qgemv_q6k_mma(out, dev.sm_count, pdl, dev.stream), "qgemv launch");
@@ -690,8 +702,10 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
 }
 
 void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_buffer *const *buffers, size_t n_buffers,
-                   ActSlot *slot) {
+                   ActSlot *slot, PendingGroup *pend) {
     MoePlan p = plan_matmul_id(dev, l);
+    const bool grouped = pend && p.decode && !p.noop && !p.zero_k && (is_iquant(l.b_dtype) || l.b_dtype == LAPID_B200_DTYPE_MXFP4);
+    if (pend && !grouped) pend->flush(dev);
     auto get = [&](uint32_t id) -> lapid_b200_buffer * {
         if (id >= n_buffers || !buffers[id])
             fail("invalid_launch", "buffer id " + std::to_string(id) + " out of range (" + std::to_string(n_buffers) + " buffers)");
@@ -719,6 +733,13 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
     else dev.ensure_scratch(p.scratch);
     char *base = (char *)dev.scratch + off;
     if (p.decode) {
+        ActSlot *quantized = slot && slot->records == ActSlot::MOE_ACT ? slot - (slot->owner >= 0 ? slot->owner : 0) : nullptr;
+        auto quantize = [&](const lb::ActQuantArgs &q) {
+            if (quantized && quantized->done) return;
+            cuda_check(lb::launch_act_quant(q, dev.sm_count, dev.pdl_launch(), dev.stream), "act_quant launch");
+            dev.launches++;
+            if (quantized) quantized->done = true;
+        };
         size_t qa_b = align_up(p.t * l.k, 256), sc_b = align_up(p.t * (l.k / 32) * 4, 256);
         lb::ActQuantArgs q{};
         q.a = (const float *)x->ptr;
@@ -730,7 +751,6 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         q.da = (float *)(base + qa_b);
         q.bs = has_min_term(l.b_dtype) ? (float *)(base + qa_b + sc_b) : nullptr;
         q.records = p.fast ? 1 : 0;
-        cuda_check(lb::launch_act_quant(q, dev.sm_count, dev.pdl_launch(), dev.stream), "act_quant launch");
         lb::GemvArgs g{};
         g.w = (const uint8_t *)w->ptr;
         g.w_bytes = w->bytes;
@@ -749,18 +769,23 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         g.id_stride = p.wl.total;
         g.id_r = (uint32_t)p.r;
         g.id_e = (uint32_t)p.e;
+        if (grouped) {  // gate and up: the same tokens and ids
+            using Range = PendingGroup::Range;
+            auto whole = [](const lapid_b200_buffer *b) { return Range{(const char *)b->ptr, (const char *)b->ptr + b->bytes}; };
+            const Range wr{(const char *)out->ptr, (const char *)out->ptr + pairs * l.n * 4}, in[3] = {whole(x), whole(w), whole(ids)};
+            if (!pend->accepts(l.b_dtype, 5, g, wr, in, 3)) pend->flush(dev);
+            quantize(q);  // (no pending launch writes its input)
+            pend->add(l.b_dtype, 5, g, wr, in, 3);
+            return;
+        }
+        quantize(q);
         const bool pdl = dev.pdl_launch();
         if (l.b_dtype == LAPID_B200_DTYPE_INT4) cuda_check(lb::launch_qgemv_i4(g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
-        else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
-        else if (is_iquant(l.b_dtype)) {
-            lb::GemvGroup one{};
-            one.count = 1;
-            one.item[0] = g;
-            cuda_check(lb::launch_qgemv_iq(l.b_dtype, one, dev.sm_count, pdl, dev.stream), "matmul_id launch");
-        }
+        else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(one_of(g), dev.sm_count, pdl, dev.stream), "matmul_id launch");
+        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, one_of(g), dev.sm_count, pdl, dev.stream), "matmul_id launch");
         else if (p.fast) cuda_check(lb::launch_qgemv_kq_moe(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         else cuda_check(lb::launch_qgemv_moe(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
-        dev.launches += 2;
+        dev.launches++;
         return;
     }
     lb::MoeRouteArgs route{};
@@ -824,8 +849,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
         return;
     }
     if (l.kind == LAPID_B200_KERNEL_MATMUL_ID) {
-        if (pend) pend->flush(dev);
-        run_matmul_id(dev, l, buffers, n_buffers, slot);
+        run_matmul_id(dev, l, buffers, n_buffers, slot, pend);
         return;
     }
     Plan p = plan_launch(dev, l);
@@ -958,14 +982,15 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
         g.a_bs = q.a_bs;
         g.a_rs = q.a_rs;
         g.status = dev.status_dev;
-        if (pend && (is_iquant(l.b_dtype) || (slot->records && l.b_dtype != LAPID_B200_DTYPE_MXFP4))) {  // (the MXFP4 kernels take one launch at a time)
+        const bool row_kernel = is_iquant(l.b_dtype) || (l.b_dtype == LAPID_B200_DTYPE_MXFP4 && !slot->records);
+        if (pend && (row_kernel || (slot->records && l.b_dtype != LAPID_B200_DTYPE_MXFP4))) {  // (the MXFP4 tensor-core kernel takes one launch at a time)
             using Range = PendingGroup::Range;
             const char *ob = (const char *)out->ptr;
             Range wr{ob + 4 * l.out.offset, ob + 4 * last};
             Range in[3];
             int n_in = 0;
             for (int i = 0; i < l.n_inputs; i++) in[n_in++] = Range{(const char *)ins[i]->ptr, (const char *)ins[i]->ptr + ins[i]->bytes};
-            const int mode = is_iquant(l.b_dtype) ? 4 : slot->records == 2 && p.stream ? 3 : slot->records;
+            const int mode = row_kernel ? 4 : slot->records == 2 && p.stream ? 3 : slot->records;
             g.early = slot->hoisted ? 1 : 0;  // gated again when the group goes out
             if (!pend->accepts(l.b_dtype, mode, g, wr, in, n_in)) pend->flush(dev);
             if (!slot->done) {  // its input is not written by a pending launch (checked above), so it may run first
@@ -1006,13 +1031,8 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
         else if (l.b_dtype == LAPID_B200_DTYPE_INT4 && p.fast_i8 && ((uintptr_t)g.w & 15) == 0 && (g.scales_offset & 15) == 0)
             cuda_check(lb::launch_qgemv_i4_fast(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (l.b_dtype == LAPID_B200_DTYPE_INT4) cuda_check(lb::launch_qgemv_i4(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        else if (is_iquant(l.b_dtype)) {
-            lb::GemvGroup one{};
-            one.count = 1;
-            one.item[0] = g;
-            cuda_check(lb::launch_qgemv_iq(l.b_dtype, one, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        }
+        else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(one_of(g), dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, one_of(g), dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (p.fast_i8 && ((uintptr_t)g.w & 15) == 0) cuda_check(lb::launch_qgemv_i8_fast(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else cuda_check(lb::launch_qgemv(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         dev.launches += dev.stream_ws.kernels > ws_before ? dev.stream_ws.kernels - ws_before : 1;  // (the stream kernel may take two)
@@ -1137,21 +1157,22 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
                 sl.offset = scratch_total;
                 // the routing tables and the gathered rows of an earlier launch with the same tokens and ids (gate and up), as long as nothing
                 // since has written either buffer
-                if (p.tc && xb && ib) {
-                    sl.records = ActSlot::MOE_COPY;
+                const bool act = p.decode && !p.noop && !p.zero_k;  // the quantized tokens of an earlier launch that reads them in the same layout
+                if ((p.tc || act) && xb && ib) {
+                    sl.records = act ? ActSlot::MOE_ACT : ActSlot::MOE_COPY;
                     sl.ptr = xb->ptr;
-                    sl.ids = ib->ptr;
+                    sl.ids = act ? nullptr : ib->ptr;
                     sl.rows = (uint32_t)p.t;
-                    sl.m = (uint32_t)p.r;
+                    sl.m = act ? 0 : (uint32_t)p.r;
                     sl.k = (uint32_t)l.k;
-                    sl.off = p.e;
+                    sl.off = act ? (p.fast ? 1 : 0) + (has_min_term(l.b_dtype) ? 2 : 0) : p.e;
                     sl.rs = p.mt;
                     sl.written_before = written.size();
                     for (size_t s2 = slots.size(); s2-- > 0 && dev->act_reuse;) {
                         if (!slots[s2].same(sl) || slots[s2].ids != sl.ids || slots[s2].owner >= 0) continue;
                         bool clean = true;
                         for (size_t w = slots[s2].written_before; w < written.size(); w++)
-                            for (const lapid_b200_buffer *b : {xb, ib})
+                            for (const lapid_b200_buffer *b : {xb, act ? xb : ib})
                                 if ((const char *)b->ptr < written[w].hi && written[w].lo < (const char *)b->ptr + b->bytes) clean = false;
                         if (clean) {
                             sl.owner = (int)(slots.size() - s2);
@@ -1698,7 +1719,7 @@ lapid_b200_status lapid_b200_device_set_option(lapid_b200_device *dev, const cha
         } else if (k == "gemv_mxfp4_k_split") {
             lb::qgemv_mxfp4_set_k_split(std::atoi(value));
         } else if (k == "gemv_mxfp4_staged") {
-            lb::qgemv_mxfp4_set_staged(std::atoi(value));
+            // accepted, without effect: the MXFP4 decode kernel has one form
         } else if (k == "gemv_iq_k_split") {
             lb::qgemv_iq_set_k_split(std::atoi(value));
         } else if (k == "gemv_iq_rows") {  // weight rows per warp of the i-quant decode kernel: 1, 2 (0: per launch)

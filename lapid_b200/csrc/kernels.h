@@ -132,14 +132,12 @@ cudaError_t launch_qgemv(int fmt, const GemvArgs &args, int sm_count, bool pdl, 
 cudaError_t launch_qgemv_moe(int fmt, const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream);
 // ---- qgemv_i4.cu: Int4 nibble planes, 1..8 rows (and the expert-indexed form: args.ids set, rows = tokens)
 cudaError_t launch_qgemv_i4(const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream);
-// ---- qgemv_mxfp4.cu: MXFP4 blocks, 1..8 rows (and the expert-indexed form: args.ids set, rows = tokens); reads the planes
-cudaError_t launch_qgemv_mxfp4(const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream);
+// ---- qgemv_mxfp4.cu (launch_qgemv_mxfp4 below): MXFP4 blocks, 1..8 rows (and the expert-indexed form: args.ids set, rows = tokens); reads the planes
 // qgemv_mxfp4_mma.cu: the same blocks on the int8 tensor-core instruction (K a multiple of 512; the activation tiles
 // of the K-quant kernels)
 bool qgemv_mxfp4_mma_shape_ok(uint32_t rows, uint32_t k);
 cudaError_t launch_qgemv_mxfp4_mma(const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream);
-void qgemv_mxfp4_set_k_split(int ways);  // warps per row of the direct form: 0: per launch (default); 1, 2, 4: forced
-void qgemv_mxfp4_set_staged(int on);  // 1 (default): rows staged through shared memory where K allows; 0: direct loads only
+void qgemv_mxfp4_set_k_split(int ways);  // warps per row: 0: per launch (default); 1, 2, 4: forced
 
 // ---- qgemv_iq.cu: the grid-based i-quants (IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS), 1..8 rows (and the expert-indexed form);
 // reads the activation planes, the codebooks from the per-device table of iquant.cu
@@ -214,6 +212,7 @@ template <int N> struct GemvGroupT {
 };
 using GemvGroup = GemvGroupT<GEMV_GROUP_MAX>;
 using GemvSingle = GemvGroupT<1>;  // what a lone launch passes to the kernel: a sixth of the parameter bytes
+cudaError_t launch_qgemv_mxfp4(const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);         // ... (and the same ids)
 cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);  // members read the same activations
 size_t qgemv_kq_group_smem(int fmt, GemvGroup &group);  // dynamic shared memory the group would need
 cudaError_t launch_qgemv_kq_group(int fmt, GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);

@@ -284,11 +284,10 @@ template <int FMT, int M> static cudaError_t launch_m(const GemvGroup &a, const 
 template <int FMT> static cudaError_t launch_fmt(const GemvGroup &args, const uint8_t *grid, int sm_count, bool pdl, cudaStream_t stream) {
     const GemvArgs &a = args.item[0];
     if (a.ids) {  // one-row GEMV per (token, slot) pair
-        if (args.count != 1 || a.id_r == 0 || a.id_e == 0 || a.rows > 8 || (uint64_t)a.rows * a.id_r > 65535 || (a.id_stride & 1))
+        if (a.id_r == 0 || a.id_e == 0 || a.rows > 8 || (uint64_t)a.rows * a.id_r > 65535 || (a.id_stride & 1))
             return cudaErrorInvalidValue;
         GemvGroup one = args;
-        one.item[0].rows = 1;
-        one.item[0].m = 1;
+        for (int i = 0; i < args.count; i++) one.item[i].rows = one.item[i].m = 1;
         return launch_m<FMT, 1>(one, grid, a.rows * a.id_r, sm_count, pdl, stream);
     }
     switch (a.rows) {
@@ -311,7 +310,7 @@ void qgemv_iq_set_k_split(int ways) { iq::g_k_split = ways == 1 || ways == 2 || 
 
 cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &args, int sm_count, bool pdl, cudaStream_t stream) {
     if (args.count < 1 || args.count > GEMV_GROUP_MAX) return cudaErrorInvalidValue;
-    for (int i = 0; i < args.count; i++) {  // members: same rows, k and activations, none of them empty
+    for (int i = 0; i < args.count; i++) {  // members: same rows, k, activations and ids, none of them empty
         const GemvArgs &a = args.item[i];
         if (args.count == 1 && (a.n == 0 || a.rows == 0)) return cudaSuccess;
         if (!is_iq(fmt) || a.n == 0 || a.k % QK != 0 || ((uintptr_t)a.w & 1) != 0 || ((uintptr_t)a.qa & 15) != 0) return cudaErrorInvalidValue;

@@ -5,249 +5,96 @@
 //
 //     acc += d * da_g * f32(sum_32 qa * KV[q])          one activation group per weight block
 //
-// One warp per weight row; a lane takes every 32nd block of the row. Blocks are 17 bytes long, so they start on
-// any byte boundary: the 16 nibble bytes are fetched as aligned 32-bit words and funnel-shifted into place. Four
-// codes become four int8 KV values with three byte-permutes and three logic operations (mxfp4_kv4 in common.cuh: the
-// four nibbles of a 16-bit half are used as the permute's selector as they are), multiplied with `dp4a` against the
-// activation planes (served by L1/L2), whose bytes one more permute per word brings into the same element order.
-// Two forms. When a weight row is a multiple of 16 bytes (K a multiple of 512) every warp streams its rows through a
-// shared-memory double buffer with 16-byte `cp.async` copies: the copy of the next row is in flight while the current
-// one is multiplied (one and two activation rows, K up to 8192: 4096 x 4096 at one row 7.6 against 9.2 us, 14336 x 4096
-// 15.8 against 17.2 us). Other launches read the blocks straight from global memory. Either way the kernel is bound
-// by the instructions that unpack a block (some 120 per 32 weights at one row), not by HBM (0.2-0.3 of its rate);
-// from three rows on the launches go to the tensor-core kernel of qgemv_mxfp4_mma.cu.
+// on the skeleton of row_stream.cuh (its unit is a block). Blocks are 17 bytes long, so they start on any byte boundary: they are fetched as the aligned
+// 32-bit words around them and funnel-shifted into place. The four nibbles of a 16-bit half are the codes of elements j, j + 16, j + 1, j + 17 and exactly
+// a `prmt` selector over the table of magnitudes; the activations are put into that order once, when they are copied to shared memory.
+// One and two rows: bit 3 of a selector nibble replicates the chosen byte's top bit, which no magnitude has, so one `prmt` gives the magnitudes of the positive
+// codes and 0 elsewhere, a second, on the word with all the sign bits turned round, those of the negative codes: the sum is the difference of two `dp4a`
+// chains, and nothing is spent on signs. From three rows on (K no multiple of 512; the others go to qgemv_mxfp4_mma.cu) the signed values are made once (mxfp4_kv4).
+// Before (a row at a time per warp, activations read from L1 for every row, seven operations for four signed values, rows staged through shared memory by 16-byte
+// copies where K allowed) -> now, us: 14336 x 4096 17.0 -> 13.3, 28672 x 4096 29.5 -> 20.7, 4096 x 14336 18.9 -> 13.9, 4096 x 4096 6.7 -> 6.3, two rows on 14336 x 4096
+// 19.2 -> 16.1, six experts of 2304 x 5120 22.1 -> 15.7, of 5120 x 2304 25.7 -> 18.6, five rows on 4096 x 2880 14.4 -> 10.2. The six experts' 37.6 MB need 5.8 us.
 #include "common.cuh"
 #include "kernels.h"
+#include "row_stream.cuh"
 
 namespace lb {
 namespace mx {
 
-constexpr int WARPS = 8;
-
-// One 17-byte block at `b` (global or shared memory, any alignment) against activation group g of every row.
-template <int M> __device__ __forceinline__ void block_dot(const uint8_t *b, const GemvArgs &p, uint32_t g, uint32_t k, uint32_t kg, float (&acc)[M]) {
-    const float d = e8m0_half(*b);
-    // the 16 nibble bytes b[1..16] from the aligned words around them
-    const uintptr_t q0 = (uintptr_t)(b + 1);
-    const uint32_t *wp = (const uint32_t *)(q0 & ~(uintptr_t)3);
-    const uint32_t sh = (uint32_t)(q0 & 3) * 8;
-    uint32_t raw[5];
-#pragma unroll
-    for (int i = 0; i < 4; i++) raw[i] = wp[i];
-    raw[4] = sh ? wp[4] : 0u;  // (aligned blocks end with the fourth word: nothing is read behind them)
-    // word i holds the codes of elements 4i..4i+3 (low nibbles) and 16+4i.. (high nibbles): q[2i] = KV of elements
-    // (4i, 4i+16, 4i+1, 4i+17), q[2i+1] of (4i+2, 4i+18, 4i+3, 4i+19) as int8 (mxfp4_kv4)
-    uint32_t q[8];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint32_t w = __funnelshift_r(raw[i], raw[i + 1], sh);
-        q[2 * i] = mxfp4_kv4(w);
-        q[2 * i + 1] = mxfp4_kv4(w >> 16);
-    }
-#pragma unroll
-    for (int r = 0; r < M; r++) {
-        const uint4 *ap = (const uint4 *)(p.qa + (uint64_t)r * k + (uint64_t)g * GROUP);
-        const uint4 a0 = __ldg(ap), a1 = __ldg(ap + 1);
-        const float da = __ldg(p.da + (uint64_t)r * kg + g);
-        const uint32_t al[4] = {a0.x, a0.y, a0.z, a0.w}, ah[4] = {a1.x, a1.y, a1.z, a1.w};
-        int dp = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {  // the activations in the same element order
-            dp = __dp4a((int)q[2 * i], (int)prmt(al[i], ah[i], 0x5140u), dp);
-            dp = __dp4a((int)q[2 * i + 1], (int)prmt(al[i], ah[i], 0x7362u), dp);
-        }
-        acc[r] = fmaf(d * da, (float)dp, acc[r]);
-    }
-}
-
-// KS warps share a row and split its blocks (matrices with few rows and a long K would otherwise leave most warp slots of
-// an SM empty); their partial sums meet in shared memory and are added in warp order.
-template <int M, int KS> __global__ void __launch_bounds__(WARPS * 32) qgemv_mxfp4_kernel(GemvArgs p) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t k = p.k, kg = k / GROUP;
-    if (p.ids) {
-        // Expert-indexed launch (Kernel::MatMulId at decode sizes): grid row y is one (token, slot) pair
-        const uint32_t pair = blockIdx.y, token = pair / p.id_r;
-        const int32_t id = p.ids[pair];
-        const bool bad = id < 0 || (uint32_t)id >= p.id_e;
-        if (bad && p.status && threadIdx.x == 0) atomicOr(p.status, 128);
-        p.w += bad ? 0 : (uint64_t)id * p.id_stride;
-        p.qa += (uint64_t)token * k;
-        p.da += (uint64_t)token * kg;
-        p.out_off += (uint64_t)pair * p.n;
-    }
-    constexpr int RPC = WARPS / KS;  // rows of a CTA per pass
-    const int wg = warp / KS, ks = warp % KS;
-    __shared__ float part[KS > 1 ? WARPS * M : 1];
-    for (uint32_t base = blockIdx.x * RPC; base < p.n; base += gridDim.x * RPC) {  // (the same number of passes for every warp of the CTA)
-        const uint32_t row = base + wg, rrow = row < p.n ? row : p.n - 1;  // (a row past the end repeats the last one; not stored)
-        float acc[M];
-#pragma unroll
-        for (int r = 0; r < M; r++) acc[r] = 0.0f;
-        const uint8_t *wrow = p.w + (uint64_t)rrow * kg * MXFP4_BYTES;
-        for (uint32_t g = lane + 32 * ks; g < kg; g += 32 * KS) block_dot<M>(wrow + (uint64_t)g * MXFP4_BYTES, p, g, k, kg, acc);
-#pragma unroll
-        for (int r = 0; r < M; r++) {
-            float v = acc[r];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if constexpr (KS > 1) {
-                if (lane == 0) part[warp * M + r] = v;
-            } else if (lane == 0 && row < p.n) {
-                const uint32_t bt = r / p.m, i = r % p.m;
-                if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)row * p.ex_s2];
-                p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
-            }
-        }
-        if constexpr (KS > 1) {
-            __syncthreads();
-            if (ks == 0 && lane < M && row < p.n) {
-                const int r = lane;
-                float v = part[warp * M + r];
-#pragma unroll
-                for (int s2 = 1; s2 < KS; s2++) v += part[(warp + s2) * M + r];
-                const uint32_t bt = r / p.m, i = r % p.m;
-                if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)row * p.ex_s2];
-                p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
-            }
-            __syncthreads();  // the partial sums are read: the next pass may overwrite them
-        }
-    }
-}
-
-// K a multiple of 512 (weight rows are multiples of 16 bytes): the same arithmetic with every warp's rows streamed
-// through its own double buffer in shared memory. The weights do not depend on the launch before this one, so the
-// first row is requested before that launch's results are waited for.
-template <int M> __global__ void __launch_bounds__(WARPS * 32) qgemv_mxfp4_staged_kernel(GemvArgs p) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t k = p.k, kg = k / GROUP, rowb = kg * MXFP4_BYTES;
-    const uint32_t slot = rowb + 16;  // (the aligned loads around a block's last nibble bytes may reach up to three bytes past the row)
-    uint8_t *buf = smem + (size_t)warp * 2 * slot;
-    if (p.ids) {
-        // Expert-indexed launch (Kernel::MatMulId at decode sizes): grid row y is one (token, slot) pair; the ids may
-        // come from the launch before this one
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        const uint32_t pair = blockIdx.y, token = pair / p.id_r;
-        const int32_t id = p.ids[pair];
-        const bool bad = id < 0 || (uint32_t)id >= p.id_e;
-        if (bad && p.status && threadIdx.x == 0) atomicOr(p.status, 128);
-        p.w += bad ? 0 : (uint64_t)id * p.id_stride;
-        p.qa += (uint64_t)token * k;
-        p.da += (uint64_t)token * kg;
-        p.out_off += (uint64_t)pair * p.n;
-    }
-    auto request = [&](uint32_t row, uint8_t *dst) {
-        const uint8_t *src = p.w + (uint64_t)row * rowb;
-        for (uint32_t c = lane; c < rowb / 16; c += 32)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + 16 * c)), "l"(src + 16 * (size_t)c) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
+template <bool SPLIT> struct Format {  // SPLIT: positive and negative codes apart
+    static constexpr int M_MIN = SPLIT ? 1 : 3, M_MAX = SPLIT ? 2 : 8;
+    static constexpr uint32_t STEP_BYTES = 32 * MXFP4_BYTES;
+    static constexpr float FACTOR = 1.0f;
+    static __host__ __device__ uint64_t row_bytes(uint32_t k) { return (uint64_t)(k / GROUP) * MXFP4_BYTES; }
+    static __device__ __forceinline__ uint32_t lane_offset(int lane) { return lane * MXFP4_BYTES; }
+    struct Raw {
+        uint32_t w[5], sh;  // the aligned words that hold the block's 17 bytes, each of them some of them; bits before the first
     };
-    const uint32_t stride = gridDim.x * WARPS;
-    uint32_t row = blockIdx.x * WARPS + warp;
-    if (row < p.n) request(row, buf);
-    if (!p.ids) asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (int cur = 0; row < p.n; row += stride, cur ^= 1) {
-        if (row + stride < p.n) {
-            request(row + stride, buf + (cur ^ 1) * slot);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    static __device__ __forceinline__ Raw none() { return Raw{{0u, 0u, 0u, 0u, 0u}, 0u}; }
+    static __device__ __forceinline__ Raw load(const uint8_t *base, uint32_t at, int) {
+        const uint32_t *a = (const uint32_t *)(base + (at & ~3u));
+        Raw r;
+#pragma unroll
+        for (int i = 0; i < 5; i++) r.w[i] = __ldg(a + i);
+        r.sh = (at & 3u) * 8;
+        return r;
+    }
+    struct W {
+        uint32_t q[8];  // SPLIT: q[i] the nibbles of four elements (low half) of each kind; else the values
+        float d;
+    };
+    static __device__ __forceinline__ W unpack(const Raw &r) {
+        W o;
+        o.d = e8m0_half((r.w[0] >> r.sh) & 255u);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t w = __funnelshift_rc(r.w[i], r.w[i + 1], r.sh + 8);  // elements 4i.. (low nibbles), 16 + 4i.. (high nibbles)
+            if constexpr (SPLIT) o.q[i] = w, o.q[4 + i] = 0;
+            else o.q[2 * i] = mxfp4_kv4(w), o.q[2 * i + 1] = mxfp4_kv4(w >> 16);
         }
-        __syncwarp();  // every lane's part of the row has landed
-        float acc[M];
+        return o;
+    }
+    static __device__ __forceinline__ float dot(const W &w, const uint32_t (&a)[8]) {
+        // |sum| <= 32 * 127 * 12 < 2^22: added to the bit pattern of 1.5 * 2^23 it lands in the mantissa, and one exact subtraction makes it a float
+        int pos = 0x4B400000, neg = 0;
+        if constexpr (SPLIT) {
 #pragma unroll
-        for (int r = 0; r < M; r++) acc[r] = 0.0f;
-        const uint8_t *wrow = buf + cur * slot;
-        for (uint32_t g = lane; g < kg; g += 32) block_dot<M>(wrow + g * MXFP4_BYTES, p, g, k, kg, acc);
-#pragma unroll
-        for (int r = 0; r < M; r++) {
-            float v = acc[r];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) {
-                const uint32_t bt = r / p.m, i = r % p.m;
-                if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)row * p.ex_s2];
-                p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
+            for (int i = 0; i < 4; i++) {
+                const uint32_t p = w.q[i], n = p ^ 0x88888888u;
+                pos = __dp4a((int)prmt(0x03020100u, 0x0C080604u, p), (int)a[2 * i], pos);
+                neg = __dp4a((int)prmt(0x03020100u, 0x0C080604u, n), (int)a[2 * i], neg);
+                pos = __dp4a((int)prmt(0x03020100u, 0x0C080604u, p >> 16), (int)a[2 * i + 1], pos);
+                neg = __dp4a((int)prmt(0x03020100u, 0x0C080604u, n >> 16), (int)a[2 * i + 1], neg);
             }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) pos = __dp4a((int)w.q[i], (int)a[i], pos), neg = __dp4a((int)w.q[4 + i], (int)a[4 + i], neg);
         }
-        __syncwarp();  // the buffer is refilled one iteration from now: every lane is done reading it
+        return __int_as_float(SPLIT ? pos - neg : pos + neg) - 12582912.0f;
     }
-}
+    // bytes of a group in the order of the nibbles: (0, 16, 1, 17), (2, 18, 3, 19), ...
+    static __device__ __forceinline__ void order(uint4 &lo, uint4 &hi) {
+        const uint4 l = lo, h = hi;
+        lo = make_uint4(prmt(l.x, h.x, 0x5140u), prmt(l.x, h.x, 0x7362u), prmt(l.y, h.y, 0x5140u), prmt(l.y, h.y, 0x7362u));
+        hi = make_uint4(prmt(l.z, h.z, 0x5140u), prmt(l.z, h.z, 0x7362u), prmt(l.w, h.w, 0x5140u), prmt(l.w, h.w, 0x7362u));
+    }
+};
 
-static bool g_staged = true;  // (tests switch the staged form off to reach the other one at the same shapes)
-static int g_k_split = 0;     // warps per row of the direct form: 0: chosen per launch; 1, 2, 4: forced
-template <int M> static cudaError_t launch_m(const GemvArgs &a, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
-    const uint32_t want = (a.n + WARPS - 1) / WARPS;
-    uint32_t cap = (uint32_t)sm_count * 8;
-    if (pairs > 1) cap = cap / pairs > 0 ? cap / pairs : 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(want < cap ? want : cap, pairs);
-    cfg.blockDim = dim3(WARPS * 32);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    // rows of 16-byte multiples at 16-byte aligned addresses: the staged form, for one and two activation rows (beyond
-    // that the `dp4a` work hides the loads anyway) and while at least three CTAs' buffers fit an SM
-    // (4096 x 14336 at eight rows: 83 us staged with one CTA per SM, 45 us direct)
-    const size_t smem = (size_t)WARPS * 2 * ((size_t)a.k / GROUP * MXFP4_BYTES + 16);
-    const bool aligned = a.k % 512 == 0 && ((uintptr_t)a.w & 15) == 0 && (!a.ids || (a.id_stride & 15) == 0);
-    if (aligned && M <= 2 && smem <= 72 * 1024 && g_staged) {
-        static DynamicSmemOptIn optin;
-        cudaError_t e = optin.raise((const void *)qgemv_mxfp4_staged_kernel<M>, smem);
-        if (e != cudaSuccess) return e;
-        cfg.dynamicSmemBytes = smem;
-        return cudaLaunchKernelEx(&cfg, qgemv_mxfp4_staged_kernel<M>, a);
-    }
-    // direct loads: one warp per row, or two / four warps per row when the rows alone leave most warp slots empty
-    // and are long enough to split
-    const uint64_t rows = (uint64_t)a.n * pairs, slots = (uint64_t)sm_count * 32, steps = a.k / GROUP / 32;
-    int ksp = 1;
-    if (g_k_split) ksp = g_k_split;
-    else
-        while (ksp < 4 && rows * ksp < slots && steps / (2 * ksp) >= 2) ksp *= 2;
-    if (ksp > 1) {
-        const uint32_t rpc = WARPS / ksp, want2 = (a.n + rpc - 1) / rpc;
-        cfg.gridDim = dim3(want2 < cap ? want2 : cap, pairs);
-        if (ksp == 2) return cudaLaunchKernelEx(&cfg, qgemv_mxfp4_kernel<M, 2>, a);
-        return cudaLaunchKernelEx(&cfg, qgemv_mxfp4_kernel<M, 4>, a);
-    }
-    return cudaLaunchKernelEx(&cfg, qgemv_mxfp4_kernel<M, 1>, a);
-}
+static int g_k_split = 0;  // warps per row: 0: chosen per launch; 1, 2, 4: forced
 
 }  // namespace mx
 
-void qgemv_mxfp4_set_staged(int on) { mx::g_staged = on != 0; }
 void qgemv_mxfp4_set_k_split(int ways) { mx::g_k_split = ways == 1 || ways == 2 || ways == 4 ? ways : 0; }
 
-cudaError_t launch_qgemv_mxfp4(const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream) {
-    if (args.n == 0 || args.rows == 0) return cudaSuccess;
-    if (args.k % GROUP != 0 || ((uintptr_t)args.w & 3) != 0) return cudaErrorInvalidValue;
-    if (args.ids) {  // one-row GEMV per (token, slot) pair
-        if (args.id_r == 0 || args.id_e == 0 || args.rows > 8 || (uint64_t)args.rows * args.id_r > 65535 || (args.id_stride & 3))
-            return cudaErrorInvalidValue;
-        GemvArgs one = args;
-        one.rows = 1;
-        one.m = 1;
-        return mx::launch_m<1>(one, args.rows * args.id_r, sm_count, pdl, stream);
+cudaError_t launch_qgemv_mxfp4(const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream) {
+    if (group.count < 1 || group.count > GEMV_GROUP_MAX) return cudaErrorInvalidValue;
+    for (int i = 0; i < group.count; i++) {  // members: same rows, k, ids and activations, none of them empty
+        const GemvArgs &a = group.item[i];
+        if (group.count == 1 && (a.n == 0 || a.rows == 0)) return cudaSuccess;
+        if (a.n == 0 || a.k % GROUP != 0 || ((uintptr_t)a.w & 3) != 0 || (a.ids && (a.id_stride & 3))) return cudaErrorInvalidValue;
     }
-    switch (args.rows) {
-        case 1: return mx::launch_m<1>(args, 1, sm_count, pdl, stream);
-        case 2: return mx::launch_m<2>(args, 1, sm_count, pdl, stream);
-        case 3: return mx::launch_m<3>(args, 1, sm_count, pdl, stream);
-        case 4: return mx::launch_m<4>(args, 1, sm_count, pdl, stream);
-        case 5: return mx::launch_m<5>(args, 1, sm_count, pdl, stream);
-        case 6: return mx::launch_m<6>(args, 1, sm_count, pdl, stream);
-        case 7: return mx::launch_m<7>(args, 1, sm_count, pdl, stream);
-        case 8: return mx::launch_m<8>(args, 1, sm_count, pdl, stream);
-        default: return cudaErrorInvalidValue;
-    }
+    if (group.item[0].ids || group.item[0].rows <= 2) return rs::launch_group<mx::Format<true>>(group, mx::g_k_split, sm_count, pdl, stream);
+    return rs::launch_group<mx::Format<false>>(group, mx::g_k_split, sm_count, pdl, stream);
 }
 
 }  // namespace lb

@@ -1,0 +1,315 @@
+// Decode GEMV skeleton for formats whose weights become int8 by byte permutes (MXFP4), 1..8 activation rows.
+// A unit is 32 weights of one matrix row: one lane's work, multiplied with one activation group. A warp step is 32 consecutive units of a row.
+//
+// What bounds these formats is instruction issue and the load / store unit, not HBM (2 to 4 bits a weight), so the kernel is laid out to spend
+// little of either beside the unpacking itself:
+//   * every CTA owns an equal share of the matrix rows (of all members of a grouped launch, concatenated), its warps are G groups of rows x KS
+//     slices of k, and a warp takes RB rows at a time: the activations of a step are read once for RB rows, their packed bytes are requested one
+//     step ahead, and RB sums are reduced by one transposing shuffle tree;
+//   * the quantized activations are copied to shared memory once, in two planes of 16 bytes a group (conflict-free wide loads), zeros behind the
+//     end of k, so that the last step of a row needs no masks beside its loads;
+// The first packed bytes do not depend on the kernel in front and are fetched before the dependency wait. One CTA of sixteen warps an SM: more and smaller ones
+// copy the activations more often (three of eight warps: 4096 x 4096 6.8 against 6.3 us, six experts of 5120 x 2304 19.1 against 18.6).
+//
+// The integer sums of a group are exact and the products those of the reference; only the order in which the groups' f32 terms are added differs.
+//
+// A format F gives: M_MIN and M_MAX (activation rows), STEP_BYTES and lane_offset() (where a lane's unit of a row
+// lies), Raw and load() (its packed bytes, as they lie), W and unpack() (int8 weights and scale), dot() (a unit's integer sum as a float), FACTOR (a power of
+// two that all of a row's scales share), order() (the activation group's bytes in the order of the weights).
+#pragma once
+#include "common.cuh"
+#include "kernels.h"
+
+namespace lb {
+namespace rs {
+
+constexpr int WARPS = 16, THREADS = WARPS * 32, PART_FLOATS = 4096;
+
+// Lane l gets the warp's sum of v[row_of(l)]: RB - 1 exchanges halve the rows, the rest is a plain tree.
+template <int RB> __device__ __forceinline__ float reduce_rows(float (&v)[RB], int lane) {
+    static_assert(RB == 1 || RB == 2 || RB == 4, "rows");
+    int o = 16;
+    float x[RB];
+#pragma unroll
+    for (int j = 0; j < RB; j++) x[j] = v[j];
+#pragma unroll
+    for (int n = RB; n > 1; n /= 2, o /= 2) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < n / 2; j++) {
+            const float keep = up ? x[2 * j + 1] : x[2 * j], send = up ? x[2 * j] : x[2 * j + 1];
+            x[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    float s = x[0];
+#pragma unroll
+    for (int p = 16 / RB; p; p /= 2) s += __shfl_xor_sync(0xffffffffu, s, p);
+    return s;
+}
+template <int RB> __device__ __forceinline__ int row_of(int lane) {
+    return RB == 4 ? 2 * ((lane >> 3) & 1) + ((lane >> 4) & 1) : RB == 2 ? (lane >> 4) & 1 : 0;
+}
+
+// ks_count: warps that share a row; pass_rows: matrix rows of a CTA between two exchanges of their partial sums
+template <class F, int M, int RB, bool ACT_SMEM, int NG>
+__global__ void __launch_bounds__(THREADS, 1)
+row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t ks_count, uint32_t pass_rows) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    // the member of the launch this CTA works for (task_end: CTAs), and its share of the rows
+    int it = 0;
+    if constexpr (NG > 1) {
+#pragma unroll
+        for (int i = 1; i < NG; i++)
+            if (i < grp.count && blockIdx.x >= grp.task_end[i - 1]) it = i;
+    }
+    const GemvArgs &p = grp.item[it];
+    const uint32_t cta = NG > 1 && it ? blockIdx.x - grp.task_end[it - 1] : blockIdx.x, ctas = NG > 1 ? grp.task_end[it] - (it ? grp.task_end[it - 1] : 0u) : gridDim.x;
+    const uint32_t c0 = (uint32_t)((uint64_t)p.n * cta / ctas), rows = (uint32_t)((uint64_t)p.n * (cta + 1) / ctas) - c0;
+
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t k = p.k, units = k / GROUP, steps = (units + 31) / 32, whole = units / 32, sg = steps * 32;  // sg: groups of the padded planes
+    float *part = (float *)smem;
+    uint8_t *acts = smem + (ks_count > 1 ? PART_FLOATS * 4 : 0);
+    float *act_d = (float *)(acts + (size_t)M * sg * GROUP);
+    const uint32_t groups = WARPS / ks_count, ks = warp % ks_count, group = warp / ks_count;
+    const int8_t *qa = p.qa;
+    const float *da = p.da;
+    float *out = p.out + p.out_off;
+    const uint8_t *w = p.w + (uint64_t)c0 * F::row_bytes(k);
+    const uint32_t row_bytes = (uint32_t)F::row_bytes(k);
+
+    // this warp's rows of a pass that starts at p0: [r0, r1), counted from c0
+    auto slice = [&](uint32_t p0, uint32_t &r0, uint32_t &r1) {
+        const uint32_t n = min(pass_rows, rows - p0);
+        r0 = p0 + n * group / groups, r1 = p0 + n * (group + 1) / groups;
+    };
+    // The packed bytes are requested one step ahead: of this warp's next step, rows or pass. A CTA's rows lie within 4 GB of their first byte.
+    typename F::Raw raw[RB];
+    const uint8_t *base = (const uint8_t *)((uintptr_t)w & ~(uintptr_t)3);
+    uint32_t at[RB];     // this lane's unit of the rows being requested, from `base`
+    uint32_t ahead = 0;  // their step
+    auto rows_at = [&](uint32_t row, uint32_t end) {
+        ahead = ks;
+        const uint32_t first = (uint32_t)((uintptr_t)w & 3) + F::lane_offset(lane) + ks * F::STEP_BYTES;
+#pragma unroll
+        for (int j = 0; j < RB; j++) at[j] = (row + j < end ? row + j : row) * row_bytes + first;
+    };
+    auto request = [&]() {
+        if (ahead < whole || 32 * ahead + lane < units) {
+#pragma unroll
+            for (int j = 0; j < RB; j++) raw[j] = F::load(base, at[j], lane);
+        } else {
+#pragma unroll
+            for (int j = 0; j < RB; j++) raw[j] = F::none();
+        }
+#pragma unroll
+        for (int j = 0; j < RB; j++) at[j] += ks_count * F::STEP_BYTES;
+        ahead += ks_count;
+    };
+    uint32_t r0, r1;
+    slice(0, r0, r1);
+    if (!p.ids && r0 < r1) rows_at(r0, r1), request();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (p.ids) {
+        // Expert-indexed launch (Kernel::MatMulId at decode sizes): grid row y is one (token, slot) pair
+        const uint32_t pair = blockIdx.y, token = pair / p.id_r;
+        const int32_t id = p.ids[pair];
+        const bool bad = id < 0 || (uint32_t)id >= p.id_e;
+        if (bad && p.status && threadIdx.x == 0) atomicOr(p.status, 128);
+        w += bad ? 0 : (uint64_t)id * p.id_stride;
+        base = (const uint8_t *)((uintptr_t)w & ~(uintptr_t)3);
+        qa += (uint64_t)token * k;
+        da += (uint64_t)token * units;
+        out += (uint64_t)pair * p.n;
+        if (r0 < r1) rows_at(r0, r1), request();
+    }
+    if constexpr (ACT_SMEM) {
+        for (uint32_t i = threadIdx.x; i < M * sg; i += THREADS) {
+            const uint32_t r = M == 1 ? 0 : i / sg, g = M == 1 ? i : i % sg;
+            uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+            float d = 0.0f;
+            if (g < units) {
+                const uint4 *src = (const uint4 *)(qa + (uint64_t)r * k + (uint64_t)g * GROUP);
+                lo = src[0], hi = src[1];
+                d = da[(uint64_t)r * units + g];
+                F::order(lo, hi);
+            }
+            *(uint4 *)(acts + ((size_t)(2 * r) * sg + g) * 16) = lo;
+            *(uint4 *)(acts + ((size_t)(2 * r + 1) * sg + g) * 16) = hi;
+            act_d[(size_t)r * sg + g] = d;
+        }
+    }
+    __syncthreads();
+    auto store = [&](uint32_t row, uint32_t r, float v) {
+        const uint32_t bt = M == 1 ? 0 : r / p.m, i = M == 1 ? 0 : r % p.m, col = c0 + row;
+        if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)col * p.ex_s2];
+        out[(uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + col] = v;
+    };
+    for (uint32_t p0 = 0; p0 < rows; p0 += pass_rows) {
+        for (uint32_t row = r0; row < r1; row += RB) {
+            const uint32_t left = r1 - row;
+            float acc[M][RB];
+#pragma unroll
+            for (int r = 0; r < M; r++)
+#pragma unroll
+                for (int j = 0; j < RB; j++) acc[r][j] = 0.0f;
+            for (uint32_t step = ks; step < steps; step += ks_count) {
+                typename F::W wv[RB];
+                if (left >= RB) {
+#pragma unroll
+                    for (int j = 0; j < RB; j++) wv[j] = F::unpack(raw[j]);
+                } else {  // (the rows that are missing cost their loads alone)
+#pragma unroll
+                    for (int j = 0; j < RB; j++)
+                        if (j == 0 || j < left) wv[j] = F::unpack(raw[j]);
+                        else wv[j] = wv[0];
+                }
+                // the packed bytes of what comes next are on their way while this is multiplied and other warps unpack theirs
+                if (ahead < steps) request();
+                else if (row + RB < r1) rows_at(row + RB, r1), request();
+                const uint32_t g = 32 * step + lane;
+#pragma unroll
+                for (int r = 0; r < M; r++) {
+                    uint4 lo, hi;
+                    float d;
+                    if constexpr (ACT_SMEM) {
+                        lo = *(const uint4 *)(acts + ((size_t)(2 * r) * sg + g) * 16), hi = *(const uint4 *)(acts + ((size_t)(2 * r + 1) * sg + g) * 16);
+                        d = act_d[(size_t)r * sg + g];
+                    } else {
+                        lo = make_uint4(0, 0, 0, 0), hi = lo, d = 0.0f;
+                        if (g < units) {
+                            const uint4 *src = (const uint4 *)(qa + (uint64_t)r * k + (uint64_t)g * GROUP);
+                            lo = __ldg(src), hi = __ldg(src + 1);
+                            d = __ldg(da + (uint64_t)r * units + g);
+                            F::order(lo, hi);
+                        }
+                    }
+                    const uint32_t a[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                    for (int j = 0; j < RB; j++) acc[r][j] = fmaf(wv[j].d * d, F::dot(wv[j], a), acc[r][j]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < M; r++) {
+                const float v = F::FACTOR * reduce_rows<RB>(acc[r], lane);
+                const uint32_t mine = row + row_of<RB>(lane);
+                if (lane % (32 / RB) == 0 && mine < r1) {
+                    if (ks_count > 1) part[((mine - p0) * ks_count + ks) * M + r] = v;
+                    else store(mine, r, v);
+                }
+            }
+        }
+        const uint32_t n = min(pass_rows, rows - p0);
+        if (n < rows - p0) {
+            slice(p0 + pass_rows, r0, r1);
+            if (r0 < r1) rows_at(r0, r1), request();
+        }
+        if (ks_count > 1) {
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < n * M; i += THREADS) {
+                const uint32_t row = i / M, r = i % M;
+                float v = part[row * ks_count * M + r];
+                for (uint32_t s = 1; s < ks_count; s++) v += part[(row * ks_count + s) * M + r];
+                store(p0 + row, r, v);
+            }
+            __syncthreads();  // the partial sums are read: the next pass may overwrite them
+        }
+    }
+}
+
+// Shared memory of a launch.
+static size_t smem_bytes(uint32_t rows, uint32_t k, uint32_t ks, bool acts) {
+    const size_t sg = ((size_t)k / GROUP + 31) / 32 * 32;
+    return (ks > 1 ? PART_FLOATS * 4 : 0) + (acts ? (size_t)rows * sg * (GROUP + 4) : 0);
+}
+
+template <class F, int M, int RB, bool ACT_SMEM, int NG>
+static cudaError_t launch(const GemvGroup &all, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+    GemvGroupT<NG> g{};
+    uint64_t rows = 0;
+    g.count = all.count;
+    for (int i = 0; i < all.count; i++) g.item[i] = all.item[i], rows += all.item[i].n;
+    const uint32_t k = g.item[0].k, steps = (k / GROUP + 31) / 32;
+    // CTAs: one per SM ; a share of them for
+    // each pair of an expert-indexed launch, and for each member as many as its rows are worth
+    uint32_t ctas = (uint32_t)sm_count;
+    if (pairs > 1) ctas = ctas / pairs ? ctas / pairs : 1;
+    const uint64_t least = (rows * F::row_bytes(k) >> 31) + all.count;  // (offsets inside a CTA's share have 32 bits)
+    if (ctas < least) ctas = (uint32_t)least;
+    uint64_t mine = 0, seen = 0;  // rows of the busiest CTA
+    uint32_t end = 0;
+    for (int i = 0; i < all.count; i++) {
+        const uint64_t n = g.item[i].n;
+        seen += n;
+        uint64_t to = (seen * ctas + rows / 2) / rows;
+        if (to <= end) to = end + 1;
+        if (to - end > n) to = end + n;
+        const uint64_t each = (n + (to - end) - 1) / (to - end);
+        if (each > mine) mine = each;
+        g.task_end[i] = end = (uint32_t)to;
+    }
+    if ((mine + 1) * F::row_bytes(k) >> 32) return cudaErrorInvalidValue;
+    // warps per row: the fewest steps for the slowest warp; a row's reduction costs about a sixth of a step, an exchange as much again
+    uint32_t ks = 1;
+    double cost = 1e30;
+    for (uint32_t c = 1; c <= WARPS && c <= steps; c *= 2) {
+        const uint64_t r = (mine * c + WARPS - 1) / WARPS;
+        const double v = (double)r * ((double)((steps + c - 1) / c) + (c > 1 ? 0.33 : 0.17));
+        if (v < cost) cost = v, ks = c;
+    }
+    if (force_ks && (uint32_t)force_ks <= steps) ks = (uint32_t)force_ks;
+    const uint32_t pass = ks > 1 ? PART_FLOATS / (ks * M) : (uint32_t)mine;  // (one pass where nothing is exchanged)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(end, pairs);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem_bytes(M, k, ks, ACT_SMEM);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    static DynamicSmemOptIn optin;
+    cudaError_t e = optin.raise((const void *)row_stream_kernel<F, M, RB, ACT_SMEM, NG>, cfg.dynamicSmemBytes);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchKernelEx(&cfg, row_stream_kernel<F, M, RB, ACT_SMEM, NG>, g, ks, pass);
+}
+
+// Four rows of a warp share the activation loads and give the schedulers more independent work, two leave fewer of them idle at the end of a CTA's share:
+// MXFP4, one row, 14336 x 4096 13.3 against 14.6 us, 28672 x 4096 20.7 against 23.3, but 4096 x 4096 8.9 against 6.3 and 4096 x 14336 18.1 against 13.9.
+constexpr uint32_t FOUR_ROWS_FROM = 64;  // matrix rows of a CTA
+template <class F, int M, int NG> static cudaError_t launch_rows(const GemvGroup &g, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+    const bool acts = smem_bytes(M, g.item[0].k, 2, true) <= 200 * 1024;
+    if constexpr (M <= 2) {
+        uint64_t rows = 0;
+        for (int i = 0; i < g.count; i++) rows += g.item[i].n;
+        if (acts && rows * pairs >= (uint64_t)FOUR_ROWS_FROM * sm_count) return launch<F, M, 4, true, NG>(g, pairs, force_ks, sm_count, pdl, stream);
+    }
+    if (acts) return launch<F, M, 2, true, NG>(g, pairs, force_ks, sm_count, pdl, stream);
+    return launch<F, M, 2, false, NG>(g, pairs, force_ks, sm_count, pdl, stream);
+}
+
+// F::M_MIN..F::M_MAX activation rows
+template <class F, int NG, int M = F::M_MIN> static cudaError_t launch_m(const GemvGroup &g, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+    if (g.item[0].rows == M) return launch_rows<F, M, NG>(g, 1, force_ks, sm_count, pdl, stream);
+    if constexpr (M < F::M_MAX) return launch_m<F, NG, M + 1>(g, force_ks, sm_count, pdl, stream);
+    else return cudaErrorInvalidValue;
+}
+
+// One launch for the members of `g` (same format, rows, k and activations). Expert-indexed (same ids too): one-row work for each pair.
+template <class F> static cudaError_t launch_group(const GemvGroup &g, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+    if (g.count < 1 || g.count > GEMV_GROUP_MAX) return cudaErrorInvalidValue;
+    const GemvArgs &a = g.item[0];
+    if (F::M_MIN == 1 && a.ids) {
+        if (a.id_r == 0 || a.id_e == 0 || a.rows > 8 || (uint64_t)a.rows * a.id_r > 65535) return cudaErrorInvalidValue;
+        GemvGroup one = g;
+        for (int i = 0; i < g.count; i++) one.item[i].rows = one.item[i].m = 1;
+        return g.count == 1 ? launch_rows<F, F::M_MIN, 1>(one, a.rows * a.id_r, force_ks, sm_count, pdl, stream)
+                            : launch_rows<F, F::M_MIN, GEMV_GROUP_MAX>(one, a.rows * a.id_r, force_ks, sm_count, pdl, stream);
+    }
+    return g.count == 1 ? launch_m<F, 1>(g, force_ks, sm_count, pdl, stream) : launch_m<F, GEMV_GROUP_MAX>(g, force_ks, sm_count, pdl, stream);
+}
+
+}  // namespace rs
+}  // namespace lb
