@@ -31,9 +31,11 @@
 
 namespace lb {
 
-// What one thread fetches for eight consecutive weights of a row, before anything waits for it ...
+// What one thread fetches for eight consecutive weights of a row, before anything waits for it: the values as they are loaded, since a shift or
+// a table lookup here would wait for a load. With those in expand8, us before -> after: MXFP4, 20 rows through 3 layers 8384 -> 5637, i-quants, 86 rows through
+// 11 layers 18450 -> 16050; 12 rows on 4096 x 2048: MXFP4 69 -> 47, Q6_K 69 -> 53, IQ3_XXS 66 -> 52, Int4 as before; one loses: IQ2_S, 64 rows on 3584 x 3584 160 -> 170.
 template <int FMT> struct Raw8 {
-    uint32_t w[FMT == FMT_Q5K ? 8 : FMT == FMT_Q4K ? 6 : FMT == FMT_Q6K ? 6 : FMT == FMT_MXFP4 ? 4 : is_iq(FMT) ? 4 : 3];
+    uint32_t w[FMT == FMT_Q5K ? 8 : FMT == FMT_Q4K ? 6 : FMT == FMT_Q6K ? 10 : FMT == FMT_MXFP4 ? 5 : is_iq(FMT) ? 5 : 3];
 };
 template <int FMT> __device__ __forceinline__ void load_raw8(const GemmF32Args &p, uint32_t row, uint32_t k0, Raw8<FMT> &r) {
     if constexpr (FMT == FMT_Q4K || FMT == FMT_Q5K) {  // header (d, dmin, scales), then the eight bytes that hold the nibbles (and the fifth bits)
@@ -50,22 +52,30 @@ template <int FMT> __device__ __forceinline__ void load_raw8(const GemmF32Args &
         const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * Q6K_BYTES;
         const uint32_t e = k0 % QK, nh = e >> 7, w = (e >> 5) & 3, l0 = e & 31;
         const uint8_t *ql = b + 64 * nh + 32 * (w & 1) + l0, *qh = b + 128 + 32 * nh + l0;
-        r.w[0] = ld32_by16(ql), r.w[1] = ld32_by16(ql + 4), r.w[2] = ld32_by16(qh), r.w[3] = ld32_by16(qh + 4);
-        r.w[4] = ld16(b + 208);
-        r.w[5] = b[192 + 8 * nh + 2 * w + (l0 >> 4)];
+#pragma unroll
+        for (int i = 0; i < 4; i++) r.w[i] = ld16(ql + 2 * i), r.w[4 + i] = ld16(qh + 2 * i);
+        r.w[8] = ld16(b + 208);
+        r.w[9] = b[192 + 8 * nh + 2 * w + (l0 >> 4)];
     } else if constexpr (FMT == FMT_MXFP4) {  // unaligned blocks: the aligned words around the eight bytes
         const uint8_t *b = p.w + (((uint64_t)row * p.k + k0) / GROUP) * MXFP4_BYTES;
         const uintptr_t at = (uintptr_t)(b + 1 + (k0 & 15));
         const uint32_t *a = (const uint32_t *)(at & ~(uintptr_t)3);
-        const uint32_t sh = 8 * (uint32_t)(at & 3), w0 = a[0], w1 = a[1], w2 = sh ? a[2] : 0u;
-        r.w[0] = b[0];
-        r.w[1] = __funnelshift_r(w0, w1, sh);
-        r.w[2] = __funnelshift_r(w1, w2, sh);
-    } else if constexpr (is_iq(FMT)) {  // grid bytes, sign bits, scale
+        r.w[0] = b[0], r.w[1] = a[0], r.w[2] = a[1], r.w[3] = 0;
+        r.w[4] = 8 * (uint32_t)(at & 3);
+        if (r.w[4]) r.w[3] = a[2];
+    } else if constexpr (is_iq(FMT)) {  // index, signs, scales, d of 8-group j (iquant.cuh has the layouts)
         const uint8_t *b = p.w + ((uint64_t)row * (p.k / QK) + k0 / QK) * iq_block_bytes(FMT);
-        const uint32_t e = k0 % QK;
-        iq_group8<FMT>(b, (int)(e >> 3), p.iq_grid, r.w[0], r.w[1], r.w[2]);
-        r.w[3] = __float_as_uint(iq_half_scale<FMT>(b, (int)(e >> 4)));
+        const uint32_t j = (k0 % QK) >> 3, ib = j >> 2, l = j & 3;
+        r.w[3] = ld16(b);
+        if constexpr (FMT == FMT_IQ2XXS) {
+            r.w[0] = b[2 + 8 * ib + l], r.w[1] = ld16(b + 6 + 8 * ib), r.w[2] = ld16(b + 8 + 8 * ib);
+        } else if constexpr (FMT == FMT_IQ2XS) {
+            r.w[0] = ld16(b + 2 + 2 * j), r.w[1] = b[66 + ib];
+        } else if constexpr (FMT == FMT_IQ2S) {
+            r.w[0] = b[2 + j], r.w[1] = b[66 + ib], r.w[2] = b[34 + j], r.w[4] = b[74 + ib];
+        } else {
+            r.w[0] = ld16(b + 2 + 8 * ib + 2 * l), r.w[1] = ld16(b + 66 + 4 * ib), r.w[2] = ld16(b + 68 + 4 * ib);
+        }
     } else {
         const uint64_t g = ((uint64_t)row * p.k + k0) / GROUP;
         const uint2 q = FMT == FMT_INT4 ? *(const uint2 *)(p.w + g * 16 + (k0 & 15)) : *(const uint2 *)(p.w + (uint64_t)row * p.k + k0);
@@ -77,7 +87,7 @@ __device__ __forceinline__ float byte_float(uint32_t w, int i, float bias) {
     return xsub(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u | (uint32_t)i)), 8388608.0f + bias);
 }
 // ... and the weights themselves, bit-exact dequant (each operation rounded on its own, as the reference rounds it).
-template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, uint32_t k0, float (&y)[8]) {
+template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, uint32_t k0, const uint8_t *grid, float (&y)[8]) {
     if constexpr (FMT == FMT_Q4K || FMT == FMT_Q5K) {
         const uint32_t e = k0 % QK, j = e >> 6, h = (e >> 5) & 1;
         const float d = half_bits_to_float(r.w[0] & 0xffffu), dmin = half_bits_to_float(r.w[0] >> 16);
@@ -92,23 +102,37 @@ template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, u
         }
     } else if constexpr (FMT == FMT_Q6K) {
         const uint32_t w = ((k0 % QK) >> 5) & 3;
-        const float t = xmul(half_bits_to_float(r.w[4]), (float)(int8_t)r.w[5]);
+        const float t = xmul(half_bits_to_float(r.w[8]), (float)(int8_t)r.w[9]);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const int lo = (r.w[i >> 2] >> (8 * (i & 3) + 4 * (w >> 1))) & 15, hi = (r.w[2 + (i >> 2)] >> (8 * (i & 3) + 2 * w)) & 3;
+            const int lo = (r.w[i >> 1] >> (8 * (i & 1) + 4 * (w >> 1))) & 15, hi = (r.w[4 + (i >> 1)] >> (8 * (i & 1) + 2 * w)) & 3;
             y[i] = xmul(t, (float)((lo | (hi << 4)) - 32));
         }
     } else if constexpr (FMT == FMT_MXFP4) {
         const float d = e8m0_half(r.w[0]);
         const int sh = (k0 & 16) ? 4 : 0;
+        const uint32_t q[2] = {__funnelshift_r(r.w[1], r.w[2], r.w[4]), __funnelshift_r(r.w[2], r.w[3], r.w[4])};
 #pragma unroll
-        for (int i = 0; i < 8; i++) y[i] = xmul((float)mxfp4_kv((r.w[1 + (i >> 2)] >> (8 * (i & 3) + sh)) & 15u), d);
+        for (int i = 0; i < 8; i++) y[i] = xmul((float)mxfp4_kv((q[i >> 2] >> (8 * (i & 3) + sh)) & 15u), d);
     } else if constexpr (is_iq(FMT)) {  // y = db * grid byte * sign (crates/lapid-quant/src/iq2.rs:38-90, iq3.rs:18-39)
-        const float db = __uint_as_float(r.w[3]);
+        const uint32_t j = (k0 % QK) >> 3, l = j & 3, a = r.w[1] | r.w[2] << 16;
+        uint32_t s, signs, g[2];
+        if constexpr (FMT == FMT_IQ3XXS) {
+            g[0] = *(const uint32_t *)(grid + 4 * (r.w[0] & 255u)), g[1] = *(const uint32_t *)(grid + 4 * (r.w[0] >> 8));
+            signs = iq_ksign((a >> (7 * l)) & 127u), s = a >> 28;
+        } else {
+            const uint32_t idx = FMT == FMT_IQ2XXS ? r.w[0] : FMT == FMT_IQ2XS ? r.w[0] & 511u : r.w[0] | ((r.w[1] << (8 - 2 * l)) & 0x300u);
+            const uint2 v = *(const uint2 *)(grid + 8 * idx);
+            g[0] = v.x, g[1] = v.y;
+            signs = FMT == FMT_IQ2XXS ? iq_ksign((a >> (7 * l)) & 127u) : FMT == FMT_IQ2XS ? iq_ksign(r.w[0] >> 9) : r.w[2];
+            const uint32_t sc = FMT == FMT_IQ2XS ? r.w[1] : r.w[4];
+            s = FMT == FMT_IQ2XXS ? a >> 28 : (j & 2) ? sc >> 4 : sc & 15u;  // (a half of 16 weights is two groups)
+        }
+        const float db = xmul(xmul(half_bits_to_float(r.w[3]), xadd(0.5f, (float)s)), FMT == FMT_IQ3XXS ? 0.5f : 0.25f);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const float v = xmul(db, (float)((r.w[i >> 2] >> (8 * (i & 3))) & 255u));
-            y[i] = (r.w[2] >> i) & 1u ? -v : v;
+            const float v = xmul(db, (float)((g[i >> 2] >> (8 * (i & 3))) & 255u));
+            y[i] = (signs >> i) & 1u ? -v : v;
         }
     } else if constexpr (FMT == FMT_INT4) {
         const float d = half_bits_to_float(r.w[2]);
@@ -215,7 +239,7 @@ qgemm_f32_kernel(GemmF32Args p) {
             const int u = tid + t * THREADS, k = 8 * (u % WP);
             if (BK == 64 && k0 + (uint32_t)k >= p.k) continue;
             float y[8];
-            expand8<FMT>(wv[t], k0 + (uint32_t)k, y);
+            expand8<FMT>(wv[t], k0 + (uint32_t)k, p.iq_grid, y);
 #pragma unroll
             for (int i = 0; i < 8; i++) Bs[buf][k + i][(u / WP) ^ swz_b(k + i)] = y[i];
         }
@@ -469,25 +493,27 @@ template <int FMT> __global__ void __launch_bounds__(CONSUMERS + PRODUCERS, 1) q
                 }
             }
             const int ak = 4 * (tid & 3), arow = tid >> 2, wk = 8 * (tid & 1), wcol = tid >> 1;
-            float av[2][AN][4];
-            Raw8<FMT> wv[2][WN];
+            uint32_t av[2][AN][4];  // four activations as they lie: f32 bits, or halves in pairs (a_vec) or one by one, widened when they are written
+            Raw8<FMT> wv[2][WN];    // (widening them here would wait for the load: IQ2_XS, 200 bf16 rows on 13306 x 5632 1278 us, so 886)
             auto fetch = [&](int set, uint32_t k0) {
 #pragma unroll
                 for (int i = 0; i < AN; i++) {
                     const uint32_t k = k0 + ak;
+                    uint32_t (&a)[4] = av[set][i];
                     if (!aptr[i]) {
-#pragma unroll
-                        for (int l = 0; l < 4; l++) av[set][i][l] = 0.0f;
+                        a[0] = a[1] = a[2] = a[3] = 0;
                     } else if (p.a_vec && p.a_type == ACT_F32) {
-                        const float4 v = *(const float4 *)((const float *)aptr[i] + k);
-                        av[set][i][0] = v.x, av[set][i][1] = v.y, av[set][i][2] = v.z, av[set][i][3] = v.w;
+                        const uint4 v = *(const uint4 *)((const float *)aptr[i] + k);
+                        a[0] = v.x, a[1] = v.y, a[2] = v.z, a[3] = v.w;
                     } else if (p.a_vec) {
                         const uint2 v = *(const uint2 *)((const uint16_t *)aptr[i] + k);
+                        a[0] = v.x, a[1] = v.y;
+                    } else if (p.a_type == ACT_F32) {
 #pragma unroll
-                        for (int l = 0; l < 4; l++) av[set][i][l] = widen_act(((l < 2 ? v.x : v.y) >> (16 * (l & 1))) & 0xffffu, p.a_type);
+                        for (int l = 0; l < 4; l++) a[l] = ((const uint32_t *)aptr[i])[k + l];
                     } else {
 #pragma unroll
-                        for (int l = 0; l < 4; l++) av[set][i][l] = load_act(aptr[i], k + l, p.a_type);
+                        for (int l = 0; l < 4; l++) a[l] = ((const uint16_t *)aptr[i])[k + l];
                     }
                 }
 #pragma unroll
@@ -500,15 +526,25 @@ template <int FMT> __global__ void __launch_bounds__(CONSUMERS + PRODUCERS, 1) q
                 if (!pipe::mbar_wait(empty + stage, phase ^ 1, WAIT_LIMIT)) return false;
                 float *As = ring + stage * STAGE_FLOATS, *Bs = As + A_FLOATS;
 #pragma unroll
-                for (int i = 0; i < AN; i++)
+                for (int i = 0; i < AN; i++) {
+                    const uint32_t (&a)[4] = av[set][i];
+                    float x[4];
+                    if (p.a_type == ACT_F32) {
 #pragma unroll
-                    for (int l = 0; l < 4; l++) As[(ak + l) * BM + ((arow + i * (PRODUCERS / 4)) ^ (2 * ak))] = av[set][i][l];
+                        for (int l = 0; l < 4; l++) x[l] = __uint_as_float(a[l]);
+                    } else {
+#pragma unroll
+                        for (int l = 0; l < 4; l++) x[l] = widen_act(p.a_vec ? (a[l >> 1] >> (16 * (l & 1))) & 0xffffu : a[l], p.a_type);
+                    }
+#pragma unroll
+                    for (int l = 0; l < 4; l++) As[(ak + l) * BM + ((arow + i * (PRODUCERS / 4)) ^ (2 * ak))] = x[l];
+                }
 #pragma unroll
                 for (int i = 0; i < WN; i++) {
                     const uint32_t c = (uint32_t)wcol + i * (PRODUCERS / 2);
                     if (c >= cols) continue;
                     float y[8];
-                    expand8<FMT>(wv[set][i], k0 + wk, y);
+                    expand8<FMT>(wv[set][i], k0 + wk, p.iq_grid, y);
 #pragma unroll
                     for (int l = 0; l < 8; l++) Bs[(wk + l) * BN + (c ^ (2 * wk + 8 * (l >> 2)))] = y[l];
                 }
@@ -576,7 +612,7 @@ template <int FMT> static cudaError_t launch_ws(const GemmF32Args &a, int sm_cou
 }
 
 // The tiles, and what one costs: an SM with `per` tiles takes about fixed + per * each (us for k = 4096 on a launch that gives every SM
-// that many; measured with int8 weights, the other formats within a tenth). The producer / consumer kernel (bm 128) multiplies fastest, small
+// that many; measured with int8 weights, the other formats within a tenth; 86 rows on 9728 x 3584: 32 x 128 tiles 229 us, 128 rows 239). The producer / consumer kernel (bm 128) multiplies fastest, small
 // tiles fill the chip and waste less on a ragged last tile: 128 rows on 1024 x 4096 weights take 94 us on 16 x 32 tiles, 157 on 64 x 64 and 250
 // on 128 rows; 64 rows on 14336 x 4096 245 us on 64 x 64 and 343 on 128 rows (the 16 x 32 tile has become a tenth faster since its constants
 // were measured: 12 rows on 2048 x 4096 74 us).
@@ -584,7 +620,7 @@ struct F32Tile {
     uint32_t bm, bn;
     double fixed, each, least;
 };
-static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 122, 0}, {16, 32, 15, 35, 84}};
+static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 110, 0}, {16, 32, 15, 35, 84}};
 static int pick_tile(uint64_t matrices, double rows, uint64_t n, int sm_count) {  // `matrices` products of `rows` rows each
     int best = 0;
     double cost = 1e30;

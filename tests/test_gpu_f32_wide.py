@@ -50,6 +50,25 @@ def test_tiles_rows_and_strides(be, fmt, m, n, k, pad, out_pad, bias):
     assert np.all(got[0][:, n:].view(np.float32) == -7.0)
 
 
+@pytest.mark.parametrize("a_dtype", [lp.DType.F16, lp.DType.BF16])
+@pytest.mark.parametrize("pad", [0, 1])   # four activations by one load, one by one
+def test_half_activations(be, a_dtype, pad):
+    """Half activations are widened exactly: the bits of the launch over their f32 values."""
+    m, n, k = 130, 7000, 96
+    rs = k + pad
+    x32 = O.normal(70, m * rs)
+    bits = x32.astype(np.float16).view(np.uint16) if a_dtype == lp.DType.F16 else (x32.view(np.uint32) >> 16).astype(np.uint16)
+    wide = bits.view(np.float16).astype(np.float32) if a_dtype == lp.DType.F16 else (bits.astype(np.uint32) << 16).view(np.float32)
+    w = np.random.default_rng(71).standard_normal(n * k, dtype=np.float32) * np.float32(0.02)
+    qb = be.upload(quant.quantize(be, lp.DType.Int8, w, n, k))
+    got = []
+    for a, code in ((bits.view(np.uint8), a_dtype), (wide, lp.DType.F32)):
+        bufs = [be.upload(a), qb, be.alloc(m * n * 4)]
+        be.execute([matmul_launch(lp.DType.Int8, m, n, k, a_dtype=code, inputs=(0, 1), output=2, a=MatView(0, m * rs, rs))], bufs)
+        got.append(bufs[2].download().view(np.uint32))
+    assert np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("fmt", [lp.DType.Int8, lp.DType.MXFP4])
 def test_experts(be, fmt):
     """Expert-indexed launches of that many rows an expert: the bits of each expert's own product."""
