@@ -1,5 +1,6 @@
 """Decode kernels of the formats that become int8 by lookups (MXFP4: csrc/row_stream.cuh, csrc/qgemv_mxfp4.cu; i-quants: csrc/qgemv_iq.cu): shares of the CTAs,
-steps of k and batches of rows at their edges, and launches that go out as one because they read the same activations.
+steps of k and batches of rows at their edges, and launches that go out as one because they read the same activations. The Int8 / Int4 kernel
+(csrc/qgemv_i8_mma.cu): units of a tile and a chunk that the warps take in order.
 
 Bar: integer sums are exact and products the oracle's, f32 terms are added in another order: max_rel <= 2e-5, as for every decode kernel."""
 import numpy as np
@@ -104,3 +105,23 @@ def test_expert_launches_of_the_same_tokens_go_out_together(be, oracle, fmt, t, 
     with pytest.raises(lp.LapidError) as err:
         be.execute([mm(1, 3, 7), mm(2, 3, 8)], bufs)
     assert err.value.code == "index_out_of_range"
+
+
+@pytest.mark.parametrize("fmt", [lp.DType.Int8, lp.DType.Int4])
+@pytest.mark.parametrize("m,n,k", [
+    (1, 33, 32), (3, 40, 288),         # one chunk, two: most warps without a unit
+    (2, 11847, 96), (5, 9500, 544),    # several tiles between two barriers, the last of a share alone
+    (8, 300, 4128), (4, 2400, 3584),   # more chunks than warps; seven chunks of 512 to eight warps
+    (8, 2500, 1024), (3, 100, 8192),   # two chunks; every warp has its place
+    (8, 40, 15008), (7, 40, 15616),    # activations that leave room for fewer warps
+])
+def test_int8_units_of_tiles_and_chunks(be, oracle, fmt, m, n, k):
+    qb, a, bias = oracle.quantize(int(fmt), O.normal(n, n * k, 0.02), n, k), O.normal(7 + n, m * k), O.normal(8 + n, n)
+    want, path = oracle.matmul(int(fmt), a, qb, n, k, m=m, bias=bias)
+    assert path == "int8_act"
+    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4), be.upload(bias)]
+    be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
+    first = bufs[2].download().view(np.float32).copy()
+    assert _max_rel(first, want) <= 2e-5
+    be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
+    assert np.array_equal(first, bufs[2].download().view(np.float32))   # the order of the sums does not depend on timing
