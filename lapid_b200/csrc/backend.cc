@@ -651,6 +651,7 @@ struct MoePlan {
     uint64_t t = 0, r = 0, e = 0;
     lapid_b200_layout wl{};
     size_t route_bytes = 0, scratch = 0;
+    bool together = false;  // decode sizes: may share with its neighbours in the list
 };
 
 MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l) {
@@ -683,6 +684,10 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
         size_t qa = align_up(p.t * l.k, 256), sc = align_up(p.t * (l.k / 32) * 4, 256);
         size_t rec = align_up(p.t * ((l.k + 255) / 256) * lb::REC, 256);
         p.scratch = p.fast ? rec : qa + 2 * sc;
+        // Launches over the same tokens (gate, up) share the quantized tokens, and MXFP4 and the i-quants a kernel, unless their matrices exceed the L2
+        // (126 MB): pairs that name the same expert then meet there only while their CTAs run in step, which a second matrix beside them ends. Two blocks of
+        // MXFP4, apart / together, us: 8 tokens with 6 of 32 experts of 8960 x 2048 2208 / 2383, one token with 6 of 32 of 2304 x 5120 94 / 85.
+        p.together = p.t * p.r * p.wl.total <= (126ull << 20);
     } else {
         p.tc = !dev.gemm_f32 && lb::qgemm_tc_moe_supported(l.b_dtype, p.e, l.n, l.k, nullptr);
         if (p.tc) {
@@ -704,7 +709,7 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
 void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_buffer *const *buffers, size_t n_buffers,
                    ActSlot *slot, PendingGroup *pend) {
     MoePlan p = plan_matmul_id(dev, l);
-    const bool grouped = pend && p.decode && !p.noop && !p.zero_k && (is_iquant(l.b_dtype) || l.b_dtype == LAPID_B200_DTYPE_MXFP4);
+    const bool grouped = pend && p.together && (is_iquant(l.b_dtype) || l.b_dtype == LAPID_B200_DTYPE_MXFP4);
     if (pend && !grouped) pend->flush(dev);
     auto get = [&](uint32_t id) -> lapid_b200_buffer * {
         if (id >= n_buffers || !buffers[id])
@@ -1157,7 +1162,7 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
                 sl.offset = scratch_total;
                 // the routing tables and the gathered rows of an earlier launch with the same tokens and ids (gate and up), as long as nothing
                 // since has written either buffer
-                const bool act = p.decode && !p.noop && !p.zero_k;  // the quantized tokens of an earlier launch that reads them in the same layout
+                const bool act = p.together;  // the quantized tokens of an earlier launch that reads them in the same layout
                 if ((p.tc || act) && xb && ib) {
                     sl.records = act ? ActSlot::MOE_ACT : ActSlot::MOE_COPY;
                     sl.ptr = xb->ptr;

@@ -614,13 +614,12 @@ template <int FMT> static cudaError_t launch_ws(const GemmF32Args &a, int sm_cou
 // The tiles, and what one costs: an SM with `per` tiles takes about fixed + per * each (us for k = 4096 on a launch that gives every SM
 // that many; measured with int8 weights, the other formats within a tenth; 86 rows on 9728 x 3584: 32 x 128 tiles 229 us, 128 rows 239). The producer / consumer kernel (bm 128) multiplies fastest, small
 // tiles fill the chip and waste less on a ragged last tile: 128 rows on 1024 x 4096 weights take 94 us on 16 x 32 tiles, 157 on 64 x 64 and 250
-// on 128 rows; 64 rows on 14336 x 4096 245 us on 64 x 64 and 343 on 128 rows (the 16 x 32 tile has become a tenth faster since its constants
-// were measured: 12 rows on 2048 x 4096 74 us).
+// on 128 rows; 64 rows on 14336 x 4096 245 us on 64 x 64 and 343 on 128 rows.
 struct F32Tile {
     uint32_t bm, bn;
     double fixed, each, least;
 };
-static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 110, 0}, {16, 32, 15, 35, 84}};
+static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 110, 0}, {16, 32, 15, 32, 84}};
 static int pick_tile(uint64_t matrices, double rows, uint64_t n, int sm_count) {  // `matrices` products of `rows` rows each
     int best = 0;
     double cost = 1e30;
