@@ -31,6 +31,7 @@ SOURCES = {
     "qgemv_mxfp4.cu": [],
     "qgemv_mxfp4_mma.cu": [],
     "qgemv_iq.cu": [],
+    "qgemv_iq_rows.cu": [],
     "iquant.cu": ["-DLAPID_B200_IQ_GRIDS_FILE=" + os.path.join(CSRC, "iq_grids.bin")],
     "qgemv_i8_mma.cu": [],
     "qgemm_f32.cu": [],

@@ -141,7 +141,7 @@ void qgemv_mxfp4_set_k_split(int ways);  // warps per row: 0: per launch (defaul
 
 // ---- qgemv_iq.cu: the grid-based i-quants (IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS), 1..8 rows (and the expert-indexed form);
 // reads the activation planes, the codebooks from the per-device table of iquant.cu
-void qgemv_iq_set_rows_per_warp(int rows);  // 0: per launch (default); 1, 2: forced
+void qgemv_iq_set_rows_per_warp(int rows);  // 0: per launch (default); 1, 2: forced (on the kernel of qgemv_iq.cu)
 void qgemv_iq_set_k_split(int ways);        // warps per row at one row per warp: 0: per launch (default); 1, 2, 4: forced
 // iquant.cu: uploads the codebooks to the current device (once; outside stream captures)
 cudaError_t iq_grids_upload();
@@ -214,6 +214,9 @@ using GemvGroup = GemvGroupT<GEMV_GROUP_MAX>;
 using GemvSingle = GemvGroupT<1>;  // what a lone launch passes to the kernel: a sixth of the parameter bytes
 cudaError_t launch_qgemv_mxfp4(const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);         // ... (and the same ids)
 cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);  // members read the same activations
+// qgemv_iq_rows.cu: the i-quants at several rows (`grid`: the format's codebook on the device; force_ks: warps per row, 0: per launch)
+bool qgemv_iq_rows_pays(int fmt, uint32_t rows, uint64_t n, uint32_t k, int sm_count);
+cudaError_t launch_qgemv_iq_rows(int fmt, const GemvGroup &group, const uint8_t *grid, int force_ks, int sm_count, bool pdl, cudaStream_t stream);
 size_t qgemv_kq_group_smem(int fmt, GemvGroup &group);  // dynamic shared memory the group would need
 cudaError_t launch_qgemv_kq_group(int fmt, GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);
 // Q4_K decode on the warp-level int8 tensor-core instruction (2..8 rows pay off); activations as

@@ -318,6 +318,12 @@ cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &args, int sm_count, bool p
     const uint8_t *grids = iq_grids();
     if (!grids) return cudaErrorNotReady;
     const uint8_t *grid = grids + iq_grid_offset(fmt);
+    const GemvArgs &a = args.item[0];
+    uint64_t n = 0;
+    for (int i = 0; i < args.count; i++) n += args.item[i].n;
+    bool words = !a.ids;  // its loads of the packed bytes are 4-byte aligned
+    for (int i = 0; i < args.count; i++) words = words && ((uintptr_t)args.item[i].w & 3) == 0;
+    if (words && !iq::g_rows_per_warp && qgemv_iq_rows_pays(fmt, a.rows, n, a.k, sm_count)) return launch_qgemv_iq_rows(fmt, args, grid, iq::g_k_split, sm_count, pdl, stream);
     switch (fmt) {
         case FMT_IQ2XXS: return iq::launch_fmt<FMT_IQ2XXS>(args, grid, sm_count, pdl, stream);
         case FMT_IQ2XS: return iq::launch_fmt<FMT_IQ2XS>(args, grid, sm_count, pdl, stream);

@@ -23,6 +23,12 @@ namespace mx {
 
 template <bool SPLIT> struct Format {  // SPLIT: positive and negative codes apart
     static constexpr int M_MIN = SPLIT ? 1 : 3, M_MAX = SPLIT ? 2 : 8;
+    static constexpr bool DIRECT = true, AHEAD = false;
+    static constexpr size_t TABLE_BYTES = 0;  // no lookups
+    static __device__ __forceinline__ void fill(uint8_t *, const uint8_t *, int, int) {}
+    struct Tables {
+        __device__ __forceinline__ Tables(const uint8_t *, int) {}
+    };
     static constexpr uint32_t STEP_BYTES = 32 * MXFP4_BYTES;
     static constexpr float FACTOR = 1.0f;
     static __host__ __device__ uint64_t row_bytes(uint32_t k) { return (uint64_t)(k / GROUP) * MXFP4_BYTES; }
@@ -43,7 +49,7 @@ template <bool SPLIT> struct Format {  // SPLIT: positive and negative codes apa
         uint32_t q[8];  // SPLIT: q[i] the nibbles of four elements (low half) of each kind; else the values
         float d;
     };
-    static __device__ __forceinline__ W unpack(const Raw &r) {
+    static __device__ __forceinline__ W unpack(const Raw &r, const Tables &) {
         W o;
         o.d = e8m0_half((r.w[0] >> r.sh) & 255u);
 #pragma unroll
@@ -93,8 +99,8 @@ cudaError_t launch_qgemv_mxfp4(const GemvGroup &group, int sm_count, bool pdl, c
         if (group.count == 1 && (a.n == 0 || a.rows == 0)) return cudaSuccess;
         if (a.n == 0 || a.k % GROUP != 0 || ((uintptr_t)a.w & 3) != 0 || (a.ids && (a.id_stride & 3))) return cudaErrorInvalidValue;
     }
-    if (group.item[0].ids || group.item[0].rows <= 2) return rs::launch_group<mx::Format<true>>(group, mx::g_k_split, sm_count, pdl, stream);
-    return rs::launch_group<mx::Format<false>>(group, mx::g_k_split, sm_count, pdl, stream);
+    if (group.item[0].ids || group.item[0].rows <= 2) return rs::launch_group<mx::Format<true>>(group, nullptr, mx::g_k_split, sm_count, pdl, stream);
+    return rs::launch_group<mx::Format<false>>(group, nullptr, mx::g_k_split, sm_count, pdl, stream);
 }
 
 }  // namespace lb

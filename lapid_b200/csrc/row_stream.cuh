@@ -1,4 +1,4 @@
-// Decode GEMV skeleton for formats whose weights become int8 by byte permutes (MXFP4), 1..8 activation rows.
+// Decode GEMV skeleton for formats whose weights become int8 by byte permutes or lookups (MXFP4; the i-quants at several rows), 1..8 activation rows.
 // A unit is 32 weights of one matrix row: one lane's work, multiplied with one activation group. A warp step is 32 consecutive units of a row.
 //
 // What bounds these formats is instruction issue and the load / store unit, not HBM (2 to 4 bits a weight), so the kernel is laid out to spend
@@ -13,7 +13,8 @@
 //
 // The integer sums of a group are exact and the products those of the reference; only the order in which the groups' f32 terms are added differs.
 //
-// A format F gives: M_MIN and M_MAX (activation rows), STEP_BYTES and lane_offset() (where a lane's unit of a row
+// A format F gives: M_MIN and M_MAX (activation rows), DIRECT (activations that do not fit shared memory are read where they lie), TABLE_BYTES, fill() and
+// Tables (lookup tables in shared memory, and where a lane reads them), AHEAD (packed bytes requested before the present ones are unpacked), STEP_BYTES and lane_offset() (where a lane's unit of a row
 // lies), Raw and load() (its packed bytes, as they lie), W and unpack() (int8 weights and scale), dot() (a unit's integer sum as a float), FACTOR (a power of
 // two that all of a row's scales share), order() (the activation group's bytes in the order of the weights).
 #pragma once
@@ -53,7 +54,7 @@ template <int RB> __device__ __forceinline__ int row_of(int lane) {
 // ks_count: warps that share a row; pass_rows: matrix rows of a CTA between two exchanges of their partial sums
 template <class F, int M, int RB, bool ACT_SMEM, int NG>
 __global__ void __launch_bounds__(THREADS, 1)
-row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t ks_count, uint32_t pass_rows) {
+row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__restrict__ table, uint32_t ks_count, uint32_t pass_rows) {
     extern __shared__ __align__(16) uint8_t smem[];
     // the member of the launch this CTA works for (task_end: CTAs), and its share of the rows
     int it = 0;
@@ -68,8 +69,8 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t ks_count,
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t k = p.k, units = k / GROUP, steps = (units + 31) / 32, whole = units / 32, sg = steps * 32;  // sg: groups of the padded planes
-    float *part = (float *)smem;
-    uint8_t *acts = smem + (ks_count > 1 ? PART_FLOATS * 4 : 0);
+    float *part = (float *)(smem + F::TABLE_BYTES);
+    uint8_t *acts = smem + F::TABLE_BYTES + (ks_count > 1 ? PART_FLOATS * 4 : 0);
     float *act_d = (float *)(acts + (size_t)M * sg * GROUP);
     const uint32_t groups = WARPS / ks_count, ks = warp % ks_count, group = warp / ks_count;
     const int8_t *qa = p.qa;
@@ -109,6 +110,7 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t ks_count,
     uint32_t r0, r1;
     slice(0, r0, r1);
     if (!p.ids && r0 < r1) rows_at(r0, r1), request();
+    F::fill(smem, table, threadIdx.x, THREADS);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (p.ids) {
@@ -141,6 +143,7 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t ks_count,
         }
     }
     __syncthreads();
+    const typename F::Tables tables(smem, lane);
     auto store = [&](uint32_t row, uint32_t r, float v) {
         const uint32_t bt = M == 1 ? 0 : r / p.m, i = M == 1 ? 0 : r % p.m, col = c0 + row;
         if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)col * p.ex_s2];
@@ -156,18 +159,26 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t ks_count,
                 for (int j = 0; j < RB; j++) acc[r][j] = 0.0f;
             for (uint32_t step = ks; step < steps; step += ks_count) {
                 typename F::W wv[RB];
+                // the packed bytes of what comes next are on their way while this is unpacked and multiplied (F::AHEAD; else while it is multiplied, which
+                // saves the copies)
+                auto next = [&]() {
+                    if (ahead < steps) request();
+                    else if (row + RB < r1) rows_at(row + RB, r1), request();
+                };
+                typename F::Raw cur[RB];
+#pragma unroll
+                for (int j = 0; j < RB; j++) cur[j] = raw[j];
+                if (F::AHEAD) next();
                 if (left >= RB) {
 #pragma unroll
-                    for (int j = 0; j < RB; j++) wv[j] = F::unpack(raw[j]);
+                    for (int j = 0; j < RB; j++) wv[j] = F::unpack(cur[j], tables);
                 } else {  // (the rows that are missing cost their loads alone)
 #pragma unroll
                     for (int j = 0; j < RB; j++)
-                        if (j == 0 || j < left) wv[j] = F::unpack(raw[j]);
+                        if (j == 0 || j < left) wv[j] = F::unpack(cur[j], tables);
                         else wv[j] = wv[0];
                 }
-                // the packed bytes of what comes next are on their way while this is multiplied and other warps unpack theirs
-                if (ahead < steps) request();
-                else if (row + RB < r1) rows_at(row + RB, r1), request();
+                if (!F::AHEAD) next();
                 const uint32_t g = 32 * step + lane;
 #pragma unroll
                 for (int r = 0; r < M; r++) {
@@ -219,13 +230,13 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t ks_count,
 }
 
 // Shared memory of a launch.
-static size_t smem_bytes(uint32_t rows, uint32_t k, uint32_t ks, bool acts) {
+template <class F> static size_t smem_bytes(uint32_t rows, uint32_t k, uint32_t ks, bool acts) {
     const size_t sg = ((size_t)k / GROUP + 31) / 32 * 32;
-    return (ks > 1 ? PART_FLOATS * 4 : 0) + (acts ? (size_t)rows * sg * (GROUP + 4) : 0);
+    return F::TABLE_BYTES + (ks > 1 ? PART_FLOATS * 4 : 0) + (acts ? (size_t)rows * sg * (GROUP + 4) : 0);
 }
 
 template <class F, int M, int RB, bool ACT_SMEM, int NG>
-static cudaError_t launch(const GemvGroup &all, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+static cudaError_t launch(const GemvGroup &all, const uint8_t *table, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
     GemvGroupT<NG> g{};
     uint64_t rows = 0;
     g.count = all.count;
@@ -263,7 +274,7 @@ static cudaError_t launch(const GemvGroup &all, uint32_t pairs, int force_ks, in
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(end, pairs);
     cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem_bytes(M, k, ks, ACT_SMEM);
+    cfg.dynamicSmemBytes = smem_bytes<F>(M, k, ks, ACT_SMEM);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -273,42 +284,44 @@ static cudaError_t launch(const GemvGroup &all, uint32_t pairs, int force_ks, in
     static DynamicSmemOptIn optin;
     cudaError_t e = optin.raise((const void *)row_stream_kernel<F, M, RB, ACT_SMEM, NG>, cfg.dynamicSmemBytes);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, row_stream_kernel<F, M, RB, ACT_SMEM, NG>, g, ks, pass);
+    return cudaLaunchKernelEx(&cfg, row_stream_kernel<F, M, RB, ACT_SMEM, NG>, g, table, ks, pass);
 }
 
 // Four rows of a warp share the activation loads and give the schedulers more independent work, two leave fewer of them idle at the end of a CTA's share:
 // MXFP4, one row, 14336 x 4096 13.3 against 14.6 us, 28672 x 4096 20.7 against 23.3, but 4096 x 4096 8.9 against 6.3 and 4096 x 14336 18.1 against 13.9.
 constexpr uint32_t FOUR_ROWS_FROM = 64;  // matrix rows of a CTA
-template <class F, int M, int NG> static cudaError_t launch_rows(const GemvGroup &g, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
-    const bool acts = smem_bytes(M, g.item[0].k, 2, true) <= 200 * 1024;
+constexpr size_t ACT_SMEM_MAX = 200 * 1024;
+template <class F, int M, int NG> static cudaError_t launch_rows(const GemvGroup &g, const uint8_t *table, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+    const bool acts = smem_bytes<F>(M, g.item[0].k, 2, true) <= ACT_SMEM_MAX;
     if constexpr (M <= 2) {
         uint64_t rows = 0;
         for (int i = 0; i < g.count; i++) rows += g.item[i].n;
-        if (acts && rows * pairs >= (uint64_t)FOUR_ROWS_FROM * sm_count) return launch<F, M, 4, true, NG>(g, pairs, force_ks, sm_count, pdl, stream);
+        if (acts && rows * pairs >= (uint64_t)FOUR_ROWS_FROM * sm_count) return launch<F, M, 4, true, NG>(g, table, pairs, force_ks, sm_count, pdl, stream);
     }
-    if (acts) return launch<F, M, 2, true, NG>(g, pairs, force_ks, sm_count, pdl, stream);
-    return launch<F, M, 2, false, NG>(g, pairs, force_ks, sm_count, pdl, stream);
+    if (acts) return launch<F, M, 2, true, NG>(g, table, pairs, force_ks, sm_count, pdl, stream);
+    if constexpr (F::DIRECT) return launch<F, M, 2, false, NG>(g, table, pairs, force_ks, sm_count, pdl, stream);
+    return cudaErrorInvalidValue;
 }
 
 // F::M_MIN..F::M_MAX activation rows
-template <class F, int NG, int M = F::M_MIN> static cudaError_t launch_m(const GemvGroup &g, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
-    if (g.item[0].rows == M) return launch_rows<F, M, NG>(g, 1, force_ks, sm_count, pdl, stream);
-    if constexpr (M < F::M_MAX) return launch_m<F, NG, M + 1>(g, force_ks, sm_count, pdl, stream);
+template <class F, int NG, int M = F::M_MIN> static cudaError_t launch_m(const GemvGroup &g, const uint8_t *table, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+    if (g.item[0].rows == M) return launch_rows<F, M, NG>(g, table, 1, force_ks, sm_count, pdl, stream);
+    if constexpr (M < F::M_MAX) return launch_m<F, NG, M + 1>(g, table, force_ks, sm_count, pdl, stream);
     else return cudaErrorInvalidValue;
 }
 
 // One launch for the members of `g` (same format, rows, k and activations). Expert-indexed (same ids too): one-row work for each pair.
-template <class F> static cudaError_t launch_group(const GemvGroup &g, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
+template <class F> static cudaError_t launch_group(const GemvGroup &g, const uint8_t *table, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
     if (g.count < 1 || g.count > GEMV_GROUP_MAX) return cudaErrorInvalidValue;
     const GemvArgs &a = g.item[0];
     if (F::M_MIN == 1 && a.ids) {
         if (a.id_r == 0 || a.id_e == 0 || a.rows > 8 || (uint64_t)a.rows * a.id_r > 65535) return cudaErrorInvalidValue;
         GemvGroup one = g;
         for (int i = 0; i < g.count; i++) one.item[i].rows = one.item[i].m = 1;
-        return g.count == 1 ? launch_rows<F, F::M_MIN, 1>(one, a.rows * a.id_r, force_ks, sm_count, pdl, stream)
-                            : launch_rows<F, F::M_MIN, GEMV_GROUP_MAX>(one, a.rows * a.id_r, force_ks, sm_count, pdl, stream);
+        return g.count == 1 ? launch_rows<F, F::M_MIN, 1>(one, table, a.rows * a.id_r, force_ks, sm_count, pdl, stream)
+                            : launch_rows<F, F::M_MIN, GEMV_GROUP_MAX>(one, table, a.rows * a.id_r, force_ks, sm_count, pdl, stream);
     }
-    return g.count == 1 ? launch_m<F, 1>(g, force_ks, sm_count, pdl, stream) : launch_m<F, GEMV_GROUP_MAX>(g, force_ks, sm_count, pdl, stream);
+    return g.count == 1 ? launch_m<F, 1>(g, table, force_ks, sm_count, pdl, stream) : launch_m<F, GEMV_GROUP_MAX>(g, table, force_ks, sm_count, pdl, stream);
 }
 
 }  // namespace rs

@@ -53,8 +53,24 @@ def test_mxfp4_shares_steps_and_rows(be, oracle, m, n, k):
     assert _max_rel(got[:, :n], want) <= 2e-5 and np.all(got[:, n:] == -7.0)
 
 
+@pytest.mark.parametrize("fmt", [lp.DType.Iq2Xxs, lp.DType.Iq2Xs, lp.DType.Iq2S, lp.DType.Iq3Xxs])
+@pytest.mark.parametrize("m,n,k", [
+    (8, 3, 256), (8, 150, 1280),                   # one block; a step that is partly there
+    (8, 2501, 2304), (8, 33, 13824),               # blocks on odd halves of a word in every other row; more steps than warps
+    (3, 8192, 1024), (4, 4097, 2304), (5, 2050, 4352),   # eight million weights and more
+    (8, 12, 16640),                                # activations that do not fit: the other kernel
+])
+def test_iquants_at_several_rows(be, oracle, fmt, m, n, k):
+    qb, a, bias = iq_matrix(fmt, n, k, m + n), O.normal(7 + n, m * k), O.normal(8 + n, n)
+    want, path = oracle.matmul(int(fmt), a, qb, n, k, m=m, bias=bias)
+    assert path == "int8_act"
+    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4), be.upload(bias)]
+    be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
+    assert _max_rel(bufs[2].download().view(np.float32), want) <= 2e-5
+
+
 @pytest.mark.parametrize("fmt", [MX, IQ])
-@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("m", [1, 2, 8])
 def test_projections_of_one_operand_go_out_together(be, oracle, fmt, m):
     """q, k, v and a launch that reads what q wrote: three in one kernel, the fourth behind it; ragged member sizes."""
     k, sizes = 1024, (1024, 129, 7)
