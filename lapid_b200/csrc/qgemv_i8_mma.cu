@@ -91,7 +91,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(const __gri
 
     // A CTA's work is its (tile, chunk) units in order, dealt out to the warps one by one. Producer cursor: unit, as tile and chunk, and ring slot. One
     // stage = 512 (RAGGED or Int4: half of that) + 32 sixteen-byte copies.
-    uint32_t pt = EVEN ? t_lo : t_lo + warp / iters, pit = EVEN ? warp : warp % iters, pslot = 0;
+    uint32_t pt = t_lo, pit = warp, pslot = 0;
+    if constexpr (!EVEN)
+        while (pit >= iters) pit -= iters, pt++;
+    uint32_t ct = pt, it = pit;  // the unit being multiplied
     auto issue = [&]() {
         if (pt < t_hi) {
             uint32_t local;
@@ -146,7 +149,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(const __gri
     const uint32_t colq = (uint32_t)gq < M ? gq : 0;      // activation row of this lane's B fragment
     const uint32_t cp = (uint32_t)(2 * t4) < M ? t4 : 0;  // activation row pair of this lane's C fragment
     uint32_t cslot = 0, par = 0;
-    uint32_t ct = EVEN ? t_lo : t_lo + warp / iters, it = EVEN ? warp : warp % iters;  // this warp's unit
     for (uint32_t t0 = t_lo; t0 < t_hi; t0 += round_tiles) {
         const uint32_t t1 = min(t0 + round_tiles, t_hi);
         while (ct < t1) {

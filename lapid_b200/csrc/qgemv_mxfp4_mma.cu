@@ -192,10 +192,16 @@ template <int WARPS> static cudaError_t launch_w(const GemvArgs &a, int sm_count
         const double eff = (double)tasks / ((double)g * ((tasks + g - 1) / g));
         if (eff >= best) best = eff, grid = g;
     }
+    // One CTA per SM: ask for so much shared memory that two do not fit. CTAs are launched while those of the kernel in front leave, so two of them come to an SM
+    // where both places are free while another SM has none, and the launch takes as long as those two (eight rows, whose activations leave room for one, never did). Three
+    // rows, 148 CTAs, us: 14336 x 4096 30.0 -> 21.0, 28672 x 4096 57.9 -> 36.2, 9728 x 2560 19.9 -> 14.8.
+    constexpr size_t MORE_THAN_HALF = 116 * 1024;
+    const size_t pad = grid <= (uint32_t)sm_count && smem < MORE_THAN_HALF ? MORE_THAN_HALF : smem;
+    if (cudaError_t e = opted.raise((const void *)kern, pad); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(WARPS * 32);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = pad;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
