@@ -529,7 +529,7 @@ def gemv_kernel_name(fmt: int, m: int, n: int = 0, k: int = 0) -> str:
     if fmt == 5:
         return "qgemv_i8_mma_kernel<int4>" if m >= 2 or k % 512 else "qgemv_i8_fast_kernel<int4>"
     if fmt == 9:
-        return "qgemv_mxfp4_mma_kernel" if m >= 3 and k % 512 == 0 else "qgemv_mxfp4_kernel"
+        return "qgemv_mxfp4_mma_kernel" if m >= 3 and k % 512 == 0 else "row_stream_kernel<mxfp4>"
     if fmt >= 10:
         return "qgemv_iq_kernel"
     return "qgemv_i8_mma_kernel" if m >= 2 or k % 512 else "qgemv_i8_fast_kernel"
