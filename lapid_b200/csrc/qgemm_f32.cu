@@ -577,7 +577,7 @@ template <int FMT, int BM, int BN, int BK, int TM, int TN> static cudaError_t la
     return cudaGetLastError();
 }
 
-// Tiles per block of 128 rows: of the numbers that fill whole rounds of CTAs, the one whose tiles cost least. A CTA takes about 92 + 35 W us
+// Tiles per block of 128 rows: of the numbers that fill whole rounds of CTAs, the one whose tiles cost least. A CTA takes about 100 + 35 W us
 // for a tile of W units of 16 columns (k = 4096; W below 4 costs what 4 costs), so few rounds of wide tiles win until a round more
 // makes them fit: 512 rows on 4096 columns, one round of 7 units 353 us, two of 4 466; on 14336, four rounds of 6 1191 us, five of 5 1310.
 static ws::Cut ws_cut(uint64_t row_blocks, uint64_t n, int sm_count, double &cost) {
@@ -592,7 +592,7 @@ static ws::Cut ws_cut(uint64_t row_blocks, uint64_t n, int sm_count, double &cos
         if (per > c.units) per = c.units;
         const double widest = ceil((double)c.units / (double)per), mean = (double)c.units / (double)per;
         // (with several rounds the wider tiles spread over the CTAs)
-        const double wide = rounds == 1 ? widest : mean + (widest - mean) / (double)rounds, us = 15 + (double)rounds * (92 + 35 * (wide < 4 ? 4 : wide));
+        const double wide = rounds == 1 ? widest : mean + (widest - mean) / (double)rounds, us = 15 + (double)rounds * (100 + 35 * (wide < 4 ? 4 : wide));
         if (us < cost) cost = us, c.per_block = (uint32_t)per;
     }
     c.tiles = (uint64_t)c.per_block * row_blocks;
@@ -614,12 +614,12 @@ template <int FMT> static cudaError_t launch_ws(const GemmF32Args &a, int sm_cou
 // The tiles, and what one costs: an SM with `per` tiles takes about fixed + per * each (us for k = 4096 on a launch that gives every SM
 // that many; measured with int8 weights, the other formats within a tenth; 86 rows on 9728 x 3584: 32 x 128 tiles 229 us, 128 rows 239). The producer / consumer kernel (bm 128) multiplies fastest, small
 // tiles fill the chip and waste less on a ragged last tile: 128 rows on 1024 x 4096 weights take 94 us on 16 x 32 tiles, 157 on 64 x 64 and 250
-// on 128 rows; 64 rows on 14336 x 4096 245 us on 64 x 64 and 343 on 128 rows.
+// on 128 rows; 64 rows on 14336 x 4096 245 us on 64 x 64 and 343 on 128 rows, 564 rows on 6144 x 1728 270 and 289, 512 on 4096 x 1024 119 and 93.
 struct F32Tile {
     uint32_t bm, bn;
     double fixed, each, least;
 };
-static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 107, 0}, {32, 128, 45, 110, 0}, {16, 32, 15, 32, 84}};
+static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 100, 0}, {32, 128, 45, 110, 0}, {16, 32, 15, 32, 84}};
 static int pick_tile(uint64_t matrices, double rows, uint64_t n, int sm_count) {  // `matrices` products of `rows` rows each
     int best = 0;
     double cost = 1e30;

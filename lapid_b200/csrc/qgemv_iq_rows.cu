@@ -172,12 +172,12 @@ template <int FMT> struct Format {
 // L1 for every one or two matrix rows. IQ2_XXS, IQ2_XS from three rows on and 8 M weights: 4096 x 4096, 3 rows 11.2 / 9.2, 4096 x 14336 27.5 / 17.4, 8 rows
 // 54 / 26, 14336 x 4096, 3 rows 19.0 / 18.9, 8 rows 36.7 / 29.3; 2048 x 2048, 6 rows 7.5 / 8.4, 8 rows 11.3 / 9.3. IQ2_S and IQ3_XXS unpack in more
 // instructions and lose to the other kernel where it has matrix rows enough for two a warp (14336 x 4096, 6 rows 28.7 / 31.6; 8 rows 37.5 / 35.7) and win
-// below that from four rows on (4096 x 14336, 4 rows 31.1 / 26.9).
+// below that from six rows on (4096 x 4096, 6 rows 15.0 / 13.4; 2111 x 7168, 4 rows 32.4 / 34.0) or, on long rows, from four (4096 x 14336, 4 rows 31.1 / 26.9).
 bool qgemv_iq_rows_pays(int fmt, uint32_t rows, uint64_t n, uint32_t k, int sm_count) {
     if (rows < 3 || rs::smem_bytes<iqr::Format<FMT_IQ2XXS>>(rows, k, 2, true) > rs::ACT_SMEM_MAX) return false;
     if (rows >= 8) return true;
     if (n * k < (8u << 20)) return false;
-    return fmt == FMT_IQ2XXS || fmt == FMT_IQ2XS || (rows >= 4 && n < 2 * 32 * (uint64_t)sm_count);
+    return fmt == FMT_IQ2XXS || fmt == FMT_IQ2XS || (rows >= (k >= 8192 ? 4 : 6) && n < 2 * 32 * (uint64_t)sm_count);
 }
 
 cudaError_t launch_qgemv_iq_rows(int fmt, const GemvGroup &group, const uint8_t *grid, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
