@@ -106,12 +106,14 @@ template <int FMT> struct Format {
 
     struct W {
         uint32_t w[8];
-        float d;     // IQ2_XXS, IQ3_XXS: block scale times (0.5 + scale); IQ2_XS, IQ2_S: block scale
+        float d;     // the reference's scale: block scale times (0.5 + scale) / 4 (IQ3_XXS: / 2); IQ2_XS, IQ2_S: block scale / 8
         int m0, m1;  // IQ2_XS, IQ2_S: 2 scale + 1 of each half
     };
-    static constexpr float FACTOR = IQ3 ? 0.5f : FMT == FMT_IQ2XXS ? 0.25f : 0.125f;
-    // 0.5 + the top four bits of x, exactly: as the low bits of 2^23
-    static __device__ __forceinline__ float half_more(uint32_t x) { return xsub(__uint_as_float(x >> 28 | 0x4B000000u), 8388607.5f); }
+    // (0.5 + the top four bits of x) / 4 (IQ3_XXS: / 2), exactly: as the low bits of 2^21 (2^22), whose last place is 1/4 (1/2). The whole scale goes into every term:
+    // a power of two taken out of the sum would let it overflow where the reference's does not.
+    static __device__ __forceinline__ float half_more(uint32_t x) {
+        return IQ3 ? xsub(__uint_as_float(x >> 28 | 0x4A800000u), 4194303.75f) : xsub(__uint_as_float(x >> 28 | 0x4A000000u), 2097151.875f);
+    }
     static __device__ __forceinline__ W unpack(const Raw &r, const Tables &t) {
         W o;
         const float d = half_bits_to_float(r.d);
@@ -139,12 +141,12 @@ template <int FMT> struct Format {
                     idx[l] = q & 511u, sg[l] = (q >> 9) & 127u;
                 }
                 o.m0 = 2 * (int)(r.x & 15u) + 1, o.m1 = 2 * (int)(r.x >> 4) + 1;
-                o.d = d;
+                o.d = xmul(d, 0.125f);
             } else {
 #pragma unroll
                 for (int l = 0; l < 4; l++) idx[l] = ((q0 >> (8 * l)) & 255u) | (((r.x >> (2 * l)) & 3u) << 8), sg[l] = (q1 >> (8 * l)) & 255u;
                 o.m0 = 2 * (int)((r.x >> 8) & 15u) + 1, o.m1 = 2 * (int)(r.x >> 12) + 1;
-                o.d = d;
+                o.d = xmul(d, 0.125f);
             }
 #pragma unroll
             for (int l = 0; l < 4; l++) {

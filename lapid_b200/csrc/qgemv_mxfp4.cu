@@ -30,7 +30,6 @@ template <bool SPLIT> struct Format {  // SPLIT: positive and negative codes apa
         __device__ __forceinline__ Tables(const uint8_t *, int) {}
     };
     static constexpr uint32_t STEP_BYTES = 32 * MXFP4_BYTES;
-    static constexpr float FACTOR = 1.0f;
     static __host__ __device__ uint64_t row_bytes(uint32_t k) { return (uint64_t)(k / GROUP) * MXFP4_BYTES; }
     static __device__ __forceinline__ uint32_t lane_offset(int lane) { return lane * MXFP4_BYTES; }
     struct Raw {

@@ -15,8 +15,7 @@
 //
 // A format F gives: M_MIN and M_MAX (activation rows), DIRECT (activations that do not fit shared memory are read where they lie), TABLE_BYTES, fill() and
 // Tables (lookup tables in shared memory, and where a lane reads them), AHEAD (packed bytes requested before the present ones are unpacked), STEP_BYTES and lane_offset() (where a lane's unit of a row
-// lies), Raw and load() (its packed bytes, as they lie), W and unpack() (int8 weights and scale), dot() (a unit's integer sum as a float), FACTOR (a power of
-// two that all of a row's scales share), order() (the activation group's bytes in the order of the weights).
+// lies), Raw and load() (its packed bytes, as they lie), W and unpack() (int8 weights and scale), dot() (a unit's integer sum as a float), order() (the activation group's bytes in the order of the weights).
 #pragma once
 #include "common.cuh"
 #include "kernels.h"
@@ -203,7 +202,7 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
             }
 #pragma unroll
             for (int r = 0; r < M; r++) {
-                const float v = F::FACTOR * reduce_rows<RB>(acc[r], lane);
+                const float v = reduce_rows<RB>(acc[r], lane);
                 const uint32_t mine = row + row_of<RB>(lane);
                 if (lane % (32 / RB) == 0 && mine < r1) {
                     if (ks_count > 1) part[((mine - p0) * ks_count + ks) * M + r] = v;

@@ -141,3 +141,19 @@ def test_int8_units_of_tiles_and_chunks(be, oracle, fmt, m, n, k):
     assert _max_rel(first, want) <= 2e-5
     be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
     assert np.array_equal(first, bufs[2].download().view(np.float32))   # the order of the sums does not depend on timing
+
+
+@pytest.mark.parametrize("fmt", [lp.DType.Iq2Xxs, lp.DType.Iq2Xs, lp.DType.Iq2S, lp.DType.Iq3Xxs])
+def test_iquant_sums_overflow_no_earlier_than_the_reference(be, oracle, fmt):
+    """Activations of one size and with the signs of the weights: the sum, of terms of one sign, is 2e38, and twice that is not finite."""
+    m, n, k = 8, 1, 512
+    qb = iq_matrix(fmt, n, k, 3)
+    w = oracle.dequantize(int(fmt), qb, n, k).reshape(n, k)
+    size = 2e38 / np.abs(w[0].astype(np.float64)).sum()
+    a = np.tile(np.where(w[0] < 0, -size, size).astype(np.float32), m)
+    want, path = oracle.matmul(int(fmt), a, qb, n, k, m=m)
+    assert path == "int8_act" and np.isfinite(want).all() and want.max() > 1.9e38
+    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4)]
+    be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)], bufs)
+    got = bufs[2].download().view(np.float32)
+    assert np.isfinite(got).all() and _max_rel(got, want) <= 2e-5
