@@ -92,25 +92,26 @@ __device__ __forceinline__ void unpack32(const Raw32 &raw, const uint8_t *grid, 
     sc1 = xmul(xmul(d, xadd(0.5f, (float)s1)), F);
 }
 
+// A launch of one takes its arguments by value: behind the table of a grouped one the compiler allots other registers (IQ3_XXS, six rows on 2048 x 2048 7.3
+// against 9.0 us, IQ2_S, one row on 14336 x 4096 15.9 against 16.8).
+__device__ __forceinline__ GemvArgs &own(GemvArgs &a, uint32_t &, uint32_t &) { return a; }
+// A grouped launch (projections that read the same activations: q and k, gate and up) gives each member a range of CTAs (task_end counts CTAs).
+__device__ __forceinline__ GemvArgs own(const GemvGroup &g, uint32_t &cta, uint32_t &ctas) {
+    int it = 0;
+#pragma unroll
+    for (int i = 1; i < GEMV_GROUP_MAX; i++)
+        if (i < g.count && cta >= g.task_end[i - 1]) it = i;
+    const uint32_t first = it ? g.task_end[it - 1] : 0;
+    cta -= first, ctas = g.task_end[it] - first;
+    return g.item[it];
+}
+
 // KS warps share the rows of a warp group and split their blocks (matrices with few rows and a long K would otherwise
 // leave most warp slots of an SM empty); their partial sums meet in shared memory and are added in warp order.
-// A grouped launch (projections that read the same activations: q and k, gate and up) gives each member a range of CTAs (task_end counts CTAs).
-template <int FMT, int M, int ROWS, int WARPS, int KS, int NG>
-__global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__restrict__ grid_global) {
-    uint32_t cta = blockIdx.x, ctas = gridDim.x;
-    int it = 0;
-    if constexpr (NG > 1) {
-#pragma unroll
-        for (int i = 1; i < NG; i++)
-            if (i < grp.count && blockIdx.x >= grp.task_end[i - 1]) it = i;
-        ctas = grp.task_end[it];
-        if (it) cta -= grp.task_end[it - 1], ctas -= grp.task_end[it - 1];
-    }
-    const GemvArgs &p = grp.item[it];
-    const uint8_t *w_base = p.w;
-    const int8_t *qa = p.qa;
-    const float *da_base = p.da;
-    float *out = p.out + p.out_off;
+template <int FMT, int M, int ROWS, int WARPS, int KS, class ARGS>
+__global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(ARGS args, const uint8_t *__restrict__ grid_global) {
+    uint32_t cta = blockIdx.x, ctas = gridDim.x;  // this CTA's number among those of its matrix
+    auto &&p = own(args, cta, ctas);
     __shared__ __align__(16) uint8_t grid[iq_grid_bytes(FMT)];
     {  // the codebook never changes: it may be read before the launch this one depends on has finished
         const uint4 *src = (const uint4 *)grid_global;
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_const
 #pragma unroll
         for (int j = 0; j < ROWS; j++) {
             const uint32_t row = row0 + j < p.n ? row0 + j : p.n - 1;  // (a row past the end repeats the last one; not stored)
-            raw[j] = load32<FMT>(w_base + ((uint64_t)row * nblk + blk) * BB, ib);
+            raw[j] = load32<FMT>(p.w + ((uint64_t)row * nblk + blk) * BB, ib);
         }
     };
     const uint32_t blk0 = (lane >> 3) + 4 * ks;
@@ -146,10 +147,10 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_const
         const int32_t id = p.ids[pair];
         const bool bad = id < 0 || (uint32_t)id >= p.id_e;
         if (bad && p.status && threadIdx.x == 0) atomicOr(p.status, 128);
-        w_base += bad ? 0 : (uint64_t)id * p.id_stride;
-        qa += (uint64_t)token * k;
-        da_base += (uint64_t)token * kg;
-        out += (uint64_t)pair * p.n;
+        p.w += bad ? 0 : (uint64_t)id * p.id_stride;
+        p.qa += (uint64_t)token * k;
+        p.da += (uint64_t)token * kg;
+        p.out_off += (uint64_t)pair * p.n;
         if (cta * RPC < p.n) fetch(cta * RPC + wg * ROWS, blk0);
     }
     __shared__ float part[KS > 1 ? WARPS * ROWS * M : 1];
@@ -172,9 +173,9 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_const
             const uint32_t g = blk * 8 + ib;  // activation group of this sub-block
 #pragma unroll
             for (int r = 0; r < M; r++) {
-                const uint4 *ap = (const uint4 *)(qa + (uint64_t)r * k + (uint64_t)g * GROUP);
+                const uint4 *ap = (const uint4 *)(p.qa + (uint64_t)r * k + (uint64_t)g * GROUP);
                 const uint4 a0 = __ldg(ap), a1 = __ldg(ap + 1);
-                const float da = __ldg(da_base + (uint64_t)r * kg + g);
+                const float da = __ldg(p.da + (uint64_t)r * kg + g);
 #pragma unroll
                 for (int j = 0; j < ROWS; j++) {
                     int d0 = __dp4a((int)w[j][0], (int)a0.x, 0);
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_const
                 } else if (lane == 0 && row < p.n) {
                     const uint32_t bt = r / p.m, i = r % p.m;
                     if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)row * p.ex_s2];
-                    out[(uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
+                    p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
                 }
             }
         }
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_const
                 if (row < p.n) {
                     const uint32_t bt = r / p.m, i = r % p.m;
                     if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)row * p.ex_s2];
-                    out[(uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
+                    p.out[p.out_off + (uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + row] = v;
                 }
             }
             __syncthreads();  // the partial sums are read: the next pass may overwrite them
@@ -227,17 +228,15 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(const __grid_const
     }
 }
 
-template <int FMT, int M, int ROWS, int WARPS, int KS, int NG> static cudaError_t launch_g(const GemvGroup &all, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
+template <int FMT, int M, int ROWS, int WARPS, int KS = 1> static cudaError_t launch_r(const GemvGroup &all, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
     constexpr uint32_t RPC = WARPS / KS * ROWS;
     uint64_t want = 0;
     for (int i = 0; i < all.count; i++) want += (all.item[i].n + RPC - 1) / RPC;
     uint32_t cap = (uint32_t)sm_count * 8 * (8 / WARPS);
     if (pairs > 1) cap = cap / pairs > 0 ? cap / pairs : 1;
-    GemvGroupT<NG> g{};
-    g.count = all.count;
+    GemvGroup g = all;
     uint32_t end = 0;
     for (int i = 0; i < all.count; i++) {  // each member as many CTAs as it has tiles, or its share of the cap
-        g.item[i] = all.item[i];
         const uint64_t tiles = (all.item[i].n + RPC - 1) / RPC;
         uint64_t c = want <= cap ? tiles : (tiles * cap + want - 1) / want;
         g.task_end[i] = end += (uint32_t)(c ? c : 1);
@@ -251,11 +250,8 @@ template <int FMT, int M, int ROWS, int WARPS, int KS, int NG> static cudaError_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, qgemv_iq_kernel<FMT, M, ROWS, WARPS, KS, NG>, g, grid);
-}
-template <int FMT, int M, int ROWS, int WARPS, int KS = 1> static cudaError_t launch_r(const GemvGroup &g, const uint8_t *grid, uint32_t pairs, int sm_count, bool pdl, cudaStream_t stream) {
-    if (g.count == 1) return launch_g<FMT, M, ROWS, WARPS, KS, 1>(g, grid, pairs, sm_count, pdl, stream);
-    return launch_g<FMT, M, ROWS, WARPS, KS, GEMV_GROUP_MAX>(g, grid, pairs, sm_count, pdl, stream);
+    if (g.count == 1) return cudaLaunchKernelEx(&cfg, qgemv_iq_kernel<FMT, M, ROWS, WARPS, KS, GemvArgs>, g.item[0], grid);
+    return cudaLaunchKernelEx(&cfg, qgemv_iq_kernel<FMT, M, ROWS, WARPS, KS, GemvGroup>, g, grid);
 }
 
 // Two weight rows per warp share the activation loads and give the scheduler two independent decode chains: the
