@@ -9,7 +9,9 @@
 //   * the quantized activations are copied to shared memory once, in two planes of 16 bytes a group (conflict-free wide loads), zeros behind the
 //     end of k, so that the last step of a row needs no masks beside its loads;
 // The first packed bytes do not depend on the kernel in front and are fetched before the dependency wait. One CTA of sixteen warps an SM: more and smaller ones
-// copy the activations more often (three of eight warps: 4096 x 4096 6.8 against 6.3 us, six experts of 5120 x 2304 19.1 against 18.6).
+// copy the activations more often (three of eight warps: 4096 x 4096 6.8 against 6.3 us, six experts of 5120 x 2304 19.1 against 18.6). A CTA takes three
+// quarters of the registers (launch bounds of 640 threads: 96 each): with all of them the small kernel in front or behind (the activations' quantization) finds no
+// room beside it and cannot overlap (IQ2_XXS, four rows on 2048 x 4096 8.9 -> 7.3 us, MXFP4, two rows on 2304 x 1024 4.9 -> 4.3).
 //
 // The integer sums of a group are exact and the products those of the reference; only the order in which the groups' f32 terms are added differs.
 //
@@ -50,10 +52,10 @@ template <int RB> __device__ __forceinline__ int row_of(int lane) {
     return RB == 4 ? 2 * ((lane >> 3) & 1) + ((lane >> 4) & 1) : RB == 2 ? (lane >> 4) & 1 : 0;
 }
 
-// ks_count: warps that share a row; pass_rows: matrix rows of a CTA between two exchanges of their partial sums
+// ks_log: log2 of the warps that share a row; pass_rows: matrix rows of a CTA between two exchanges of their partial sums
 template <class F, int M, int RB, bool ACT_SMEM, int NG>
-__global__ void __launch_bounds__(THREADS, 1)
-row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__restrict__ table, uint32_t ks_count, uint32_t pass_rows) {
+__global__ void __launch_bounds__(THREADS + 128, 1)
+row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__restrict__ table, uint32_t ks_log, uint32_t pass_rows) {
     extern __shared__ __align__(16) uint8_t smem[];
     // the member of the launch this CTA works for (task_end: CTAs), and its share of the rows
     int it = 0;
@@ -64,14 +66,18 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
     }
     const GemvArgs &p = grp.item[it];
     const uint32_t cta = NG > 1 && it ? blockIdx.x - grp.task_end[it - 1] : blockIdx.x, ctas = NG > 1 ? grp.task_end[it] - (it ? grp.task_end[it - 1] : 0u) : gridDim.x;
-    const uint32_t c0 = (uint32_t)((uint64_t)p.n * cta / ctas), rows = (uint32_t)((uint64_t)p.n * (cta + 1) / ctas) - c0;
+    const uint32_t each = p.n / ctas, more = p.n - each * ctas;  // (the first `more` CTAs take one row more; 64-bit divisions would take longer than the smallest launches' sums)
+    const uint32_t c0 = cta * each + min(cta, more), rows = each + (cta < more ? 1 : 0);
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t ks_count = 1u << ks_log;
     const uint32_t k = p.k, units = k / GROUP, steps = (units + 31) / 32, whole = units / 32, sg = steps * 32;  // sg: groups of the padded planes
     float *part = (float *)(smem + F::TABLE_BYTES);
     uint8_t *acts = smem + F::TABLE_BYTES + (ks_count > 1 ? PART_FLOATS * 4 : 0);
     float *act_d = (float *)(acts + (size_t)M * sg * GROUP);
-    const uint32_t groups = WARPS / ks_count, ks = warp % ks_count, group = warp / ks_count;
+    constexpr int WARPS_LOG = 4;
+    static_assert(1 << WARPS_LOG == WARPS, "warps");
+    const uint32_t ks = warp & (ks_count - 1), group = warp >> ks_log;
     const int8_t *qa = p.qa;
     const float *da = p.da;
     float *out = p.out + p.out_off;
@@ -81,7 +87,7 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
     // this warp's rows of a pass that starts at p0: [r0, r1), counted from c0
     auto slice = [&](uint32_t p0, uint32_t &r0, uint32_t &r1) {
         const uint32_t n = min(pass_rows, rows - p0);
-        r0 = p0 + n * group / groups, r1 = p0 + n * (group + 1) / groups;
+        r0 = p0 + (n * group >> (WARPS_LOG - ks_log)), r1 = p0 + (n * (group + 1) >> (WARPS_LOG - ks_log));
     };
     // The packed bytes are requested one step ahead: of this warp's next step, rows or pass. A CTA's rows lie within 4 GB of their first byte.
     typename F::Raw raw[RB];
@@ -110,6 +116,8 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
     slice(0, r0, r1);
     if (!p.ids && r0 < r1) rows_at(r0, r1), request();
     F::fill(smem, table, threadIdx.x, THREADS);
+    // The arguments that the end of the kernel reads are fetched before the wait: a launch's arguments are in no cache yet.
+    asm volatile("" ::"r"(p.m), "l"(p.out_bs), "l"(p.out_rs), "l"(p.extra), "r"(p.epi.n), "l"(p.ex_off), "l"(p.ex_s2));
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (p.ids) {
@@ -127,7 +135,10 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
     }
     if constexpr (ACT_SMEM) {
         for (uint32_t i = threadIdx.x; i < M * sg; i += THREADS) {
-            const uint32_t r = M == 1 ? 0 : i / sg, g = M == 1 ? i : i % sg;
+            uint32_t r = 0, g = i;
+#pragma unroll
+            for (int j = 1; j < M; j++)
+                if (g >= sg) g -= sg, r++;
             uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
             float d = 0.0f;
             if (g < units) {
@@ -144,7 +155,9 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
     __syncthreads();
     const typename F::Tables tables(smem, lane);
     auto store = [&](uint32_t row, uint32_t r, float v) {
-        const uint32_t bt = M == 1 ? 0 : r / p.m, i = M == 1 ? 0 : r % p.m, col = c0 + row;
+        const uint32_t col = c0 + row;
+        uint32_t bt = 0, i = r;
+        if (M > 1 && r >= p.m) bt = r / p.m, i = r % p.m;
         if (p.extra && !p.epi.n) v += p.extra[p.ex_off + (int64_t)bt * p.ex_s0 + (int64_t)i * p.ex_s1 + (int64_t)col * p.ex_s2];
         out[(uint64_t)bt * p.out_bs + (uint64_t)i * p.out_rs + col] = v;
     };
@@ -205,7 +218,7 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
                 const float v = reduce_rows<RB>(acc[r], lane);
                 const uint32_t mine = row + row_of<RB>(lane);
                 if (lane % (32 / RB) == 0 && mine < r1) {
-                    if (ks_count > 1) part[((mine - p0) * ks_count + ks) * M + r] = v;
+                    if (ks_count > 1) part[((((mine - p0) << ks_log) + ks)) * M + r] = v;
                     else store(mine, r, v);
                 }
             }
@@ -219,8 +232,8 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
             __syncthreads();
             for (uint32_t i = threadIdx.x; i < n * M; i += THREADS) {
                 const uint32_t row = i / M, r = i % M;
-                float v = part[row * ks_count * M + r];
-                for (uint32_t s = 1; s < ks_count; s++) v += part[(row * ks_count + s) * M + r];
+                float v = part[(row << ks_log) * M + r];
+                for (uint32_t s = 1; s < ks_count; s++) v += part[((row << ks_log) + s) * M + r];
                 store(p0 + row, r, v);
             }
             __syncthreads();  // the partial sums are read: the next pass may overwrite them
@@ -234,44 +247,58 @@ template <class F> static size_t smem_bytes(uint32_t rows, uint32_t k, uint32_t 
     return F::TABLE_BYTES + (ks > 1 ? PART_FLOATS * 4 : 0) + (acts ? (size_t)rows * sg * (GROUP + 4) : 0);
 }
 
-template <class F, int M, int RB, bool ACT_SMEM, int NG>
-static cudaError_t launch(const GemvGroup &all, const uint8_t *table, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
-    GemvGroupT<NG> g{};
-    uint64_t rows = 0;
-    g.count = all.count;
-    for (int i = 0; i < all.count; i++) g.item[i] = all.item[i], rows += all.item[i].n;
-    const uint32_t k = g.item[0].k, steps = (k / GROUP + 31) / 32;
-    // CTAs: one per SM ; a share of them for
-    // each pair of an expert-indexed launch, and for each member as many as its rows are worth
-    uint32_t ctas = (uint32_t)sm_count;
-    if (pairs > 1) ctas = ctas / pairs ? ctas / pairs : 1;
-    const uint64_t least = (rows * F::row_bytes(k) >> 31) + all.count;  // (offsets inside a CTA's share have 32 bits)
+// How a launch is cut.
+struct Cut {
+    uint32_t grid, end[GEMV_GROUP_MAX];  // CTAs in all (for each pair), and up to each member's end
+    uint64_t mine;                       // matrix rows of the busiest CTA
+};
+// One CTA per SM; a share of them for each pair of an expert-indexed launch, and for each member as many as its rows are worth.
+template <class F> static Cut cut_rows(const GemvGroup &g, uint32_t pairs, int sm_count) {
+    Cut c{};
+    uint64_t rows = 0, seen = 0;
+    for (int i = 0; i < g.count; i++) rows += g.item[i].n;
+    uint32_t ctas = (uint32_t)sm_count / pairs;
+    const uint64_t least = (rows * F::row_bytes(g.item[0].k) >> 31) + g.count;  // (offsets inside a CTA's share have 32 bits)
     if (ctas < least) ctas = (uint32_t)least;
-    uint64_t mine = 0, seen = 0;  // rows of the busiest CTA
-    uint32_t end = 0;
-    for (int i = 0; i < all.count; i++) {
+    for (int i = 0; i < g.count; i++) {
         const uint64_t n = g.item[i].n;
         seen += n;
         uint64_t to = (seen * ctas + rows / 2) / rows;
-        if (to <= end) to = end + 1;
-        if (to - end > n) to = end + n;
-        const uint64_t each = (n + (to - end) - 1) / (to - end);
-        if (each > mine) mine = each;
-        g.task_end[i] = end = (uint32_t)to;
+        if (to <= c.grid) to = c.grid + 1;
+        if (to - c.grid > n) to = c.grid + n;
+        const uint64_t each = (n + (to - c.grid) - 1) / (to - c.grid);
+        if (each > c.mine) c.mine = each;
+        c.end[i] = c.grid = (uint32_t)to;
     }
-    if ((mine + 1) * F::row_bytes(k) >> 32) return cudaErrorInvalidValue;
-    // warps per row: the fewest steps for the slowest warp; a row's reduction costs about a sixth of a step, an exchange as much again
-    uint32_t ks = 1;
-    double cost = 1e30;
+    return c;
+}
+// Matrix rows that a warp takes at a time (RB: 1, 2) and warps per row (KS): the least time of the slowest warp, in steps of one row. A step of two rows
+// takes 1.4 (one activation row) to 1.9 (eight) steps of one, and as much when the second row is missing; a reduction about a sixth of a step, an exchange as
+// much again. One row at a time only where a warp has no second one: else the activations' loads are what two rows share (eight rows, IQ2_XXS, 14336 x 4096 26.8
+// against 35.0 us). MXFP4, one activation row: 2304 x 1024 one row, one warp 3.52, two rows 3.80; 1024 x 14336 one row, two warps 7.9, two rows, four warps 6.7.
+static void pick(uint32_t m, uint64_t mine, uint32_t steps, int force_ks, int &rb, uint32_t &ks) {
+    double best = 1e30;
     for (uint32_t c = 1; c <= WARPS && c <= steps; c *= 2) {
+        if (force_ks && (uint32_t)force_ks <= steps && c != (uint32_t)force_ks) continue;
         const uint64_t r = (mine * c + WARPS - 1) / WARPS;
-        const double v = (double)r * ((double)((steps + c - 1) / c) + (c > 1 ? 0.33 : 0.17));
-        if (v < cost) cost = v, ks = c;
+        const double row = (double)((steps + c - 1) / c) + (c > 1 ? 0.33 : 0.17), pair = row * (double)((r + 1) / 2) * (1.35 + 0.07 * m);
+        if (r == 1 && row < best) best = row, rb = 1, ks = c;
+        if (pair < best) best = pair, rb = 2, ks = c;
     }
-    if (force_ks && (uint32_t)force_ks <= steps) ks = (uint32_t)force_ks;
-    const uint32_t pass = ks > 1 ? PART_FLOATS / (ks * M) : (uint32_t)mine;  // (one pass where nothing is exchanged)
+}
+
+template <class F, int M, int RB, bool ACT_SMEM, int NG>
+static cudaError_t launch(const GemvGroup &all, const uint8_t *table, const Cut &cut, uint32_t ks, uint32_t pairs, bool pdl, cudaStream_t stream) {
+    GemvGroupT<NG> g{};
+    g.count = all.count;
+    for (int i = 0; i < all.count; i++) g.item[i] = all.item[i], g.task_end[i] = cut.end[i];
+    const uint32_t k = g.item[0].k;
+    if ((cut.mine + 1) * F::row_bytes(k) >> 32) return cudaErrorInvalidValue;
+    uint32_t ks_log = 0;
+    while (2u << ks_log <= ks) ks_log++;
+    const uint32_t pass = ks > 1 ? PART_FLOATS / (ks * M) : (uint32_t)cut.mine;  // (one pass where nothing is exchanged)
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(end, pairs);
+    cfg.gridDim = dim3(cut.grid, pairs);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem_bytes<F>(M, k, ks, ACT_SMEM);
     cfg.stream = stream;
@@ -283,22 +310,30 @@ static cudaError_t launch(const GemvGroup &all, const uint8_t *table, uint32_t p
     static DynamicSmemOptIn optin;
     cudaError_t e = optin.raise((const void *)row_stream_kernel<F, M, RB, ACT_SMEM, NG>, cfg.dynamicSmemBytes);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, row_stream_kernel<F, M, RB, ACT_SMEM, NG>, g, table, ks, pass);
+    return cudaLaunchKernelEx(&cfg, row_stream_kernel<F, M, RB, ACT_SMEM, NG>, g, table, ks_log, pass);
 }
 
-// Four rows of a warp share the activation loads and give the schedulers more independent work, two leave fewer of them idle at the end of a CTA's share:
-// MXFP4, one row, 14336 x 4096 13.3 against 14.6 us, 28672 x 4096 20.7 against 23.3, but 4096 x 4096 8.9 against 6.3 and 4096 x 14336 18.1 against 13.9.
+// One activation row over many matrix rows: four of them share the activation loads and give the schedulers more independent work, two leave fewer warps idle at the
+// end of a CTA's share: MXFP4, 14336 x 4096 12.2 against 14.6 us, 28672 x 4096 19.5 against 23.3, but 4096 x 4096 8.9 against 6.3 and 4096 x 14336 18.1 against
+// 13.9. Two activation rows have no registers for four (14336 x 4096 17.2, with spills, against 15.5).
+// One activation row and at most one step for each warp: the activations are read where they lie, once, instead of copied (256 x 1024 3.29 -> 3.24, 2304 x 1024
+// 3.52 -> 3.34; 2304 x 2048, two steps, 3.91 -> 3.93; two activation rows 256 x 1024 3.90 -> 4.04).
 constexpr uint32_t FOUR_ROWS_FROM = 64;  // matrix rows of a CTA
 constexpr size_t ACT_SMEM_MAX = 200 * 1024;
 template <class F, int M, int NG> static cudaError_t launch_rows(const GemvGroup &g, const uint8_t *table, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
-    const bool acts = smem_bytes<F>(M, g.item[0].k, 2, true) <= ACT_SMEM_MAX;
-    if constexpr (M <= 2) {
-        uint64_t rows = 0;
-        for (int i = 0; i < g.count; i++) rows += g.item[i].n;
-        if (acts && rows * pairs >= (uint64_t)FOUR_ROWS_FROM * sm_count) return launch<F, M, 4, true, NG>(g, table, pairs, force_ks, sm_count, pdl, stream);
+    const uint32_t k = g.item[0].k, steps = (k / GROUP + 31) / 32;
+    const bool acts = smem_bytes<F>(M, k, 2, true) <= ACT_SMEM_MAX;
+    const Cut cut = cut_rows<F>(g, pairs, sm_count);
+    int rb = 2;
+    uint32_t ks = 1;
+    pick(M, cut.mine, steps, force_ks, rb, ks);
+    if constexpr (M == 1) {
+        if (F::DIRECT && cut.mine * steps <= WARPS) return launch<F, M, 1, false, NG>(g, table, cut, ks, pairs, pdl, stream);
+        if (acts && cut.mine >= FOUR_ROWS_FROM) return launch<F, M, 4, true, NG>(g, table, cut, ks, pairs, pdl, stream);
     }
-    if (acts) return launch<F, M, 2, true, NG>(g, table, pairs, force_ks, sm_count, pdl, stream);
-    if constexpr (F::DIRECT) return launch<F, M, 2, false, NG>(g, table, pairs, force_ks, sm_count, pdl, stream);
+    if (acts && rb == 1) return launch<F, M, 1, true, NG>(g, table, cut, ks, pairs, pdl, stream);
+    if (acts) return launch<F, M, 2, true, NG>(g, table, cut, ks, pairs, pdl, stream);
+    if constexpr (F::DIRECT) return launch<F, M, 2, false, NG>(g, table, cut, ks, pairs, pdl, stream);
     return cudaErrorInvalidValue;
 }
 

@@ -40,6 +40,8 @@ def _max_rel(got, want):
     (1, 9473, 96), (2, 9500, 1024),    # four rows a warp, the last ones of a share missing
     (1, 700, 16384), (1, 40, 20480),   # sixteen slices of k and more steps than that
     (1, 5, 230400), (2, 5, 92160),     # activations that do not fit shared memory
+    (1, 2300, 1024), (1, 1200, 4096), (2, 2100, 1056), (5, 600, 2880),   # a matrix row for each warp at most; one row, activations not copied
+    (2, 1000, 14336), (3, 2048, 8224), # two rows a warp, several warps to a row
     (3, 77, 2880), (8, 40, 160), (8, 33, 23072),
 ])
 def test_mxfp4_shares_steps_and_rows(be, oracle, m, n, k):
