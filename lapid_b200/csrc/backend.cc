@@ -231,6 +231,7 @@ struct lapid_b200_device {
     // MXFP4 decode launches with at least this many rows use the int8 tensor-core kernel (0 = never): about 18.5 us on
     // 14336 x 4096 whatever the row count, against 15.8 / 17.9 / 25.4 / 42.9 us of the dp4a kernel at 1 / 2 / 4 / 8 rows
     uint32_t mxfp4_mma_rows = 3;
+    int iq_row_kernel = 0;  // option "gemv_iq_row_kernel": i-quants at three to eight rows: 0 per launch, 1 on the row kernel where it fits, 2 never
     bool small_dp4a = true;  // small Q5_K / Q6_K matrices at 3 and 4 rows on the dp4a kernel (see plan_launch)
     bool two_row_dp4a = false;    // two early Q4_K rows on the dp4a kernel (see execute_impl)
     lb::StreamWs stream_ws{};    // workspace of that kernel: partial sums in flight between CTAs (all zero between launches)
@@ -438,7 +439,7 @@ struct PendingGroup {
         const uint64_t before = dev.stream_ws.kernels;
         if (mode == 3) cuda_check(lb::launch_qgemv_kq_stream(fmt, out, dev.stream_ws, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (mode >= 4 && fmt == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(out, dev.sm_count, pdl, dev.stream), "qgemv launch");
-        else if (mode >= 4) cuda_check(lb::launch_qgemv_iq(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (mode >= 4) cuda_check(lb::launch_qgemv_iq(fmt, out, dev.iq_row_kernel, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (fmt == LAPID_B200_DTYPE_INT8 || fmt == LAPID_B200_DTYPE_INT4)
             cuda_check(lb::launch_qgemv_i8_mma(fmt, out, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (mode == 2 && fmt == LAPID_B200_DTYPE_Q6_K) cuda_check(lb::launch_qgemv_q6k_mma(out, dev.sm_count, pdl, dev.stream), "qgemv launch");
@@ -787,7 +788,7 @@ void run_matmul_id(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b20
         const bool pdl = dev.pdl_launch();
         if (l.b_dtype == LAPID_B200_DTYPE_INT4) cuda_check(lb::launch_qgemv_i4(g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(one_of(g), dev.sm_count, pdl, dev.stream), "matmul_id launch");
-        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, one_of(g), dev.sm_count, pdl, dev.stream), "matmul_id launch");
+        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, one_of(g), dev.iq_row_kernel, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         else if (p.fast) cuda_check(lb::launch_qgemv_kq_moe(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         else cuda_check(lb::launch_qgemv_moe(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "matmul_id launch");
         dev.launches++;
@@ -1037,7 +1038,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
             cuda_check(lb::launch_qgemv_i4_fast(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (l.b_dtype == LAPID_B200_DTYPE_INT4) cuda_check(lb::launch_qgemv_i4(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (l.b_dtype == LAPID_B200_DTYPE_MXFP4) cuda_check(lb::launch_qgemv_mxfp4(one_of(g), dev.sm_count, pdl, dev.stream), "qgemv launch");
-        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, one_of(g), dev.sm_count, pdl, dev.stream), "qgemv launch");
+        else if (is_iquant(l.b_dtype)) cuda_check(lb::launch_qgemv_iq(l.b_dtype, one_of(g), dev.iq_row_kernel, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else if (p.fast_i8 && ((uintptr_t)g.w & 15) == 0) cuda_check(lb::launch_qgemv_i8_fast(g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         else cuda_check(lb::launch_qgemv(l.b_dtype, g, dev.sm_count, pdl, dev.stream), "qgemv launch");
         dev.launches += dev.stream_ws.kernels > ws_before ? dev.stream_ws.kernels - ws_before : 1;  // (the stream kernel may take two)
@@ -1729,6 +1730,10 @@ lapid_b200_status lapid_b200_device_set_option(lapid_b200_device *dev, const cha
             lb::qgemv_iq_set_k_split(std::atoi(value));
         } else if (k == "gemv_iq_rows") {  // weight rows per warp of the i-quant decode kernel: 1, 2 (0: per launch)
             lb::qgemv_iq_set_rows_per_warp(std::atoi(value));
+        } else if (k == "gemv_iq_row_kernel") {
+            int r = std::atoi(value);
+            if (r < 0 || r > 2) fail("invalid_argument", "gemv_iq_row_kernel must be 0 (per launch), 1 (where it fits) or 2 (never)");
+            dev->iq_row_kernel = r;
         } else if (k == "gemv_ctas_per_sm") {
             lb::qgemv_q4k_fast_set_cta_cap(std::atoi(value));
         } else if (k == "gemm_wide" || k == "gemm_tall") {

@@ -213,8 +213,10 @@ template <int N> struct GemvGroupT {
 using GemvGroup = GemvGroupT<GEMV_GROUP_MAX>;
 using GemvSingle = GemvGroupT<1>;  // what a lone launch passes to the kernel: a sixth of the parameter bytes
 cudaError_t launch_qgemv_mxfp4(const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);         // ... (and the same ids)
-cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &group, int sm_count, bool pdl, cudaStream_t stream);  // members read the same activations
+// i-quants: members read the same activations; row_kernel: 0 the kernel is chosen per launch, 1 that of qgemv_iq_rows.cu where it fits, 2 the other one
+cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &group, int row_kernel, int sm_count, bool pdl, cudaStream_t stream);
 // qgemv_iq_rows.cu: the i-quants at several rows (`grid`: the format's codebook on the device; force_ks: warps per row, 0: per launch)
+bool qgemv_iq_rows_fits(uint32_t rows, uint32_t k);
 bool qgemv_iq_rows_pays(int fmt, uint32_t rows, uint64_t n, uint32_t k, int sm_count);
 cudaError_t launch_qgemv_iq_rows(int fmt, const GemvGroup &group, const uint8_t *grid, int force_ks, int sm_count, bool pdl, cudaStream_t stream);
 size_t qgemv_kq_group_smem(int fmt, GemvGroup &group);  // dynamic shared memory the group would need

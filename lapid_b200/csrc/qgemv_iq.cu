@@ -304,7 +304,7 @@ template <int FMT> static cudaError_t launch_fmt(const GemvGroup &args, const ui
 void qgemv_iq_set_rows_per_warp(int rows) { iq::g_rows_per_warp = rows == 1 || rows == 2 ? rows : 0; }
 void qgemv_iq_set_k_split(int ways) { iq::g_k_split = ways == 1 || ways == 2 || ways == 4 ? ways : 0; }
 
-cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &args, int sm_count, bool pdl, cudaStream_t stream) {
+cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &args, int row_kernel, int sm_count, bool pdl, cudaStream_t stream) {
     if (args.count < 1 || args.count > GEMV_GROUP_MAX) return cudaErrorInvalidValue;
     for (int i = 0; i < args.count; i++) {  // members: same rows, k, activations and ids, none of them empty
         const GemvArgs &a = args.item[i];
@@ -317,9 +317,10 @@ cudaError_t launch_qgemv_iq(int fmt, const GemvGroup &args, int sm_count, bool p
     const GemvArgs &a = args.item[0];
     uint64_t n = 0;
     for (int i = 0; i < args.count; i++) n += args.item[i].n;
-    bool words = !a.ids;  // its loads of the packed bytes are 4-byte aligned
+    bool words = true;  // that kernel's loads of the packed bytes are 4-byte aligned
     for (int i = 0; i < args.count; i++) words = words && ((uintptr_t)args.item[i].w & 3) == 0;
-    if (words && !iq::g_rows_per_warp && qgemv_iq_rows_pays(fmt, a.rows, n, a.k, sm_count)) return launch_qgemv_iq_rows(fmt, args, grid, iq::g_k_split, sm_count, pdl, stream);
+    if (row_kernel != 2 && !a.ids && words && qgemv_iq_rows_fits(a.rows, a.k) && (row_kernel == 1 || (!iq::g_rows_per_warp && qgemv_iq_rows_pays(fmt, a.rows, n, a.k, sm_count))))
+        return launch_qgemv_iq_rows(fmt, args, grid, iq::g_k_split, sm_count, pdl, stream);
     switch (fmt) {
         case FMT_IQ2XXS: return iq::launch_fmt<FMT_IQ2XXS>(args, grid, sm_count, pdl, stream);
         case FMT_IQ2XS: return iq::launch_fmt<FMT_IQ2XS>(args, grid, sm_count, pdl, stream);

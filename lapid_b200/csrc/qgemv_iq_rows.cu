@@ -170,16 +170,19 @@ template <int FMT> struct Format {
 
 }  // namespace iqr
 
-// Where this kernel beats qgemv_iq.cu's, us there / here. Its tables cost a CTA some 2 us to fill, the activations are copied once instead of being read from
-// L1 for every one or two matrix rows. IQ2_XXS, IQ2_XS from three rows on and 8 M weights: 4096 x 4096, 3 rows 11.2 / 9.2, 4096 x 14336 27.5 / 17.4, 8 rows
-// 54 / 26, 14336 x 4096, 3 rows 19.0 / 18.9, 8 rows 36.7 / 29.3; 2048 x 2048, 6 rows 7.5 / 8.4, 8 rows 11.3 / 9.3. IQ2_S and IQ3_XXS unpack in more
-// instructions and lose to the other kernel where it has matrix rows enough for two a warp (14336 x 4096, 6 rows 28.7 / 31.6; 8 rows 37.5 / 35.7) and win
-// below that from six rows on (4096 x 4096, 6 rows 15.0 / 13.4; 2111 x 7168, 4 rows 32.4 / 34.0) or, on long rows, from four (4096 x 14336, 4 rows 31.1 / 26.9).
+bool qgemv_iq_rows_fits(uint32_t rows, uint32_t k) { return rows >= 3 && rows <= 8 && rs::smem_bytes<iqr::Format<FMT_IQ2XXS>>(rows, k, 2, true) <= rs::ACT_SMEM_MAX; }
+// Where this kernel beats qgemv_iq.cu's, us there / here. The activations are copied once instead of being read from L1 for every one or two matrix rows; its tables
+// cost a CTA some 2 us to fill, which the pre-pass hides. Three rows and K below 2048 do too little to win it back (IQ2_XS 1024 x 1024 3.5 / 4.0, 14336 x 1024
+// 8.3 / 8.9; IQ2_XXS 1024 x 2048 5.2 / 4.2; IQ2_XS, whose other kernel is the quickest, 3000 x 2048 5.5 / 5.8, 4096 x 2048 6.3 / 5.8). IQ2_XXS and IQ2_XS else always: 256 x 1024, 4 rows 4.1 / 4.0, 8 rows 6.4 / 5.2; 2048 x 4096, 3 rows 6.6 / 5.4, 4096 x 14336
+// 29.6 / 14.0, 14336 x 4096, 8 rows 35.7 / 26.8. IQ2_S and IQ3_XXS unpack in more instructions and lose at three to five rows to the other kernel's two matrix
+// rows a warp (28672 x 4096, 3 rows 33.6 / 37.9, 5 rows 45.5 / 46.7; 4096 x 4096, 5 rows 14.4 / 10.5; 28672 x 4096, 6 rows 54.7 / 49.8), IQ3_XXS at five and six also
+// where few columns of many steps leave warps idle here (1536 x 4096, 6 rows 7.2 / 7.6, 512 x 8192, 5 rows 6.1 / 6.7; 2048 x 4096, 5 rows 7.7 / 7.4).
 bool qgemv_iq_rows_pays(int fmt, uint32_t rows, uint64_t n, uint32_t k, int sm_count) {
-    if (rows < 3 || rs::smem_bytes<iqr::Format<FMT_IQ2XXS>>(rows, k, 2, true) > rs::ACT_SMEM_MAX) return false;
-    if (rows >= 8) return true;
-    if (n * k < (8u << 20)) return false;
-    return fmt == FMT_IQ2XXS || fmt == FMT_IQ2XS || (rows >= (k >= 8192 ? 4 : 6) && n < 2 * 32 * (uint64_t)sm_count);
+    if (rows == 3 && (k < 2048 || (fmt == FMT_IQ2XS && n * k < (8u << 20)))) return false;
+    if (fmt == FMT_IQ2XXS || fmt == FMT_IQ2XS) return true;
+    if (rows <= 5 && n >= 2 * 32 * (uint64_t)sm_count) return false;
+    if (fmt == FMT_IQ3XXS) return !((rows == 5 || rows == 6) && k >= 4096 && n < 12 * (uint64_t)sm_count);
+    return rows != 4 || k >= 2048;
 }
 
 cudaError_t launch_qgemv_iq_rows(int fmt, const GemvGroup &group, const uint8_t *grid, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {

@@ -1,4 +1,4 @@
-"""Decode kernels of the formats that become int8 by lookups (MXFP4: csrc/row_stream.cuh, csrc/qgemv_mxfp4.cu; i-quants: csrc/qgemv_iq.cu): shares of the CTAs,
+"""Decode kernels of the formats that become int8 by lookups (MXFP4: csrc/row_stream.cuh, csrc/qgemv_mxfp4.cu; i-quants: csrc/qgemv_iq.cu, csrc/qgemv_iq_rows.cu): shares of the CTAs,
 steps of k and batches of rows at their edges, and launches that go out as one because they read the same activations. The Int8 / Int4 kernel
 (csrc/qgemv_i8_mma.cu): units of a tile and a chunk that the warps take in order.
 
@@ -55,20 +55,38 @@ def test_mxfp4_shares_steps_and_rows(be, oracle, m, n, k):
     assert _max_rel(got[:, :n], want) <= 2e-5 and np.all(got[:, n:] == -7.0)
 
 
+@pytest.mark.parametrize("row_kernel", ["1", "2"])   # on csrc/qgemv_iq_rows.cu, on csrc/qgemv_iq.cu
 @pytest.mark.parametrize("fmt", [lp.DType.Iq2Xxs, lp.DType.Iq2Xs, lp.DType.Iq2S, lp.DType.Iq3Xxs])
 @pytest.mark.parametrize("m,n,k", [
     (8, 3, 256), (8, 150, 1280),                   # one block; a step that is partly there
     (8, 2501, 2304), (8, 33, 13824),               # blocks on odd halves of a word in every other row; more steps than warps
-    (3, 8192, 1024), (4, 4097, 2304), (5, 2050, 4352),   # eight million weights and more
-    (8, 12, 16640),                                # activations that do not fit: the other kernel
+    (3, 2400, 1024), (4, 4097, 2304), (5, 2050, 4352), (6, 1500, 768), (7, 301, 2560),
 ])
-def test_iquants_at_several_rows(be, oracle, fmt, m, n, k):
+def test_iquants_at_several_rows(be, oracle, fmt, m, n, k, row_kernel):
     qb, a, bias = iq_matrix(fmt, n, k, m + n), O.normal(7 + n, m * k), O.normal(8 + n, n)
     want, path = oracle.matmul(int(fmt), a, qb, n, k, m=m, bias=bias)
     assert path == "int8_act"
     bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4), be.upload(bias)]
-    be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
+    be.set_option("gemv_iq_row_kernel", row_kernel)
+    try:
+        be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
+    finally:
+        be.set_option("gemv_iq_row_kernel", "0")
     assert _max_rel(bufs[2].download().view(np.float32), want) <= 2e-5
+
+
+def test_iquant_activations_that_do_not_fit(be, oracle):
+    """Eight rows of 16640: the row kernel has no room for them, forced or not."""
+    m, n, k, fmt = 8, 12, 16640, lp.DType.Iq2Xs
+    qb, a = iq_matrix(fmt, n, k, 1), O.normal(9, m * k)
+    want, _ = oracle.matmul(int(fmt), a, qb, n, k, m=m)
+    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4)]
+    for row_kernel in ("1", "0"):
+        be.set_option("gemv_iq_row_kernel", row_kernel)
+        be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)], bufs)
+        assert _max_rel(bufs[2].download().view(np.float32), want) <= 2e-5
+    with pytest.raises(lp.LapidError):
+        be.set_option("gemv_iq_row_kernel", "3")
 
 
 @pytest.mark.parametrize("fmt", [MX, IQ])
@@ -156,6 +174,8 @@ def test_iquant_sums_overflow_no_earlier_than_the_reference(be, oracle, fmt):
     want, path = oracle.matmul(int(fmt), a, qb, n, k, m=m)
     assert path == "int8_act" and np.isfinite(want).all() and want.max() > 1.9e38
     bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4)]
-    be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)], bufs)
-    got = bufs[2].download().view(np.float32)
-    assert np.isfinite(got).all() and _max_rel(got, want) <= 2e-5
+    for row_kernel in ("1", "2", "0"):
+        be.set_option("gemv_iq_row_kernel", row_kernel)
+        be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)], bufs)
+        got = bufs[2].download().view(np.float32)
+        assert np.isfinite(got).all() and _max_rel(got, want) <= 2e-5
