@@ -32,8 +32,8 @@
 namespace lb {
 
 // What one thread fetches for eight consecutive weights of a row, before anything waits for it: the values as they are loaded, since a shift or
-// a table lookup here would wait for a load. With those in expand8, us before -> after: MXFP4, 20 rows through 3 layers 8384 -> 5637, i-quants, 86 rows through
-// 11 layers 18450 -> 16050; 12 rows on 4096 x 2048: MXFP4 69 -> 47, Q6_K 69 -> 53, IQ3_XXS 66 -> 52, Int4 as before; one loses: IQ2_S, 64 rows on 3584 x 3584 160 -> 170.
+// a table lookup here would wait for a load. With those in expand8 (lookups: Entry8), us before -> after: 12 rows on 4096 x 2048: MXFP4 69 -> 47, Q6_K 69 -> 53,
+// Int4 as before.
 template <int FMT> struct Raw8 {
     uint32_t w[FMT == FMT_Q5K ? 8 : FMT == FMT_Q4K ? 6 : FMT == FMT_Q6K ? 10 : FMT == FMT_MXFP4 ? 5 : is_iq(FMT) ? 5 : 3];
 };
@@ -86,8 +86,24 @@ template <int FMT> __device__ __forceinline__ void load_raw8(const GemmF32Args &
 __device__ __forceinline__ float byte_float(uint32_t w, int i, float bias) {
     return xsub(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u | (uint32_t)i)), 8388608.0f + bias);
 }
+// i-quants: the grid's bytes. Their address is in what was loaded, so they are a load behind a load: asked for when the raw values have arrived (a step after they
+// were asked for), a step before they are expanded. us, looked up with the raw values / when they are expanded / in between: IQ2_S, 64 rows on 4096 x 4096
+// 172 / 201 / 170, 16 rows on 14336 x 4096 177 / 200 / 171, 600 rows on 4096 x 14336 2033 / 2185 / 1987.
+template <int FMT> struct Entry8 {
+    uint32_t g[is_iq(FMT) ? 2 : 1];
+};
+template <int FMT> __device__ __forceinline__ void look8(const Raw8<FMT> &r, uint32_t k0, const uint8_t *grid, Entry8<FMT> &e) {
+    if constexpr (FMT == FMT_IQ3XXS) {
+        e.g[0] = *(const uint32_t *)(grid + 4 * (r.w[0] & 255u)), e.g[1] = *(const uint32_t *)(grid + 4 * (r.w[0] >> 8));
+    } else if constexpr (is_iq(FMT)) {
+        const uint32_t l = ((k0 % QK) >> 3) & 3;
+        const uint32_t idx = FMT == FMT_IQ2XXS ? r.w[0] : FMT == FMT_IQ2XS ? r.w[0] & 511u : r.w[0] | ((r.w[1] << (8 - 2 * l)) & 0x300u);
+        const uint2 v = *(const uint2 *)(grid + 8 * idx);
+        e.g[0] = v.x, e.g[1] = v.y;
+    }
+}
 // ... and the weights themselves, bit-exact dequant (each operation rounded on its own, as the reference rounds it).
-template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, uint32_t k0, const uint8_t *grid, float (&y)[8]) {
+template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, const Entry8<FMT> &en, uint32_t k0, float (&y)[8]) {
     if constexpr (FMT == FMT_Q4K || FMT == FMT_Q5K) {
         const uint32_t e = k0 % QK, j = e >> 6, h = (e >> 5) & 1;
         const float d = half_bits_to_float(r.w[0] & 0xffffu), dmin = half_bits_to_float(r.w[0] >> 16);
@@ -116,14 +132,10 @@ template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, u
         for (int i = 0; i < 8; i++) y[i] = xmul((float)mxfp4_kv((q[i >> 2] >> (8 * (i & 3) + sh)) & 15u), d);
     } else if constexpr (is_iq(FMT)) {  // y = db * grid byte * sign (crates/lapid-quant/src/iq2.rs:38-90, iq3.rs:18-39)
         const uint32_t j = (k0 % QK) >> 3, l = j & 3, a = r.w[1] | r.w[2] << 16;
-        uint32_t s, signs, g[2];
+        uint32_t s, signs;
         if constexpr (FMT == FMT_IQ3XXS) {
-            g[0] = *(const uint32_t *)(grid + 4 * (r.w[0] & 255u)), g[1] = *(const uint32_t *)(grid + 4 * (r.w[0] >> 8));
             signs = iq_ksign((a >> (7 * l)) & 127u), s = a >> 28;
         } else {
-            const uint32_t idx = FMT == FMT_IQ2XXS ? r.w[0] : FMT == FMT_IQ2XS ? r.w[0] & 511u : r.w[0] | ((r.w[1] << (8 - 2 * l)) & 0x300u);
-            const uint2 v = *(const uint2 *)(grid + 8 * idx);
-            g[0] = v.x, g[1] = v.y;
             signs = FMT == FMT_IQ2XXS ? iq_ksign((a >> (7 * l)) & 127u) : FMT == FMT_IQ2XS ? iq_ksign(r.w[0] >> 9) : r.w[2];
             const uint32_t sc = FMT == FMT_IQ2XS ? r.w[1] : r.w[4];
             s = FMT == FMT_IQ2XXS ? a >> 28 : (j & 2) ? sc >> 4 : sc & 15u;  // (a half of 16 weights is two groups)
@@ -131,7 +143,7 @@ template <int FMT> __device__ __forceinline__ void expand8(const Raw8<FMT> &r, u
         const float db = xmul(xmul(half_bits_to_float(r.w[3]), xadd(0.5f, (float)s)), FMT == FMT_IQ3XXS ? 0.5f : 0.25f);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const float v = xmul(db, (float)((g[i >> 2] >> (8 * (i & 3))) & 255u));
+            const float v = xmul(db, (float)((en.g[i >> 2] >> (8 * (i & 3))) & 255u));
             y[i] = (signs >> i) & 1u ? -v : v;
         }
     } else if constexpr (FMT == FMT_INT4) {
@@ -199,7 +211,8 @@ qgemm_f32_kernel(GemmF32Args p) {
     }
 
     float av[AN][4];
-    Raw8<FMT> wv[WN];
+    Raw8<FMT> wv[WN], wv2[WN];  // (the second one: i-quants)
+    Entry8<FMT> entry[WN];
     auto fetch = [&](uint32_t k0) {
 #pragma unroll
         for (int t = 0; t < AN; t++) {
@@ -219,15 +232,24 @@ qgemm_f32_kernel(GemmF32Args p) {
                 for (int i = 0; i < 4; i++) av[t][i] = load_act(aptr[t], k + i, p.a_type);
             }
         }
+    };
+    auto fetch_weights = [&](uint32_t k0, Raw8<FMT> (&to)[WN]) {
 #pragma unroll
         for (int t = 0; t < WN; t++) {
             const int u = tid + t * THREADS;
             const uint32_t wrow = col0 + (uint32_t)(u / WP);
             const uint32_t k = k0 + 8 * (uint32_t)(u % WP);
-            if (BK == 16 || k < p.k) load_raw8<FMT>(p, wrow < p.n ? wrow : p.n - 1, k, wv[t]);  // columns past the matrix are not stored
+            if (BK == 16 || k < p.k) load_raw8<FMT>(p, wrow < p.n ? wrow : p.n - 1, k, to[t]);  // columns past the matrix are not stored
         }
     };
-    auto stage = [&](int buf, uint32_t k0) {
+    auto look_up = [&](uint32_t k0, const Raw8<FMT> (&wv)[WN]) {
+#pragma unroll
+        for (int t = 0; t < WN; t++) {
+            const uint32_t k = k0 + 8 * (uint32_t)((tid + t * THREADS) % WP);
+            if (BK == 16 || k < p.k) look8<FMT>(wv[t], k, p.iq_grid, entry[t]);
+        }
+    };
+    auto stage = [&](int buf, uint32_t k0, const Raw8<FMT> (&wv)[WN]) {
 #pragma unroll
         for (int t = 0; t < AN; t++) {
             const int u = tid + t * THREADS, k = a_k(u);
@@ -239,7 +261,7 @@ qgemm_f32_kernel(GemmF32Args p) {
             const int u = tid + t * THREADS, k = 8 * (u % WP);
             if (BK == 64 && k0 + (uint32_t)k >= p.k) continue;
             float y[8];
-            expand8<FMT>(wv[t], k0 + (uint32_t)k, p.iq_grid, y);
+            expand8<FMT>(wv[t], entry[t], k0 + (uint32_t)k, y);
 #pragma unroll
             for (int i = 0; i < 8; i++) Bs[buf][k + i][(u / WP) ^ swz_b(k + i)] = y[i];
         }
@@ -248,12 +270,22 @@ qgemm_f32_kernel(GemmF32Args p) {
     // k is a multiple of 32: the last step of BK = 64 may be half full and then ends there (a term 0 * 0 more would turn an accumulator
     // of -0, which a negative product that underflows leaves, into +0).
     fetch(0);
-    stage(0, 0);
+    fetch_weights(0, wv);
+    look_up(0, wv);
+    stage(0, 0, wv);
+    if (is_iq(FMT) && BK < p.k) fetch_weights(BK, wv);
     __syncthreads();
-    int buf = 0;
-    for (uint32_t k0 = 0; k0 < p.k; k0 += BK, buf ^= 1) {
+    auto step = [&](uint32_t k0, int buf, Raw8<FMT> (&next)[WN], Raw8<FMT> (&after)[WN]) {  // `after`: i-quants, whose raw values come two steps ahead
         const bool more = k0 + BK < p.k;
-        if (more) fetch(k0 + BK);
+        if (more) {
+            fetch(k0 + BK);
+            if constexpr (is_iq(FMT)) {
+                look_up(k0 + BK, next);
+                if (k0 + 2 * BK < p.k) fetch_weights(k0 + 2 * BK, after);
+            } else {
+                fetch_weights(k0 + BK, next);
+            }
+        }
         // operands of step kk + 1 are on their way while kk is multiplied
         uint64_t a2[2][TM / 2];
         float b[2][TN];
@@ -286,9 +318,18 @@ qgemm_f32_kernel(GemmF32Args p) {
         if (BK == 64 && p.k - k0 < BK) multiply(std::integral_constant<int, BK / 2>());
         else multiply(std::integral_constant<int, BK>());
         if (more) {
-            stage(buf ^ 1, k0 + BK);  // the other buffer's readers passed the barrier of the step before
+            stage(buf ^ 1, k0 + BK, next);  // the other buffer's readers passed the barrier of the step before
             __syncthreads();
         }
+    };
+    if constexpr (is_iq(FMT)) {
+        for (uint32_t k0 = 0; k0 < p.k; k0 += 2 * BK) {
+            step(k0, 0, wv, wv2);
+            if (k0 + BK < p.k) step(k0 + BK, 1, wv2, wv);
+        }
+    } else {
+        int buf = 0;
+        for (uint32_t k0 = 0; k0 < p.k; k0 += BK, buf ^= 1) step(k0, buf, wv, wv);
     }
 #pragma unroll
     for (int i = 0; i < TM; i++) {
@@ -522,6 +563,12 @@ template <int FMT> __global__ void __launch_bounds__(CONSUMERS + PRODUCERS, 1) q
                     if (c < cols) load_raw8<FMT>(p, row < p.n ? row : p.n - 1, k0 + wk, wv[set][i]);  // columns past the matrix are not stored
                 }
             };
+            Entry8<FMT> entry[2][WN];
+            auto look_up = [&](int set, uint32_t k0) {  // (i-quants; the raw values were asked for a step ago)
+#pragma unroll
+                for (int i = 0; i < WN; i++)
+                    if ((uint32_t)wcol + i * (PRODUCERS / 2) < cols) look8<FMT>(wv[set][i], k0 + wk, p.iq_grid, entry[set][i]);
+            };
             auto put = [&](int set, uint32_t k0) {
                 if (!pipe::mbar_wait(empty + stage, phase ^ 1, WAIT_LIMIT)) return false;
                 float *As = ring + stage * STAGE_FLOATS, *Bs = As + A_FLOATS;
@@ -544,7 +591,7 @@ template <int FMT> __global__ void __launch_bounds__(CONSUMERS + PRODUCERS, 1) q
                     const uint32_t c = (uint32_t)wcol + i * (PRODUCERS / 2);
                     if (c >= cols) continue;
                     float y[8];
-                    expand8<FMT>(wv[set][i], k0 + wk, p.iq_grid, y);
+                    expand8<FMT>(wv[set][i], entry[set][i], k0 + wk, y);
 #pragma unroll
                     for (int l = 0; l < 8; l++) Bs[(wk + l) * BN + (c ^ (2 * wk + 8 * (l >> 2)))] = y[l];
                 }
@@ -556,9 +603,11 @@ template <int FMT> __global__ void __launch_bounds__(CONSUMERS + PRODUCERS, 1) q
             // the operands of the step after the one being written are on their way (k is a multiple of 32: steps come in pairs)
             fetch(0, 0);
             for (uint32_t k0 = 0; k0 < p.k && ok; k0 += 2 * BK) {
+                look_up(0, k0);
                 fetch(1, k0 + BK);
                 ok = put(0, k0);
                 if (!ok) break;
+                look_up(1, k0 + BK);
                 if (k0 + 2 * BK < p.k) fetch(0, k0 + 2 * BK);
                 ok = put(1, k0 + BK);
             }
