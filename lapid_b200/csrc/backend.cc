@@ -236,6 +236,7 @@ struct lapid_b200_device {
     bool two_row_dp4a = false;    // two early Q4_K rows on the dp4a kernel (see execute_impl)
     lb::StreamWs stream_ws{};    // workspace of that kernel: partial sums in flight between CTAs (all zero between launches)
     lb::GemmTcTuning gemm_tc;  // options "gemm_splitk", "gemm_pair"
+    uint32_t f32_tile = 0;  // option "gemm_f32_tile": activation rows per tile of the exact-f32 GEMM (0: chosen per launch)
     bool gemm_f32 = false;  // true: rows > gemv_max_rows always take the exact-f32 GEMM instead of the tensor cores
     // option "profile": every launch of an execute list is bracketed by events (launches run one by one then: nothing is
     // grouped) and its GPU time added to its kernel kind; lapid_b200_take_profile drains the totals
@@ -697,7 +698,7 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
             // prefer the tile that holds an expert's expected rows (plus the spread of a random routing) in one piece
             p.mt = avg <= 48 ? 64 : avg <= 100 ? 128 : 256;
         } else {
-            p.mt = lb::qgemm_f32_moe_tile(p.t * p.r, p.e, l.n, dev.sm_count);
+            p.mt = dev.f32_tile ? dev.f32_tile : lb::qgemm_f32_moe_tile(p.t * p.r, p.e, l.n, dev.sm_count);
         }
         if ((uint64_t)lb::moe_max_tiles(p.t * p.r, p.e, p.mt) * p.mt >= lim) fail("too_large", "b200 matmul_id: tile space exceeds 32-bit indexing");
         p.route_bytes = lb::moe_route_bytes(p.t * p.r, p.e, p.mt);
@@ -1108,6 +1109,7 @@ void run_launch(lapid_b200_device &dev, const lapid_b200_launch &l, lapid_b200_b
     f.n = g.n;
     f.k = g.k;
     f.status = dev.status_dev;
+    f.tile = dev.f32_tile;
     cuda_check(lb::launch_qgemm_f32(l.b_dtype, f, dev.sm_count, dev.stream), "qgemm_f32 launch");
     dev.launches++;
     expr_pass();
@@ -1742,6 +1744,10 @@ lapid_b200_status lapid_b200_device_set_option(lapid_b200_device *dev, const cha
             dev->gemm_tc.splitk = std::atoi(value);
         } else if (k == "gemm_pair") {
             dev->gemm_tc.pair = std::atoi(value);
+        } else if (k == "gemm_f32_tile") {
+            int r = std::atoi(value);
+            if (r != 0 && r != 16 && r != 32 && r != 64 && r != 128) fail("invalid_argument", "gemm_f32_tile must be 0 (per launch), 16, 32, 64 or 128");
+            dev->f32_tile = (uint32_t)r;
         } else if (k == "gemm") {
             if (v == "f32") dev->gemm_f32 = true;
             else if (v == "tc") dev->gemm_f32 = false;

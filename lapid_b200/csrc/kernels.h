@@ -295,6 +295,7 @@ struct GemmF32Args {
     int64_t ex_s0, ex_s1, ex_s2;
     uint32_t rows, m, n, k;
     int *status;                 // host-visible status word of bounded waits (may be nullptr)
+    uint32_t tile;               // rows of an activation tile: 0: chosen per launch; 16, 32, 64, 128: forced (128: the producer / consumer kernel)
     bool a_vec;                  // four activations of a row can be fetched with one aligned load (set by the launcher)
     // Expert-indexed launches (moe.cu): rows = the tile space (tiles of mt rows: qgemm_f32_moe_tile), w = the expert stack
     uint32_t mt;

@@ -698,7 +698,7 @@ uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts, uint64_t n, int sm
 }
 
 template <int FMT> static cudaError_t launch_fmt(const GemmF32Args &a, int sm_count, cudaStream_t stream) {
-    switch (a.tile_expert ? a.mt : F32_TILES[pick_tile(1, a.rows, a.n, sm_count)].bm) {
+    switch (a.tile_expert ? a.mt : a.tile ? a.tile : F32_TILES[pick_tile(1, a.rows, a.n, sm_count)].bm) {
         case 128: return launch_ws<FMT>(a, sm_count, stream);
         case 64: return launch_tile<FMT, 64, 64, 16, 8, 4>(a, stream);
         case 32: return launch_tile<FMT, 32, 128, 16, 8, 4>(a, stream);
