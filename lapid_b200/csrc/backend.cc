@@ -698,7 +698,7 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
             // prefer the tile that holds an expert's expected rows (plus the spread of a random routing) in one piece
             p.mt = avg <= 48 ? 64 : avg <= 100 ? 128 : 256;
         } else {
-            p.mt = dev.f32_tile ? dev.f32_tile : lb::qgemm_f32_moe_tile(p.t * p.r, p.e, l.n, dev.sm_count);
+            p.mt = dev.f32_tile ? dev.f32_tile : lb::qgemm_f32_moe_tile(l.b_dtype, p.t * p.r, p.e, l.n, (uint32_t)l.k, dev.sm_count);
         }
         if ((uint64_t)lb::moe_max_tiles(p.t * p.r, p.e, p.mt) * p.mt >= lim) fail("too_large", "b200 matmul_id: tile space exceeds 32-bit indexing");
         p.route_bytes = lb::moe_route_bytes(p.t * p.r, p.e, p.mt);

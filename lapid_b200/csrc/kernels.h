@@ -306,7 +306,7 @@ struct GemmF32Args {
     const uint8_t *iq_grid;      // i-quants: the format's codebook on this device (set by the launcher)
 };
 cudaError_t launch_qgemm_f32(int fmt, const GemmF32Args &args, int sm_count, cudaStream_t stream);
-uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts, uint64_t n, int sm_count);  // activation rows per tile of an expert-indexed launch
+uint32_t qgemm_f32_moe_tile(int fmt, uint64_t pairs, uint64_t experts, uint64_t n, uint32_t k, int sm_count);  // activation rows per tile of an expert-indexed launch
 
 // ---- qgemm_tc.cu: tcgen05 tensor-core GEMM (Q4_K weights, bf16 operands, f32 accumulation)
 struct GemmTcArgs {

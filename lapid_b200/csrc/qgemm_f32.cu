@@ -626,10 +626,20 @@ template <int FMT, int BM, int BN, int BK, int TM, int TN> static cudaError_t la
     return cudaGetLastError();
 }
 
-// Tiles per block of 128 rows: of the numbers that fill whole rounds of CTAs, the one whose tiles cost least. A CTA takes about 100 + 35 W us
-// for a tile of W units of 16 columns (k = 4096; W below 4 costs what 4 costs), so few rounds of wide tiles win until a round more
+// Time of a tile of W units of 16 columns on a CTA of the producer / consumer kernel, us, K = 4096 (int8 weights; the other formats within a tenth; W below 4 costs
+// what 4 costs). On long rows narrow tiles take more than their share (4 units, K = 14336: 960 us, 14336 / 4096 of 241 is 844), and of i-quants, whose
+// expansion the producers then wait for (IQ3_XXS 279).
+static double ws_tile_us(double w, uint32_t k, bool iq) {
+    static const double SHORT[] = {241, 268, 305, 330, 390}, LONG[] = {262, 278, 305, 330, 390}, IQ[] = {280, 290, 305, 330, 390};  // W = 4..8
+    const double *us = iq ? IQ : k < 8192 ? SHORT : LONG;
+    if (w <= 4) return us[0];
+    if (w >= ws::W_MAX) return us[4];
+    const int i = (int)w - 4;
+    return us[i] + (us[i + 1] - us[i]) * (w - 4 - i);
+}
+// Tiles per block of 128 rows: of the numbers that fill whole rounds of CTAs, the one whose tiles cost least. Few rounds of wide tiles win until a round more
 // makes them fit: 512 rows on 4096 columns, one round of 7 units 353 us, two of 4 466; on 14336, four rounds of 6 1191 us, five of 5 1310.
-static ws::Cut ws_cut(uint64_t row_blocks, uint64_t n, int sm_count, double &cost) {
+static ws::Cut ws_cut(bool iq, uint64_t row_blocks, uint64_t n, uint32_t k, int sm_count, double &cost) {
     ws::Cut c{};
     c.row_blocks = (uint32_t)row_blocks;
     c.units = (uint32_t)((n + ws::TX - 1) / ws::TX);
@@ -641,7 +651,7 @@ static ws::Cut ws_cut(uint64_t row_blocks, uint64_t n, int sm_count, double &cos
         if (per > c.units) per = c.units;
         const double widest = ceil((double)c.units / (double)per), mean = (double)c.units / (double)per;
         // (with several rounds the wider tiles spread over the CTAs)
-        const double wide = rounds == 1 ? widest : mean + (widest - mean) / (double)rounds, us = 15 + (double)rounds * (100 + 35 * (wide < 4 ? 4 : wide));
+        const double us = (double)rounds * ws_tile_us(rounds == 1 ? widest : mean + (widest - mean) / (double)rounds, k, iq);
         if (us < cost) cost = us, c.per_block = (uint32_t)per;
     }
     c.tiles = (uint64_t)c.per_block * row_blocks;
@@ -652,7 +662,7 @@ template <int FMT> static cudaError_t launch_ws(const GemmF32Args &a, int sm_cou
     const uint64_t row_blocks = ((uint64_t)a.rows + ws::BM - 1) / ws::BM;
     if (row_blocks > GRID_Y_MAX) return cudaErrorInvalidValue;
     double cost;
-    const ws::Cut c = ws_cut(row_blocks, a.n, sm_count, cost);
+    const ws::Cut c = ws_cut(is_iq(FMT), row_blocks, a.n, a.k, sm_count, cost);
     static DynamicSmemOptIn optin;
     cudaError_t e = optin.raise((const void *)ws::qgemm_f32_ws_kernel<FMT>, ws::SMEM);
     if (e != cudaSuccess) return e;
@@ -660,45 +670,52 @@ template <int FMT> static cudaError_t launch_ws(const GemmF32Args &a, int sm_cou
     return cudaGetLastError();
 }
 
-// The tiles, and what one costs: an SM with `per` tiles takes about fixed + per * each (us for k = 4096 on a launch that gives every SM
-// that many; measured with int8 weights, the other formats within a tenth; 86 rows on 9728 x 3584: 32 x 128 tiles 229 us, 128 rows 239). The producer / consumer kernel (bm 128) multiplies fastest, small
-// tiles fill the chip and waste less on a ragged last tile: 128 rows on 1024 x 4096 weights take 94 us on 16 x 32 tiles, 157 on 64 x 64 and 250
-// on 128 rows; 64 rows on 14336 x 4096 245 us on 64 x 64 and 343 on 128 rows, 564 rows on 6144 x 1728 270 and 289, 512 on 4096 x 1024 119 and 93.
+// The tiles, and what a launch on them takes: us at K = 4096 for an SM with 1, 2, .. of them (several run side by side), then `more` for each further one, all but
+// `start` in proportion to K (int8 weights, every SM with that many; measured at 9 to 600 rows on 512 to 14336 columns and K 1024, 4096 and 14336: of 250 shapes the choice
+// is the fastest or within 1 % of it). The last round costs a tenth of a tile less where it reaches part of the SMs. Activation rows that lie a multiple of 4096 bytes apart
+// share cache sets, which the kernel above feels (`uneven`: where they don't). Examples, us, 16 x 32 / 32 x 128 / 64 x 64 / 128 rows: 64 rows on 4096 x 4096 150 / 171 / 155 /
+// 231, 300 on 3000 x 4096 - / 283 / 245 / 237, on 3000 x 1024 - / 69 / 60 / 65, 86 on 9728 x 4096 - / 282 / 350 / 269, 86 on 9728 x 2560 - / 164 / 210 / 169.
 struct F32Tile {
     uint32_t bm, bn;
-    double fixed, each, least;
+    double start, more, uneven;
+    int counted;
+    double us[7];
 };
-static const F32Tile F32_TILES[] = {{128, 0, 0, 0, 0}, {64, 64, 45, 100, 0}, {32, 128, 45, 110, 0}, {16, 32, 15, 32, 84}};
-static int pick_tile(uint64_t matrices, double rows, uint64_t n, int sm_count) {  // `matrices` products of `rows` rows each
+static const F32Tile F32_TILES[] = {{128, 0, 10, 0, 1, 0, {}},  // ws_tile_us
+                                    {64, 64, 2, 105, 0.95, 4, {152, 246, 358, 462}},
+                                    {32, 128, 0, 125, 0.93, 4, {168, 280, 410, 532}},
+                                    {16, 32, 4, 29.5, 1, 7, {75, 92, 121, 146, 185, 206, 238}}};
+static int pick_tile(bool iq, uint64_t matrices, double rows, uint64_t n, uint32_t k, int sm_count) {  // `matrices` products of `rows` rows each
     int best = 0;
     double cost = 1e30;
     for (int i = 0; i < 4; i++) {
         const F32Tile &t = F32_TILES[i];
         const uint64_t blocks = matrices * (uint64_t)ceil(rows / t.bm);
-        double c;
+        double us;
         if (t.bn) {
             const uint64_t tiles = blocks * ((n + t.bn - 1) / t.bn), per = (tiles + sm_count - 1) / sm_count;
-            c = t.fixed + t.each * (double)per;
+            us = per <= (uint64_t)t.counted ? t.us[per - 1] : t.us[t.counted - 1] + t.more * (double)(per - t.counted);
+            if (t.bm > 16 && per > 1) us -= 0.1 * t.more * ((double)per - (double)tiles / sm_count);
         } else {
-            ws_cut(blocks, n, sm_count, c);
+            ws_cut(iq, blocks, n, k, sm_count, us);
         }
-        if (c < t.least) c = t.least;
-        if (c < cost) cost = c, best = i;
+        us = t.start + (us - t.start) * (double)k / 4096.0 * (k % 1024 ? t.uneven : 1.0);
+        if (us < cost) cost = us, best = i;
     }
     return best;
 }
 // Expert-indexed launches: the tile for the experts' expected rows plus the spread of a random routing.
-uint32_t qgemm_f32_moe_tile(uint64_t pairs, uint64_t experts, uint64_t n, int sm_count) {
+uint32_t qgemm_f32_moe_tile(int fmt, uint64_t pairs, uint64_t experts, uint64_t n, uint32_t k, int sm_count) {
     const uint64_t used = experts < pairs ? experts : pairs;
     if (!used) return 64;
     const double avg = (double)pairs / (double)used;
-    int i = pick_tile(used, avg + (avg > 1 ? sqrt(avg) : 0), n, sm_count);
+    int i = pick_tile(is_iq(fmt), used, avg + (avg > 1 ? sqrt(avg) : 0), n, k, sm_count);
     while (i > 0 && moe_max_tiles(pairs, experts, F32_TILES[i].bm) > GRID_Y_MAX) i--;  // tens of thousands of experts: taller tiles, fewer of them
     return F32_TILES[i].bm;
 }
 
 template <int FMT> static cudaError_t launch_fmt(const GemmF32Args &a, int sm_count, cudaStream_t stream) {
-    switch (a.tile_expert ? a.mt : a.tile ? a.tile : F32_TILES[pick_tile(1, a.rows, a.n, sm_count)].bm) {
+    switch (a.tile_expert ? a.mt : a.tile ? a.tile : F32_TILES[pick_tile(is_iq(FMT), 1, a.rows, a.n, a.k, sm_count)].bm) {
         case 128: return launch_ws<FMT>(a, sm_count, stream);
         case 64: return launch_tile<FMT, 64, 64, 16, 8, 4>(a, stream);
         case 32: return launch_tile<FMT, 32, 128, 16, 8, 4>(a, stream);
