@@ -26,6 +26,7 @@
 // eight with 512. Tile by tile with eight warps -> units in order with sixteen, us: three rows int8 15360 x 2880 16.8 -> 14.7, seven rows 4096 x 11008 19.6 -> 14.7,
 // three rows Int4 15360 x 2880 22.4 -> 13.4; a token of three rows through 12 layers of 2880 / 7680 606 -> 574. Where K is a multiple of 512, eight warps stay
 // (sixteen with 256: 14336 x 4096 15.6 -> 17.2), units in order: eight rows int8 8192 x 1024 6.2 -> 5.5, four rows Int4 4096 x 4096 7.5 -> 6.4; EVEN as before.
+// Less than a tile for every CTA pays 0.1 us for the order (eight rows int8 512 x 1024 3.66 -> 3.77, 3.89 while the warps' places were found by subtracting in a loop).
 //
 // Several projections over the same activations (q, k, v; gate, up) run as one launch over the concatenated tiles. Early
 // mode (GemvArgs::early): activations are read and tiles computed before the dependency wait, which comes before the first store.
@@ -62,7 +63,7 @@ __host__ __device__ constexpr uint32_t act_block_bytes(uint32_t rows) { return 2
 
 // EVEN: a tile's chunks divide evenly over the warps, which then keep their places from tile to tile.
 template <bool I4, bool RAGGED, bool EVEN, int WARPS, int NG>
-__global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t round_in, uint32_t buffers_in) {
+__global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(const __grid_constant__ GemvGroupT<NG> grp, uint32_t round_in, uint32_t buffers_in, uint32_t inverse) {
     const uint32_t round_tiles = EVEN ? 1 : round_in, buffers = EVEN ? 2 : buffers_in;
     constexpr int THREADS = WARPS * 32;
     constexpr int KC = chunk_of(RAGGED), CPR = KC / (I4 ? 32 : 16), RPI = 32 / CPR;  // 16-byte copies a row, rows an instruction
@@ -91,9 +92,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(const __gri
 
     // A CTA's work is its (tile, chunk) units in order, dealt out to the warps one by one. Producer cursor: unit, as tile and chunk, and ring slot. One
     // stage = 512 (RAGGED or Int4: half of that) + 32 sixteen-byte copies.
-    uint32_t pt = t_lo, pit = warp, pslot = 0;
-    if constexpr (!EVEN)
-        while (pit >= iters) pit -= iters, pt++;
+    // `inverse` divides numbers up to WARPS by `iters`: subtracting in a loop takes longer than the smallest launches' products.
+    const uint32_t first_tile = EVEN ? 0 : warp * inverse >> 16, step_tiles = EVEN ? 0 : WARPS * inverse >> 16, step = WARPS - step_tiles * iters;
+    uint32_t pt = t_lo + first_tile, pit = warp - first_tile * iters, pslot = 0;
     uint32_t ct = pt, it = pit;  // the unit being multiplied
     auto issue = [&]() {
         if (pt < t_hi) {
@@ -119,11 +120,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(const __gri
                 copy16(dst + Q_BYTES + 16 * lane, p.w + p.scales_offset + ((size_t)row * kg + (size_t)pit * (KC / GROUP)) * 2 + 16 * (lane & 1), 16);
             }
             pslot ^= 1;
-            pit += WARPS;
             if constexpr (EVEN) {
+                pit += WARPS;
                 if (pit >= iters) pit = warp, pt++;
             } else {
-                while (pit >= iters) pit -= iters, pt++;
+                pit += step, pt += step_tiles;
+                if (pit >= iters) pit -= iters, pt++;
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group keeps the count in step
@@ -215,11 +217,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1) qgemv_i8_mma_kernel(const __gri
                 __syncwarp();  // every lane is done reading the slot before it is refilled
                 issue();
                 cslot ^= 1;
-                it += WARPS;
                 if constexpr (EVEN) {
+                    it += WARPS;
                     if (it >= iters) it = warp, ct++;
                 } else {
-                    while (it >= iters) it -= iters, ct++;
+                    it += step, ct += step_tiles;
+                    if (it >= iters) it -= iters, ct++;
                 }
             } while (ct == tile);
             float *mine = red + ((size_t)(par * round_tiles + tile - t0) * WARPS + warp) * 128;
@@ -318,7 +321,8 @@ template <bool I4, bool RAGGED, bool EVEN, int WARPS, int NG> static cudaError_t
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, g, round, buffers);
+    const uint32_t iters = (k + chunk_of(RAGGED) - 1) / chunk_of(RAGGED);
+    return cudaLaunchKernelEx(&cfg, kern, g, round, buffers, 65536 / iters + 1);
 }
 template <bool I4, bool RAGGED, int WARPS, int NG> static cudaError_t launch_w(const GemvGroup &g, int sm_count, bool pdl, cudaStream_t stream) {
     const uint32_t iters = g.item[0].k / chunk_of(RAGGED);
