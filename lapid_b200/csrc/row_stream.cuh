@@ -9,9 +9,9 @@
 //   * the quantized activations are copied to shared memory once, in two planes of 16 bytes a group (conflict-free wide loads), zeros behind the
 //     end of k, so that the last step of a row needs no masks beside its loads;
 // The first packed bytes do not depend on the kernel in front and are fetched before the dependency wait. One CTA of sixteen warps an SM: more and smaller ones
-// copy the activations more often (three of eight warps: 4096 x 4096 6.8 against 6.3 us, six experts of 5120 x 2304 19.1 against 18.6). A CTA takes three
-// quarters of the registers (launch bounds of 640 threads: 96 each): with all of them the small kernel in front or behind (the activations' quantization) finds no
-// room beside it and cannot overlap (IQ2_XXS, four rows on 2048 x 4096 8.9 -> 7.3 us, MXFP4, two rows on 2304 x 1024 4.9 -> 4.3).
+// copy the activations more often (three of eight warps: 4096 x 4096 6.8 against 6.3 us, six experts of 5120 x 2304 19.1 against 18.6). ROOM: a CTA takes
+// three quarters of the registers (launch bounds of 640 threads: 96 each): with all of them the small kernel in front or behind (the activations' quantization)
+// finds no room beside it and cannot overlap (IQ2_XXS, four rows on 2048 x 4096 8.9 -> 7.3 us, MXFP4, two rows on 2304 x 1024 4.9 -> 4.3).
 //
 // The integer sums of a group are exact and the products those of the reference; only the order in which the groups' f32 terms are added differs.
 //
@@ -53,8 +53,8 @@ template <int RB> __device__ __forceinline__ int row_of(int lane) {
 }
 
 // ks_log: log2 of the warps that share a row; pass_rows: matrix rows of a CTA between two exchanges of their partial sums
-template <class F, int M, int RB, bool ACT_SMEM, int NG>
-__global__ void __launch_bounds__(THREADS + 128, 1)
+template <class F, int M, int RB, bool ACT_SMEM, int NG, bool ROOM>
+__global__ void __launch_bounds__(ROOM ? THREADS + 128 : THREADS, 1)
 row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__restrict__ table, uint32_t ks_log, uint32_t pass_rows) {
     extern __shared__ __align__(16) uint8_t smem[];
     // the member of the launch this CTA works for (task_end: CTAs), and its share of the rows
@@ -287,7 +287,7 @@ static void pick(uint32_t m, uint64_t mine, uint32_t steps, int force_ks, int &r
     }
 }
 
-template <class F, int M, int RB, bool ACT_SMEM, int NG>
+template <class F, int M, int RB, bool ACT_SMEM, int NG, bool ROOM = true>
 static cudaError_t launch(const GemvGroup &all, const uint8_t *table, const Cut &cut, uint32_t ks, uint32_t pairs, bool pdl, cudaStream_t stream) {
     GemvGroupT<NG> g{};
     g.count = all.count;
@@ -308,17 +308,19 @@ static cudaError_t launch(const GemvGroup &all, const uint8_t *table, const Cut 
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     static DynamicSmemOptIn optin;
-    cudaError_t e = optin.raise((const void *)row_stream_kernel<F, M, RB, ACT_SMEM, NG>, cfg.dynamicSmemBytes);
+    cudaError_t e = optin.raise((const void *)row_stream_kernel<F, M, RB, ACT_SMEM, NG, ROOM>, cfg.dynamicSmemBytes);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, row_stream_kernel<F, M, RB, ACT_SMEM, NG>, g, table, ks_log, pass);
+    return cudaLaunchKernelEx(&cfg, row_stream_kernel<F, M, RB, ACT_SMEM, NG, ROOM>, g, table, ks_log, pass);
 }
 
 // One activation row over many matrix rows: four of them share the activation loads and give the schedulers more independent work, two leave fewer warps idle at the
 // end of a CTA's share: MXFP4, 14336 x 4096 12.2 against 14.6 us, 28672 x 4096 19.5 against 23.3, but 4096 x 4096 8.9 against 6.3 and 4096 x 14336 18.1 against
-// 13.9. Two activation rows have no registers for four (14336 x 4096 17.2, with spills, against 15.5).
+// 13.9. Two activation rows have no registers for four (14336 x 4096 17.2, with spills, against 15.5). Long launches of that kind and those of several expert pairs
+// gain more from all registers than from what runs beside them: us, 96 / 128 registers, 11008 x 4096 10.6 / 11.5, 28672 x 4096 19.5 / 20.0, 128256 x 2048 36.1 /
+// 35.3, six experts of 2304 x 5120, gate and up, 21.7 / 20.9, 64 of 1408 x 2048 54.7 / 51.5.
 // One activation row and at most one step for each warp: the activations are read where they lie, once, instead of copied (256 x 1024 3.29 -> 3.24, 2304 x 1024
 // 3.52 -> 3.34; 2304 x 2048, two steps, 3.91 -> 3.93; two activation rows 256 x 1024 3.90 -> 4.04).
-constexpr uint32_t FOUR_ROWS_FROM = 64;  // matrix rows of a CTA
+constexpr uint32_t FOUR_ROWS_FROM = 64, SHORT_STEPS = 800;  // matrix rows of a CTA; times the steps of a row
 constexpr size_t ACT_SMEM_MAX = 200 * 1024;
 template <class F, int M, int NG> static cudaError_t launch_rows(const GemvGroup &g, const uint8_t *table, uint32_t pairs, int force_ks, int sm_count, bool pdl, cudaStream_t stream) {
     const uint32_t k = g.item[0].k, steps = (k / GROUP + 31) / 32;
@@ -329,7 +331,9 @@ template <class F, int M, int NG> static cudaError_t launch_rows(const GemvGroup
     pick(M, cut.mine, steps, force_ks, rb, ks);
     if constexpr (M == 1) {
         if (F::DIRECT && cut.mine * steps <= WARPS) return launch<F, M, 1, false, NG>(g, table, cut, ks, pairs, pdl, stream);
-        if (acts && cut.mine >= FOUR_ROWS_FROM) return launch<F, M, 4, true, NG>(g, table, cut, ks, pairs, pdl, stream);
+        if (acts && cut.mine >= FOUR_ROWS_FROM)
+            return pairs == 1 && cut.mine * steps <= SHORT_STEPS ? launch<F, M, 4, true, NG>(g, table, cut, ks, pairs, pdl, stream)
+                                                                 : launch<F, M, 4, true, NG, false>(g, table, cut, ks, pairs, pdl, stream);
     }
     if (acts && rb == 1) return launch<F, M, 1, true, NG>(g, table, cut, ks, pairs, pdl, stream);
     if (acts) return launch<F, M, 2, true, NG>(g, table, cut, ks, pairs, pdl, stream);
