@@ -653,7 +653,7 @@ struct MoePlan {
     uint64_t t = 0, r = 0, e = 0;
     lapid_b200_layout wl{};
     size_t route_bytes = 0, scratch = 0;
-    bool together = false;  // decode sizes: may share with its neighbours in the list
+    bool together = false;  // decode sizes: may share a kernel with its neighbours in the list
 };
 
 MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l) {
@@ -686,9 +686,10 @@ MoePlan plan_matmul_id(const lapid_b200_device &dev, const lapid_b200_launch &l)
         size_t qa = align_up(p.t * l.k, 256), sc = align_up(p.t * (l.k / 32) * 4, 256);
         size_t rec = align_up(p.t * ((l.k + 255) / 256) * lb::REC, 256);
         p.scratch = p.fast ? rec : qa + 2 * sc;
-        // Launches over the same tokens (gate, up) share the quantized tokens, and MXFP4 and the i-quants a kernel, unless their matrices exceed the L2
-        // (126 MB): pairs that name the same expert then meet there only while their CTAs run in step, which a second matrix beside them ends. Two blocks of
-        // MXFP4, apart / together, us: 8 tokens with 6 of 32 experts of 8960 x 2048 2208 / 2383, one token with 6 of 32 of 2304 x 5120 94 / 85.
+        // MXFP4 and i-quant launches over the same tokens (gate, up) are one kernel while the matrices that their pairs read, counted pair by pair, are no more than
+        // the L2 (126 MB): pairs that name the same expert meet there only while their CTAs run in step, which a second matrix beside them ends. Gate and up,
+        // us, apart / together: MXFP4, one token with 4 of 8 experts of 14336 x 4096 66 / 61, with 2 40 / 36, 8 tokens with 6 of 32 of 8960 x 2048 201 / 308; IQ3_XXS, 8 with 4
+        // of 8 of 4096 x 4096 242 / 263, though these eight would fit twice; 8 with 8 of 64 of 1408 x 2048 97 / 86.
         p.together = p.t * p.r * p.wl.total <= (126ull << 20);
     } else {
         p.tc = !dev.gemm_f32 && lb::qgemm_tc_moe_supported(l.b_dtype, p.e, l.n, l.k, nullptr);
@@ -1165,7 +1166,7 @@ void execute_locked(lapid_b200_device *dev, const lapid_b200_launch *launches, s
                 sl.offset = scratch_total;
                 // the routing tables and the gathered rows of an earlier launch with the same tokens and ids (gate and up), as long as nothing
                 // since has written either buffer
-                const bool act = p.together;  // the quantized tokens of an earlier launch that reads them in the same layout
+                const bool act = p.decode;  // the quantized tokens of an earlier launch that reads them in the same layout
                 if ((p.tc || act) && xb && ib) {
                     sl.records = act ? ActSlot::MOE_ACT : ActSlot::MOE_COPY;
                     sl.ptr = xb->ptr;

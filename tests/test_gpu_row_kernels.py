@@ -143,6 +143,27 @@ def test_expert_launches_of_the_same_tokens_go_out_together(be, oracle, fmt, t, 
     assert err.value.code == "index_out_of_range"
 
 
+@pytest.mark.parametrize("fmt", [MX, lp.DType.Q4K, lp.DType.Q6K, lp.DType.Int8])
+def test_expert_launches_share_the_quantized_tokens_whatever_their_size(be, oracle, fmt):
+    """gate and up of 8 tokens with 8 slots each: their 64 pairs read more than the L2 holds, so they are two kernels, but the tokens are quantized once."""
+    t, r, e, n, k = 8, 8, 8, 2048, 2048   # (each expert eight times: above that the reference multiplies in f32)
+    total = oracle.layout(int(fmt), n, k).total
+    one = _weights(fmt, n, k, 5) if fmt == MX else oracle.quantize(int(fmt), O.normal(5, n * k, 0.02), n, k)
+    stack = np.zeros(e * total, np.uint8)
+    for i in range(e):   # every expert another matrix: the first 16 i rows of its quants are zeros
+        stack[i * total:i * total + one.size] = one
+        stack[i * total:i * total + 16 * i * (one.size // n)] = 0
+    ids = np.array([(i // r + i) % e for i in range(t * r)], np.int32)
+    x = O.normal(62, t * k)
+    bufs = [be.upload(x), be.upload(stack), be.upload(stack), be.upload(ids.view(np.uint8))] + [be.alloc(t * r * n * 4) for _ in range(2)]
+    be.take_launch_count()
+    be.execute([matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 1 + i, 3), output=4 + i) for i in (0, 1)], bufs)
+    assert be.take_launch_count() == 3
+    want = oracle.matmul_id(int(fmt), x, stack, ids, t, r, e, n, k)
+    for b in bufs[4:]:
+        assert _max_rel(b.download().view(np.float32), want) <= 2e-5
+
+
 @pytest.mark.parametrize("fmt", [lp.DType.Int8, lp.DType.Int4])
 @pytest.mark.parametrize("m,n,k", [
     (1, 33, 32), (3, 40, 288),         # one chunk, two: most warps without a unit
