@@ -228,9 +228,10 @@ struct lapid_b200_device {
     // balanced-stream tensor-core decode kernel (qgemv_kq_stream.cu): 0 never; 1 (default) Q5_K always and Q4_K where
     // it is the faster one (launch_qgemv_q4k_mma decides); 2 both formats always
     int gemv_stream = 1;
-    // MXFP4 decode launches with at least this many rows use the int8 tensor-core kernel (0 = never): about 18.5 us on
-    // 14336 x 4096 whatever the row count, against 15.8 / 17.9 / 25.4 / 42.9 us of the dp4a kernel at 1 / 2 / 4 / 8 rows
-    uint32_t mxfp4_mma_rows = 3;
+    // Option "gemv_mxfp4_mma_rows": MXFP4 decode launches with at least this many rows use the int8 tensor-core kernel (0: never). Until it is set the kernel is
+    // chosen per launch (qgemv_mxfp4_mma_pays).
+    uint32_t mxfp4_mma_rows = MXFP4_PER_LAUNCH;
+    static constexpr uint32_t MXFP4_PER_LAUNCH = ~0u;
     int iq_row_kernel = 0;  // option "gemv_iq_row_kernel": i-quants at three to eight rows: 0 per launch, 1 on the row kernel where it fits, 2 never
     bool small_dp4a = true;  // small Q5_K / Q6_K matrices at 3 and 4 rows on the dp4a kernel (see plan_launch)
     bool two_row_dp4a = false;    // two early Q4_K rows on the dp4a kernel (see execute_impl)
@@ -545,7 +546,8 @@ Plan plan_launch(const lapid_b200_device &dev, const lapid_b200_launch &l) {
                  // (one row: the bulk-copy kernel where it takes the shape)
                  ((l.b_dtype == LAPID_B200_DTYPE_INT8 || l.b_dtype == LAPID_B200_DTYPE_INT4) && (p.rows >= dev.gemv_mma_rows || (p.rows == 1 && !p.fast_i8)) &&
                   lb::qgemv_i8_mma_shape_ok(l.b_dtype, p.rows, (uint32_t)l.k)) ||
-                 (l.b_dtype == LAPID_B200_DTYPE_MXFP4 && dev.mxfp4_mma_rows > 0 && p.rows >= dev.mxfp4_mma_rows &&
+                 (l.b_dtype == LAPID_B200_DTYPE_MXFP4 &&
+                  (dev.mxfp4_mma_rows == dev.MXFP4_PER_LAUNCH ? lb::qgemv_mxfp4_mma_pays(p.rows, (uint32_t)l.n, (uint32_t)l.k) : dev.mxfp4_mma_rows > 0 && p.rows >= dev.mxfp4_mma_rows) &&
                   lb::qgemv_mxfp4_mma_shape_ok(p.rows, (uint32_t)l.k)));
         // Small Q5_K / Q6_K matrices at three and four rows: their tensor-core kernels cost about 5 us whatever the size
         // (1024 x 4096: 5.0-5.5 us), the dp4a kernel 3.8-4.6 us; from five rows on, and from 4096 x 4096 on, the
@@ -1723,8 +1725,8 @@ lapid_b200_status lapid_b200_device_set_option(lapid_b200_device *dev, const cha
             lb::qgemv_q6k_mma_set_config(std::atoi(value));
         } else if (k == "gemv_mxfp4_mma_rows") {
             int r = std::atoi(value);
-            if (r < 0 || r > 8) fail("invalid_argument", "gemv_mxfp4_mma_rows must be in 0..8");
-            dev->mxfp4_mma_rows = (uint32_t)r;
+            if (r < 0 || r > 8) fail("invalid_argument", "gemv_mxfp4_mma_rows must be in 0..8, or auto");
+            dev->mxfp4_mma_rows = v == "auto" ? lapid_b200_device::MXFP4_PER_LAUNCH : (uint32_t)r;
         } else if (k == "gemv_mxfp4_k_split") {
             lb::qgemv_mxfp4_set_k_split(std::atoi(value));
         } else if (k == "gemv_mxfp4_staged") {

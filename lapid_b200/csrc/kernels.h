@@ -136,6 +136,7 @@ cudaError_t launch_qgemv_i4(const GemvArgs &args, int sm_count, bool pdl, cudaSt
 // qgemv_mxfp4_mma.cu: the same blocks on the int8 tensor-core instruction (K a multiple of 512; the activation tiles
 // of the K-quant kernels)
 bool qgemv_mxfp4_mma_shape_ok(uint32_t rows, uint32_t k);
+bool qgemv_mxfp4_mma_pays(uint32_t rows, uint32_t n, uint32_t k);
 cudaError_t launch_qgemv_mxfp4_mma(const GemvArgs &args, int sm_count, bool pdl, cudaStream_t stream);
 void qgemv_mxfp4_set_k_split(int ways);  // warps per row: 0: per launch (default); 1, 2, 4: forced
 

@@ -214,6 +214,19 @@ template <int WARPS> static cudaError_t launch_w(const GemvArgs &a, int sm_count
 }  // namespace mxm
 
 // K a multiple of 512: whole stages, and every row and chunk of the packed matrix a multiple of 16 bytes.
+// Where it beats the row kernel (qgemv_mxfp4.cu). Its time hardly depends on the rows, and a launch costs it 1 to 1.5 us more. us, row kernel / this one: three rows
+// 1024 x 4096 4.8 / 5.4, 14336 x 4096 18.9 / 20.9, 4096 x 14336 20.6 / 20.7, but 4096 x 4096 8.6 / 8.3 and 2048 x 7680 9.1 / 8.4; four 1024 x 4096 5.1 / 5.4, 4096 x 2048
+// 6.3 / 5.9, 8192 x 4096 14.2 / 13.5, 14336 x 4096 20.5 / 21.1, 1024 x 14336 10.1 / 11.7; five 1024 x 2048 4.5 / 5.1, 2048 x 2048 5.6 / 5.3, 14336 x 1024 11.7 / 14.3; six
+// 14336 x 4096 24.4 / 21.1; eight 64 x 512 4.8 / 4.7, 1024 x 4096 6.6 / 5.7. The row kernel also takes projections of one operand as one launch.
+bool qgemv_mxfp4_mma_pays(uint32_t rows, uint32_t n, uint32_t k) {
+    const uint64_t weights = (uint64_t)n * k;
+    if (rows < 3) return false;
+    if (rows == 3) return n >= 2048 && n <= 4096 && k >= 4096 && k <= 8192;
+    if (rows == 4) return weights > (4u << 20) && n >= 2048 && n < 14336;
+    if (rows <= 6) return weights > (2u << 20) && k > 1024;
+    return true;
+}
+
 bool qgemv_mxfp4_mma_shape_ok(uint32_t rows, uint32_t k) {
     if (rows < 1 || rows > 8 || k < mxm::KC || k % mxm::KC != 0) return false;
     return mxm::smem_bytes(4, rows, k) <= 227 * 1024 - 256;

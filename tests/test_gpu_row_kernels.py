@@ -55,6 +55,32 @@ def test_mxfp4_shares_steps_and_rows(be, oracle, m, n, k):
     assert _max_rel(got[:, :n], want) <= 2e-5 and np.all(got[:, n:] == -7.0)
 
 
+@pytest.mark.parametrize("m,n,k,mma", [
+    (3, 1024, 4096, False), (3, 2048, 4096, True), (3, 4097, 4096, False), (3, 2048, 8704, False), (4, 2048, 2048, False), (4, 2304, 5120, True),
+    (4, 14336, 512, False), (5, 1024, 2048, False), (5, 2048, 1536, True), (6, 8192, 1024, False), (8, 64, 512, True), (8, 64, 544, False),
+])
+def test_mxfp4_kernel_choice(oracle, m, n, k, mma):
+    """Three to eight rows go to the row kernel or to the tensor cores by size: the bits are those of the kernel named."""
+    be = lp.Backend(0)
+    qb, a = _weights(MX, n, k, m + n), O.normal(7 + n, m * k)
+    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4)]
+    got = []
+    for option in (None, "1" if mma else "0", "auto"):
+        if option:
+            be.set_option("gemv_mxfp4_mma_rows", option)
+        be.execute([matmul_launch(MX, m, n, k, inputs=(0, 1), output=2)], bufs)
+        got.append(bufs[2].download().view(np.uint32).copy())
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+    be.set_option("gemv_mxfp4_mma_rows", "0" if mma else "1")
+    be.execute([matmul_launch(MX, m, n, k, inputs=(0, 1), output=2)], bufs)
+    other = bufs[2].download().view(np.float32)
+    if k % 512 == 0:
+        assert not np.array_equal(got[0], other.view(np.uint32))
+    assert _max_rel(other, got[0].view(np.float32)) <= 2e-5
+    want, _ = oracle.matmul(O.MXFP4, a, qb, n, k, m=m)
+    assert _max_rel(got[0].view(np.float32), want) <= 2e-5
+
+
 @pytest.mark.parametrize("row_kernel", ["1", "2"])   # on csrc/qgemv_iq_rows.cu, on csrc/qgemv_iq.cu
 @pytest.mark.parametrize("fmt", [lp.DType.Iq2Xxs, lp.DType.Iq2Xs, lp.DType.Iq2S, lp.DType.Iq3Xxs])
 @pytest.mark.parametrize("m,n,k", [
