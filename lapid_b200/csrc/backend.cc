@@ -1128,7 +1128,11 @@ void check_status_word(lapid_b200_device *dev) {
     cudaMemsetAsync(dev->stream_ws.pairs, 0, dev->stream_ws.total_bytes, dev->stream);
     cudaStreamSynchronize(dev->stream);
     if (st == 128) fail("index_out_of_range", "an index of a gather or an expert id of a matmul_id is out of range; the rows it selects were not computed");
-    fail("backend", "a device-side wait gave up (status " + std::to_string(st) + "); the results of this call are invalid");
+    // (which kernel sets which bit: 1 decode, 2 to 32 the waits of the tensor-core prefill, 64 tensor-parallel exchange, 128 a bad index, 256 exact-f32 GEMM)
+    std::string who;
+    for (auto [bits, name] : {std::pair<int, const char *>{1, "decode"}, {2 | 4 | 8 | 16 | 32, "tensor-core prefill"}, {64, "tensor-parallel exchange"}, {256, "exact-f32 GEMM"}})
+        if (st & bits) who += (who.empty() ? ": " : ", ") + std::string(name);
+    fail("backend", "a device-side wait gave up (status " + std::to_string(st) + who + "); the results of this call are invalid");
 }
 
 // (the caller holds dev->mu and has made the device current)

@@ -613,7 +613,7 @@ template <int FMT> __global__ void __launch_bounds__(CONSUMERS + PRODUCERS, 1) q
             }
         }
     }
-    if (!ok && p.status) atomicOr(p.status, 8);
+    if (!ok && p.status) atomicOr(p.status, 256);
 }
 
 }  // namespace ws

@@ -104,3 +104,16 @@ def test_launch_marshalling_matches_header_struct():
     assert list(c.expr)[:11] == [1, 1, 16, 17, 2, 0x3F800000, 32, 21, 34, 1 | 1 << 8, 34] and list(c.extra.strides) == [128, 64, 1]
     c = lp.backend.matmul_launch(lp.DType.Q4K, 2, 64, 256, expr=lp.backend.Expr.load(0).tanh()).to_c()
     assert (c.n_inputs, c.n_expr) == (2, 2)
+
+
+def test_status_bits_say_which_kernel_gave_up():
+    """The kernels whose bounded waits share a bit of the host-visible status word are those the error text names together."""
+    csrc = os.path.join(ROOT, "lapid_b200", "csrc")
+    bits = {}
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh")):
+            for bit in re.findall(r"atomicOr\([\w.\[\]]*status, (\d+)\)", open(os.path.join(csrc, name)).read()):
+                bits.setdefault(int(bit), set()).add(name)
+    assert set(bits) == {1, 2, 4, 8, 16, 32, 64, 128, 256}
+    assert all(bits[b] == {"qgemm_tc.cu"} for b in (2, 4, 8, 16, 32)) and bits[256] == {"qgemm_f32.cu"}
+    assert all(n.startswith("qgemv") for n in bits[1]) and bits[64] == {"glue.cu", "tp_allreduce.cu"}
