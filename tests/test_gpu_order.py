@@ -92,8 +92,8 @@ def test_captured_decode_step_gives_the_bits_of_the_serial_one(mix, m, fuse_act)
     be.synchronize()
 
 
-@pytest.mark.parametrize("fmt", [DType.Q4K, DType.Q6K, DType.Int8, DType.Iq3Xxs])
-@pytest.mark.parametrize("m", [1, 4])
+@pytest.mark.parametrize("fmt", [DType.Q4K, DType.Q6K, DType.Int8, DType.MXFP4, DType.Iq3Xxs])
+@pytest.mark.parametrize("m", [1, 3, 4, 8])   # (MXFP4 and the i-quants: two kernels each)
 def test_captured_weights_written_between_the_glue_kernel_and_the_list(fmt, m):
     """A list behind a glue kernel may request weights early only when nothing stands between the two: here a copy (then a kernel) rewrites
     the weights there, in every replay with other ones."""
@@ -249,6 +249,52 @@ def test_weights_written_by_an_earlier_launch_of_the_list(fmt, m, writer_rows):
                 out.zero_()
                 run()
                 got = out.view(torch.int32).clone()
+            s1.synchronize()
+            assert torch.equal(got, wants[rep % 2]), rep
+    serial.synchronize()
+    be.synchronize()
+
+
+@pytest.mark.parametrize("fmt", [DType.MXFP4, DType.Iq2Xxs])
+@pytest.mark.parametrize("m", [1, 3, 8])
+def test_decode_weights_copied_by_a_gather_of_the_list(fmt, m):
+    """A Gather (of one f32 row: it copies bytes) writes the weights of two decode launches that share a kernel: they must read the copied ones."""
+    import torch
+    serial, s0 = _device(pdl="0")
+    be, s1 = _device()
+    n, k = 2048, 2048
+    if fmt == DType.MXFP4:
+        sets = [_weights(be, int(fmt), n, k, 1100 + i) for i in range(2)]
+    else:
+        sets = [torch.randint(0, 256, (n * k // 256, 66), dtype=torch.uint8, device="cuda") for _ in range(2)]
+        for b in sets:
+            b[:, :2] = torch.full((len(b),), 1e-3, device="cuda").half().view(torch.uint8).view(-1, 2)
+        sets = [torch.cat([b.reshape(-1), b.new_zeros(tp.layout_total(int(fmt), n, k) - b.numel())]) for b in sets]
+    other = sets[0].clone()
+    source, w = sets[0].clone(), torch.zeros_like(sets[0])
+    x, outs = torch.from_numpy(O.normal(1110, m * k).reshape(m, k)).cuda(), [torch.zeros(m, n, device="cuda") for _ in range(2)]
+    row = torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ls = [gather_launch(DType.F32, 1, w.numel() // 4, 1, inputs=(3, 4), output=1), matmul_launch(fmt, m, n, k, inputs=(0, 5), output=6),
+          matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)]
+    tensors = (x, w, outs[0], source, row, other, outs[1])
+    wants = []
+    for a in sets:
+        source.copy_(a)
+        torch.cuda.synchronize()
+        serial.execute(ls, [serial.wrap_tensor(t) for t in tensors])
+        wants.append(outs[0].clone())
+    assert not torch.equal(*wants)
+    bufs = [be.wrap_tensor(t) for t in tensors]
+    torch.cuda.synchronize()
+    graph = _capture(be, s1, lambda: be.execute_async(ls, bufs))
+    for rep in range(20):
+        for run in (lambda: be.execute_async(ls, bufs), graph.replay):
+            with torch.cuda.stream(s1):
+                source.copy_(sets[rep % 2])
+                outs[0].zero_()
+                run()
+                got = outs[0].clone()
             s1.synchronize()
             assert torch.equal(got, wants[rep % 2]), rep
     serial.synchronize()
