@@ -25,7 +25,7 @@ __device__ __forceinline__ uint32_t spread_signs(uint32_t s8) {
 template <int FMT> struct Format {
     static constexpr int GRID_WORDS = 8192;
     static constexpr int M_MIN = 3, M_MAX = 8;
-    static constexpr bool DIRECT = false, AHEAD = true;
+    static constexpr bool DIRECT = false, AHEAD = true, CHUNKS = false;
     static constexpr bool IQ3 = FMT == FMT_IQ3XXS;
     static constexpr int ENTRIES = iq_grid_bytes(FMT) / (IQ3 ? 4 : 8), COPIES = GRID_WORDS / ENTRIES;  // 32 KB of grid words: 32, 16 (IQ2_XS), 8 (IQ2_S) copies
     static constexpr int SIGNS = FMT == FMT_IQ2S ? 256 : 128, SIGN_COPIES = GRID_WORDS / 2 / SIGNS / (IQ3 ? 2 : 1);

@@ -23,7 +23,7 @@ namespace mx {
 
 template <bool SPLIT> struct Format {  // SPLIT: positive and negative codes apart
     static constexpr int M_MIN = SPLIT ? 1 : 3, M_MAX = SPLIT ? 2 : 8;
-    static constexpr bool DIRECT = true, AHEAD = false;
+    static constexpr bool DIRECT = true, AHEAD = false, CHUNKS = true;
     static constexpr size_t TABLE_BYTES = 0;  // no lookups
     static __device__ __forceinline__ void fill(uint8_t *, const uint8_t *, int, int) {}
     struct Tables {

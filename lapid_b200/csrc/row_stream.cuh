@@ -13,10 +13,14 @@
 // three quarters of the registers (launch bounds of 640 threads: 96 each): with all of them the small kernel in front or behind (the activations' quantization)
 // finds no room beside it and cannot overlap (IQ2_XXS, four rows on 2048 x 4096 8.9 -> 7.3 us, MXFP4, two rows on 2304 x 1024 4.9 -> 4.3).
 //
-// The integer sums of a group are exact and the products those of the reference; only the order in which the groups' f32 terms are added differs.
+// The integer sums of a group are exact and the products those of the reference; only the order in which the groups' f32 terms are added differs. It keeps the error no
+// larger than that of the kernels before, which gave a row to up to four warps: every four steps by themselves (F::CHUNKS: MXFP4), the warps of a row, each with one
+// rounding less, without roundings in between (against f64, MXFP4, one row on 4096 x 14336: before 8.2e-8, here 8.3e-8, as one chain 9.3e-8, on 1500 x 14336
+// 8.3e-8, 6.8e-8, 8.8e-8). The i-quants' two halves of a unit are one
+// exact sum here, two terms there.
 //
 // A format F gives: M_MIN and M_MAX (activation rows), DIRECT (activations that do not fit shared memory are read where they lie), TABLE_BYTES, fill() and
-// Tables (lookup tables in shared memory, and where a lane reads them), AHEAD (packed bytes requested before the present ones are unpacked), STEP_BYTES and lane_offset() (where a lane's unit of a row
+// Tables (lookup tables in shared memory, and where a lane reads them), AHEAD (packed bytes requested before the present ones are unpacked), CHUNKS (see above), STEP_BYTES and lane_offset() (where a lane's unit of a row
 // lies), Raw and load() (its packed bytes, as they lie), W and unpack() (int8 weights and scale), dot() (a unit's integer sum as a float), order() (the activation group's bytes in the order of the weights).
 #pragma once
 #include "common.cuh"
@@ -25,10 +29,10 @@
 namespace lb {
 namespace rs {
 
-constexpr int WARPS = 16, THREADS = WARPS * 32, PART_FLOATS = 4096;
+constexpr int WARPS = 16, THREADS = WARPS * 32, PARTS = 2048;
 
-// Lane l gets the warp's sum of v[row_of(l)]: RB - 1 exchanges halve the rows, the rest is a plain tree.
-template <int RB> __device__ __forceinline__ float reduce_rows(float (&v)[RB], int lane) {
+// Lane l gets the warp's sum of v[row_of(l)]: RB - 1 exchanges halve the rows, the rest is a plain tree, the last addition left to the caller.
+template <int RB> __device__ __forceinline__ float2 reduce_rows(float (&v)[RB], int lane) {
     static_assert(RB == 1 || RB == 2 || RB == 4, "rows");
     int o = 16;
     float x[RB];
@@ -45,11 +49,23 @@ template <int RB> __device__ __forceinline__ float reduce_rows(float (&v)[RB], i
     }
     float s = x[0];
 #pragma unroll
-    for (int p = 16 / RB; p; p /= 2) s += __shfl_xor_sync(0xffffffffu, s, p);
-    return s;
+    for (int p = 16 / RB; p > 1; p /= 2) s += __shfl_xor_sync(0xffffffffu, s, p);
+    return make_float2(s, __shfl_xor_sync(0xffffffffu, s, 1));
 }
 template <int RB> __device__ __forceinline__ int row_of(int lane) {
     return RB == 4 ? 2 * ((lane >> 3) & 1) + ((lane >> 4) & 1) : RB == 2 ? (lane >> 4) & 1 : 0;
+}
+
+// The sum of n (up to WARPS) numbers that lie `STRIDE` apart.
+template <int STRIDE> __device__ __forceinline__ float sum_parts(const double *x, uint32_t n) {
+    double v[WARPS];
+#pragma unroll
+    for (int i = 0; i < WARPS; i++) v[i] = (uint32_t)i < n ? x[i * STRIDE] : 0.0;
+#pragma unroll
+    for (int w = 1; w < WARPS; w *= 2)
+#pragma unroll
+        for (int i = 0; i < WARPS; i += 2 * w) v[i] += v[i + w];
+    return (float)v[0];
 }
 
 // ks_log: log2 of the warps that share a row; pass_rows: matrix rows of a CTA between two exchanges of their partial sums
@@ -72,8 +88,8 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t ks_count = 1u << ks_log;
     const uint32_t k = p.k, units = k / GROUP, steps = (units + 31) / 32, whole = units / 32, sg = steps * 32;  // sg: groups of the padded planes
-    float *part = (float *)(smem + F::TABLE_BYTES);
-    uint8_t *acts = smem + F::TABLE_BYTES + (ks_count > 1 ? PART_FLOATS * 4 : 0);
+    double *part = (double *)(smem + F::TABLE_BYTES);
+    uint8_t *acts = smem + F::TABLE_BYTES + (ks_count > 1 ? PARTS * 8 : 0);
     float *act_d = (float *)(acts + (size_t)M * sg * GROUP);
     constexpr int WARPS_LOG = 4;
     static_assert(1 << WARPS_LOG == WARPS, "warps");
@@ -164,11 +180,15 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
     for (uint32_t p0 = 0; p0 < rows; p0 += pass_rows) {
         for (uint32_t row = r0; row < r1; row += RB) {
             const uint32_t left = r1 - row;
-            float acc[M][RB];
+            // Every four steps are summed by themselves. More activation rows have no registers to spare (pick() splits k instead), and where a CTA has matrix rows for
+            // four a warp, a row had one warp before, too.
+            constexpr bool CHUNKS = F::CHUNKS && M <= 2 && RB <= 2;
+            float acc[M][RB], total[M][RB];
+            uint32_t left_in_chunk = 4;
 #pragma unroll
             for (int r = 0; r < M; r++)
 #pragma unroll
-                for (int j = 0; j < RB; j++) acc[r][j] = 0.0f;
+                for (int j = 0; j < RB; j++) acc[r][j] = total[r][j] = 0.0f;
             for (uint32_t step = ks; step < steps; step += ks_count) {
                 typename F::W wv[RB];
                 // the packed bytes of what comes next are on their way while this is unpacked and multiplied (F::AHEAD; else while it is multiplied, which
@@ -212,14 +232,29 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
 #pragma unroll
                     for (int j = 0; j < RB; j++) acc[r][j] = fmaf(wv[j].d * d, F::dot(wv[j], a), acc[r][j]);
                 }
+                if (CHUNKS && --left_in_chunk == 0) {
+                    left_in_chunk = 4;
+#pragma unroll
+                    for (int r = 0; r < M; r++)
+#pragma unroll
+                        for (int j = 0; j < RB; j++) total[r][j] += acc[r][j], acc[r][j] = 0.0f;
+                }
             }
+            float2 v[M];
 #pragma unroll
             for (int r = 0; r < M; r++) {
-                const float v = reduce_rows<RB>(acc[r], lane);
-                const uint32_t mine = row + row_of<RB>(lane);
-                if (lane % (32 / RB) == 0 && mine < r1) {
-                    if (ks_count > 1) part[((((mine - p0) << ks_log) + ks)) * M + r] = v;
-                    else store(mine, r, v);
+#pragma unroll
+                for (int j = 0; CHUNKS && j < RB; j++) acc[r][j] += total[r][j];
+                v[r] = reduce_rows<RB>(acc[r], lane);
+            }
+            const uint32_t mine = row + row_of<RB>(lane);
+            if (lane % (32 / RB) == 0 && mine < r1) {
+                if (ks_count > 1) {
+#pragma unroll
+                    for (int r = 0; r < M; r++) part[(((mine - p0) << ks_log) + ks) * M + r] = (double)v[r].x + (double)v[r].y;
+                } else {
+#pragma unroll
+                    for (int r = 0; r < M; r++) store(mine, r, v[r].x + v[r].y);
                 }
             }
         }
@@ -232,9 +267,7 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
             __syncthreads();
             for (uint32_t i = threadIdx.x; i < n * M; i += THREADS) {
                 const uint32_t row = i / M, r = i % M;
-                float v = part[(row << ks_log) * M + r];
-                for (uint32_t s = 1; s < ks_count; s++) v += part[((row << ks_log) + s) * M + r];
-                store(p0 + row, r, v);
+                store(p0 + row, r, sum_parts<M>(part + (row << ks_log) * M + r, ks_count));
             }
             __syncthreads();  // the partial sums are read: the next pass may overwrite them
         }
@@ -244,7 +277,7 @@ row_stream_kernel(const __grid_constant__ GemvGroupT<NG> grp, const uint8_t *__r
 // Shared memory of a launch.
 template <class F> static size_t smem_bytes(uint32_t rows, uint32_t k, uint32_t ks, bool acts) {
     const size_t sg = ((size_t)k / GROUP + 31) / 32 * 32;
-    return F::TABLE_BYTES + (ks > 1 ? PART_FLOATS * 4 : 0) + (acts ? (size_t)rows * sg * (GROUP + 4) : 0);
+    return F::TABLE_BYTES + (ks > 1 ? PARTS * 8 : 0) + (acts ? (size_t)rows * sg * (GROUP + 4) : 0);
 }
 
 // How a launch is cut.
@@ -275,10 +308,10 @@ template <class F> static Cut cut_rows(const GemvGroup &g, uint32_t pairs, int s
 // Matrix rows that a warp takes at a time (RB: 1, 2) and warps per row (KS): the least time of the slowest warp, in steps of one row. A step of two rows
 // takes 1.4 (one activation row) to 1.9 (eight) steps of one, and as much when the second row is missing; a reduction about a sixth of a step, an exchange as
 // much again. One row at a time only where a warp has no second one: else the activations' loads are what two rows share (eight rows, IQ2_XXS, 14336 x 4096 26.8
-// against 35.0 us). MXFP4, one activation row: 2304 x 1024 one row, one warp 3.52, two rows 3.80; 1024 x 14336 one row, two warps 7.9, two rows, four warps 6.7.
-static void pick(uint32_t m, uint64_t mine, uint32_t steps, int force_ks, int &rb, uint32_t &ks) {
+// against 35.0 us). At least `least` warps. MXFP4, one activation row: 2304 x 1024 one row, one warp 3.52, two rows 3.80; 1024 x 14336 one row, two warps 7.9, two rows, four warps 6.7.
+static void pick(uint32_t m, uint64_t mine, uint32_t steps, uint32_t least, int force_ks, int &rb, uint32_t &ks) {
     double best = 1e30;
-    for (uint32_t c = 1; c <= WARPS && c <= steps; c *= 2) {
+    for (uint32_t c = least; c <= WARPS && c <= steps; c *= 2) {
         if (force_ks && (uint32_t)force_ks <= steps && c != (uint32_t)force_ks) continue;
         const uint64_t r = (mine * c + WARPS - 1) / WARPS;
         const double row = (double)((steps + c - 1) / c) + (c > 1 ? 0.33 : 0.17), pair = row * (double)((r + 1) / 2) * (1.35 + 0.07 * m);
@@ -296,7 +329,7 @@ static cudaError_t launch(const GemvGroup &all, const uint8_t *table, const Cut 
     if ((cut.mine + 1) * F::row_bytes(k) >> 32) return cudaErrorInvalidValue;
     uint32_t ks_log = 0;
     while (2u << ks_log <= ks) ks_log++;
-    const uint32_t pass = ks > 1 ? PART_FLOATS / (ks * M) : (uint32_t)cut.mine;  // (one pass where nothing is exchanged)
+    const uint32_t pass = ks > 1 ? PARTS / (ks * M) : (uint32_t)cut.mine;  // (one pass where nothing is exchanged)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cut.grid, pairs);
     cfg.blockDim = dim3(THREADS);
@@ -328,7 +361,8 @@ template <class F, int M, int NG> static cudaError_t launch_rows(const GemvGroup
     const Cut cut = cut_rows<F>(g, pairs, sm_count);
     int rb = 2;
     uint32_t ks = 1;
-    pick(M, cut.mine, steps, force_ks, rb, ks);
+    // (three MXFP4 rows and more: few matrix rows had two warps each before, too)
+    pick(M, cut.mine, steps, F::CHUNKS && M > 2 && cut.mine < 32 && steps > 4 && !force_ks ? 2 : 1, force_ks, rb, ks);
     if constexpr (M == 1) {
         if (F::DIRECT && cut.mine * steps <= WARPS) return launch<F, M, 1, false, NG>(g, table, cut, ks, pairs, pdl, stream);
         if (acts && cut.mine >= FOUR_ROWS_FROM)

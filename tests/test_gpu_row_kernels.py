@@ -226,3 +226,25 @@ def test_iquant_sums_overflow_no_earlier_than_the_reference(be, oracle, fmt):
         be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)], bufs)
         got = bufs[2].download().view(np.float32)
         assert np.isfinite(got).all() and _max_rel(got, want) <= 2e-5
+
+
+@pytest.mark.parametrize("fmt,n,k,members,bound", [
+    (MX, 1500, 14336, 1, 8.4e-8),      # several warps to a row
+    (MX, 4096, 14336, 1, 8.6e-8),      # one warp, fourteen steps
+    (IQ, 4096, 11008, 2, 9.8e-8),      # a group's members have fewer warps to a row than each would alone
+])
+def test_f32_sums_are_as_close_to_f64_as_with_more_warps_to_a_row(be, oracle, fmt, n, k, members, bound):
+    """One activation row against f64 sums of the same quantized operands. The bounds lie between what these sums show (6.5e-8, 8.2e-8, 9.0e-8; with two or four
+    warps to a row, one chain each: 8.2e-8, 8.3e-8, 9.1e-8) and one chain over a longer k (8.8e-8, 9.2e-8, 1.02e-7); 2-norms over all outputs, inputs fixed."""
+    a = O.normal(71, k)
+    q, d = oracle.quantize_row_sums(a, want_bs=False)[:2]
+    x = (np.asarray(q, np.float64).reshape(-1, 32) * np.asarray(d, np.float64).reshape(-1, 1)).reshape(-1)
+    ws = [_weights(fmt, n, k, 72 + i) for i in range(members)]
+    bufs = [be.upload(a)] + [be.upload(w) for w in ws] + [be.alloc(n * 4) for _ in ws]
+    be.execute([matmul_launch(fmt, 1, n, k, inputs=(0, 1 + i), output=1 + members + i) for i in range(members)], bufs)
+    off = total = 0.0
+    for i, w in enumerate(ws):
+        want = oracle.dequantize(int(fmt), w, n, k).reshape(n, k).astype(np.float64) @ x
+        off += ((bufs[1 + members + i].download().view(np.float32) - want) ** 2).sum()
+        total += (want ** 2).sum()
+    assert (off / total) ** 0.5 <= bound
