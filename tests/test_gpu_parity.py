@@ -1445,8 +1445,9 @@ def test_small_matrices_at_three_and_four_rows_take_the_dp4a_kernel(oracle, fmt,
         assert np.array_equal(got, plain) == dp4a, (m, n, k)
 
 
-def test_mxfp4_decode_row_kernel(be, oracle):
-    """The MXFP4 row kernel at one to eight rows with one, two and four warps per row and with the launch's own choice,
+def test_mxfp4_decode_staged_and_direct_forms(be, oracle):
+    """The MXFP4 decode kernel streams rows through shared memory when K is a multiple of 512 and reads them directly
+    otherwise: same arithmetic in the same order, so the two forms agree bit for bit on shapes both can run; both
     against the oracle; the expert-indexed launch included."""
     from lapid_b200.backend import matmul_id_launch
     rng = np.random.default_rng(21)
@@ -1456,12 +1457,20 @@ def test_mxfp4_decode_row_kernel(be, oracle):
         qb = np.concatenate([raw, np.zeros((-raw.size) % 256, np.uint8)])
         a = O.normal(1900 + m, m * k)
         want, _ = oracle.matmul(O.MXFP4, a, qb, n, k, m=m)
-        be.set_option("gemv_mxfp4_mma_rows", "0")       # (the row kernel at every row count)
-        for split in ("1", "2", "4", "0"):              # one, two and four warps per row, then the launch's own choice
+        got = {}
+        be.set_option("gemv_mxfp4_mma_rows", "0")       # (the dp4a kernel at every row count)
+        be.set_option("gemv_mxfp4_k_split", "1")
+        for staged in ("1", "0"):
+            be.set_option("gemv_mxfp4_staged", staged)
+            got[staged] = run_matmul(be, lp.DType.MXFP4, a, qb, m, n, k)
+            assert max_rel(got[staged], want) <= 2e-5, (m, n, k, staged)
+        assert np.array_equal(got["0"], got["1"]), (m, n, k)
+        for split in ("2", "4", "0"):                   # two and four warps per row, then the launch's own choice
             be.set_option("gemv_mxfp4_k_split", split)
             assert max_rel(run_matmul(be, lp.DType.MXFP4, a, qb, m, n, k), want) <= 2e-5, (m, n, k, split)
-        be.set_option("gemv_mxfp4_mma_rows", "auto")
-    t, r, e, n, k = 3, 2, 4, 200, 1024   # (an expert-indexed launch is one-row work per pair)
+        be.set_option("gemv_mxfp4_staged", "1")
+        be.set_option("gemv_mxfp4_mma_rows", "3")
+    t, r, e, n, k = 3, 2, 4, 200, 1024   # (an expert-indexed launch is one-row work per pair: staged)
     one = oracle.layout(O.MXFP4, n, k).total
     stack = np.zeros(e * one, np.uint8)
     for x in range(e):
@@ -1472,11 +1481,14 @@ def test_mxfp4_decode_row_kernel(be, oracle):
     ids = np.array([(i * 3 + 1) % e for i in range(t * r)], np.int32)
     want = oracle.matmul_id(O.MXFP4, xs, stack, ids, t, r, e, n, k)
     bufs = [be.upload(xs), be.upload(stack), be.upload(ids.view(np.uint8)), be.alloc(t * r * n * 4)]
-    for split in ("1", "2", "0"):
-        be.set_option("gemv_mxfp4_k_split", split)
+    res = {}
+    for staged in ("1", "0"):
+        be.set_option("gemv_mxfp4_staged", staged)
         be.execute([matmul_id_launch(lp.DType.MXFP4, t, r, e, n, k)], bufs)
-        assert max_rel(bufs[3].download().view(np.float32), want) <= 2e-5, split
-    be.set_option("gemv_mxfp4_staged", "0")             # (accepted, without effect)
+        res[staged] = bufs[3].download().view(np.float32).copy()
+        assert max_rel(res[staged], want) <= 2e-5
+    be.set_option("gemv_mxfp4_staged", "1")
+    assert np.array_equal(res["0"], res["1"])
 
 
 def test_gemv_mxfp4_tensor_core_decode_kernel(be, oracle):
@@ -1505,7 +1517,7 @@ def test_gemv_mxfp4_tensor_core_decode_kernel(be, oracle):
             assert max_rel(got, want) <= 2e-5, (m, n, k, max_rel(got, want))
             assert max_rel(got, ref) <= 2e-5, (m, n, k)
     finally:
-        be.set_option("gemv_mxfp4_mma_rows", "auto")
+        be.set_option("gemv_mxfp4_mma_rows", "3")
 
 
 def test_gemv_int4_bulk_copy_kernel(be, oracle):

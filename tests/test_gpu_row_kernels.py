@@ -1,4 +1,4 @@
-"""Decode kernels of the formats that become int8 by lookups (MXFP4: csrc/row_stream.cuh, csrc/qgemv_mxfp4.cu; i-quants: csrc/qgemv_iq.cu, csrc/qgemv_iq_rows.cu): shares of the CTAs,
+"""Decode kernels of the formats that become int8 by lookups (MXFP4: csrc/row_stream.cuh, csrc/qgemv_mxfp4.cu; i-quants: csrc/qgemv_iq.cu): shares of the CTAs,
 steps of k and batches of rows at their edges, and launches that go out as one because they read the same activations. The Int8 / Int4 kernel
 (csrc/qgemv_i8_mma.cu): units of a tile and a chunk that the warps take in order.
 
@@ -40,8 +40,6 @@ def _max_rel(got, want):
     (1, 9473, 96), (2, 9500, 1024),    # four rows a warp, the last ones of a share missing
     (1, 700, 16384), (1, 40, 20480),   # sixteen slices of k and more steps than that
     (1, 5, 230400), (2, 5, 92160),     # activations that do not fit shared memory
-    (1, 2300, 1024), (1, 1200, 4096), (2, 2100, 1056), (5, 600, 2880),   # a matrix row for each warp at most; one row, activations not copied
-    (2, 1000, 14336), (3, 2048, 8224), # two rows a warp, several warps to a row
     (3, 77, 2880), (8, 40, 160), (8, 33, 23072),
 ])
 def test_mxfp4_shares_steps_and_rows(be, oracle, m, n, k):
@@ -55,64 +53,20 @@ def test_mxfp4_shares_steps_and_rows(be, oracle, m, n, k):
     assert _max_rel(got[:, :n], want) <= 2e-5 and np.all(got[:, n:] == -7.0)
 
 
-@pytest.mark.parametrize("m,n,k,mma", [
-    (3, 1024, 4096, False), (3, 2048, 4096, True), (3, 4097, 4096, False), (3, 2048, 8704, False), (4, 2048, 2048, False), (4, 2304, 5120, True),
-    (4, 14336, 512, False), (5, 1024, 2048, False), (5, 2048, 1536, True), (6, 8192, 1024, False), (8, 64, 512, True), (8, 64, 544, False),
-])
-def test_mxfp4_kernel_choice(oracle, m, n, k, mma):
-    """Three to eight rows go to the row kernel or to the tensor cores by size: the bits are those of the kernel named."""
-    be = lp.Backend(0)
-    qb, a = _weights(MX, n, k, m + n), O.normal(7 + n, m * k)
-    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4)]
-    got = []
-    for option in (None, "1" if mma else "0", "auto"):
-        if option:
-            be.set_option("gemv_mxfp4_mma_rows", option)
-        be.execute([matmul_launch(MX, m, n, k, inputs=(0, 1), output=2)], bufs)
-        got.append(bufs[2].download().view(np.uint32).copy())
-    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
-    be.set_option("gemv_mxfp4_mma_rows", "0" if mma else "1")
-    be.execute([matmul_launch(MX, m, n, k, inputs=(0, 1), output=2)], bufs)
-    other = bufs[2].download().view(np.float32)
-    if k % 512 == 0:
-        assert not np.array_equal(got[0], other.view(np.uint32))
-    assert _max_rel(other, got[0].view(np.float32)) <= 2e-5
-    want, _ = oracle.matmul(O.MXFP4, a, qb, n, k, m=m)
-    assert _max_rel(got[0].view(np.float32), want) <= 2e-5
-
-
-@pytest.mark.parametrize("row_kernel", ["1", "2"])   # on csrc/qgemv_iq_rows.cu, on csrc/qgemv_iq.cu
 @pytest.mark.parametrize("fmt", [lp.DType.Iq2Xxs, lp.DType.Iq2Xs, lp.DType.Iq2S, lp.DType.Iq3Xxs])
 @pytest.mark.parametrize("m,n,k", [
     (8, 3, 256), (8, 150, 1280),                   # one block; a step that is partly there
     (8, 2501, 2304), (8, 33, 13824),               # blocks on odd halves of a word in every other row; more steps than warps
-    (3, 2400, 1024), (4, 4097, 2304), (5, 2050, 4352), (6, 1500, 768), (7, 301, 2560),
+    (3, 8192, 1024), (4, 4097, 2304), (5, 2050, 4352),   # eight million weights and more
+    (8, 12, 16640),                                # activations that do not fit: the other kernel
 ])
-def test_iquants_at_several_rows(be, oracle, fmt, m, n, k, row_kernel):
+def test_iquants_at_several_rows(be, oracle, fmt, m, n, k):
     qb, a, bias = iq_matrix(fmt, n, k, m + n), O.normal(7 + n, m * k), O.normal(8 + n, n)
     want, path = oracle.matmul(int(fmt), a, qb, n, k, m=m, bias=bias)
     assert path == "int8_act"
     bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4), be.upload(bias)]
-    be.set_option("gemv_iq_row_kernel", row_kernel)
-    try:
-        be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
-    finally:
-        be.set_option("gemv_iq_row_kernel", "0")
+    be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
     assert _max_rel(bufs[2].download().view(np.float32), want) <= 2e-5
-
-
-def test_iquant_activations_that_do_not_fit(be, oracle):
-    """Eight rows of 16640: the row kernel has no room for them, forced or not."""
-    m, n, k, fmt = 8, 12, 16640, lp.DType.Iq2Xs
-    qb, a = iq_matrix(fmt, n, k, 1), O.normal(9, m * k)
-    want, _ = oracle.matmul(int(fmt), a, qb, n, k, m=m)
-    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4)]
-    for row_kernel in ("1", "0"):
-        be.set_option("gemv_iq_row_kernel", row_kernel)
-        be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)], bufs)
-        assert _max_rel(bufs[2].download().view(np.float32), want) <= 2e-5
-    with pytest.raises(lp.LapidError):
-        be.set_option("gemv_iq_row_kernel", "3")
 
 
 @pytest.mark.parametrize("fmt", [MX, IQ])
@@ -169,27 +123,6 @@ def test_expert_launches_of_the_same_tokens_go_out_together(be, oracle, fmt, t, 
     assert err.value.code == "index_out_of_range"
 
 
-@pytest.mark.parametrize("fmt", [MX, lp.DType.Q4K, lp.DType.Q6K, lp.DType.Int8])
-def test_expert_launches_share_the_quantized_tokens_whatever_their_size(be, oracle, fmt):
-    """gate and up of 8 tokens with 8 slots each: their 64 pairs read more than the L2 holds, so they are two kernels, but the tokens are quantized once."""
-    t, r, e, n, k = 8, 8, 8, 2048, 2048   # (each expert eight times: above that the reference multiplies in f32)
-    total = oracle.layout(int(fmt), n, k).total
-    one = _weights(fmt, n, k, 5) if fmt == MX else oracle.quantize(int(fmt), O.normal(5, n * k, 0.02), n, k)
-    stack = np.zeros(e * total, np.uint8)
-    for i in range(e):   # every expert another matrix: the first 16 i rows of its quants are zeros
-        stack[i * total:i * total + one.size] = one
-        stack[i * total:i * total + 16 * i * (one.size // n)] = 0
-    ids = np.array([(i // r + i) % e for i in range(t * r)], np.int32)
-    x = O.normal(62, t * k)
-    bufs = [be.upload(x), be.upload(stack), be.upload(stack), be.upload(ids.view(np.uint8))] + [be.alloc(t * r * n * 4) for _ in range(2)]
-    be.take_launch_count()
-    be.execute([matmul_id_launch(fmt, t, r, e, n, k, inputs=(0, 1 + i, 3), output=4 + i) for i in (0, 1)], bufs)
-    assert be.take_launch_count() == 3
-    want = oracle.matmul_id(int(fmt), x, stack, ids, t, r, e, n, k)
-    for b in bufs[4:]:
-        assert _max_rel(b.download().view(np.float32), want) <= 2e-5
-
-
 @pytest.mark.parametrize("fmt", [lp.DType.Int8, lp.DType.Int4])
 @pytest.mark.parametrize("m,n,k", [
     (1, 33, 32), (3, 40, 288),         # one chunk, two: most warps without a unit
@@ -208,43 +141,3 @@ def test_int8_units_of_tiles_and_chunks(be, oracle, fmt, m, n, k):
     assert _max_rel(first, want) <= 2e-5
     be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2, bias_input=3)], bufs)
     assert np.array_equal(first, bufs[2].download().view(np.float32))   # the order of the sums does not depend on timing
-
-
-@pytest.mark.parametrize("fmt", [lp.DType.Iq2Xxs, lp.DType.Iq2Xs, lp.DType.Iq2S, lp.DType.Iq3Xxs])
-def test_iquant_sums_overflow_no_earlier_than_the_reference(be, oracle, fmt):
-    """Activations of one size and with the signs of the weights: the sum, of terms of one sign, is 2e38, and twice that is not finite."""
-    m, n, k = 8, 1, 512
-    qb = iq_matrix(fmt, n, k, 3)
-    w = oracle.dequantize(int(fmt), qb, n, k).reshape(n, k)
-    size = 2e38 / np.abs(w[0].astype(np.float64)).sum()
-    a = np.tile(np.where(w[0] < 0, -size, size).astype(np.float32), m)
-    want, path = oracle.matmul(int(fmt), a, qb, n, k, m=m)
-    assert path == "int8_act" and np.isfinite(want).all() and want.max() > 1.9e38
-    bufs = [be.upload(a), be.upload(qb), be.alloc(m * n * 4)]
-    for row_kernel in ("1", "2", "0"):
-        be.set_option("gemv_iq_row_kernel", row_kernel)
-        be.execute([matmul_launch(fmt, m, n, k, inputs=(0, 1), output=2)], bufs)
-        got = bufs[2].download().view(np.float32)
-        assert np.isfinite(got).all() and _max_rel(got, want) <= 2e-5
-
-
-@pytest.mark.parametrize("fmt,n,k,members,bound", [
-    (MX, 1500, 14336, 1, 8.4e-8),      # several warps to a row
-    (MX, 4096, 14336, 1, 8.6e-8),      # one warp, fourteen steps
-    (IQ, 4096, 11008, 2, 9.8e-8),      # a group's members have fewer warps to a row than each would alone
-])
-def test_f32_sums_are_as_close_to_f64_as_with_more_warps_to_a_row(be, oracle, fmt, n, k, members, bound):
-    """One activation row against f64 sums of the same quantized operands. The bounds lie between what these sums show (6.5e-8, 8.2e-8, 9.0e-8; with two or four
-    warps to a row, one chain each: 8.2e-8, 8.3e-8, 9.1e-8) and one chain over a longer k (8.8e-8, 9.2e-8, 1.02e-7); 2-norms over all outputs, inputs fixed."""
-    a = O.normal(71, k)
-    q, d = oracle.quantize_row_sums(a, want_bs=False)[:2]
-    x = (np.asarray(q, np.float64).reshape(-1, 32) * np.asarray(d, np.float64).reshape(-1, 1)).reshape(-1)
-    ws = [_weights(fmt, n, k, 72 + i) for i in range(members)]
-    bufs = [be.upload(a)] + [be.upload(w) for w in ws] + [be.alloc(n * 4) for _ in ws]
-    be.execute([matmul_launch(fmt, 1, n, k, inputs=(0, 1 + i), output=1 + members + i) for i in range(members)], bufs)
-    off = total = 0.0
-    for i, w in enumerate(ws):
-        want = oracle.dequantize(int(fmt), w, n, k).reshape(n, k).astype(np.float64) @ x
-        off += ((bufs[1 + members + i].download().view(np.float32) - want) ** 2).sum()
-        total += (want ** 2).sum()
-    assert (off / total) ** 0.5 <= bound
