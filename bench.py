@@ -529,9 +529,11 @@ def gemv_kernel_name(fmt: int, m: int, n: int = 0, k: int = 0) -> str:
     if fmt == 5:
         return "qgemv_i8_mma_kernel<int4>" if m >= 2 or k % 512 else "qgemv_i8_fast_kernel<int4>"
     if fmt == 9:
-        return "qgemv_mxfp4_mma_kernel" if m >= 3 and k % 512 == 0 else "row_stream_kernel<mxfp4>"
+        pays = {1: False, 2: False, 3: 2048 <= n <= 4096 and 4096 <= k <= 8192, 4: n * k > (4 << 20) and 2048 <= n < 14336}.get(m, m > 6 or (n * k > (2 << 20) and k > 1024))
+        return "qgemv_mxfp4_mma_kernel" if pays and k % 512 == 0 else "row_stream_kernel<mxfp4>"
     if fmt >= 10:
-        return "qgemv_iq_kernel"
+        # from three rows on one of two kernels, by size, format and the shared memory that the activations need
+        return "qgemv_iq_kernel" if m <= 2 else "row_stream_kernel<iq> or qgemv_iq_kernel"
     return "qgemv_i8_mma_kernel" if m >= 2 or k % 512 else "qgemv_i8_fast_kernel"
 
 

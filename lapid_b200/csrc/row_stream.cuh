@@ -7,7 +7,7 @@
 //     slices of k, and a warp takes RB rows at a time: the activations of a step are read once for RB rows, their packed bytes are requested one
 //     step ahead, and RB sums are reduced by one transposing shuffle tree;
 //   * the quantized activations are copied to shared memory once, in two planes of 16 bytes a group (conflict-free wide loads), zeros behind the
-//     end of k, so that the last step of a row needs no masks beside its loads;
+//     end of k, so that the last step of a row needs no masks beside its loads.
 // The first packed bytes do not depend on the kernel in front and are fetched before the dependency wait. One CTA of sixteen warps an SM: more and smaller ones
 // copy the activations more often (three of eight warps: 4096 x 4096 6.8 against 6.3 us, six experts of 5120 x 2304 19.1 against 18.6). ROOM: a CTA takes
 // three quarters of the registers (launch bounds of 640 threads: 96 each): with all of them the small kernel in front or behind (the activations' quantization)
@@ -15,8 +15,8 @@
 //
 // The integer sums of a group are exact and the products those of the reference; only the order in which the groups' f32 terms are added differs. It keeps the error no
 // larger than that of the kernels before, which gave a row to up to four warps: every four steps by themselves (F::CHUNKS: MXFP4), the warps of a row, each with one
-// rounding less, without roundings in between (against f64, MXFP4, one row on 4096 x 14336: before 8.2e-8, here 8.3e-8, as one chain 9.3e-8, on 1500 x 14336
-// 8.3e-8, 6.8e-8, 8.8e-8). The i-quants' two halves of a unit are one
+// rounding less, without roundings in between (against f64, MXFP4, one row on 4096 x 14336: before 8.3e-8, here 8.2e-8, as one chain 9.2e-8, on 1500 x 14336
+// 8.2e-8, 6.5e-8, 8.8e-8). The i-quants' two halves of a unit are one
 // exact sum here, two terms there.
 //
 // A format F gives: M_MIN and M_MAX (activation rows), DIRECT (activations that do not fit shared memory are read where they lie), TABLE_BYTES, fill() and
@@ -285,7 +285,8 @@ struct Cut {
     uint32_t grid, end[GEMV_GROUP_MAX];  // CTAs in all (for each pair), and up to each member's end
     uint64_t mine;                       // matrix rows of the busiest CTA
 };
-// One CTA per SM; a share of them for each pair of an expert-indexed launch, and for each member as many as its rows are worth.
+// A launch has one CTA per SM. Its members get as many of them as their rows are worth. Each pair of an expert-indexed launch gets the same number, rounded down, so that
+// up to a third of the SMs stay without a CTA (56 pairs: 112 CTAs).
 template <class F> static Cut cut_rows(const GemvGroup &g, uint32_t pairs, int sm_count) {
     Cut c{};
     uint64_t rows = 0, seen = 0;
