@@ -14,8 +14,6 @@
 // `dp4a` against each activation row's 32 int8 values (two 16-byte loads per row from the activation planes, shared
 // by the ROWS weight rows). The sums over 16 elements are exact and the products are the reference's; only the
 // order in which the halves are added differs (lanes, then a shuffle tree).
-#include <type_traits>
-
 #include "common.cuh"
 #include "iquant.cuh"
 #include "kernels.h"
@@ -158,15 +156,11 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(ARGS args, const u
     __shared__ float part[KS > 1 ? WARPS * ROWS * M : 1];
     for (uint32_t base = cta * RPC; base < p.n; base += ctas * RPC) {  // (the same number of passes for every warp of the CTA)
         const uint32_t row0 = base + wg * ROWS;
-        // A grouped launch has fewer warps to a row than its members would have alone: it sums every two steps by themselves, which is as close to f64
-        // (gate and up of 4096 x 11008, IQ2_XXS, one row: alone 9.4e-8, grouped 9.0e-8, with one sum 1.07e-7).
-        constexpr bool CHUNKS = std::is_same<ARGS, GemvGroup>::value && M <= 4;
-        bool odd = false;
-        float acc[ROWS][M], total[ROWS][M];
+        float acc[ROWS][M];
 #pragma unroll
         for (int j = 0; j < ROWS; j++)
 #pragma unroll
-            for (int r = 0; r < M; r++) acc[j][r] = total[j][r] = 0.0f;
+            for (int r = 0; r < M; r++) acc[j][r] = 0.0f;
         for (uint32_t blk = blk0; blk < nblk; blk += 4 * KS) {
             Raw32 cur[ROWS];
 #pragma unroll
@@ -196,19 +190,13 @@ __global__ void __launch_bounds__(WARPS * 32) qgemv_iq_kernel(ARGS args, const u
                     acc[j][r] += (sc[j][1] * da) * (float)d1;
                 }
             }
-            if (CHUNKS && odd)
-#pragma unroll
-                for (int j = 0; j < ROWS; j++)
-#pragma unroll
-                    for (int r = 0; r < M; r++) total[j][r] += acc[j][r], acc[j][r] = 0.0f;
-            odd = !odd;
         }
         if (base + ctas * RPC < p.n) fetch(row0 + ctas * RPC, blk0);  // the next pass
 #pragma unroll
         for (int j = 0; j < ROWS; j++) {
 #pragma unroll
             for (int r = 0; r < M; r++) {
-                float v = CHUNKS ? acc[j][r] + total[j][r] : acc[j][r];
+                float v = acc[j][r];
 #pragma unroll
                 for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
                 const uint32_t row = row0 + j;
